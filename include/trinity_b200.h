@@ -305,7 +305,7 @@ int trn_profile_entry(int i, char* name, int name_len, long long* launches, doub
  * call cudaMalloc/cudaFree: inputs and output are the caller's device
  * buffers (d_points[2V], d_tris[3T] 0-based CCW, d_solut[V] -> d_tensor[3V],
  * m11 m12 m22 per vertex), and the working memory is one fixed __device__
- * array of about 6 MB that every GPU loading this library holds until exit.
+ * array of about 7 MB that every GPU loading this library holds until exit.
  * Limits: V <= TRN_NOALLOC_MAX_NODES, T <= TRN_NOALLOC_MAX_ELEMS, at most
  * TRN_NOALLOC_BUCKET triangles around a vertex; larger inputs return
  * TRN_ERR_CAPACITY. The tensors are those of trn_metric_run on the same mesh

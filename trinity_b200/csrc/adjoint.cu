@@ -43,6 +43,7 @@
  */
 #include "trn_internal.h"
 #include "trn_mixed.cuh"
+#include "trn_patch.cuh"
 
 #include <algorithm>
 
@@ -380,7 +381,36 @@ __device__ __forceinline__ int patch_owners(const DMesh& m, int4 n, int* ids) {
   return trn_iunique(ids, k);
 }
 
-/* ge[t] = area_t * sum over the patch owners i of gv[i] (NC components) */
+/* the same owners in registers: the three adjacency rows, merged with the
+ * three vertices themselves; false when a row does not fit */
+constexpr int kOwnerKeys = 4 * kRowRegs;
+
+__device__ __forceinline__ bool owner_keys(const DMesh& m, int4 n, int* key) {
+  if (m.bucket & 3) return false;   /* rows not 16-byte aligned */
+  const int c[3] = {n.x, n.y, n.z};
+  const int nv[3] = {m.vdeg[n.x], m.vdeg[n.y], m.vdeg[n.z]};
+  if (nv[0] > kRowRegs || nv[1] > kRowRegs || nv[2] > kRowRegs) return false;
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) ok &= patch_row(m.vic + (size_t) c[j] * m.bucket, nv[j], key + j * kRowRegs);
+  if (!ok) return false;
+#pragma unroll
+  for (int j = 0; j < kRowRegs; ++j) key[3 * kRowRegs + j] = j < 3 ? c[j] : kNoId;
+  patch_cmp(key[3 * kRowRegs], key[3 * kRowRegs + 1]);
+  patch_cmp(key[3 * kRowRegs + 1], key[3 * kRowRegs + 2]);
+  patch_cmp(key[3 * kRowRegs], key[3 * kRowRegs + 1]);
+  patch_merge_rows<kOwnerKeys>(key);
+  return true;
+}
+
+template <class R, int NC>
+struct alignas(sizeof(R) * NC) OwnerRec {
+  R c[NC];
+};
+
+/* ge[t] = area_t * sum over the patch owners i of gv[i] (NC components), in
+ * ascending vertex order: merged in registers where the rows are short, else
+ * sorted in local memory; the same sums */
 template <bool F32, int NC>
 __global__ void k_adj_elem_patch(DMesh m, int nb_elems, const AReal<F32>* __restrict__ gv,
                                  AReal<F32>* __restrict__ ge) {
@@ -392,9 +422,25 @@ __global__ void k_adj_elem_patch(DMesh m, int nb_elems, const AReal<F32>* __rest
     R acc[NC];
     for (int c = 0; c < NC; ++c) acc[c] = R(0);
     if (n.x >= 0) {
-      const int k = patch_owners(m, n, ids);
-      for (int a = 0; a < k; ++a)
-        for (int c = 0; c < NC; ++c) acc[c] += gv[NC * (size_t) ids[a] + c];
+      int key[kOwnerKeys];
+      if (owner_keys(m, n, key)) {
+#pragma unroll
+        for (int a = 0; a < kOwnerKeys; a += 4) {
+          OwnerRec<R, NC> r[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (key[a + j] != kNoId && (a + j == 0 || key[a + j] != key[a + j - 1]))
+              r[j] = reinterpret_cast<const OwnerRec<R, NC>*>(gv)[key[a + j]];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (key[a + j] != kNoId && (a + j == 0 || key[a + j] != key[a + j - 1]))
+              for (int c = 0; c < NC; ++c) acc[c] += r[j].c[c];
+        }
+      } else {
+        const int k = patch_owners(m, n, ids);
+        for (int a = 0; a < k; ++a)
+          for (int c = 0; c < NC; ++c) acc[c] += gv[NC * (size_t) ids[a] + c];
+      }
       const double2 p0 = m.pts[n.x], p1 = m.pts[n.y], p2 = m.pts[n.z];
       const R area = R(0.5 * ((p1.x - p0.x) * (p2.y - p0.y) - (p2.x - p0.x) * (p1.y - p0.y)));
       for (int c = 0; c < NC; ++c) acc[c] *= area;
@@ -513,7 +559,7 @@ static void adjoint_impl(const DMesh& m, int nb_nodes, int nb_elems, const doubl
     DMesh g = f;
     g.lten = nullptr;
     metric_run(g, nb_nodes, nb_elems, um->solut, um->grad, um->terms, ws.scal + 0, um->exact_sum,
-               um->p, s, &keep);
+               um->p, um->ws, s, &keep);
   }
   log_cache(f, nb_nodes, F32, s);
   /* the solution's adjoint only when its output is asked for */
@@ -546,7 +592,7 @@ static void adjoint_impl(const DMesh& m, int nb_nodes, int nb_elems, const doubl
   sum_tree(ws.vfact, nb_nodes, ws.vfact + nb_nodes, ws.scal + 2, s);
   k_adj_star_area<<<grid_for(nb_nodes), TRN_THREADS, 0, s>>>(f, nb_nodes, ws.astar);
   note_launch();
-  R* graw = reinterpret_cast<R*>(ws.vbuf) + 3 * (size_t) nb_nodes;
+  R* graw = reinterpret_cast<R*>(ws.vbuf) + 4 * (size_t) nb_nodes;   /* records of 4: aligned to their size */
   k_adj_local<F32><<<grid_for(nb_nodes), TRN_THREADS, 0, s>>>(
       f, nb_nodes, ws.hsym, ws.mloc, ws.astar, ws.atot, ws.scal + 0, ws.scal + 2, um->p.target,
       um->p.scale_exp, gm, graw);

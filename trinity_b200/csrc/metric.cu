@@ -1,110 +1,134 @@
 /*
  * metric.cu — Hessian-based metric recovery (Metrics::run, metric.cpp:59-70).
  *
- *   k_gradient        per vertex: area-weighted mean of the P1 gradients over
- *                     the 2-ring element patch (hessian.cpp:24-83)
- *   k_hessian_local   per vertex: the same on the gradient field, symmetrised
+ *   k_elem_gradient   per element: its signed area and area x P1 gradient
+ *   k_patch_sum<GradSum>  per vertex: area-weighted mean of those over the
+ *                     2-ring element patch (hessian.cpp:24-83)
+ *   k_elem_hessian    per element: area x the gradient field's derivatives
+ *   k_patch_sum<HessSum>  per vertex: their mean, symmetrised
  *                     (hessian.cpp:86-153), then |H| eigen-clamp and local L^p
  *                     scale det^(-1/(2p+2)) (metric.cpp:100-150), fused
- *   k_complexity_term per element: area * mean_k sqrt(det M_k) (metric.cpp:159-181)
- *   k_sum_*           the complexity sum: either one thread in element order
- *                     (bit-identical to the reference's 1-thread sum) or a
- *                     deterministic two-level tree
+ *   k_sum_terms       per element: area * mean_k sqrt(det M_k)
+ *                     (metric.cpp:159-181), summed by a deterministic
+ *                     two-level tree (k_sum_final), or
+ *   k_complexity_term, k_sum_sequential  by one thread in element order
+ *                     (bit-identical to the reference's 1-thread sum)
  *   k_normalize       global scale target/complexity and eigenvalue clamp to
  *                     [1/h_max^2, 1/h_min^2] (metric.cpp:188-238)
- *   k_*_f32           the same recovery in FP32 for the mixed-precision form
+ *   k_elem_edges, *Sum32, k_normalize_f32   the same recovery in FP32 for the
+ *                     mixed-precision form
  *
  * Patch order matters: the reference sums over the patch in ascending element
- * id (std::set order, mesh.cpp:396-432), so each thread gathers the stencils
- * of the vertex and of its neighbours, sorts and deduplicates them first.
+ * id (std::set order, mesh.cpp:396-432), so the union of the stencils of the
+ * vertex and of its neighbours is sorted and deduplicated first
+ * (trn_patch.cuh): in registers where the rows are short, by a warp for the
+ * vertices that the first pass lists as not fitting.
  */
 #include "trn_internal.h"
 #include "trn_mixed.cuh"
+#include "trn_patch.cuh"
 
 namespace trn {
 
-__device__ __forceinline__ int gather_patch(const DMesh& m, int v, int* patch) {
-  int k = 0;
-  const int* s = m.stenc + (size_t) v * m.bucket;
-  int d = trn_deg(m, v);
-  for (int a = 0; a < d && k < TRN_MAX_PATCH; ++a) patch[k++] = s[a];
-  const int* vc = m.vic + (size_t) v * m.bucket;
-  int nv = m.vdeg[v];
-  for (int b = 0; b < nv; ++b) {
-    int w = vc[b];
-    const int* sw = m.stenc + (size_t) w * m.bucket;
-    int dw = trn_deg(m, w);
-    for (int a = 0; a < dw; ++a) {
-      if (k == TRN_MAX_PATCH) {
-        trn_set_error(m.err, TRN_DERR_BUCKET);
-        break;
-      }
-      patch[k++] = sw[a];
+/* An element's share of a patch sum depends on the element alone, and an
+ * element lies in the patches of about 12 vertices: it is computed once into a
+ * 32-byte record (one sector a gather) instead of once per patch. What bounds
+ * the patch sums: the record gathers (24 a vertex, mostly L1/L2 hits) and the
+ * integer merge of the rows. One vertex a thread that gathered, sorted in
+ * local memory and computed every element of its patch took 582 us for the
+ * gradient and 650 us for the Hessian of the 2M-triangle mesh; records and
+ * register merge take 30 + 194 and 30 + 202 us (cold caches). */
+__global__ void k_elem_gradient(DMesh m, int nb_elems, const double* __restrict__ solut,
+                                double4* __restrict__ rec) {
+  if (trn_failed(m)) return;
+  for (int t = trn_tid(); t < nb_elems; t += trn_grid_stride()) {
+    if (m.tri[t].x < 0) {
+      rec[t] = make_double4(0.0, 0.0, 0.0, 0.0);
+      continue;
     }
+    const ElemGrad g = elem_grad(m, t);
+    const double s0 = solut[g.v.x], s1 = solut[g.v.y], s2 = solut[g.v.z];
+    double ex = 0, ey = 0;
+    ex += s0 * g.d[0];
+    ey += s0 * g.d[1];
+    ex += s1 * g.d[2];
+    ey += s1 * g.d[3];
+    ex += s2 * g.d[4];
+    ey += s2 * g.d[5];
+    rec[t] = make_double4(g.area, g.area * ex, g.area * ey, 0.0);
   }
-  trn_isort(patch, k);
-  return trn_iunique(patch, k);
 }
 
-__global__ void k_gradient(DMesh m, int nb_nodes, const double* __restrict__ solut,
-                           double2* __restrict__ grad, double* __restrict__ atot) {
+__global__ void k_elem_hessian(DMesh m, int nb_elems, const double2* __restrict__ grad,
+                               double4* __restrict__ rec) {
   if (trn_failed(m)) return;
-  int patch[TRN_MAX_PATCH];
-  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    int n = gather_patch(m, v, patch);
-    double total_area = 0.;
-    double gx = 0., gy = 0.;
-    /* the reference stores per-element (area, grad) and sums afterwards in the
-     * same element order; interleaving the two loops keeps every sum's order */
-    for (int i = 0; i < n; ++i) {
-      ElemGrad g = elem_grad(m, patch[i]);
-      total_area += g.area;
-      double s0 = solut[g.v.x], s1 = solut[g.v.y], s2 = solut[g.v.z];
-      double ex = 0, ey = 0;
-      ex += s0 * g.d[0];
-      ey += s0 * g.d[1];
-      ex += s1 * g.d[2];
-      ey += s1 * g.d[3];
-      ex += s2 * g.d[4];
-      ey += s2 * g.d[5];
-      gx += (g.area * ex);
-      gy += (g.area * ey);
+  for (int t = trn_tid(); t < nb_elems; t += trn_grid_stride()) {
+    if (m.tri[t].x < 0) {
+      rec[t] = make_double4(0.0, 0.0, 0.0, 0.0);
+      continue;
     }
+    const ElemGrad g = elem_grad(m, t);
+    const double2 g0 = grad[g.v.x], g1 = grad[g.v.y], g2 = grad[g.v.z];
+    double dl[4] = {0, 0, 0, 0};
+    dl[0] += (g0.x * g.d[0]);
+    dl[1] += (g0.x * g.d[1]);
+    dl[2] += (g0.y * g.d[0]);
+    dl[3] += (g0.y * g.d[1]);
+    dl[0] += (g1.x * g.d[2]);
+    dl[1] += (g1.x * g.d[3]);
+    dl[2] += (g1.y * g.d[2]);
+    dl[3] += (g1.y * g.d[3]);
+    dl[0] += (g2.x * g.d[4]);
+    dl[1] += (g2.x * g.d[5]);
+    dl[2] += (g2.y * g.d[4]);
+    dl[3] += (g2.y * g.d[5]);
+    rec[t] = make_double4(g.area * dl[0], g.area * dl[1], g.area * dl[2], g.area * dl[3]);
+  }
+}
+
+/* the sums over one patch: load() the record of an element, add() them in
+ * ascending element order, finish() the vertex. The reference stores the
+ * per-element values and sums afterwards in the same element order;
+ * interleaving its loops keeps every sum's order. */
+struct GradSum {
+  const double4* rec;
+  double2* grad;
+  double* atot;   /* patch areas, for the Hessian's mean too */
+  double total_area = 0, gx = 0, gy = 0;
+  using Rec = double4;
+  __device__ __forceinline__ void begin(const DMesh&, int) {}
+  __device__ __forceinline__ Rec load(const DMesh&, int t) const { return rec[t]; }
+  __device__ __forceinline__ void add(const Rec& r) {
+    total_area += r.x;
+    gx += r.y;
+    gy += r.z;
+  }
+  __device__ __forceinline__ void finish(const DMesh&, int v) {
     gx /= total_area;
     gy /= total_area;
     grad[v] = make_double2(gx, gy);
-    if (atot) atot[v] = total_area;
+    atot[v] = total_area;
   }
-}
+};
 
-__global__ void k_hessian_local(DMesh m, int nb_nodes, const double2* __restrict__ grad,
-                                double scale_exp, double4* __restrict__ hsym,
-                                double4* __restrict__ mloc) {
-  if (trn_failed(m)) return;
-  int patch[TRN_MAX_PATCH];
-  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    int n = gather_patch(m, v, patch);
-    double total_area = 0;
-    double h[4] = {0, 0, 0, 0};
-    for (int i = 0; i < n; ++i) {
-      ElemGrad g = elem_grad(m, patch[i]);
-      total_area += g.area;
-      double2 g0 = grad[g.v.x], g1 = grad[g.v.y], g2 = grad[g.v.z];
-      double dl[4] = {0, 0, 0, 0};
-      dl[0] += (g0.x * g.d[0]);
-      dl[1] += (g0.x * g.d[1]);
-      dl[2] += (g0.y * g.d[0]);
-      dl[3] += (g0.y * g.d[1]);
-      dl[0] += (g1.x * g.d[2]);
-      dl[1] += (g1.x * g.d[3]);
-      dl[2] += (g1.y * g.d[2]);
-      dl[3] += (g1.y * g.d[3]);
-      dl[0] += (g2.x * g.d[4]);
-      dl[1] += (g2.x * g.d[5]);
-      dl[2] += (g2.y * g.d[4]);
-      dl[3] += (g2.y * g.d[5]);
-      for (int j = 0; j < 4; ++j) h[j] += g.area * dl[j];
-    }
+struct HessSum {
+  const double4* rec;
+  const double* atot;   /* the gradient pass's sums: the same areas in the same order */
+  double scale_exp;
+  double4* hsym;
+  double4* mloc;
+  double h[4] = {0, 0, 0, 0};
+  using Rec = double4;
+  __device__ __forceinline__ void begin(const DMesh&, int) {}
+  __device__ __forceinline__ Rec load(const DMesh&, int t) const { return rec[t]; }
+  __device__ __forceinline__ void add(const Rec& r) {
+    h[0] += r.x;
+    h[1] += r.y;
+    h[2] += r.z;
+    h[3] += r.w;
+  }
+  __device__ __forceinline__ void finish(const DMesh& m, int v) {
+    const double total_area = atot[v];
     for (int j = 0; j < 4; ++j) h[j] /= total_area;
     /* symmetrise (hessian.cpp:149-152) */
     double t0 = h[0];
@@ -125,7 +149,7 @@ __global__ void k_hessian_local(DMesh m, int nb_nodes, const double2* __restrict
     m.ten[v] = r;
     if (mloc) mloc[v] = r;
   }
-}
+};
 
 /* ---- the mixed-precision form of the recovery ----
  * The same patch means in FP32. Every coordinate difference is taken in
@@ -136,65 +160,82 @@ __global__ void k_hessian_local(DMesh m, int nb_nodes, const double2* __restrict
  * afford); area x basis gradient is formed directly from the rotated edges
  * (area x 2/area x edge), so no division per element. The eigen-clamp, the
  * local L^p scale and the global scaling are FP32 too; the complexity sum
- * stays FP64. */
-__device__ __forceinline__ void elem_edges_f32(const DMesh& m, int4 t, float* area, float* ey, float* ex) {
-  const double2 p0 = m.pts[t.x], p1 = m.pts[t.y], p2 = m.pts[t.z];
-  /* rotated edges: area x d[2j] = 2 ey[j], area x d[2j+1] = 2 ex[j] */
-  ey[0] = (float) (p1.y - p2.y);
-  ex[0] = (float) (p2.x - p1.x);
-  ey[1] = (float) (p2.y - p0.y);
-  ex[1] = (float) (p0.x - p2.x);
-  ey[2] = (float) (p0.y - p1.y);
-  ex[2] = (float) (p1.x - p0.x);
-  const float c0 = (float) (p1.x - p0.x), c1 = (float) (p2.x - p0.x);
-  const float c2 = (float) (p1.y - p0.y), c3 = (float) (p2.y - p0.y);
-  *area = 0.5f * (c0 * c3 - c1 * c2);
-}
+ * stays FP64. An element's record holds its area and rotated edges; the
+ * differences to the centre are the patch's own. */
+struct Edges32 {
+  float4 a, b;   /* area, ey[3]; ex[3], unused */
+};
 
-__global__ void k_gradient_f32(DMesh m, int nb_nodes, const double* __restrict__ solut,
-                               double2* __restrict__ grad) {
+__global__ void k_elem_edges(DMesh m, int nb_elems, float4* __restrict__ rec) {
   if (trn_failed(m)) return;
-  int patch[TRN_MAX_PATCH];
-  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    const int n = gather_patch(m, v, patch);
-    const double uv = solut[v];
-    float tot = 0.f, gx = 0.f, gy = 0.f;
-    for (int i = 0; i < n; ++i) {
-      const int4 t = m.tri[patch[i]];
-      float area, ey[3], ex[3];
-      elem_edges_f32(m, t, &area, ey, ex);
-      const float s[3] = {(float) (solut[t.x] - uv), (float) (solut[t.y] - uv), (float) (solut[t.z] - uv)};
-      tot += area;
-      gx += 2.f * (s[0] * ey[0] + s[1] * ey[1] + s[2] * ey[2]);
-      gy += 2.f * (s[0] * ex[0] + s[1] * ex[1] + s[2] * ex[2]);
-    }
-    const float it = __frcp_rn(tot);
-    grad[v] = make_double2((double) (gx * it), (double) (gy * it));
+  for (int i = trn_tid(); i < nb_elems; i += trn_grid_stride()) {
+    const int4 t = m.tri[i];
+    if (t.x < 0) continue;
+    const double2 p0 = m.pts[t.x], p1 = m.pts[t.y], p2 = m.pts[t.z];
+    /* rotated edges: area x d[2j] = 2 ey[j], area x d[2j+1] = 2 ex[j] */
+    const float c0 = (float) (p1.x - p0.x), c1 = (float) (p2.x - p0.x);
+    const float c2 = (float) (p1.y - p0.y), c3 = (float) (p2.y - p0.y);
+    rec[2 * (size_t) i] = make_float4(0.5f * (c0 * c3 - c1 * c2), (float) (p1.y - p2.y), (float) (p2.y - p0.y),
+                                      (float) (p0.y - p1.y));
+    rec[2 * (size_t) i + 1] = make_float4((float) (p2.x - p1.x), (float) (p0.x - p2.x), (float) (p1.x - p0.x), 0.f);
   }
 }
 
-__global__ void k_hessian_local_f32(DMesh m, int nb_nodes, const double2* __restrict__ grad, float scale_exp) {
-  if (trn_failed(m)) return;
-  int patch[TRN_MAX_PATCH];
-  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    const int n = gather_patch(m, v, patch);
-    const double2 gv = grad[v];
-    float tot = 0.f, h[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int i = 0; i < n; ++i) {
-      const int4 t = m.tri[patch[i]];
-      float area, ey[3], ex[3];
-      elem_edges_f32(m, t, &area, ey, ex);
-      const int id[3] = {t.x, t.y, t.z};
-      tot += area;
-      for (int j = 0; j < 3; ++j) {
-        const double2 g = grad[id[j]];
-        const float dx = (float) (g.x - gv.x), dy = (float) (g.y - gv.y);
-        h[0] += 2.f * (dx * ey[j]);
-        h[1] += 2.f * (dx * ex[j]);
-        h[2] += 2.f * (dy * ey[j]);
-        h[3] += 2.f * (dy * ex[j]);
-      }
+struct GradSum32 {
+  const float4* rec;
+  const double* solut;
+  double2* grad;
+  double uv = 0;
+  float tot = 0.f, gx = 0.f, gy = 0.f;
+  struct Rec {
+    Edges32 e;
+    double u[3];
+  };
+  __device__ __forceinline__ void begin(const DMesh&, int v) { uv = solut[v]; }
+  __device__ __forceinline__ Rec load(const DMesh& m, int i) const {
+    const int4 t = m.tri[i];
+    return Rec{{rec[2 * (size_t) i], rec[2 * (size_t) i + 1]}, {solut[t.x], solut[t.y], solut[t.z]}};
+  }
+  __device__ __forceinline__ void add(const Rec& r) {
+    const float s[3] = {(float) (r.u[0] - uv), (float) (r.u[1] - uv), (float) (r.u[2] - uv)};
+    tot += r.e.a.x;
+    gx += 2.f * (s[0] * r.e.a.y + s[1] * r.e.a.z + s[2] * r.e.a.w);
+    gy += 2.f * (s[0] * r.e.b.x + s[1] * r.e.b.y + s[2] * r.e.b.z);
+  }
+  __device__ __forceinline__ void finish(const DMesh&, int v) {
+    const float it = __frcp_rn(tot);
+    grad[v] = make_double2((double) (gx * it), (double) (gy * it));
+  }
+};
+
+struct HessSum32 {
+  const float4* rec;
+  const double2* grad;
+  float scale_exp;
+  double2 gv = {0, 0};
+  float tot = 0.f, h[4] = {0.f, 0.f, 0.f, 0.f};
+  struct Rec {
+    Edges32 e;
+    double2 g[3];
+  };
+  __device__ __forceinline__ void begin(const DMesh&, int v) { gv = grad[v]; }
+  __device__ __forceinline__ Rec load(const DMesh& m, int i) const {
+    const int4 t = m.tri[i];
+    return Rec{{rec[2 * (size_t) i], rec[2 * (size_t) i + 1]}, {grad[t.x], grad[t.y], grad[t.z]}};
+  }
+  __device__ __forceinline__ void add(const Rec& r) {
+    tot += r.e.a.x;
+    const float ey[3] = {r.e.a.y, r.e.a.z, r.e.a.w}, ex[3] = {r.e.b.x, r.e.b.y, r.e.b.z};
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const float dx = (float) (r.g[j].x - gv.x), dy = (float) (r.g[j].y - gv.y);
+      h[0] += 2.f * (dx * ey[j]);
+      h[1] += 2.f * (dx * ex[j]);
+      h[2] += 2.f * (dy * ey[j]);
+      h[3] += 2.f * (dy * ex[j]);
     }
+  }
+  __device__ __forceinline__ void finish(const DMesh& m, int v) {
     const float it = __frcp_rn(tot);
     const float t0 = h[0] * it, t1 = 0.5f * (h[1] + h[2]) * it, t2 = h[3] * it;
     float mm[4] = {t0, t1, t1, t2}, val[2], vec[4];
@@ -208,32 +249,83 @@ __global__ void k_hessian_local_f32(DMesh m, int nb_nodes, const double2* __rest
     m.ten[v] = make_double4((double) (vec[0] * c0 + vec[1] * c2), (double) (vec[0] * c1 + vec[1] * c3),
                             (double) (vec[2] * c1 + vec[3] * c3), 0.0);
   }
+};
+
+/* one thread a vertex, its patch merged in registers; a vertex whose rows do
+ * not fit goes onto rest[*rest_n] (when given; the second pass over the same
+ * rows finds the same ones) */
+constexpr int kPatchThreads = 128;
+
+template <class Sum, int Batch>
+__global__ void __launch_bounds__(kPatchThreads) k_patch_sum(DMesh m, int nb_nodes, Sum zero, int* rest,
+                                                             int* rest_n) {
+  if (trn_failed(m)) return;
+  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
+    int key[kPatchKeys];
+    if (!patch_keys(m, v, key)) {
+      if (rest) trn_append(rest, rest_n, v);
+      continue;
+    }
+    Sum s = zero;
+    s.begin(m, v);
+#pragma unroll
+    for (int c = 0; c < kPatchKeys; c += Batch) {
+      typename Sum::Rec r[Batch];
+#pragma unroll
+      for (int j = 0; j < Batch; ++j)
+        if (key[c + j] != kNoId && (c + j == 0 || key[c + j] != key[c + j - 1])) r[j] = s.load(m, key[c + j]);
+#pragma unroll
+      for (int j = 0; j < Batch; ++j)
+        if (key[c + j] != kNoId && (c + j == 0 || key[c + j] != key[c + j - 1])) s.add(r[j]);
+    }
+    s.finish(m, v);
+  }
+}
+
+/* the listed vertices, a warp each: every lane walks the sorted patch (the
+ * loads are warp-wide broadcasts) and the first writes */
+template <class Sum>
+__global__ void __launch_bounds__(kPatchThreads) k_patch_sum_rest(DMesh m, Sum zero, const int* rest,
+                                                                  const int* rest_n) {
+  __shared__ int s_buf[kPatchThreads / 32][TRN_MAX_PATCH];
+  if (trn_failed(m)) return;
+  const int n = *rest_n;
+  int* buf = s_buf[threadIdx.x >> 5];
+  for (int q = trn_tid() >> 5; q < n; q += trn_grid_stride() >> 5) {
+    const int v = rest[q];
+    const int k = patch_sort_warp(m, v, buf);
+    Sum s = zero;
+    s.begin(m, v);
+    for (int i = 0; i < k; ++i)
+      if (i == 0 || buf[i] != buf[i - 1]) s.add(s.load(m, buf[i]));
+    if ((threadIdx.x & 31) == 0) s.finish(m, v);
+    __syncwarp();
+  }
+}
+
+__device__ __forceinline__ double complexity_term(const DMesh& m, int i) {
+  const int4 v = m.tri[i];
+  if (v.x < 0) return 0.0;
+  double2 p0 = m.pts[v.x], p1 = m.pts[v.y], p2 = m.pts[v.z];
+  double s0 = p1.x - p0.x;
+  double s1 = p2.x - p0.x;
+  double s2 = p1.y - p0.y;
+  double s3 = p2.y - p0.y;
+  double area = 0.5 * (s0 * s3 - s1 * s2);
+  double rho = 0.;
+  int ids[3] = {v.x, v.y, v.z};
+  for (int j = 0; j < 3; ++j) {
+    double4 t = m.ten[ids[j]];
+    double det = t.x * t.z - trn_pow(t.y, 2);
+    rho += sqrt(det);
+  }
+  rho /= 3;
+  return rho * area;
 }
 
 __global__ void k_complexity_term(DMesh m, int nb_elems, double* __restrict__ terms) {
   if (trn_failed(m)) return;
-  for (int i = trn_tid(); i < nb_elems; i += trn_grid_stride()) {
-    int4 v = m.tri[i];
-    if (v.x < 0) {
-      terms[i] = 0.0;
-      continue;
-    }
-    double2 p0 = m.pts[v.x], p1 = m.pts[v.y], p2 = m.pts[v.z];
-    double s0 = p1.x - p0.x;
-    double s1 = p2.x - p0.x;
-    double s2 = p1.y - p0.y;
-    double s3 = p2.y - p0.y;
-    double area = 0.5 * (s0 * s3 - s1 * s2);
-    double rho = 0.;
-    int ids[3] = {v.x, v.y, v.z};
-    for (int j = 0; j < 3; ++j) {
-      double4 t = m.ten[ids[j]];
-      double det = t.x * t.z - trn_pow(t.y, 2);
-      rho += sqrt(det);
-    }
-    rho /= 3;
-    terms[i] = rho * area;
-  }
+  for (int i = trn_tid(); i < nb_elems; i += trn_grid_stride()) terms[i] = complexity_term(m, i);
 }
 
 /* one thread, element order: the 1-thread reference's summation */
@@ -252,10 +344,8 @@ __global__ void k_sum_sequential(const double* __restrict__ terms, int n, double
 }
 
 /* deterministic tree: fixed per-block partials, then one block in order */
-__global__ void k_sum_partial(const double* __restrict__ terms, int n, double* partial) {
+__device__ __forceinline__ void block_partial(double s, double* partial) {
   __shared__ double sm[TRN_THREADS];
-  double s = 0;
-  for (int i = trn_tid(); i < n; i += trn_grid_stride()) s += terms[i];
   sm[threadIdx.x] = s;
   __syncthreads();
   for (int o = TRN_THREADS / 2; o > 0; o >>= 1) {
@@ -263,6 +353,20 @@ __global__ void k_sum_partial(const double* __restrict__ terms, int n, double* p
     __syncthreads();
   }
   if (threadIdx.x == 0) partial[blockIdx.x] = sm[0];
+}
+
+__global__ void k_sum_partial(const double* __restrict__ terms, int n, double* partial) {
+  double s = 0;
+  for (int i = trn_tid(); i < n; i += trn_grid_stride()) s += terms[i];
+  block_partial(s, partial);
+}
+
+/* the elements' complexity terms straight into the tree's first level */
+__global__ void k_sum_terms(DMesh m, int nb_elems, double* partial) {
+  double s = 0;
+  if (!trn_failed(m))
+    for (int i = trn_tid(); i < nb_elems; i += trn_grid_stride()) s += complexity_term(m, i);
+  block_partial(s, partial);
 }
 
 __global__ void k_sum_final(const double* __restrict__ partial, int nb, double* out) {
@@ -325,65 +429,89 @@ void sum_tree(const double* in, int n, double* partial, double* out, cudaStream_
   note_launch();
 }
 
-void metric_run(const DMesh& m, int nb_nodes, int nb_elems, const double* solut, double2* grad,
-                double* terms, double* complexity, bool exact_sum, const MetricParams& p,
-                cudaStream_t s, const MetricSaves* keep, bool fp32) {
+/* a patch mean: the elements' records are ready in ws.rec; the vertices
+ * that the register merge cannot take are listed by the first pass (collect)
+ * and served by the second kernel, which returns at once when there are none */
+template <int Batch, class Sum>
+static void patch_sum(const DMesh& m, int nb_nodes, const Sum& zero, const MetricWs& ws, bool collect,
+                      cudaStream_t s) {
+  auto* fast = k_patch_sum<Sum, Batch>;
+  auto* rest = k_patch_sum_rest<Sum>;
+  fast<<<TRN_RESIDENT(fast, grid_for(nb_nodes, kPatchThreads), kPatchThreads), kPatchThreads, 0, s>>>(
+      m, nb_nodes, zero, collect ? ws.rest : nullptr, ws.rest_n);
+  note_launch();
+  rest<<<TRN_RESIDENT(rest, grid_for(32LL * nb_nodes, kPatchThreads), kPatchThreads), kPatchThreads, 0, s>>>(
+      m, zero, ws.rest, ws.rest_n);
+  note_launch();
+}
+
+void metric_patches(const DMesh& m, int nb_nodes, int nb_elems, const double* solut, double2* grad,
+                    const MetricWs& ws, double scale_exp, cudaStream_t s, const MetricSaves* keep, bool fp32) {
+  const double V = nb_nodes, E = nb_elems;
+  const int ge = grid_for(nb_elems);
+  cudaMemsetAsync(ws.rest_n, 0, sizeof(int), s);
   if (fp32) {
-    const double V = nb_nodes, E = nb_elems;
+    float4* rec = reinterpret_cast<float4*>(ws.rec);
     {
     ProfScope ps("metric_gradient", s, V * (2 * kIdx + kAvgDeg * kIdx * 2 + 8 + kPt + 16) + E * kTri);
-    k_gradient_f32<<<grid_for(nb_nodes), TRN_THREADS, 0, s>>>(m, nb_nodes, solut, grad);
+    k_elem_edges<<<ge, TRN_THREADS, 0, s>>>(m, nb_elems, rec);
     note_launch();
+    GradSum32 z{rec, solut, grad};
+    patch_sum<2>(m, nb_nodes, z, ws, true, s);
     }
-    {
     ProfScope ps("metric_hessian", s, V * (2 * kIdx + kAvgDeg * kIdx * 2 + 16 + kPt + kTen) + E * kTri);
-    k_hessian_local_f32<<<grid_for(nb_nodes), TRN_THREADS, 0, s>>>(m, nb_nodes, grad, (float) p.scale_exp);
-    note_launch();
-    }
-    ProfScope ps("metric_complexity", s, E * (kTri + 8) + V * (kPt + kTen));
-    k_complexity_term<<<grid_for(nb_elems), TRN_THREADS, 0, s>>>(m, nb_elems, terms);
-    note_launch();
-    if (exact_sum) {
-      k_sum_sequential<<<1, 32, 0, s>>>(terms, nb_elems, complexity);
-      note_launch();
-    } else {
-      sum_tree(terms, nb_elems, terms + m.capa_elem, complexity, s);
-    }
-    ProfScope ps2("metric_normalize", s, V * 2 * kTen);
-    k_normalize_f32<<<grid_for(nb_nodes), TRN_THREADS, 0, s>>>(m, nb_nodes, complexity, p.target,
-                                                                p.eig_min, p.eig_max);
-    note_launch();
-    check_launch("metric_run");
+    HessSum32 z{rec, grad, (float) scale_exp};
+    patch_sum<2>(m, nb_nodes, z, ws, false, s);
     return;
   }
-  double* atot = keep ? keep->atot : nullptr;
-  double4* hsym = keep ? keep->hsym : nullptr;
-  double4* mloc = keep ? keep->mloc : nullptr;
-  const double V = nb_nodes, E = nb_elems;
+  double* atot = keep && keep->atot ? keep->atot : ws.atot;
   {
   ProfScope ps("metric_gradient", s, V * (2 * kIdx + kAvgDeg * kIdx * 2 + 8 + kPt + 16) + E * kTri);
-  k_gradient<<<grid_for(nb_nodes), TRN_THREADS, 0, s>>>(m, nb_nodes, solut, grad, atot);
+  k_elem_gradient<<<ge, TRN_THREADS, 0, s>>>(m, nb_elems, solut, ws.rec);
   note_launch();
+  GradSum z{ws.rec, grad, atot};
+  patch_sum<4>(m, nb_nodes, z, ws, true, s);
   }
-  {
   ProfScope ps("metric_hessian", s, V * (2 * kIdx + kAvgDeg * kIdx * 2 + 16 + kPt + kTen) + E * kTri);
-  k_hessian_local<<<grid_for(nb_nodes), TRN_THREADS, 0, s>>>(m, nb_nodes, grad, p.scale_exp,
-                                                                hsym, mloc);
+  k_elem_hessian<<<ge, TRN_THREADS, 0, s>>>(m, nb_elems, grad, ws.rec);
   note_launch();
-  }
-  ProfScope ps("metric_complexity", s, E * (kTri + 8) + V * (kPt + kTen));
-  k_complexity_term<<<grid_for(nb_elems), TRN_THREADS, 0, s>>>(m, nb_elems, terms);
-  note_launch();
+  HessSum z{ws.rec, atot, scale_exp, keep ? keep->hsym : nullptr, keep ? keep->mloc : nullptr};
+  patch_sum<4>(m, nb_nodes, z, ws, false, s);
+}
+
+void metric_complexity(const DMesh& m, int nb_elems, double* terms, double* partial, double* complexity,
+                       bool exact_sum, cudaStream_t s) {
   if (exact_sum) {
+    k_complexity_term<<<grid_for(nb_elems), TRN_THREADS, 0, s>>>(m, nb_elems, terms);
+    note_launch();
     k_sum_sequential<<<1, 32, 0, s>>>(terms, nb_elems, complexity);
     note_launch();
-  } else {
-    /* partials live after the terms (terms has capa_elem + grid slots) */
-    sum_tree(terms, nb_elems, terms + m.capa_elem, complexity, s);
+    return;
   }
-  ProfScope ps2("metric_normalize", s, V * 2 * kTen);
-  k_normalize<<<grid_for(nb_nodes), TRN_THREADS, 0, s>>>(m, nb_nodes, complexity, p.target,
-                                                          p.eig_min, p.eig_max);
+  const int nb = grid_for(nb_elems);
+  k_sum_terms<<<nb, TRN_THREADS, 0, s>>>(m, nb_elems, partial);
+  note_launch();
+  k_sum_final<<<1, TRN_THREADS, 0, s>>>(partial, nb, complexity);
+  note_launch();
+}
+
+void metric_run(const DMesh& m, int nb_nodes, int nb_elems, const double* solut, double2* grad,
+                double* terms, double* complexity, bool exact_sum, const MetricParams& p, const MetricWs& ws,
+                cudaStream_t s, const MetricSaves* keep, bool fp32) {
+  const double V = nb_nodes, E = nb_elems;
+  metric_patches(m, nb_nodes, nb_elems, solut, grad, ws, p.scale_exp, s, keep, fp32);
+  {
+  ProfScope ps("metric_complexity", s, E * (kTri + 8) + V * (kPt + kTen));
+  /* partials live after the terms (terms has capa_elem + grid slots) */
+  metric_complexity(m, nb_elems, terms, terms + m.capa_elem, complexity, exact_sum, s);
+  }
+  ProfScope ps("metric_normalize", s, V * 2 * kTen);
+  if (fp32)
+    k_normalize_f32<<<grid_for(nb_nodes), TRN_THREADS, 0, s>>>(m, nb_nodes, complexity, p.target, p.eig_min,
+                                                              p.eig_max);
+  else
+    k_normalize<<<grid_for(nb_nodes), TRN_THREADS, 0, s>>>(m, nb_nodes, complexity, p.target, p.eig_min,
+                                                          p.eig_max);
   note_launch();
   check_launch("metric_run");
 }

@@ -12,7 +12,7 @@
  *
  * The scratch array is sized for at most TRN_NOALLOC_MAX_NODES vertices,
  * TRN_NOALLOC_MAX_ELEMS triangles and TRN_NOALLOC_BUCKET triangles around one
- * vertex; it takes about 6 MB on every GPU that loads this library, for as
+ * vertex; it takes about 7 MB on every GPU that loads this library, for as
  * long as the process lives. Every call on a device shares it: calls that
  * overlap on the GPU (other streams, other host threads) race and corrupt
  * each other's results, so serialise them. The array keeps the last call's
@@ -44,14 +44,6 @@ namespace trn {
 __global__ void k_fill_stencils(DMesh m, int nb_elems);
 __global__ void k_sort_stencils(DMesh m, int nb_nodes);
 __global__ void k_build_vicin(DMesh m, int nb_nodes, int only_flagged);
-__global__ void k_gradient(DMesh m, int nb_nodes, const double* __restrict__ solut,
-                           double2* __restrict__ grad, double* __restrict__ atot);
-__global__ void k_hessian_local(DMesh m, int nb_nodes, const double2* __restrict__ grad,
-                                double scale_exp, double4* __restrict__ hsym,
-                                double4* __restrict__ mloc);
-__global__ void k_complexity_term(DMesh m, int nb_elems, double* __restrict__ terms);
-__global__ void k_sum_partial(const double* __restrict__ terms, int n, double* partial);
-__global__ void k_sum_final(const double* __restrict__ partial, int nb, double* out);
 __global__ void k_normalize(DMesh m, int nb_nodes, const double* complexity, double target,
                             double eig_min, double eig_max);
 
@@ -75,7 +67,10 @@ constexpr size_t oVdeg = oDeg + align256(sizeof(int) * kMaxN);
 constexpr size_t oAlive = oVdeg + align256(sizeof(int) * kMaxN);
 constexpr size_t oGrad = oAlive + align256(kMaxN);
 constexpr size_t oTerms = oGrad + align256(sizeof(double2) * kMaxN);
-constexpr size_t oCplx = oTerms + align256(sizeof(double) * (kMaxE + kPartials));
+constexpr size_t oRec = oTerms + align256(sizeof(double) * kPartials);
+constexpr size_t oAtot = oRec + align256(sizeof(double4) * kMaxE);
+constexpr size_t oRest = oAtot + align256(sizeof(double) * kMaxN);
+constexpr size_t oCplx = oRest + align256(sizeof(int) * (kMaxN + 1));
 constexpr size_t oErr = oCplx + 256;
 constexpr size_t kScratchBytes = oErr + 256;
 
@@ -194,11 +189,10 @@ extern "C" int trn_metric_noalloc(int nb_nodes, int nb_elems, const double* d_po
   const double scale_exp = lp_norm ? -1. / (2 * lp_norm + 2) : 0.5;
   const double eig_min = 1 / trn_pow(h_min, 2);
   const double eig_max = 1 / trn_pow(h_max, 2);
-  k_gradient<<<gv, TRN_THREADS, 0, s>>>(d, nb_nodes, d_solut, grad, nullptr);
-  k_hessian_local<<<gv, TRN_THREADS, 0, s>>>(d, nb_nodes, grad, scale_exp, nullptr, nullptr);
-  k_complexity_term<<<ge, TRN_THREADS, 0, s>>>(d, nb_elems, terms);
-  k_sum_partial<<<ge, TRN_THREADS, 0, s>>>(terms, nb_elems, terms + kMaxE);
-  k_sum_final<<<1, TRN_THREADS, 0, s>>>(terms + kMaxE, ge, cplx);
+  int* rest = reinterpret_cast<int*>(base + oRest);
+  const MetricWs ws{reinterpret_cast<double4*>(base + oRec), reinterpret_cast<double*>(base + oAtot), rest + 1, rest};
+  metric_patches(d, nb_nodes, nb_elems, d_solut, grad, ws, scale_exp, s);
+  metric_complexity(d, nb_elems, nullptr, terms, cplx, false, s);
   k_normalize<<<gv, TRN_THREADS, 0, s>>>(d, nb_nodes, cplx, target, eig_min, eig_max);
   k_na_tensor<<<gv, TRN_THREADS, 0, s>>>(d.ten, nb_nodes, d_tensor);
   if (cudaPeekAtLastError() != cudaSuccess) return TRN_ERR_CUDA;

@@ -220,9 +220,12 @@ __global__ void k_ref_cut(DMesh m, int nb_elems, const int4* __restrict__ info,
 }
 
 void refine_ws_alloc(RefineWs* ws, int capa_node, int capa_elem) {
-  cudaMalloc(&ws->info, sizeof(int4) * (size_t) capa_elem);
-  cudaMalloc(&ws->cnt, sizeof(long long) * (size_t) capa_elem);
-  cudaMalloc(&ws->off, sizeof(long long) * (size_t) capa_elem);
+  /* one block of 32 bytes an element: the metric recovery keeps its element
+   * records there between refinements */
+  const size_t ce = (size_t) capa_elem;
+  cudaMalloc(&ws->info, (sizeof(int4) + 2 * sizeof(long long)) * ce);
+  ws->cnt = reinterpret_cast<long long*>(ws->info + ce);
+  ws->off = ws->cnt + ce;
   unsigned long long cap = 1024;
   while (cap < 2ULL * (unsigned long long) capa_node) cap <<= 1;
   ws->hcap = cap;
@@ -232,8 +235,6 @@ void refine_ws_alloc(RefineWs* ws, int capa_node, int capa_elem) {
 
 void refine_ws_free(RefineWs* ws) {
   cudaFree(ws->info);
-  cudaFree(ws->cnt);
-  cudaFree(ws->off);
   cudaFree(ws->hkey);
   cudaFree(ws->hval);
   *ws = RefineWs();

@@ -102,6 +102,14 @@ struct trn_mesh {
 
 namespace {
 
+/* the recovery works in buffers that are free meanwhile: refinement's
+ * (32 bytes an element, and 8 bytes a vertex in its edge table) and the list
+ * that a compaction fills */
+MetricWs metric_ws(trn_mesh* m) {
+  return MetricWs{reinterpret_cast<double4*>(m->rws.info), reinterpret_cast<double*>(m->rws.hval), m->list,
+                  m->scan.count};
+}
+
 int fail(trn_mesh* m, int code, const std::string& msg) {
   if (m) m->err = msg;
   return code;
@@ -908,7 +916,7 @@ int trn_metric_run(trn_mesh* m, double target_factor, int norm, double h_min, do
   p.eig_max = 1 / trn_pow(h_max, 2);
   begin_timing(m);
   metric_run(m->d, m->nb_nodes, m->nb_elems, m->solut, m->grad, m->terms, m->complexity,
-             m->exact_sum || m->replay, p, m->stream, nullptr, m->fp32);
+             m->exact_sum || m->replay, p, metric_ws(m), m->stream, nullptr, m->fp32);
   CK(cudaMemcpyAsync(m->h_status + H_WIDE, m->complexity, sizeof(double), cudaMemcpyDeviceToHost, m->stream));
   int rc = sync_status(m);
   if (rc) return rc;
@@ -1190,6 +1198,7 @@ int trn_quality_adjoint(trn_mesh* m, const double* xy, const double* solut, doub
     um.grad = m->grad;
     um.terms = m->terms;
     um.exact_sum = m->exact_sum || m->replay;
+    um.ws = metric_ws(m);
     um.p.target = (double) (int) std::floor(m->nb_nodes * target_factor);
     um.p.scale_exp = norm ? -1. / (2 * norm + 2) : 0.5;
     um.p.eig_min = 1 / trn_pow(h_min, 2);

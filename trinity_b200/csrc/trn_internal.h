@@ -192,13 +192,29 @@ struct MetricSaves {
   double4* hsym = nullptr;
   double4* mloc = nullptr;
 };
+/* scratch of the recovery: one 32-byte record per element, the patch areas,
+ * and the vertices whose patch the register merge cannot take */
+struct MetricWs {
+  double4* rec = nullptr;
+  double* atot = nullptr;
+  int* rest = nullptr;
+  int* rest_n = nullptr;
+};
+/* the recovery's two patch means, up to the locally normalised tensors; the
+ * complexity sum (partial: grid_for(nb_elems) slots; terms: nb_elems, exact_sum
+ * only) */
+void metric_patches(const DMesh& m, int nb_nodes, int nb_elems, const double* solut, double2* grad,
+                    const MetricWs& ws, double scale_exp, cudaStream_t s, const MetricSaves* keep = nullptr,
+                    bool fp32 = false);
+void metric_complexity(const DMesh& m, int nb_elems, double* terms, double* partial, double* complexity,
+                       bool exact_sum, cudaStream_t s);
 /* fp32: the mixed-precision form's recovery (FP32 patch means with FP64
  * coordinate and value differences, FP32 normalisations, FP64 complexity
  * sum; writes the FP32 tensor copy and logarithm cache too) */
 void metric_run(const DMesh& m, int nb_nodes, int nb_elems, const double* solut,
                 double2* grad, double* terms, double* complexity, bool exact_sum,
-                const MetricParams& p, cudaStream_t s, const MetricSaves* keep = nullptr,
-                bool fp32 = false);
+                const MetricParams& p, const MetricWs& ws, cudaStream_t s,
+                const MetricSaves* keep = nullptr, bool fp32 = false);
 /* deterministic two-level sum of n doubles; partial holds grid_for(n) slots */
 void sum_tree(const double* in, int n, double* partial, double* out, cudaStream_t s);
 
@@ -349,6 +365,7 @@ struct AdjMetric {
   double* terms;       /* complexity terms (capa_elem + partial slots) */
   bool exact_sum;
   MetricParams p;
+  MetricWs ws;
 };
 /* J -> ws.scal[1]; gxy (2 per vertex) and gu (per vertex) may be null; um
  * null: the metric is the mesh's own tensors */
