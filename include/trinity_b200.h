@@ -189,10 +189,9 @@ int trn_smooth_gradient_run(trn_mesh* mesh, int max_colors, int steps, double ma
  * search), cfg[4] flip block, cfg[5] lanes per smoothed vertex (1, 2, 4,
  * 8), cfg[6] variant of the smoothing kernel with 2 or more lanes (0: the
  * back-off tries in turn, up to 128 registers, two 256-thread blocks per SM;
- * 1: capped for three; 2: for four; 3: as 2, element metrics in shared
- * memory; 4, 5, 6: the five tries in one sweep, capped for four, three,
- * two blocks; 7, 8: the sweep with the element metrics in shared memory,
- * two or three blocks; one lane a vertex reads 0-2 only and treats 3-8 as
+ * 1: capped for three; 2, 3: for four; 4: the five tries in one sweep, capped
+ * for four; 5, 8: for three; 6, 7: for two; one lane a vertex reads 0-2 only
+ * and treats 3-8 as
  * 2). Defaults: 2 lanes, variant 7, 256-thread blocks. Per mesh; a
  * captured round is recaptured when they change. trn_autotune chooses them
  * on the loaded mesh, timing metric + `rounds` rounds from the input (the

@@ -292,40 +292,152 @@ __device__ __forceinline__ double4 log_pair(double t0, double t1, double t2, int
   return make_double4(cache[0], cache[1], cache[2], cache[3]);
 }
 
+/* ---- the sweep's decisions ----
+ * A try only needs to know whether every element stays CCW with quality above
+ * the old minimum; the qualities themselves are wanted for the one try that
+ * is kept. So the sweep decides with a cheap estimate whose error is bounded,
+ * evaluates exactly only what the bound leaves open (a floating-point filter,
+ * Shewchuk 1997), and the commit evaluates the kept try exactly: the same
+ * decisions and the same bits as exact qualities throughout.
+ *
+ * The element has corners (i, B, C), i moving along pini + w (o - pini). With
+ * u = B - pini, v = C - pini, d = o - pini, b = C - B, twice its area is
+ * u x v - w d x b and its squared metric edge lengths are
+ * |u|^2 - 2 w <u,d> + w^2 |d|^2, the same with v, and |b|^2: three quadratics
+ * in w whose coefficients are taken in FP64 once for the five tries. Each
+ * value is rounded to FP32, where square roots and reciprocals are one
+ * instruction. Error of the estimate, relative, in units of 1e-7: an edge 1.5
+ * (conversion 2^-24 halved by the root, root 2^-23), the perimeter p 2.7,
+ * min(p/3, 3/p) 5.1, f(2-f) 6.3, its cube 20, 1/p^2 8.4, the products 3:
+ * under 32, so 80 (kTryMargin) decides. The FP64 part must stay far below:
+ * with t = j0 + j2, every term of a squared length is at most 2 t (|u|^2 +
+ * |d|^2) and is rounded to 1e-15 of that, and the tried positions themselves
+ * are rounded to e = 1e-15 times the coordinates, which moves a squared length
+ * by a relative sqrt(t) e / length; lengths that are not 1e8 times above
+ * either, and areas that are not, are left to the exact evaluation (flat or
+ * nearly degenerate elements, anisotropy beyond 1e4). Smoothing of two rounds
+ * of the 2M-triangle workload, FP64: 8.03 ms with five exact evaluations,
+ * 6.57 ms with the estimate (2 lanes, two blocks an SM). */
+constexpr float kTryMargin = 8.e-6f;
+
+__device__ __forceinline__ float try_sqrt(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float try_rcp(float x) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+/* bits 0-4: try w passes this element; bits 5-9: try w is undecided */
+__device__ __forceinline__ unsigned try_filter(double2 pini, double2 o, double2 B, double2 C, double4 jm,
+                                               double q_min) {
+  const double dx = o.x - pini.x, dy = o.y - pini.y;
+  const double ux = B.x - pini.x, uy = B.y - pini.y, vx = C.x - pini.x, vy = C.y - pini.y;
+  const double bx = C.x - B.x, by = C.y - B.y;
+  const double mdx = __fma_rn(jm.x, dx, jm.y * dy), mdy = __fma_rn(jm.y, dx, jm.z * dy);
+  const double uu = __fma_rn(ux, __fma_rn(jm.x, ux, jm.y * uy), uy * __fma_rn(jm.y, ux, jm.z * uy));
+  const double vv = __fma_rn(vx, __fma_rn(jm.x, vx, jm.y * vy), vy * __fma_rn(jm.y, vx, jm.z * vy));
+  const double bb = __fma_rn(bx, __fma_rn(jm.x, bx, jm.y * by), by * __fma_rn(jm.y, bx, jm.z * by));
+  const double dd = __fma_rn(dx, mdx, dy * mdy);
+  const double ud = -2.0 * __fma_rn(ux, mdx, uy * mdy), vd = -2.0 * __fma_rn(vx, mdx, vy * mdy);
+  const double h = 0.5 * jm.w;
+  const double a0 = h * __fma_rn(ux, vy, -(uy * vx)), a1 = -h * __fma_rn(dx, by, -(dy * bx));
+  /* what must be exceeded: lt for the squared lengths, at for area x sqrt(det) */
+  const double e = 1.e-15 * (fabs(pini.x) + fabs(pini.y) + fabs(o.x) + fabs(o.y));
+  const double L = fabs(ux) + fabs(uy) + fabs(vx) + fabs(vy) + fabs(dx) + fabs(dy);
+  const double LL = L * L;
+  const float lt = (float) ((jm.x + jm.z) * __fma_rn(4.e-8, LL, 1.e16 * (e * e)));
+  const float at = (float) (h * __fma_rn(4.e-8, LL, 1.e8 * (e * L)));
+  const float ae = (float) (h * __fma_rn(1.e-14, LL, 1.e1 * (e * L)));
+  const float ccw = (float) (2.0 * h * TRN_EPS);
+  const float fbb = (float) bb, lb = try_sqrt(fbb);
+  const float qlo = (float) q_min * (1.f - kTryMargin), qhi = (float) q_min * (1.f + kTryMargin);
+  const bool base = fbb > lt && qlo > 1.e-20f;
+  unsigned m = 0;
+  double w = 1;
+#pragma unroll
+  for (int k = 0; k < 5; ++k, w *= 0.5) {
+    const float fu = (float) __fma_rn(w, __fma_rn(w, dd, ud), uu);
+    const float fv = (float) __fma_rn(w, __fma_rn(w, dd, vd), vv);
+    const float fa = (float) __fma_rn(w, a1, a0);
+    const float p = try_sqrt(fu) + try_sqrt(fv) + lb;
+    const float ip = try_rcp(p);
+    const float f = fminf(p * 0.333333343f, 3.f * ip);
+    const float g = f * (2.f - f);
+    const float q = fa * (20.78460969082653f * (g * g * g)) * (ip * ip);
+    const bool sure = base && fu > lt && fv > lt && fa > at && fa > (ccw + ae) * (1.f + 1.e-6f);
+    const bool flat = fa + ae < ccw * (1.f - 1.e-6f);   /* certainly not CCW */
+    if (sure && q > qhi) m |= 1u << k;
+    else if (!(flat || (sure && q < qlo))) m |= 32u << k;
+  }
+  return m;
+}
+
+/* the passing tries of one element (bit w), all five decided */
+template <bool F32>
+__device__ __forceinline__ unsigned try_mask(const DMesh& m, int i, int4 n, double2 pini, double2 o, JmT<F32> jm,
+                                             double q_min) {
+  const double2 b0 = (n.x == i) ? pini : m.pts[n.x];
+  const double2 b1 = (n.y == i) ? pini : m.pts[n.y];
+  const double2 b2 = (n.z == i) ? pini : m.pts[n.z];
+  unsigned ok = 0, open = 0x1f;
+  if constexpr (!F32) {
+    if (n.x == i || n.y == i || n.z == i) {
+      const double2 B = n.x == i ? b1 : (n.y == i ? b2 : b0), C = n.x == i ? b2 : (n.y == i ? b0 : b1);
+      const unsigned f = try_filter(pini, o, B, C, jm, q_min);
+      ok = f & 0x1f;
+      open = f >> 5;
+    }
+    if (!open) return ok;
+  }
+  double weight = 1;
+#pragma unroll
+  for (int w = 0; w < 5; ++w, weight *= 0.5) {
+    if (!F32 && !(open & (1u << w))) continue;
+    double2 pw;
+    pw.x = (1 - weight) * pini.x + weight * o.x;
+    pw.y = (1 - weight) * pini.y + weight * o.y;
+    const double2 p0 = (n.x == i) ? pw : b0;
+    const double2 p1 = (n.y == i) ? pw : b1;
+    const double2 p2 = (n.z == i) ? pw : b2;
+    if (trn_ccw(p0, p1, p2) && qgeom_x(p0, p1, p2, jm) > q_min) ok |= 1u << w;
+  }
+  return ok;
+}
+
+/* the element metric of stencil element n of vertex i, whose new logarithm is lnew */
+template <bool F32>
+__device__ __forceinline__ JmT<F32> elem_metric(const DMesh& m, int i, int4 n, LogT<F32> lnew) {
+  return qmetric_x((n.x == i) ? lnew : log_load<F32>(m, n.x), (n.y == i) ? lnew : log_load<F32>(m, n.y),
+                   (n.z == i) ? lnew : log_load<F32>(m, n.z));
+}
+
 /* V selects how the back-off runs:
  *   0  the tries in turn, element metrics in registers;
- *   1  the same with the element metrics in shared memory (KQ slots a
- *      thread, stride blockDim.x) and the lane's element records prefetched
- *      into L1 while the stencil minimum is read;
- *   2  one sweep over the lane's elements evaluates all five tries (the
- *      element's points loaded once, five independent geometry chains), the
- *      group ANDs the lanes' five-bit pass masks and keeps the first try that
- *      passes; the qualities wait in shared memory (5 x KQ a thread). A
- *      warp of 8 groups almost always runs all five tries in turn anyway
- *      (half the moves fail every try), so this costs no extra issue and
- *      turns a serial chain into parallel ones. Same tries, same arithmetic,
- *      same first passing try: the same bits;
- *   3  the sweep of 2 with the element metrics in shared memory too (before
- *      the qualities), which frees the registers the five chains need. */
+ *   1  one sweep over the lane's elements decides all five tries (try_mask),
+ *      the group ANDs the lanes' five-bit pass masks and keeps the first try
+ *      that passes, whose qualities the commit evaluates. A warp of 8 groups
+ *      or more almost always runs all five tries in turn anyway (half the
+ *      moves fail every try), so this costs no extra issue and turns a serial
+ *      chain into parallel ones. The element metrics of the lane's first KQ
+ *      elements wait in shared memory (stride blockDim.x), which frees
+ *      registers; those of later ones (long stencils) are taken again.
+ * Same tries, same arithmetic, same first passing try: the same bits. */
 template <bool F32, int G, int V>
 __device__ int move_laplacian_grp(const DMesh& m, int i, int lane, unsigned gmask, unsigned char* smem) {
   static_assert(G >= 2, "lane groups of two or more");
-  constexpr bool JS = V == 1 || V == 3;
-  constexpr bool SW = V >= 2;
+  constexpr bool SW = V == 1;
   constexpr int KQ = G >= 4 ? 2 : 3;
   JmT<F32>* js = reinterpret_cast<JmT<F32>*>(smem) + threadIdx.x;
-  double* qs = reinterpret_cast<double*>(smem + (JS ? (size_t) KQ * blockDim.x * sizeof(JmT<F32>) : 0)) +
-               threadIdx.x;
   const int* vc = m.vic + (size_t) i * m.bucket;
   const int* st = m.stenc + (size_t) i * m.bucket;
   const int deg = trn_deg(m, i);
   const int nb_neigh = m.vdeg[i];
   double q_min = 1.7976931348623157e308;
-  for (int a = lane; a < deg; a += G) {
-    const int e = st[a];
-    if constexpr (JS) asm volatile("prefetch.global.L1 [%0];" ::"l"(m.tri + e));
-    q_min = trn_dmin(q_min, m.qual[e]);
-  }
+  for (int a = lane; a < deg; a += G) q_min = trn_dmin(q_min, m.qual[st[a]]);
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) q_min = trn_dmin(q_min, __shfl_xor_sync(gmask, q_min, o, G));
   const double2 pini = m.pts[i];
@@ -378,78 +490,35 @@ __device__ int move_laplacian_grp(const DMesh& m, int i, int lane, unsigned gmas
     lnew = log_of<F32>(tn[0], tn[1], tn[2]);
   }
   const double4 tnew = make_double4(tn[0], tn[1], tn[2], 0.0);
-  /* qualities and element metrics kept per lane (a stencil of 6 elements
-   * fits: 2 a lane with 4 lanes, 3 with 2); later ones are recomputed */
-  double qv[KQ];
   /* the element metrics of this lane's first KQ elements: they do not depend
-   * on where the vertex sits, so the tries below only redo the geometry */
-  JmT<F32> jv[JS ? 1 : KQ];
-#pragma unroll
-  for (int j = 0; j < KQ; ++j) {
-    const int a = lane + j * G;
-    if (a < deg) {
-      const int4 n = m.tri[st[a]];
-      const JmT<F32> q = qmetric_x((n.x == i) ? lnew : log_load<F32>(m, n.x),
-                                   (n.y == i) ? lnew : log_load<F32>(m, n.y),
-                                   (n.z == i) ? lnew : log_load<F32>(m, n.z));
-      if constexpr (JS) js[(size_t) j * blockDim.x] = q;
-      else jv[j] = q;
-    }
-  }
+   * on where the vertex sits, so the tries below only redo the geometry (a
+   * stencil of 6 elements fits: 2 a lane with 4 lanes, 3 with 2) */
   if constexpr (SW) {
+    const double2 o = make_double2(ox, oy);
     unsigned okm = 0x1fu;   /* bit w: every element of this lane passes try w */
     int j = 0;
     for (int a = lane; a < deg; a += G, ++j) {
-      if (j < KQ) {
-        const int4 n = m.tri[st[a]];
-        const double2 b0 = (n.x == i) ? pini : m.pts[n.x];
-        const double2 b1 = (n.y == i) ? pini : m.pts[n.y];
-        const double2 b2 = (n.z == i) ? pini : m.pts[n.z];
-        JmT<F32> jm;
-        if constexpr (JS) jm = js[(size_t) j * blockDim.x];
-        else jm = reg_pick(jv, j);
-        double weight = 1;
-#pragma unroll
-        for (int w = 0; w < 5; ++w) {
-          double2 pw;
-          pw.x = (1 - weight) * pini.x + weight * ox;
-          pw.y = (1 - weight) * pini.y + weight * oy;
-          const double2 p0 = (n.x == i) ? pw : b0;
-          const double2 p1 = (n.y == i) ? pw : b1;
-          const double2 p2 = (n.z == i) ? pw : b2;
-          const bool ccw = trn_ccw(p0, p1, p2);
-          const double q = qgeom_x(p0, p1, p2, jm);
-          qs[(size_t) (w * KQ + j) * blockDim.x] = q;
-          if (!(ccw && q > q_min)) okm &= ~(1u << w);
-          weight *= 0.5;
-        }
-      } else {
-        double weight = 1;
-        for (int w = 0; w < 5; ++w) {
-          double2 pw;
-          pw.x = (1 - weight) * pini.x + weight * ox;
-          pw.y = (1 - weight) * pini.y + weight * oy;
-          double q = 0;
-          if (!(elem_quality_at<F32>(m, i, m.tri[st[a]], pw, lnew, &q) && q > q_min)) okm &= ~(1u << w);
-          weight *= 0.5;
-        }
-      }
+      const int4 n = m.tri[st[a]];
+      const JmT<F32> q = elem_metric<F32>(m, i, n, lnew);
+      if (j < KQ) js[(size_t) j * blockDim.x] = q;
+      okm &= try_mask<F32>(m, i, n, pini, o, q, q_min);
     }
 #pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) okm &= __shfl_xor_sync(gmask, okm, o, G);
+    for (int d = G / 2; d > 0; d >>= 1) okm &= __shfl_xor_sync(gmask, okm, d, G);
     if (!okm) return 0;
-    const int wsel = __ffs(okm) - 1;
     double weight = 1;
-    for (int w = 0; w < wsel; ++w) weight *= 0.5;
+    for (int w = __ffs(okm) - 1; w > 0; --w) weight *= 0.5;
     double2 pa;
     pa.x = (1 - weight) * pini.x + weight * ox;
     pa.y = (1 - weight) * pini.y + weight * oy;
     j = 0;
     for (int a = lane; a < deg; a += G, ++j) {
-      double q = 0;
-      if (j < KQ) q = qs[(size_t) (wsel * KQ + j) * blockDim.x];
-      else elem_quality_at<F32>(m, i, m.tri[st[a]], pa, lnew, &q);
-      m.qual[st[a]] = q;
+      const int4 n = m.tri[st[a]];
+      const JmT<F32> q = j < KQ ? js[(size_t) j * blockDim.x] : elem_metric<F32>(m, i, n, lnew);
+      const double2 p0 = (n.x == i) ? pa : m.pts[n.x];
+      const double2 p1 = (n.y == i) ? pa : m.pts[n.y];
+      const double2 p2 = (n.z == i) ? pa : m.pts[n.z];
+      m.qual[st[a]] = qgeom_x(p0, p1, p2, q);
     }
     if (lane == 0) {
       m.pts[i] = pa;
@@ -457,6 +526,13 @@ __device__ int move_laplacian_grp(const DMesh& m, int i, int lane, unsigned gmas
       log_store<F32>(m, i, lnew);
     }
     return 1;
+  }
+  double qv[KQ];
+  JmT<F32> jv[KQ];
+#pragma unroll
+  for (int j = 0; j < KQ; ++j) {
+    const int a = lane + j * G;
+    if (a < deg) jv[j] = elem_metric<F32>(m, i, m.tri[st[a]], lnew);
   }
   bool valid;
   int retry = 0;
@@ -476,8 +552,7 @@ __device__ int move_laplacian_grp(const DMesh& m, int i, int lane, unsigned gmas
         const double2 p2 = (n.z == i) ? pa : m.pts[n.z];
         ok = trn_ccw(p0, p1, p2);
         if (ok) {
-          if constexpr (JS) q = qgeom_x(p0, p1, p2, js[(size_t) j * blockDim.x]);
-          else q = qgeom_x(p0, p1, p2, reg_pick(jv, j));
+          q = qgeom_x(p0, p1, p2, reg_pick(jv, j));
           ok = q > q_min;
         }
         reg_put(qv, j, q);
@@ -560,20 +635,16 @@ static void smooth_launch(const DMesh& m, const int* list, int n, const int* off
   const int g = grid_for((long long) hint * lanes, t);
   const int regs = tune().smooth_regs;
   if (lanes == 8 || lanes == 4 || lanes == 2) {
-    /* smooth_regs 3: the 64-register cap with the element metrics in shared
-     * memory (KQ = 2 slots a thread for 4 or 8 lanes, 3 for 2); 4, 5, 6: all
-     * five tries in one sweep, registers capped at 64, 80, 128, with 5 x KQ
-     * qualities a thread in shared memory; 7, 8: the sweep with the element
-     * metrics in shared memory too, capped at 128, 80 */
+    /* smooth_regs 0, 1, 2 (and 3): the tries in turn, registers capped for
+     * two, three, four 256-thread blocks an SM; 4, 5 (and 8), 6 (and 7): the
+     * sweep, capped for four, three, two, with the element metrics in shared
+     * memory (KQ = 2 slots a thread for 4 or 8 lanes, 3 for 2) */
     const int kq = lanes >= 4 ? 2 : 3;
     const size_t js_smem = (size_t) kq * t * (fp32 ? sizeof(float4) : sizeof(double4));
-    const size_t sw_smem = (size_t) 5 * kq * t * sizeof(double);
 #define TRN_GRP(F, G, B, V)                                                                   \
   do {                                                                                        \
     auto* kern = k_smooth_move_grp<F, G, B, V>;                                               \
-    const size_t sm = V == 1 ? js_smem : V == 2 ? sw_smem : V == 3 ? js_smem + sw_smem : 0;   \
-    if (sm > (48u << 10))                                                                     \
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm);      \
+    const size_t sm = V == 1 ? js_smem : 0;                                                   \
     kern<<<grid_resident(reinterpret_cast<const void*>(kern), t, g, sm), t, sm, s>>>(m, list, n, off, c, \
                                                                                      counters, bc); \
   } while (0)
@@ -581,13 +652,10 @@ static void smooth_launch(const DMesh& m, const int* list, int n, const int* off
   do {                                                                                        \
     if (regs == 0) TRN_GRP(F, G, 2, 0);                                                       \
     else if (regs == 1) TRN_GRP(F, G, 3, 0);                                                  \
-    else if (regs == 2) TRN_GRP(F, G, 4, 0);                                                  \
-    else if (regs == 3) TRN_GRP(F, G, 4, 1);                                                  \
-    else if (regs == 4) TRN_GRP(F, G, 4, 2);                                                  \
-    else if (regs == 5) TRN_GRP(F, G, 3, 2);                                                  \
-    else if (regs == 6) TRN_GRP(F, G, 2, 2);                                                  \
-    else if (regs == 7) TRN_GRP(F, G, 2, 3);                                                  \
-    else TRN_GRP(F, G, 3, 3);                                                                 \
+    else if (regs <= 3) TRN_GRP(F, G, 4, 0);                                                  \
+    else if (regs == 4) TRN_GRP(F, G, 4, 1);                                                  \
+    else if (regs == 5 || regs == 8) TRN_GRP(F, G, 3, 1);                                     \
+    else TRN_GRP(F, G, 2, 1);                                                                 \
   } while (0)
     if (lanes == 8) {
       if (fp32) TRN_GRP_B(true, 8);

@@ -96,11 +96,9 @@ struct Tune {
   int group_max = 16384;      /* longest level list the grouped search takes */
   int flip_threads = 256;     /* k_swap_flip block: 128, 256, 512 */
   int smooth_lanes = 2;       /* lanes per smoothed vertex: 1, 2, 4, 8 */
-  int smooth_regs = 7;        /* smoothing registers: 0 up to 128, 1 capped at 80 (three 256-thread
-                                 blocks an SM), 2 at 64 (four), 3 at 64 with the grouped form's
-                                 element metrics in shared memory; 4, 5, 6: the grouped form's
-                                 five tries in one sweep, capped at 64, 80, 128; 7, 8: the sweep
-                                 with the element metrics in shared memory, capped at 128, 80 */
+  int smooth_regs = 7;        /* smoothing variant: 0 the tries in turn, up to 128 registers, 1 capped
+                                 at 80 (three 256-thread blocks an SM), 2 (and 3) at 64 (four); 4, 5
+                                 (and 8), 6 (and 7): the five tries in one sweep, capped at 64, 80, 128 */
   bool operator==(const Tune& o) const {
     return smooth_threads == o.smooth_threads && filter_threads == o.filter_threads &&
            group_lanes == o.group_lanes && group_max == o.group_max && flip_threads == o.flip_threads &&
