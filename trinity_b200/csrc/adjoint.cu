@@ -222,7 +222,7 @@ __global__ void k_adj_vertex(DMesh f, int nb_nodes, const AReal<F32>* __restrict
   using R = AReal<F32>;
   if (trn_failed(f)) return;
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    const int* st = f.stenc + (size_t) v * f.bucket;
+    const TrnRow st = trn_row(f.stenc, f, v);
     const int deg = f.alive[v] ? trn_deg(f, v) : 0;
     R gx = 0, gy = 0, g[3] = {0, 0, 0};
     for (int a = 0; a < deg; ++a) {
@@ -368,7 +368,7 @@ __device__ __forceinline__ int patch_owners(const DMesh& m, int4 n, int* ids) {
   int k = 0;
   const int c[3] = {n.x, n.y, n.z};
   for (int j = 0; j < 3; ++j) {
-    const int* vc = m.vic + (size_t) c[j] * m.bucket;
+    const TrnRow vc = trn_row(m.vic, m, c[j]);
     const int nv = min(m.vdeg[c[j]], m.bucket);
     if (k + 1 + nv > TRN_MAX_PATCH) {
       trn_set_error(m.err, TRN_DERR_BUCKET);
@@ -386,13 +386,12 @@ __device__ __forceinline__ int patch_owners(const DMesh& m, int4 n, int* ids) {
 constexpr int kOwnerKeys = 4 * kRowRegs;
 
 __device__ __forceinline__ bool owner_keys(const DMesh& m, int4 n, int* key) {
-  if (m.bucket & 3) return false;   /* rows not 16-byte aligned */
   const int c[3] = {n.x, n.y, n.z};
   const int nv[3] = {m.vdeg[n.x], m.vdeg[n.y], m.vdeg[n.z]};
   if (nv[0] > kRowRegs || nv[1] > kRowRegs || nv[2] > kRowRegs) return false;
   bool ok = true;
 #pragma unroll
-  for (int j = 0; j < 3; ++j) ok &= patch_row(m.vic + (size_t) c[j] * m.bucket, nv[j], key + j * kRowRegs);
+  for (int j = 0; j < 3; ++j) ok &= patch_row(trn_row(m.vic, m, c[j]), nv[j], key + j * kRowRegs);
   if (!ok) return false;
 #pragma unroll
   for (int j = 0; j < kRowRegs; ++j) key[3 * kRowRegs + j] = j < 3 ? c[j] : kNoId;
@@ -456,7 +455,7 @@ __global__ void k_adj_vertex_hess(DMesh m, int nb_nodes, const AReal<F32>* __res
   using R = AReal<F32>;
   if (trn_failed(m)) return;
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    const int* st = m.stenc + (size_t) v * m.bucket;
+    const TrnRow st = trn_row(m.stenc, m, v);
     const int deg = m.alive[v] ? trn_deg(m, v) : 0;
     R gx = 0, gy = 0;
     for (int a = 0; a < deg; ++a) {
@@ -480,7 +479,7 @@ __global__ void k_adj_vertex_u(DMesh m, int nb_nodes, const AReal<F32>* __restri
   using R = AReal<F32>;
   if (trn_failed(m)) return;
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    const int* st = m.stenc + (size_t) v * m.bucket;
+    const TrnRow st = trn_row(m.stenc, m, v);
     const int deg = m.alive[v] ? trn_deg(m, v) : 0;
     R g = 0;
     for (int a = 0; a < deg; ++a) {
@@ -498,7 +497,7 @@ __global__ void k_adj_vertex_u(DMesh m, int nb_nodes, const AReal<F32>* __restri
 __global__ void k_adj_star_area(DMesh m, int nb_nodes, double* __restrict__ astar) {
   if (trn_failed(m)) return;
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    const int* st = m.stenc + (size_t) v * m.bucket;
+    const TrnRow st = trn_row(m.stenc, m, v);
     const int deg = m.alive[v] ? trn_deg(m, v) : 0;
     double a = 0;
     for (int k = 0; k < deg; ++k) a += elem_grad(m, st[k]).area;
@@ -638,7 +637,7 @@ void quality_adjoint(const DMesh& m, int nb_nodes, int nb_elems, const double2* 
 template <bool F32>
 __device__ int move_gradient(const DMesh& m, int i, double max_len, int mode) {
   const bool use_log = (mode & 1) != 0, follow = (mode & 2) != 0;
-  const int* st = m.stenc + (size_t) i * m.bucket;
+  const TrnRow st = trn_row(m.stenc, m, i);
   const int deg = trn_deg(m, i);
   double q_min = 1.7976931348623157e308, obj = 0;
   for (int a = 0; a < deg; ++a) {
@@ -652,7 +651,7 @@ __device__ int move_gradient(const DMesh& m, int i, double max_len, int mode) {
   double4 tnew = tini;
   LogT<F32> lnew = lini;
   if (follow) {
-    const int* vc = m.vic + (size_t) i * m.bucket;
+    const TrnRow vc = trn_row(m.vic, m, i);
     const int nb_neigh = min(m.vdeg[i], m.bucket);
     if (nb_neigh == 0) return 0;
     LogSum<F32> lsum;

@@ -48,7 +48,7 @@ __device__ int identify_target(const DMesh& m, int source) {
   double lens[TRN_MAX_DEG];
   int cands[TRN_MAX_DEG];
   int nc = 0;
-  const int* vc = m.vic + (size_t) source * m.bucket;
+  const TrnRow vc = trn_row(m.vic, m, source);
   const int nv = m.vdeg[source];
   const double2 ps = m.pts[source];
   const TenT<F32> ts = ten_load<F32>(m, source);
@@ -69,7 +69,7 @@ __device__ int identify_target(const DMesh& m, int source) {
       nc++;
     }
   }
-  const int* st = m.stenc + (size_t) source * m.bucket;
+  const TrnRow st = trn_row(m.stenc, m, source);
   const int deg = trn_deg(m, source);
   int destin = -1;
   bool skip = true;
@@ -188,8 +188,8 @@ __global__ void k_coarse_filter_group(DMesh m, const int* __restrict__ act, cons
     const int nv = v >= 0 ? m.vdeg[v] : 0;
     const bool serial = nv > 32;
     const bool grp = v >= 0 && !serial;
-    const int* vc = m.vic + (size_t) (v >= 0 ? v : 0) * m.bucket;
-    const int* st = m.stenc + (size_t) (v >= 0 ? v : 0) * m.bucket;
+    const TrnRow vc = trn_row(m.vic, m, (v >= 0 ? v : 0));
+    const TrnRow st = trn_row(m.stenc, m, (v >= 0 ? v : 0));
     const bool bsrc = v >= 0 && (m.tags[v] & TRN_TAG_BOUND) != 0;
     double2 ps = make_double2(0, 0);
     TenT<F32> ts{};
@@ -301,7 +301,7 @@ __global__ void k_collapse(DMesh m, const int* __restrict__ indep, const int* co
       continue;
     }
     const int destin = target[source];
-    int* st = m.stenc + (size_t) source * m.bucket;
+    const TrnRow st = trn_row(m.stenc, m, source);
     const int deg = trn_deg(m, source);
     const int limit = (m.tags[source] & TRN_TAG_BOUND) ? 1 : 2;
     int k = 0, trash0 = -1, trash1 = -1;
@@ -339,7 +339,7 @@ __global__ void k_collapse(DMesh m, const int* __restrict__ indep, const int* co
       m.tri[rest[a]] = n;
     }
     trn_tag_fix(m, destin);
-    const int* vc = m.vic + (size_t) source * m.bucket;
+    const TrnRow vc = trn_row(m.vic, m, source);
     const int nv = m.vdeg[source];
     /* re-activate the 1-ring: independent flag atomics, newly set ids listed
      * in batches of 16 with one atomic each */

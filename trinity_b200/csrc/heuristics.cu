@@ -149,7 +149,7 @@ __device__ __forceinline__ uint8_t mis_item(const DMesh& m, const uint8_t* __res
     return sv;
   }
   const uint64_t pv = trn_prio(seed, v);
-  const int* vc = m.vic + (size_t) v * m.bucket;
+  const TrnRow vc = trn_row(m.vic, m, v);
   const int nv = m.vdeg[v];
   bool is_max = true, leave = false;
   for (int b = 0; b < nv; ++b) {
@@ -812,7 +812,7 @@ __global__ void k_color_init(DMesh m, int nb_nodes, int* list, int* n, int* colo
 __device__ __forceinline__ bool color_item(const DMesh& m, int v, int* color, uint8_t* tent, int capa,
                                            int max_col, uint64_t seed, int round) {
   const uint64_t pv = trn_prio(seed, v);
-  const int* vc = m.vic + (size_t) v * m.bucket;
+  const TrnRow vc = trn_row(m.vic, m, v);
   const int nv = m.vdeg[v];
   const uint8_t* prev = tent + (size_t) ((round - 1) & 1) * capa;
   const int mine = round > 0 ? prev[v] : 0;

@@ -169,12 +169,11 @@ extern "C" int trn_metric_noalloc(int nb_nodes, int nb_elems, const double* d_po
   double* terms = reinterpret_cast<double*>(base + oTerms);
   double* cplx = reinterpret_cast<double*>(base + oCplx);
 
-  /* what must start empty: degrees, stencil/adjacency rows, error word */
+  /* what must start empty: degrees and the error word (rows are read up to
+   * their counts) */
   if (cudaMemsetAsync(d.err, 0, sizeof(int), s) != cudaSuccess ||
       cudaMemsetAsync(d.deg, 0, sizeof(int) * (size_t) nb_nodes, s) != cudaSuccess ||
       cudaMemsetAsync(d.vdeg, 0, sizeof(int) * (size_t) nb_nodes, s) != cudaSuccess ||
-      cudaMemsetAsync(d.stenc, 0xff, sizeof(int) * (size_t) nb_nodes * kB, s) != cudaSuccess ||
-      cudaMemsetAsync(d.vic, 0xff, sizeof(int) * (size_t) nb_nodes * kB, s) != cudaSuccess ||
       cudaMemsetAsync(d.alive, 1, (size_t) nb_nodes, s) != cudaSuccess)
     return TRN_ERR_CUDA;
 

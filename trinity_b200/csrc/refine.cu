@@ -67,7 +67,7 @@ __device__ int h_get(const unsigned long long* hkey, const int* hval, unsigned l
 
 /* Mesh::getElemNeigh, mesh.cpp:437-453: element != id holding edge j -> i */
 __device__ __forceinline__ int elem_neigh(const DMesh& m, int id, int i, int j) {
-  const int* s = m.stenc + (size_t) i * m.bucket;
+  const TrnRow s = trn_row(m.stenc, m, i);
   int d = trn_deg(m, i);
   for (int a = 0; a < d; ++a) {
     int t = s[a];

@@ -42,8 +42,8 @@ using JmT = LogT<F32>;
 
 template <bool F32>
 __device__ int move_laplacian(const DMesh& m, int i, JmT<F32>* jc, int kj) {
-  const int* vc = m.vic + (size_t) i * m.bucket;
-  const int* st = m.stenc + (size_t) i * m.bucket;
+  const TrnRow vc = trn_row(m.vic, m, i);
+  const TrnRow st = trn_row(m.stenc, m, i);
   const int deg = trn_deg(m, i);
   const int nb_neigh = m.vdeg[i];
   double q_min = 1.7976931348623157e308;
@@ -152,7 +152,7 @@ __device__ unsigned long long smooth_bytes(const DMesh& m, int v, bool moved, un
   const int deg = trn_deg(m, v), nv = m.vdeg[v];
   b += 4 + 2 * (16 + kTenB + kLogB);
   b += (unsigned long long) deg * (4 + 16 + 8 + 8) + (unsigned long long) nv * 4;
-  const int* vc = m.vic + (size_t) v * m.bucket;
+  const TrnRow vc = trn_row(m.vic, m, v);
   for (int k = 0; k < nv; ++k) {
     const int w = vc[k];
     const unsigned bit = 1u << (w & 31);
@@ -432,8 +432,8 @@ __device__ int move_laplacian_grp(const DMesh& m, int i, int lane, unsigned gmas
   constexpr bool SW = V == 1;
   constexpr int KQ = G >= 4 ? 2 : 3;
   JmT<F32>* js = reinterpret_cast<JmT<F32>*>(smem) + threadIdx.x;
-  const int* vc = m.vic + (size_t) i * m.bucket;
-  const int* st = m.stenc + (size_t) i * m.bucket;
+  const TrnRow vc = trn_row(m.vic, m, i);
+  const TrnRow st = trn_row(m.stenc, m, i);
   const int deg = trn_deg(m, i);
   const int nb_neigh = m.vdeg[i];
   double q_min = 1.7976931348623157e308;
@@ -526,58 +526,59 @@ __device__ int move_laplacian_grp(const DMesh& m, int i, int lane, unsigned gmas
       log_store<F32>(m, i, lnew);
     }
     return 1;
-  }
-  double qv[KQ];
-  JmT<F32> jv[KQ];
+  } else {
+    double qv[KQ];
+    JmT<F32> jv[KQ];
 #pragma unroll
-  for (int j = 0; j < KQ; ++j) {
-    const int a = lane + j * G;
-    if (a < deg) jv[j] = elem_metric<F32>(m, i, m.tri[st[a]], lnew);
-  }
-  bool valid;
-  int retry = 0;
-  double weight = 1;
-  double2 pa;
-  do {
-    pa.x = (1 - weight) * pini.x + weight * ox;
-    pa.y = (1 - weight) * pini.y + weight * oy;
-    bool ok = true;
-    int j = 0;
-    for (int a = lane; ok && a < deg; a += G, ++j) {
-      double q = 0;
-      if (j < KQ) {
-        const int4 n = m.tri[st[a]];
-        const double2 p0 = (n.x == i) ? pa : m.pts[n.x];
-        const double2 p1 = (n.y == i) ? pa : m.pts[n.y];
-        const double2 p2 = (n.z == i) ? pa : m.pts[n.z];
-        ok = trn_ccw(p0, p1, p2);
-        if (ok) {
-          q = qgeom_x(p0, p1, p2, reg_pick(jv, j));
-          ok = q > q_min;
+    for (int j = 0; j < KQ; ++j) {
+      const int a = lane + j * G;
+      if (a < deg) jv[j] = elem_metric<F32>(m, i, m.tri[st[a]], lnew);
+    }
+    bool valid;
+    int retry = 0;
+    double weight = 1;
+    double2 pa;
+    do {
+      pa.x = (1 - weight) * pini.x + weight * ox;
+      pa.y = (1 - weight) * pini.y + weight * oy;
+      bool ok = true;
+      int j = 0;
+      for (int a = lane; ok && a < deg; a += G, ++j) {
+        double q = 0;
+        if (j < KQ) {
+          const int4 n = m.tri[st[a]];
+          const double2 p0 = (n.x == i) ? pa : m.pts[n.x];
+          const double2 p1 = (n.y == i) ? pa : m.pts[n.y];
+          const double2 p2 = (n.z == i) ? pa : m.pts[n.z];
+          ok = trn_ccw(p0, p1, p2);
+          if (ok) {
+            q = qgeom_x(p0, p1, p2, reg_pick(jv, j));
+            ok = q > q_min;
+          }
+          reg_put(qv, j, q);
+        } else {
+          ok = elem_quality_at<F32>(m, i, m.tri[st[a]], pa, lnew, &q) && (q > q_min);
         }
-        reg_put(qv, j, q);
-      } else {
-        ok = elem_quality_at<F32>(m, i, m.tri[st[a]], pa, lnew, &q) && (q > q_min);
+      }
+      valid = __all_sync(gmask, ok);
+      weight *= 0.5;
+    } while (!valid && ++retry < 5);
+    if (valid) {
+      int j = 0;
+      for (int a = lane; a < deg; a += G, ++j) {
+        double q = 0;
+        if (j < KQ) q = reg_pick(qv, j);
+        else elem_quality_at<F32>(m, i, m.tri[st[a]], pa, lnew, &q);
+        m.qual[st[a]] = q;
+      }
+      if (lane == 0) {
+        m.pts[i] = pa;
+        ten_store<F32>(m, i, tnew);
+        log_store<F32>(m, i, lnew);
       }
     }
-    valid = __all_sync(gmask, ok);
-    weight *= 0.5;
-  } while (!valid && ++retry < 5);
-  if (valid) {
-    int j = 0;
-    for (int a = lane; a < deg; a += G, ++j) {
-      double q = 0;
-      if (j < KQ) q = reg_pick(qv, j);
-      else elem_quality_at<F32>(m, i, m.tri[st[a]], pa, lnew, &q);
-      m.qual[st[a]] = q;
-    }
-    if (lane == 0) {
-      m.pts[i] = pa;
-      ten_store<F32>(m, i, tnew);
-      log_store<F32>(m, i, lnew);
-    }
+    return valid ? 1 : 0;
   }
-  return valid ? 1 : 0;
 }
 
 template <bool F32, int G, int MinB, int V>

@@ -71,7 +71,7 @@ __device__ __forceinline__ int dual_row(const DMesh& m, int k, int i, int* __res
     const int4 n = m.tri[k];
     int row[4] = {k, -1, -1, -1};
     int dn = 1;
-    const int* s0 = m.stenc + (size_t) n.x * m.bucket;
+    const TrnRow s0 = trn_row(m.stenc, m, n.x);
     const int d0 = trn_deg(m, n.x);
     for (int a = 0; dn < 3 && a < d0; ++a) {
       int t = s0[a];
@@ -82,7 +82,7 @@ __device__ __forceinline__ int dual_row(const DMesh& m, int k, int i, int* __res
           (v.z == n.x && v.x == n.z) || (v.z == n.y && v.x == n.x))
         row[dn++] = t;
     }
-    const int* s2 = m.stenc + (size_t) n.z * m.bucket;
+    const TrnRow s2 = trn_row(m.stenc, m, n.z);
     const int d2 = trn_deg(m, n.z);
     for (int a = 0; a < d2; ++a) {
       int t = s2[a];

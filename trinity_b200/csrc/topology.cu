@@ -33,7 +33,7 @@ __global__ void k_sort_stencils(DMesh m, int nb_nodes) {
   int buf[TRN_MAX_DEG];
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
     int d = trn_deg(m, v);
-    int* s = m.stenc + (size_t) v * m.bucket;
+    const TrnRow s = trn_row(m.stenc, m, v);
     for (int a = 0; a < d; ++a) buf[a] = s[a];
     trn_isort(buf, d);
     for (int a = 0; a < d; ++a) s[a] = buf[a];
@@ -57,7 +57,7 @@ __global__ void k_build_vicin(DMesh m, int nb_nodes, int only_flagged) {
 constexpr int kFixRegs = 16;
 
 __device__ __forceinline__ void fix_stencil(const DMesh& m, int v, int* buf) {
-  int* s = m.stenc + (size_t) v * m.bucket;
+  const TrnRow s = trn_row(m.stenc, m, v);
   const int d = trn_deg(m, v);
   int k = 0;
   if (d <= kFixRegs) {

@@ -310,8 +310,8 @@ int trn_mesh_create_ex(const int size[2], int bucket, int depth, int verbosity, 
   if ((rc = dmalloc(m, &d.pts, cn)) || (rc = dmalloc(m, &d.ten, cn)) || (rc = dmalloc(m, &d.lten, cn)) ||
       (rc = dmalloc(m, &d.tenf, cn)) ||
       (rc = dmalloc(m, &d.tri, ce)) ||
-      (rc = dmalloc(m, &d.stenc, cn * bucket)) || (rc = dmalloc(m, &d.deg, cn)) ||
-      (rc = dmalloc(m, &d.vic, cn * bucket)) || (rc = dmalloc(m, &d.vdeg, cn)) ||
+      (rc = dmalloc(m, &d.stenc, trn_row_ints(cn, bucket))) || (rc = dmalloc(m, &d.deg, cn)) ||
+      (rc = dmalloc(m, &d.vic, trn_row_ints(cn, bucket))) || (rc = dmalloc(m, &d.vdeg, cn)) ||
       (rc = dmalloc(m, &d.tags, cn)) || (rc = dmalloc(m, &d.alive, cn)) ||
       (rc = dmalloc(m, &d.fixes, cn + 16)) || (rc = dmalloc(m, &d.activ, std::max(cn, ce) + 16)) ||
       (rc = dmalloc(m, &d.qual, ce)) || (rc = dmalloc(m, &m->solut, cn)) ||
@@ -351,25 +351,24 @@ int trn_mesh_destroy(trn_mesh* m) {
 /* state of a freshly loaded mesh from the device copies pts0/tri0/tags0 */
 static int init_from_device(trn_mesh* m) {
   DMesh& d = m->d;
-  const size_t cn = (size_t) m->capa_node, ce = (size_t) m->capa_elem, b = (size_t) m->bucket;
+  const size_t cn = (size_t) m->capa_node, ce = (size_t) m->capa_elem;
   const int nb_nodes = m->n0_nodes, nb_elems = m->n0_elems;
   cudaStream_t s = m->stream;
-  CK(cudaMemsetAsync(d.ten, 0, sizeof(double4) * cn, s));
-  CK(cudaMemsetAsync(d.lten, 0, sizeof(double4) * cn, s));
-  CK(cudaMemsetAsync(d.pts, 0, sizeof(double2) * cn, s));
-  CK(cudaMemsetAsync(d.tri, 0xff, sizeof(int4) * ce, s));
-  CK(cudaMemsetAsync(d.stenc, 0xff, sizeof(int) * cn * b, s));
-  CK(cudaMemsetAsync(d.vic, 0xff, sizeof(int) * cn * b, s));
+  /* only what is read before it is written: the tensors of the vertices in
+   * use (an export before the first recovery), the counts and the flags.
+   * Rows are read up to their counts; a new vertex or element is written
+   * whole when it gets its slot, but for its flags. */
+  CK(cudaMemsetAsync(d.ten, 0, sizeof(double4) * (size_t) nb_nodes, s));
+  CK(cudaMemsetAsync(d.lten, 0, sizeof(double4) * (size_t) nb_nodes, s));
   CK(cudaMemsetAsync(d.vdeg, 0, sizeof(int) * cn, s));
   CK(cudaMemsetAsync(d.tags, 0, cn, s));
   CK(cudaMemsetAsync(d.alive, 1, cn, s));
   CK(cudaMemsetAsync(d.fixes, 0, cn, s));
   CK(cudaMemsetAsync(d.activ, 0, std::max(cn, ce), s));
-  CK(cudaMemsetAsync(d.qual, 0, sizeof(double) * ce, s));
+  CK(cudaMemsetAsync(d.qual, 0, sizeof(double) * (size_t) nb_elems, s));
   CK(cudaMemsetAsync(m->status, 0, sizeof(int) * S_SIZE, s));
   const int counts[2] = {nb_nodes, nb_elems};
   CK(cudaMemcpyAsync(m->status + S_NB, counts, sizeof(counts), cudaMemcpyHostToDevice, s));
-  CK(cudaMemsetAsync(m->map, 0xff, sizeof(int) * ce, s));
   CK(cudaMemcpyAsync(d.pts, m->pts0, sizeof(double2) * (size_t) nb_nodes, cudaMemcpyDeviceToDevice, s));
   CK(cudaMemcpyAsync(d.tri, m->tri0, sizeof(int4) * (size_t) nb_elems, cudaMemcpyDeviceToDevice, s));
   CK(cudaMemcpyAsync(d.tags, m->tags0, (size_t) nb_nodes, cudaMemcpyDeviceToDevice, s));

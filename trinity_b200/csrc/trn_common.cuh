@@ -7,11 +7,12 @@
  *   ten   double4[capa_node]        metric tensor (m11, m12, m22, unused):
  *                                   32-byte records, one sector per gather
  *   tri   int4[capa_elem]           vertex ids (x,y,z), x = -1 when erased
- *   stenc int[capa_node * bucket]   vertex -> incident elements (the
+ *   stenc int rows of `bucket`      vertex -> incident elements (the
  *                                   reference's "stencil", mesh.h:112), first
  *                                   deg[v] slots used, appended atomically
- *   vic   int[capa_node * bucket]   vertex -> adjacent vertices, sorted
+ *   vic   int rows of `bucket`      vertex -> adjacent vertices, sorted
  *                                   (the reference's "vicin", mesh.h:113)
+ *         rows are cut into chunks of 8 entries (TrnRow)
  *   tags/alive/fixes  uint8 per vertex; activ int8 shared by vertices and
  *                                   elements exactly like mesh.h:146
  *   qual  double[capa_elem]         cached element quality
@@ -69,6 +70,35 @@ struct DMesh {
   int capa_node;
   int capa_elem;
 };
+
+/* One vertex's row of stenc or vic. Rows are stored in chunks of kRowChunk
+ * entries, chunk c of all vertices before chunk c + 1: entry k of vertex v
+ * at ((k / 8) * capa_node + v) * 8 + k % 8. A planar triangulation averages 6
+ * entries, so nearly every row is one aligned 32-byte sector, and the rows of
+ * consecutive vertices are consecutive: a 128-byte cache line holds four of
+ * them. Rows `bucket` entries apart (512 bytes at bucket 128) spent a line on
+ * each, and the rows of a million vertices took the L2 twice over. Measured
+ * on the 2M-triangle workload: the adjacency rebuild 133 -> 100 us, the
+ * coloring 351 -> 298 us, the stencil repair 109 -> 75 us a call; a load, which
+ * no longer clears the rows, 2.9 -> 2.3 ms. */
+constexpr int kRowChunk = 8;
+
+struct TrnRow {
+  int* p;
+  size_t plane;
+  __device__ __forceinline__ int& operator[](int k) const {
+    return k < kRowChunk ? p[k] : p[(size_t) (k / kRowChunk) * plane + (k % kRowChunk)];
+  }
+};
+
+__device__ __forceinline__ TrnRow trn_row(int* base, const DMesh& m, int v) {
+  return TrnRow{base + (size_t) v * kRowChunk, (size_t) m.capa_node * kRowChunk};
+}
+
+/* ints that hold the rows of n vertices */
+__host__ __device__ constexpr size_t trn_row_ints(size_t n, int bucket) {
+  return n * (size_t) ((bucket + kRowChunk - 1) / kRowChunk) * kRowChunk;
+}
 
 __device__ __forceinline__ void trn_set_error(int* err, int code) {
   atomicCAS(err, 0, code);
@@ -182,7 +212,7 @@ __device__ __forceinline__ void trn_stenc_append(const DMesh& m, int v, int t) {
     trn_set_error(m.err, TRN_DERR_BUCKET);
     return;
   }
-  m.stenc[(size_t) v * m.bucket + k] = t;
+  trn_row(m.stenc, m, v)[k] = t;
 }
 
 __device__ __forceinline__ void trn_stenc_append_n(const DMesh& m, int v, const int* t, int n) {
@@ -191,8 +221,8 @@ __device__ __forceinline__ void trn_stenc_append_n(const DMesh& m, int v, const 
     trn_set_error(m.err, TRN_DERR_BUCKET);
     return;
   }
-  int* s = m.stenc + (size_t) v * m.bucket + k;
-  for (int i = 0; i < n; ++i) s[i] = t[i];
+  const TrnRow s = trn_row(m.stenc, m, v);
+  for (int i = 0; i < n; ++i) s[k + i] = t[i];
 }
 
 __device__ __forceinline__ void trn_isort(int* a, int n) {
@@ -223,7 +253,7 @@ constexpr int kVicRegs = 24;
 
 __device__ __forceinline__ void build_one_vicin(const DMesh& m, int v) {
   if (m.alive[v] && trn_deg(m, v) <= kVicRegs / 2) {
-    const int* s = m.stenc + (size_t) v * m.bucket;
+    const TrnRow s = trn_row(m.stenc, m, v);
     const int d = trn_deg(m, v);
     int r[kVicRegs];
 #pragma unroll
@@ -246,7 +276,7 @@ __device__ __forceinline__ void build_one_vicin(const DMesh& m, int v) {
         r[a] = lo;
         r[a + 1] = hi;
       }
-    int* out = m.vic + (size_t) v * m.bucket;
+    const TrnRow out = trn_row(m.vic, m, v);
     int k = 0;
 #pragma unroll
     for (int a = 0; a < kVicRegs; ++a)
@@ -264,7 +294,7 @@ __device__ __forceinline__ void build_one_vicin(const DMesh& m, int v) {
   int buf[2 * TRN_MAX_DEG];
   int k = 0;
   if (m.alive[v]) {
-    const int* s = m.stenc + (size_t) v * m.bucket;
+    const TrnRow s = trn_row(m.stenc, m, v);
     int d = trn_deg(m, v);
     for (int a = 0; a < d; ++a) {
       int4 n = m.tri[s[a]];
@@ -279,7 +309,7 @@ __device__ __forceinline__ void build_one_vicin(const DMesh& m, int v) {
     trn_set_error(m.err, TRN_DERR_BUCKET);
     k = m.bucket;
   }
-  int* out = m.vic + (size_t) v * m.bucket;
+  const TrnRow out = trn_row(m.vic, m, v);
   for (int a = 0; a < k; ++a) out[a] = buf[a];
   m.vdeg[v] = k;
 }

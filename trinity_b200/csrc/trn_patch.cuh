@@ -18,7 +18,7 @@
 
 #include "trn_common.cuh"
 
-constexpr int kRowRegs = 8;                 /* entries of a row kept in registers */
+constexpr int kRowRegs = kRowChunk;         /* entries of a row kept in registers */
 constexpr int kNoId = 0x7fffffff;           /* pads the unused slots, sorts last */
 constexpr int kPatchRows = 8;               /* the vertex's own row and 7 neighbours' */
 constexpr int kPatchKeys = kPatchRows * kRowRegs;
@@ -56,12 +56,12 @@ __device__ __forceinline__ void patch_merge_rows(int* a) {
   if constexpr (N >= 64) patch_merge<64>(a);
 }
 
-/* the first n entries of a row whose start is 16-byte aligned, the rest
- * kNoId; false when they are not in ascending order */
-__device__ __forceinline__ bool patch_row(const int* row, int n, int* out) {
+/* the first n entries of a row (its first chunk, one aligned sector), the
+ * rest kNoId; false when they are not in ascending order */
+__device__ __forceinline__ bool patch_row(const TrnRow& row, int n, int* out) {
   int4 a = make_int4(kNoId, kNoId, kNoId, kNoId), b = a;
-  if (n > 0) a = *reinterpret_cast<const int4*>(row);
-  if (n > 4) b = *reinterpret_cast<const int4*>(row + 4);
+  if (n > 0) a = *reinterpret_cast<const int4*>(row.p);
+  if (n > 4) b = *reinterpret_cast<const int4*>(row.p + 4);
   out[0] = n > 0 ? a.x : kNoId;
   out[1] = n > 1 ? a.y : kNoId;
   out[2] = n > 2 ? a.z : kNoId;
@@ -79,12 +79,11 @@ __device__ __forceinline__ bool patch_row(const int* row, int n, int* out) {
 /* the 2-ring element patch of v as kPatchKeys ascending ids, duplicates
  * adjacent, kNoId last; false when the rows do not fit the registers */
 __device__ __forceinline__ bool patch_keys(const DMesh& m, int v, int* key) {
-  if (m.bucket & 3) return false;   /* rows not 16-byte aligned */
   const int d = trn_deg(m, v), nv = m.vdeg[v];
   if (d > kRowRegs || nv > kPatchRows - 1) return false;
-  bool ok = patch_row(m.stenc + (size_t) v * m.bucket, d, key);
+  bool ok = patch_row(trn_row(m.stenc, m, v), d, key);
   int w[kRowRegs];
-  patch_row(m.vic + (size_t) v * m.bucket, nv, w);   /* any order will do */
+  patch_row(trn_row(m.vic, m, v), nv, w);   /* any order will do */
   int dw[kPatchRows - 1];
 #pragma unroll
   for (int b = 0; b < kPatchRows - 1; ++b) {
@@ -94,7 +93,7 @@ __device__ __forceinline__ bool patch_keys(const DMesh& m, int v, int* key) {
   if (!ok) return false;
 #pragma unroll
   for (int b = 0; b < kPatchRows - 1; ++b)
-    ok &= patch_row(m.stenc + (size_t) (b < nv ? w[b] : v) * m.bucket, dw[b], key + (b + 1) * kRowRegs);
+    ok &= patch_row(trn_row(m.stenc, m, b < nv ? w[b] : v), dw[b], key + (b + 1) * kRowRegs);
   if (!ok) return false;
   patch_merge_rows<kPatchKeys>(key);
   return true;
@@ -109,9 +108,9 @@ __device__ __forceinline__ int patch_sort_warp(const DMesh& m, int v, int* buf) 
   const int d = trn_deg(m, v), nv = m.vdeg[v];
   int k = 0;
   for (int b = -1; b < nv; ++b) {
-    const int w = b < 0 ? v : m.vic[(size_t) v * m.bucket + b];
+    const int w = b < 0 ? v : trn_row(m.vic, m, v)[b];
     const int dw = b < 0 ? d : trn_deg(m, w);
-    const int* s = m.stenc + (size_t) w * m.bucket;
+    const TrnRow s = trn_row(m.stenc, m, w);
     const int room = TRN_MAX_PATCH - k;
     if (dw > room && lane == 0) trn_set_error(m.err, TRN_DERR_BUCKET);
     const int n = dw < room ? dw : room;
