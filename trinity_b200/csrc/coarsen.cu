@@ -42,10 +42,40 @@ __global__ void k_coarse_pre(DMesh m, int nb_nodes, int* __restrict__ act, int* 
   }
 }
 
+/* is the collapse of source onto destin valid: every element that remains
+ * CCW with no edge longer than sqrt(2)? The destination's point and tensor are
+ * the caller's, so an element costs two gathers of each. */
+template <bool F32>
+__device__ __forceinline__ bool collapse_valid(const DMesh& m, int source, int destin, const TrnRow& st, int deg,
+                                               bool both_bound, double2 pd, TenT<F32> td) {
+  int shared = 0;
+  for (int k = 0; k < deg; ++k) {
+    const int4 n = m.tri[st[k]];
+    const int pos = n.x == source ? 0 : (n.y == source ? 1 : 2);
+    const int a = pos == 0 ? n.y : (pos == 1 ? n.z : n.x);
+    const int b = pos == 0 ? n.z : (pos == 1 ? n.x : n.y);
+    if (a == destin || b == destin) {
+      if (++shared > 1 && both_bound) return false;
+      continue;
+    }
+    const double2 pa = m.pts[a], pb = m.pts[b];
+    if (!trn_ccw_from(pd, pa, pb, pos)) return false;
+    const TenT<F32> ta = ten_load<F32>(m, a), tb = ten_load<F32>(m, b);
+    if (length_gt<F32>(pd, pa, td, ta, TRN_L_MAX) || length_gt<F32>(pb, pd, tb, td, TRN_L_MAX) ||
+        length_gt<F32>(pa, pb, ta, tb, TRN_L_MAX))
+      return false;
+  }
+  return true;
+}
+
+/* The candidates are tried by increasing upper bound of their length
+ * (length_below), and the exact length is computed only between two valid
+ * ones whose bounds overlap: the pick is the valid one of smallest (length,
+ * adjacency index), as the reference's multimap gives it. */
 template <bool F32>
 __device__ int identify_target(const DMesh& m, int source) {
   const bool bound_source = (m.tags[source] & TRN_TAG_BOUND) != 0;
-  double lens[TRN_MAX_DEG];
+  float lo[TRN_MAX_DEG], hi[TRN_MAX_DEG];
   int cands[TRN_MAX_DEG];
   int nc = 0;
   const TrnRow vc = trn_row(m.vic, m, source);
@@ -53,54 +83,49 @@ __device__ int identify_target(const DMesh& m, int source) {
   const double2 ps = m.pts[source];
   const TenT<F32> ts = ten_load<F32>(m, source);
   for (int b = 0; b < nv; ++b) {
-    int neigh = vc[b];
-    bool bound_destin = (m.tags[neigh] & TRN_TAG_BOUND) != 0;
-    if (bound_source && !bound_destin) continue;
-    double len;
-    if (length_lt<F32>(ps, m.pts[neigh], ts, ten_load<F32>(m, neigh), TRN_L_MIN, &len)) {
+    const int neigh = vc[b];
+    if (bound_source && !(m.tags[neigh] & TRN_TAG_BOUND)) continue;
+    float l, h;
+    if (length_below<F32>(ps, m.pts[neigh], ts, ten_load<F32>(m, neigh), TRN_L_MIN, &l, &h)) {
       int p = nc;
-      while (p > 0 && lens[p - 1] > len) {
-        lens[p] = lens[p - 1];
+      while (p > 0 && hi[p - 1] > h) {
+        hi[p] = hi[p - 1];
+        lo[p] = lo[p - 1];
         cands[p] = cands[p - 1];
         --p;
       }
-      lens[p] = len;
+      hi[p] = h;
+      lo[p] = l;
       cands[p] = neigh;
       nc++;
     }
   }
   const TrnRow st = trn_row(m.stenc, m, source);
   const int deg = trn_deg(m, source);
-  int destin = -1;
-  bool skip = true;
-  int next = 0;
-  while (skip && next < nc) {
-    destin = cands[next++];
-    skip = false;
-    int shared = 0;
-    const bool bound_destin = (m.tags[destin] & TRN_TAG_BOUND) != 0;
-    for (int a = 0; !skip && a < deg; ++a) {
-      int4 n = m.tri[st[a]];
-      if ((source == n.x && destin == n.y) || (source == n.y && destin == n.x) ||
-          (source == n.y && destin == n.z) || (source == n.z && destin == n.y) ||
-          (source == n.z && destin == n.x) || (source == n.x && destin == n.z)) {
-        skip = (++shared > 1 && bound_source && bound_destin);
-        continue;
-      }
-      int f0 = (n.x == source ? destin : n.x);
-      int f1 = (n.y == source ? destin : n.y);
-      int f2 = (n.z == source ? destin : n.z);
-      double2 p0 = m.pts[f0], p1 = m.pts[f1], p2 = m.pts[f2];
-      if (trn_ccw(p0, p1, p2)) {
-        const TenT<F32> t0 = ten_load<F32>(m, f0), t1 = ten_load<F32>(m, f1), t2 = ten_load<F32>(m, f2);
-        skip = length_gt<F32>(p0, p1, t0, t1, TRN_L_MAX) || length_gt<F32>(p1, p2, t1, t2, TRN_L_MAX) ||
-               length_gt<F32>(p2, p0, t2, t0, TRN_L_MAX);
-        continue;
-      }
-      skip = true;
+  int best = -1;
+  float best_hi = 0.f;
+  for (int k = 0; k < nc; ++k) {
+    if (best >= 0 && lo[k] > best_hi) continue;   /* certainly longer */
+    const int c = cands[k];
+    const bool both = bound_source && (m.tags[c] & TRN_TAG_BOUND) != 0;
+    const double2 pc = m.pts[c];
+    const TenT<F32> tc = ten_load<F32>(m, c);
+    if (!collapse_valid<F32>(m, source, c, st, deg, both, pc, tc)) continue;
+    if (best < 0) {
+      best = c;
+      best_hi = hi[k];
+      continue;
+    }
+    LenT<F32> s1, r1;
+    const LenT<F32> s0 = length_squares<F32>(ps, pc, ts, tc, &s1);
+    const LenT<F32> r0 = length_squares<F32>(ps, m.pts[best], ts, ten_load<F32>(m, best), &r1);
+    const double lc = (double) length_of_squares(s0, s1), lb = (double) length_of_squares(r0, r1);
+    if (lc < lb || (lc == lb && c < best)) {   /* rows are in id order */
+      best = c;
+      best_hi = hi[k] > best_hi ? hi[k] : best_hi;
     }
   }
-  return skip ? -1 : destin;
+  return best;
 }
 
 template <bool F32>
@@ -120,12 +145,19 @@ __global__ void k_coarse_filter(DMesh m, int nb_nodes, int* __restrict__ target,
   }
 }
 
+/* any block size of the tuner's, which caps the registers at 64: 32 warps an
+ * SM to hide the scan's gathers. 2M-triangle workload, coarsening of three
+ * rounds: 8.98 ms at two 256-thread blocks, 8.41 at three, 8.31 at four; with
+ * the scan that computed every candidate's length, gathered three corners an
+ * element and tested lengths with roots and logarithms, 10.08 ms. */
+constexpr int kSearchThreads = 1024;
+
 /* free mode: one pass per level rebuilds the adjacency of each active vertex,
  * finds its target and appends the candidates (in no particular order: the
  * independent set is chosen by hashed priorities, not by list position),
  * marking them undecided for the independent-set rounds */
 template <bool F32>
-__global__ void k_coarse_filter_append(DMesh m, const int* __restrict__ act, const int* act_n,
+__global__ void __launch_bounds__(kSearchThreads) k_coarse_filter_append(DMesh m, const int* __restrict__ act, const int* act_n,
                                        int* __restrict__ target, int* __restrict__ cand, int* count,
                                        uint8_t* __restrict__ state, int min_n) {
   if (blockIdx.x == 0 && threadIdx.x == 0) trn_level_clear(m, nullptr);

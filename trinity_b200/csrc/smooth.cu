@@ -320,11 +320,6 @@ __device__ __forceinline__ double4 log_pair(double t0, double t1, double t2, int
  * 6.57 ms with the estimate (2 lanes, two blocks an SM). */
 constexpr float kTryMargin = 8.e-6f;
 
-__device__ __forceinline__ float try_sqrt(float x) {
-  float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
 __device__ __forceinline__ float try_rcp(float x) {
   float r;
   asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -353,7 +348,7 @@ __device__ __forceinline__ unsigned try_filter(double2 pini, double2 o, double2 
   const float at = (float) (h * __fma_rn(4.e-8, LL, 1.e8 * (e * L)));
   const float ae = (float) (h * __fma_rn(1.e-14, LL, 1.e1 * (e * L)));
   const float ccw = (float) (2.0 * h * TRN_EPS);
-  const float fbb = (float) bb, lb = try_sqrt(fbb);
+  const float fbb = (float) bb, lb = trnf_sqrt_approx(fbb);
   const float qlo = (float) q_min * (1.f - kTryMargin), qhi = (float) q_min * (1.f + kTryMargin);
   const bool base = fbb > lt && qlo > 1.e-20f;
   unsigned m = 0;
@@ -363,7 +358,7 @@ __device__ __forceinline__ unsigned try_filter(double2 pini, double2 o, double2 
     const float fu = (float) __fma_rn(w, __fma_rn(w, dd, ud), uu);
     const float fv = (float) __fma_rn(w, __fma_rn(w, dd, vd), vv);
     const float fa = (float) __fma_rn(w, a1, a0);
-    const float p = try_sqrt(fu) + try_sqrt(fv) + lb;
+    const float p = trnf_sqrt_approx(fu) + trnf_sqrt_approx(fv) + lb;
     const float ip = try_rcp(p);
     const float f = fminf(p * 0.333333343f, 3.f * ip);
     const float g = f * (2.f - f);

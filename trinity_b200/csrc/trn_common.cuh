@@ -245,13 +245,67 @@ __device__ __forceinline__ int trn_iunique(int* a, int n) {
 }
 
 /* adjacency of v from its (canonical) stencil: the other two vertices of
- * each element, sorted, without duplicates. A stencil of up to 12 elements
+ * each element, sorted, without duplicates. Around an interior vertex the
+ * elements' next vertices are its neighbours and so are their previous ones:
+ * up to 8 elements are two 8-entry sorts that must agree, two vector stores.
+ * Otherwise a stencil of up to 12 elements
  * stays in registers (its element loads all in flight, an odd-even
  * transposition network over the 24 ids, no local memory); longer ones sort
  * in a local array. Both give the same rows. */
 constexpr int kVicRegs = 24;
 
+__device__ __forceinline__ void patch_cmp(int& a, int& b) {
+  const int lo = min(a, b), hi = max(a, b);
+  a = lo;
+  b = hi;
+}
+
+/* 8 ids into ascending order (Batcher's odd-even merge sort, 19 compares) */
+__device__ __forceinline__ void patch_sort8(int* a) {
+  patch_cmp(a[0], a[1]); patch_cmp(a[2], a[3]); patch_cmp(a[4], a[5]); patch_cmp(a[6], a[7]);
+  patch_cmp(a[0], a[2]); patch_cmp(a[1], a[3]); patch_cmp(a[4], a[6]); patch_cmp(a[5], a[7]);
+  patch_cmp(a[1], a[2]); patch_cmp(a[5], a[6]);
+  patch_cmp(a[0], a[4]); patch_cmp(a[1], a[5]); patch_cmp(a[2], a[6]); patch_cmp(a[3], a[7]);
+  patch_cmp(a[2], a[4]); patch_cmp(a[3], a[5]);
+  patch_cmp(a[1], a[2]); patch_cmp(a[3], a[4]); patch_cmp(a[5], a[6]);
+}
+
+/* the interior case of build_one_vicin; false when it is not that */
+__device__ __forceinline__ bool build_vicin_ring(const DMesh& m, int v, int d) {
+  const int* s = trn_row(m.stenc, m, v).p;
+  int4 r0 = make_int4(-1, -1, -1, -1), r1 = r0;
+  if (d > 0) r0 = *reinterpret_cast<const int4*>(s);
+  if (d > 4) r1 = *reinterpret_cast<const int4*>(s + 4);
+  const int e[kRowChunk] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+  int a[kRowChunk], b[kRowChunk];
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < kRowChunk; ++j) {
+    a[j] = b[j] = 0x7fffffff;
+    if (j < d) {
+      const int4 n = m.tri[e[j]];
+      a[j] = v == n.x ? n.y : (v == n.y ? n.z : n.x);
+      b[j] = v == n.x ? n.z : (v == n.y ? n.x : n.y);
+      ok &= v == n.x || v == n.y || v == n.z;
+    }
+  }
+  patch_sort8(a);
+  patch_sort8(b);
+#pragma unroll
+  for (int j = 0; j < kRowChunk; ++j) {
+    ok &= a[j] == b[j];
+    if (j > 0 && j < d) ok &= a[j] != a[j - 1];
+  }
+  if (!ok) return false;
+  int4* out = reinterpret_cast<int4*>(trn_row(m.vic, m, v).p);
+  out[0] = make_int4(a[0], a[1], a[2], a[3]);
+  if (d > 4) out[1] = make_int4(a[4], a[5], a[6], a[7]);
+  m.vdeg[v] = d;
+  return true;
+}
+
 __device__ __forceinline__ void build_one_vicin(const DMesh& m, int v) {
+  if (m.alive[v] && trn_deg(m, v) <= kRowChunk && build_vicin_ring(m, v, trn_deg(m, v))) return;
   if (m.alive[v] && trn_deg(m, v) <= kVicRegs / 2) {
     const TrnRow s = trn_row(m.stenc, m, v);
     const int d = trn_deg(m, v);

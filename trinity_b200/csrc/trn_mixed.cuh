@@ -139,13 +139,13 @@ __device__ __forceinline__ float4 tenf_of(double4 t) {
 __device__ __forceinline__ float4 tenf_of(float4 t) { return t; }
 
 /* metric edge length (numeric.cpp:469-497) in FP32, in the same two halves */
-__device__ __forceinline__ void trnf_dist2_ends(double2 pa, double2 pb, float4 ta, float4 tb,
-                                                float* l0, float* l1) {
+__device__ __forceinline__ void trnf_dist2_squares(double2 pa, double2 pb, float4 ta, float4 tb,
+                                                   float* s0, float* s1) {
   const float w0 = (float) (pb.x - pa.x), w1 = (float) (pb.y - pa.y);
   const float a0 = ta.x, a1 = ta.y, a2 = ta.z;
   const float b0 = tb.x, b1 = tb.y, b2 = tb.z;
-  *l0 = sqrtf(w0 * (a0 * w0 + a1 * w1) + w1 * (a1 * w0 + a2 * w1));
-  *l1 = sqrtf(w0 * (b0 * w0 + b1 * w1) + w1 * (b1 * w0 + b2 * w1));
+  *s0 = w0 * (a0 * w0 + a1 * w1) + w1 * (a1 * w0 + a2 * w1);
+  *s1 = w0 * (b0 * w0 + b1 * w1) + w1 * (b1 * w0 + b2 * w1);
 }
 
 __device__ __forceinline__ float trnf_dist2_finish(float l0, float l1) {
@@ -156,9 +156,9 @@ __device__ __forceinline__ float trnf_dist2_finish(float l0, float l1) {
 }
 
 __device__ __forceinline__ float trnf_dist2(double2 pa, double2 pb, float4 ta, float4 tb) {
-  float l0, l1;
-  trnf_dist2_ends(pa, pb, ta, tb, &l0, &l1);
-  return trnf_dist2_finish(l0, l1);
+  float s0, s1;
+  trnf_dist2_squares(pa, pb, ta, tb, &s0, &s1);
+  return trnf_dist2_finish(sqrtf(s0), sqrtf(s1));
 }
 
 __device__ __forceinline__ float trnf_dist1(double2 pa, double2 pb, float4 t) {
@@ -242,49 +242,119 @@ __device__ __forceinline__ double length_x(double2 pa, double2 pb, T ta, T tb) {
   else return trn_dist2(pa, pb, ta, tb);
 }
 
-/* Comparisons of a metric edge length with a threshold, with the answer of
- * comparing length_x itself. That length interpolates the edge's lengths
- * under its two endpoint tensors geometrically, so it lies between them: up
- * to a few units in the last place as computed, far inside the margins below
- * (1e-12 relative in FP64, 1e-5 in FP32). When the threshold lies outside
- * that range, with the margin, the answer is known without the logarithm. */
-template <bool F32, class T>
-__device__ __forceinline__ bool length_gt(double2 pa, double2 pb, T ta, T tb, double thresh) {
-  if constexpr (F32) {
-    float l0, l1;
-    trnf_dist2_ends(pa, pb, tenf_of(ta), tenf_of(tb), &l0, &l1);
-    const float t = (float) thresh;
-    if (l0 == l0 && l1 == l1) {
-      if (trnf_max(l0, l1) < t * (1.f - 1.e-5f)) return false;
-      if (trnf_min(l0, l1) > t * (1.f + 1.e-5f)) return true;
-    }
-    return (double) trnf_dist2_finish(l0, l1) > thresh;
-  } else {
-    double l0, l1;
-    trn_dist2_ends(pa, pb, ta, tb, &l0, &l1);
-    if (l0 == l0 && l1 == l1) {
-      if (trn_dmax(l0, l1) < thresh * (1 - 1.e-12)) return false;
-      if (trn_dmin(l0, l1) > thresh * (1 + 1.e-12)) return true;
-    }
-    return trn_dist2_finish(l0, l1) > thresh;
-  }
+/* ---- comparisons of a metric edge length with a threshold ----
+ * The same answer as comparing length_x itself, mostly without it. That
+ * length is the logarithmic mean (l1 - l0) / ln(l1 / l0) of the edge's lengths
+ * under its two endpoint tensors, computed to a few units in the last place.
+ *   1. It lies between the two: when the threshold's square lies outside the
+ *      two squared lengths, with a margin far above the rounding (1e-11
+ *      relative in FP64, 3e-5 in FP32), no root and no logarithm are needed.
+ *   2. With A and G the arithmetic and geometric means of the two, it lies
+ *      between (G^2 A)^(1/3) (Leach and Sholander 1983) and (2 G + A) / 3
+ *      (Carlson 1972), which differ by 4e-5 where l1 = 1.5 l0. Evaluated in
+ *      FP32 these are good to 7e-7 (G^2 A) and 4e-7; the margin kSideMargin
+ *      is 5e-6 of the length in the FP64 form, 2e-5 in the FP32 form, whose
+ *      own length is good to about 1e-6. Where the two lengths all but agree
+ *      (the computed ratio may be 1) the FP32 form is left to step 3.
+ *   3. The computed length. A NaN fails every test before and ends here.
+ * Steps 2 and 3 are met by the edges whose endpoints put the threshold
+ * between them, some 5 % on graded meshes: with step 3 alone nearly every warp
+ * paid two roots, a logarithm and three divisions for each of its tests. */
+__device__ __forceinline__ float trnf_sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
-/* length_x < thresh; *len receives length_x whenever the answer is true */
-template <bool F32, class T>
-__device__ __forceinline__ bool length_lt(double2 pa, double2 pb, T ta, T tb, double thresh,
-                                          double* len) {
-  if constexpr (F32) {
-    float l0, l1;
-    trnf_dist2_ends(pa, pb, tenf_of(ta), tenf_of(tb), &l0, &l1);
-    if (l0 == l0 && l1 == l1 && trnf_min(l0, l1) > (float) thresh * (1.f + 1.e-5f)) return false;
-    *len = (double) trnf_dist2_finish(l0, l1);
-  } else {
-    double l0, l1;
-    trn_dist2_ends(pa, pb, ta, tb, &l0, &l1);
-    if (l0 == l0 && l1 == l1 && trn_dmin(l0, l1) > thresh * (1 + 1.e-12)) return false;
-    *len = trn_dist2_finish(l0, l1);
+template <bool F32>
+constexpr float kSideMargin = F32 ? 2.e-5f : 5.e-6f;
+
+/* 1: the length is above t, -1: below, 0: undecided; s0, s1 squared lengths */
+template <bool F32>
+__device__ __forceinline__ int length_side(float s0, float s1, float t) {
+  if (!(s0 > 1.e-20f && s1 > 1.e-20f && s0 < 1.e12f && s1 < 1.e12f)) return 0;
+  if (F32 && fabsf(s0 - s1) < 1.e-4f * s0) return 0;
+  const float l0 = trnf_sqrt_approx(s0), l1 = trnf_sqrt_approx(s1);
+  const float g2 = l0 * l1, a = 0.5f * (l0 + l1);
+  if (g2 * a > t * t * t * (1.f + 3.f * kSideMargin<F32>)) return 1;
+  if (2.f * trnf_sqrt_approx(g2) + a < 3.f * t * (1.f - kSideMargin<F32>)) return -1;
+  return 0;
+}
+
+/* the computed length from the squared ones, out of line: rarely reached */
+static __device__ __noinline__ double length_of_squares(double s0, double s1) {
+  return trn_dist2_finish(sqrt(s0), sqrt(s1));
+}
+static __device__ __noinline__ float length_of_squares(float s0, float s1) {
+  return trnf_dist2_finish(sqrtf(s0), sqrtf(s1));
+}
+
+template <bool F32>
+using LenT = typename std::conditional<F32, float, double>::type;
+
+template <bool F32>
+__device__ __forceinline__ LenT<F32> length_squares(double2 pa, double2 pb, TenT<F32> ta, TenT<F32> tb,
+                                                    LenT<F32>* s1) {
+  LenT<F32> s0;
+  if constexpr (F32) trnf_dist2_squares(pa, pb, ta, tb, &s0, s1);
+  else trn_dist2_squares(pa, pb, ta, tb, &s0, s1);
+  return s0;
+}
+
+/* steps 1 and 2: 1 above thresh, -1 below, 0 undecided */
+template <bool F32>
+__device__ __forceinline__ int length_test(LenT<F32> s0, LenT<F32> s1, double thresh) {
+  using R = LenT<F32>;
+  const R t = (R) (thresh * thresh), e = F32 ? (R) 3.e-5 : (R) 1.e-11;
+  if (s0 < t * (1 - e) && s1 < t * (1 - e)) return -1;
+  if (s0 > t * (1 + e) && s1 > t * (1 + e)) return 1;
+  return length_side<F32>((float) s0, (float) s1, (float) thresh);
+}
+
+template <bool F32>
+__device__ __forceinline__ bool length_gt(double2 pa, double2 pb, TenT<F32> ta, TenT<F32> tb, double thresh) {
+  LenT<F32> s1;
+  const LenT<F32> s0 = length_squares<F32>(pa, pb, ta, tb, &s1);
+  const int side = length_test<F32>(s0, s1, thresh);
+  if (side) return side > 0;
+  return (double) length_of_squares(s0, s1) > thresh;
+}
+
+/* length_x < thresh, and float bounds of that length: the geometric mean of
+ * the endpoint lengths below it, (2 G + A) / 3 above it, each widened by
+ * kSideMargin. Endpoint lengths so small or large that the computed
+ * interpolation could overflow, or all but equal in the FP32 form, get the
+ * computed length as their bounds. */
+template <bool F32>
+__device__ __forceinline__ bool length_below(double2 pa, double2 pb, TenT<F32> ta, TenT<F32> tb, double thresh,
+                                             float* lo, float* hi) {
+  LenT<F32> s1;
+  const LenT<F32> s0 = length_squares<F32>(pa, pb, ta, tb, &s1);
+  const int side = length_test<F32>(s0, s1, thresh);
+  if (side > 0) return false;
+  const float f0 = (float) s0, f1 = (float) s1;
+  if (side < 0 && f0 > 1.e-20f && f1 > 1.e-20f && !(F32 && fabsf(f0 - f1) < 1.e-4f * f0)) {
+    const float l0 = trnf_sqrt_approx(f0), l1 = trnf_sqrt_approx(f1);
+    const float g = trnf_sqrt_approx(l0 * l1);
+    *lo = g * (1.f - kSideMargin<F32>);
+    *hi = (2.f * g + 0.5f * (l0 + l1)) * (0.333333343f * (1.f + kSideMargin<F32>));
+    return true;
   }
+  const double len = (double) length_of_squares(s0, s1);
+  *lo = *hi = (float) len;
+  *lo *= 1.f - kSideMargin<F32>;
+  *hi *= 1.f + kSideMargin<F32>;
+  return len < thresh;
+}
+
+/* the same; *len receives length_x whenever the answer is true */
+template <bool F32>
+__device__ __forceinline__ bool length_lt(double2 pa, double2 pb, TenT<F32> ta, TenT<F32> tb, double thresh,
+                                          double* len) {
+  LenT<F32> s1;
+  const LenT<F32> s0 = length_squares<F32>(pa, pb, ta, tb, &s1);
+  if (length_test<F32>(s0, s1, thresh) > 0) return false;
+  *len = (double) length_of_squares(s0, s1);
   return *len < thresh;
 }
 

@@ -187,18 +187,18 @@ __device__ __forceinline__ double trn_dist1(double2 pa, double2 pb, double4 t) {
 }
 
 /* numeric::approxRiemannDist(a, b, Ma, Mb), numeric.cpp:469-497, in two
- * halves: the edge's length under each endpoint tensor, then their
- * geometric interpolation */
-__device__ __forceinline__ void trn_dist2_ends(double2 pa, double2 pb, double4 ta, double4 tb,
-                                               double* l0, double* l1) {
+ * halves: the edge's squared length under each endpoint tensor, then the
+ * geometric interpolation of their roots */
+__device__ __forceinline__ void trn_dist2_squares(double2 pa, double2 pb, double4 ta, double4 tb,
+                                                  double* s0, double* s1) {
   double w0 = pb.x - pa.x;
   double w1 = pb.y - pa.y;
   double m0 = ta.x * w0 + ta.y * w1;
   double m1 = ta.y * w0 + ta.z * w1;
   double m2 = tb.x * w0 + tb.y * w1;
   double m3 = tb.y * w0 + tb.z * w1;
-  *l0 = sqrt(w0 * m0 + w1 * m1);
-  *l1 = sqrt(w0 * m2 + w1 * m3);
+  *s0 = w0 * m0 + w1 * m1;
+  *s1 = w0 * m2 + w1 * m3;
 }
 
 __device__ __forceinline__ double trn_dist2_finish(double l0, double l1) {
@@ -210,9 +210,9 @@ __device__ __forceinline__ double trn_dist2_finish(double l0, double l1) {
 }
 
 __device__ __forceinline__ double trn_dist2(double2 pa, double2 pb, double4 ta, double4 tb) {
-  double l0, l1;
-  trn_dist2_ends(pa, pb, ta, tb, &l0, &l1);
-  return trn_dist2_finish(l0, l1);
+  double s0, s1;
+  trn_dist2_squares(pa, pb, ta, tb, &s0, &s1);
+  return trn_dist2_finish(sqrt(s0), sqrt(s1));
 }
 
 /* numeric::computeSteinerPoint, numeric.cpp:387-445 (la, lb: cached
@@ -240,6 +240,19 @@ __device__ __forceinline__ bool trn_ccw(double2 a, double2 b, double2 c) {
   double c2 = b.y - a.y;
   double c3 = c.y - a.y;
   return 0.5 * (c0 * c3 - c1 * c2) > TRN_EPS;
+}
+
+/* trn_ccw of the element whose corners from `pos` on are d, a, b in turn. The
+ * area seen from d differs from the one the element's own first corner gives
+ * by rounding alone, under 1e-14 of the products of its extents; only within
+ * that of the threshold are the corners put in their own order. */
+__device__ __forceinline__ bool trn_ccw_from(double2 d, double2 a, double2 b, int pos) {
+  const double ux = a.x - d.x, uy = a.y - d.y, vx = b.x - d.x, vy = b.y - d.y;
+  const double area = 0.5 * (ux * vy - vx * uy);
+  const double e = 1.e-14 * ((fabs(ux) + fabs(vx)) * (fabs(uy) + fabs(vy)));
+  if (area > TRN_EPS + e) return true;
+  if (area < TRN_EPS - e) return false;
+  return pos == 0 ? trn_ccw(d, a, b) : (pos == 1 ? trn_ccw(b, d, a) : trn_ccw(a, b, d));
 }
 
 /* tensor from eigen pairs, metric.cpp:134-148 / 222-236 */

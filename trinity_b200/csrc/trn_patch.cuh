@@ -23,12 +23,6 @@ constexpr int kNoId = 0x7fffffff;           /* pads the unused slots, sorts last
 constexpr int kPatchRows = 8;               /* the vertex's own row and 7 neighbours' */
 constexpr int kPatchKeys = kPatchRows * kRowRegs;
 
-__device__ __forceinline__ void patch_cmp(int& a, int& b) {
-  const int lo = min(a, b), hi = max(a, b);
-  a = lo;
-  b = hi;
-}
-
 /* odd-even merge of the sorted halves of a[0..N) */
 template <int N>
 __device__ __forceinline__ void patch_merge(int* a) {
