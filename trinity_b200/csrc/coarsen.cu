@@ -19,6 +19,7 @@
  * repair pass sorts them.
  */
 #include "trn_internal.h"
+#include "trn_level.cuh"
 #include "trn_mixed.cuh"
 
 #include <algorithm>
@@ -180,6 +181,78 @@ __global__ void __launch_bounds__(kSearchThreads) k_coarse_filter_append(DMesh m
   }
 }
 
+/* build_one_vicin by G lanes, two elements a lane: the elements' next
+ * vertices, and the one previous vertex that is no next one (a boundary
+ * vertex), are the neighbours; a neighbour's place is the number of smaller
+ * ones, counted by shuffles. Longer or irregular stencils by the group's first
+ * lane. v < 0: no vertex; all lanes of the warp call it. */
+template <int G>
+__device__ __forceinline__ void build_vicin_group(const DMesh& m, int v) {
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
+  const unsigned gm = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << g0;
+  const int deg = v >= 0 && m.alive[v] ? trn_deg(m, v) : 0;
+  bool odd = deg > 2 * G;
+  int a[2], b[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int k = gl + h * G;
+    a[h] = b[h] = 0x7fffffff;
+    if (k < deg && !odd) {
+      const int e = trn_row(m.stenc, m, v)[k];
+      const int4 n = e >= 0 ? m.tri[e] : make_int4(-1, -1, -1, 0);
+      a[h] = v == n.x ? n.y : (v == n.y ? n.z : n.x);
+      b[h] = v == n.x ? n.z : (v == n.y ? n.x : n.y);
+      odd |= !(v == n.x || v == n.y || v == n.z);
+    }
+  }
+  /* uniform over the warp: how many entries any of its vertices has */
+  const int most = __reduce_max_sync(0xffffffffu, odd ? 0 : deg);
+  int rank[2] = {0, 0};
+  bool found[2] = {false, false};
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (h * G >= most) break;
+    for (int k = 0; k < G; ++k) {
+      if (h * G + k >= most) break;
+      const int x = __shfl_sync(0xffffffffu, a[h], k, G);
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {
+        rank[o] += x < a[o];
+        found[o] |= x == b[o];
+        odd |= a[o] != 0x7fffffff && x == a[o] && (h * G + k) != (o * G + gl);
+      }
+    }
+  }
+  int extra = 0, x = 0x7fffffff;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const unsigned miss = __ballot_sync(0xffffffffu, b[h] != 0x7fffffff && !found[h]) & gm;
+    const int from = __shfl_sync(0xffffffffu, b[h], miss ? __ffs(miss) - 1 : 0);
+    if (miss) x = from;
+    extra += __popc(miss);
+  }
+  const bool serial = (__ballot_sync(0xffffffffu, odd || extra > 1 || deg + extra > m.bucket) & gm) != 0;
+  if (!serial && v >= 0) {
+    const TrnRow row = trn_row(m.vic, m, v);
+    int below = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (a[h] != 0x7fffffff) {
+        row[rank[h] + (extra && x < a[h] ? 1 : 0)] = a[h];
+        below += a[h] < x;
+      }
+    if (extra) {
+#pragma unroll
+      for (int o = G / 2; o >= 1; o >>= 1) below += __shfl_xor_sync(gm, below, o);
+      if (gl == 0) row[below] = x;
+    }
+    if (gl == 0) m.vdeg[v] = deg + extra;
+  } else if (serial && gl == 0) {
+    build_one_vicin(m, v);
+  }
+  __syncwarp();
+}
+
 /* the same search by a group of G lanes per vertex, for the levels that
  * list few vertices, where one lane's chain of dependent gathers (adjacency,
  * stencil, triangles, points, tensors) sets the time. The lanes compute the
@@ -188,131 +261,126 @@ __global__ void __launch_bounds__(kSearchThreads) k_coarse_filter_append(DMesh m
  * the smallest (length, adjacency index) among the valid candidates, which is
  * the first valid one in the serial search's stable length order, so the
  * targets are the same. Vertices with more than 32 neighbours fall back to
- * the serial search on the group's first lane. */
-
+ * the serial search on the group's first lane. v (the same on all lanes of a
+ * group, < 0: no vertex) gets its adjacency row too; all lanes of the warp
+ * call it, and the group's first lane receives the target. */
 template <bool F32, int G>
-__global__ void k_coarse_filter_group(DMesh m, const int* __restrict__ act, const int* act_n,
-                                      int* __restrict__ target, int* __restrict__ cand, int* count,
-                                      uint8_t* __restrict__ state, int max_n) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) trn_level_clear(m, nullptr);
-  if (trn_failed(m)) return;
-  const int n = *act_n;
-  if (n > max_n) return;
+__device__ __forceinline__ int search_group(const DMesh& m, int v) {
   const int lane = threadIdx.x & 31;
   const int gl = lane & (G - 1);
-  const int gbase = lane & ~(G - 1);
-  const int per_warp = 32 / G;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int base = warp * per_warp; base < n; base += nwarps * per_warp) {
-    const int q = base + lane / G;
-    int vv = -1;
-    if (gl == 0 && q < n) {
-      const int x = act[q];
-      if (m.activ[x] > 0) {
-        m.activ[x] = 0;
-        build_one_vicin(m, x);
-        vv = x;
-      }
-    }
-    const int v = __shfl_sync(0xffffffffu, vv, gbase);
-    __syncwarp();
-    const int nv = v >= 0 ? m.vdeg[v] : 0;
-    const bool serial = nv > 32;
-    const bool grp = v >= 0 && !serial;
-    const TrnRow vc = trn_row(m.vic, m, (v >= 0 ? v : 0));
-    const TrnRow st = trn_row(m.stenc, m, (v >= 0 ? v : 0));
-    const bool bsrc = v >= 0 && (m.tags[v] & TRN_TAG_BOUND) != 0;
-    double2 ps = make_double2(0, 0);
-    TenT<F32> ts{};
-    if (grp) {
-      ps = m.pts[v];
-      ts = ten_load<F32>(m, v);
-    }
-    /* neighbours b = gl + G * k: candidates closer than 1/sqrt(2) */
-    double lenk[32 / G];
-    unsigned candm = 0, boundm = 0;
-    for (int k = 0; k < 32 / G; ++k) {
-      const int b = gl + G * k;
-      lenk[k] = 0.0;
-      if (grp && b < nv) {
-        const int w = vc[b];
-        const bool bd = (m.tags[w] & TRN_TAG_BOUND) != 0;
-        if (bd) boundm |= 1u << b;
-        if (!(bsrc && !bd)) {
-          double len;
-          if (length_lt<F32>(ps, m.pts[w], ts, ten_load<F32>(m, w), TRN_L_MIN, &len)) {
-            candm |= 1u << b;
-            lenk[k] = len;
-          }
+  build_vicin_group<G>(m, v);
+  const int nv = v >= 0 ? m.vdeg[v] : 0;
+  const bool serial = nv > 32;
+  const bool grp = v >= 0 && !serial;
+  const TrnRow vc = trn_row(m.vic, m, (v >= 0 ? v : 0));
+  const TrnRow st = trn_row(m.stenc, m, (v >= 0 ? v : 0));
+  const bool bsrc = v >= 0 && (m.tags[v] & TRN_TAG_BOUND) != 0;
+  double2 ps = make_double2(0, 0);
+  TenT<F32> ts{};
+  if (grp) {
+    ps = m.pts[v];
+    ts = ten_load<F32>(m, v);
+  }
+  /* neighbours b = gl + G * k: candidates closer than 1/sqrt(2) */
+  double lenk[32 / G];
+  unsigned candm = 0, boundm = 0;
+  for (int k = 0; k < 32 / G; ++k) {
+    const int b = gl + G * k;
+    lenk[k] = 0.0;
+    if (grp && b < nv) {
+      const int w = vc[b];
+      const bool bd = (m.tags[w] & TRN_TAG_BOUND) != 0;
+      if (bd) boundm |= 1u << b;
+      if (!(bsrc && !bd)) {
+        double len;
+        if (length_lt<F32>(ps, m.pts[w], ts, ten_load<F32>(m, w), TRN_L_MIN, &len)) {
+          candm |= 1u << b;
+          lenk[k] = len;
         }
       }
     }
-    for (int o = G / 2; o >= 1; o >>= 1) {
-      candm |= __shfl_xor_sync(0xffffffffu, candm, o);
-      boundm |= __shfl_xor_sync(0xffffffffu, boundm, o);
+  }
+  for (int o = G / 2; o >= 1; o >>= 1) {
+    candm |= __shfl_xor_sync(0xffffffffu, candm, o);
+    boundm |= __shfl_xor_sync(0xffffffffu, boundm, o);
+  }
+  /* every (candidate, element) pair of the simulated collapses */
+  const int deg = grp ? trn_deg(m, v) : 0;
+  const int np = (grp && candm) ? nv * deg : 0;
+  const int iters = __reduce_max_sync(0xffffffffu, (np + G - 1) / G);
+  unsigned failm = 0, once = 0, twice = 0;
+  for (int k = 0; k < iters; ++k) {
+    const int p = gl + G * k;
+    if (p >= np) continue;
+    const int b = p / deg, a = p - b * deg;
+    if (!((candm >> b) & 1u)) continue;
+    const unsigned bit = 1u << b;
+    const int destin = vc[b];
+    const int4 e = m.tri[st[a]];
+    if ((v == e.x && destin == e.y) || (v == e.y && destin == e.x) || (v == e.y && destin == e.z) ||
+        (v == e.z && destin == e.y) || (v == e.z && destin == e.x) || (v == e.x && destin == e.z)) {
+      twice |= once & bit;
+      once |= bit;
+      continue;
     }
-    /* every (candidate, element) pair of the simulated collapses */
-    const int deg = grp ? trn_deg(m, v) : 0;
-    const int np = (grp && candm) ? nv * deg : 0;
-    const int iters = __reduce_max_sync(0xffffffffu, (np + G - 1) / G);
-    unsigned failm = 0, once = 0, twice = 0;
-    for (int k = 0; k < iters; ++k) {
-      const int p = gl + G * k;
-      if (p >= np) continue;
-      const int b = p / deg, a = p - b * deg;
-      if (!((candm >> b) & 1u)) continue;
-      const unsigned bit = 1u << b;
-      const int destin = vc[b];
-      const int4 e = m.tri[st[a]];
-      if ((v == e.x && destin == e.y) || (v == e.y && destin == e.x) || (v == e.y && destin == e.z) ||
-          (v == e.z && destin == e.y) || (v == e.z && destin == e.x) || (v == e.x && destin == e.z)) {
-        twice |= once & bit;
-        once |= bit;
-        continue;
-      }
-      const int f0 = (e.x == v ? destin : e.x);
-      const int f1 = (e.y == v ? destin : e.y);
-      const int f2 = (e.z == v ? destin : e.z);
-      const double2 p0 = m.pts[f0], p1 = m.pts[f1], p2 = m.pts[f2];
-      if (trn_ccw(p0, p1, p2)) {
-        const TenT<F32> t0 = ten_load<F32>(m, f0), t1 = ten_load<F32>(m, f1), t2 = ten_load<F32>(m, f2);
-        if (length_gt<F32>(p0, p1, t0, t1, TRN_L_MAX) || length_gt<F32>(p1, p2, t1, t2, TRN_L_MAX) ||
-            length_gt<F32>(p2, p0, t2, t0, TRN_L_MAX))
-          failm |= bit;
-      } else {
+    const int f0 = (e.x == v ? destin : e.x);
+    const int f1 = (e.y == v ? destin : e.y);
+    const int f2 = (e.z == v ? destin : e.z);
+    const double2 p0 = m.pts[f0], p1 = m.pts[f1], p2 = m.pts[f2];
+    if (trn_ccw(p0, p1, p2)) {
+      const TenT<F32> t0 = ten_load<F32>(m, f0), t1 = ten_load<F32>(m, f1), t2 = ten_load<F32>(m, f2);
+      if (length_gt<F32>(p0, p1, t0, t1, TRN_L_MAX) || length_gt<F32>(p1, p2, t1, t2, TRN_L_MAX) ||
+          length_gt<F32>(p2, p0, t2, t0, TRN_L_MAX))
         failm |= bit;
-      }
+    } else {
+      failm |= bit;
     }
-    for (int o = G / 2; o >= 1; o >>= 1) {
-      const unsigned fo = __shfl_xor_sync(0xffffffffu, failm, o);
-      const unsigned oo = __shfl_xor_sync(0xffffffffu, once, o);
-      const unsigned to = __shfl_xor_sync(0xffffffffu, twice, o);
-      twice |= to | (once & oo);
-      once |= oo;
-      failm |= fo;
+  }
+  for (int o = G / 2; o >= 1; o >>= 1) {
+    const unsigned fo = __shfl_xor_sync(0xffffffffu, failm, o);
+    const unsigned oo = __shfl_xor_sync(0xffffffffu, once, o);
+    const unsigned to = __shfl_xor_sync(0xffffffffu, twice, o);
+    twice |= to | (once & oo);
+    once |= oo;
+    failm |= fo;
+  }
+  const unsigned valid = candm & ~failm & ~(bsrc ? (twice & boundm) : 0u);
+  /* the smallest (length, adjacency index) among the valid candidates */
+  double best = 0.0;
+  int bestb = -1;
+  for (int k = 0; k < 32 / G; ++k) {
+    const int b = gl + G * k;
+    if (b < 32 && ((valid >> b) & 1u) && (bestb < 0 || lenk[k] < best)) {
+      best = lenk[k];
+      bestb = b;
     }
-    const unsigned valid = candm & ~failm & ~(bsrc ? (twice & boundm) : 0u);
-    /* the smallest (length, adjacency index) among the valid candidates */
-    double best = 0.0;
-    int bestb = -1;
-    for (int k = 0; k < 32 / G; ++k) {
-      const int b = gl + G * k;
-      if (b < 32 && ((valid >> b) & 1u) && (bestb < 0 || lenk[k] < best)) {
-        best = lenk[k];
-        bestb = b;
-      }
+  }
+  for (int o = G / 2; o >= 1; o >>= 1) {
+    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const int obb = __shfl_xor_sync(0xffffffffu, bestb, o);
+    if (obb >= 0 && (bestb < 0 || ob < best || (ob == best && obb < bestb))) {
+      best = ob;
+      bestb = obb;
     }
-    for (int o = G / 2; o >= 1; o >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int obb = __shfl_xor_sync(0xffffffffu, bestb, o);
-      if (obb >= 0 && (bestb < 0 || ob < best || (ob == best && obb < bestb))) {
-        best = ob;
-        bestb = obb;
-      }
-    }
+  }
+  if (gl != 0 || v < 0) return -1;
+  return serial ? identify_target<F32>(m, v) : (bestb >= 0 ? vc[bestb] : -1);
+}
+
+/* the listed vertices by the groups of the warps warp, warp + nwarps, ... */
+template <bool F32, int G>
+__device__ __forceinline__ void search_list(const DMesh& m, const int* act, int n, int warp, int nwarps, int* target,
+                                            int* cand, int* count, uint8_t* state) {
+  constexpr int per_warp = 32 / G;
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+  for (int base = warp * per_warp; base < n; base += nwarps * per_warp) {
+    const int q = base + lane / G;
+    int v = q < n ? act[q] : -1;
+    if (v >= 0 && m.activ[v] <= 0) v = -1;
+    __syncwarp();
+    if (gl == 0 && v >= 0) m.activ[v] = 0;
+    const int t = search_group<F32, G>(m, v);
     if (gl == 0 && v >= 0) {
-      const int t = serial ? identify_target<F32>(m, v) : (bestb >= 0 ? vc[bestb] : -1);
       target[v] = t;
       if (t > -1) {
         state[v] = 1;
@@ -322,74 +390,354 @@ __global__ void k_coarse_filter_group(DMesh m, const int* __restrict__ act, cons
   }
 }
 
-__global__ void k_collapse(DMesh m, const int* __restrict__ indep, const int* count,
-                           const int* __restrict__ target, const uint8_t* __restrict__ cand_flag) {
+template <bool F32, int G>
+__global__ void k_coarse_filter_group(DMesh m, const int* __restrict__ act, const int* act_n,
+                                      int* __restrict__ target, int* __restrict__ cand, int* count,
+                                      uint8_t* __restrict__ state, int max_n) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) trn_level_clear(m, nullptr);
   if (trn_failed(m)) return;
-  const int n_indep = *count;
-  for (int q = trn_tid(); q < n_indep; q += trn_grid_stride()) {
-    const int source = indep[q];
-    if (source < 0 || source >= m.capa_node || (cand_flag && !cand_flag[source])) {
-      trn_set_error(m.err, TRN_DERR_REPLAY);
+  const int n = *act_n;
+  if (n > max_n) return;
+  search_list<F32, G>(m, act, n, trn_tid() >> 5, trn_grid_stride() >> 5, target, cand, count, state);
+}
+
+/* one collapse (Coarse::collapseEdge) by one lane: long stencils */
+__device__ __noinline__ void collapse_serial(const DMesh& m, int source, int destin) {
+  const TrnRow st = trn_row(m.stenc, m, source);
+  const int deg = trn_deg(m, source);
+  const int limit = (m.tags[source] & TRN_TAG_BOUND) ? 1 : 2;
+  int k = 0, trash0 = -1, trash1 = -1;
+  int opp[2] = {-1, -1};
+  for (int a = 0; k < limit && a < deg; ++a) {
+    int4 n = m.tri[st[a]];
+    int o = -2;
+    if ((source == n.x && destin == n.y) || (destin == n.x && source == n.y)) o = n.z;
+    else if ((source == n.y && destin == n.z) || (destin == n.y && source == n.z)) o = n.x;
+    else if ((source == n.z && destin == n.x) || (destin == n.z && source == n.x)) o = n.y;
+    if (o != -2) {
+      opp[k] = o;
+      if (k == 0) trash0 = a; else trash1 = a;
+      ++k;
+    }
+  }
+  int rest[TRN_MAX_DEG];
+  int nr = 0;
+  for (int a = 0; a < deg; ++a) {
+    int e = st[a];
+    if (a == trash0 || a == trash1) {
+      m.tri[e] = make_int4(-1, -1, -1, 0);
       continue;
     }
-    const int destin = target[source];
-    const TrnRow st = trn_row(m.stenc, m, source);
-    const int deg = trn_deg(m, source);
-    const int limit = (m.tags[source] & TRN_TAG_BOUND) ? 1 : 2;
-    int k = 0, trash0 = -1, trash1 = -1;
-    int opp[2] = {-1, -1};
-    for (int a = 0; k < limit && a < deg; ++a) {
-      int4 n = m.tri[st[a]];
-      int o = -2;
-      if ((source == n.x && destin == n.y) || (destin == n.x && source == n.y)) o = n.z;
-      else if ((source == n.y && destin == n.z) || (destin == n.y && source == n.z)) o = n.x;
-      else if ((source == n.z && destin == n.x) || (destin == n.z && source == n.x)) o = n.y;
-      if (o != -2) {
-        opp[k] = o;
-        if (k == 0) trash0 = a; else trash1 = a;
-        ++k;
-      }
+    rest[nr++] = e;
+  }
+  for (int j = 0; j < k; ++j)
+    if (opp[j] >= 0) trn_tag_fix(m, opp[j]);
+  trn_stenc_append_n(m, destin, rest, nr);
+  for (int a = 0; a < nr; ++a) {
+    int4 n = m.tri[rest[a]];
+    if (n.x == source) n.x = destin;
+    else if (n.y == source) n.y = destin;
+    else if (n.z == source) n.z = destin;
+    m.tri[rest[a]] = n;
+  }
+  trn_tag_fix(m, destin);
+  const TrnRow vc = trn_row(m.vic, m, source);
+  const int nv = m.vdeg[source];
+  /* re-activate the 1-ring: independent flag atomics, newly set ids listed
+   * in batches of 16 with one atomic each */
+  int ids[16], na = 0;
+  for (int b = 0; b < nv; ++b) {
+    const int t = vc[b];
+    if (trn_byte_cas01(m.activ + t)) ids[na++] = t;
+    if (na == 16) {
+      if (m.act_next) trn_list_push_n(m.act_next, m.act_next_n, ids, na);
+      na = 0;
     }
-    int rest[TRN_MAX_DEG];
-    int nr = 0;
-    for (int a = 0; a < deg; ++a) {
-      int e = st[a];
-      if (a == trash0 || a == trash1) {
-        m.tri[e] = make_int4(-1, -1, -1, 0);
-        continue;
-      }
-      rest[nr++] = e;
+  }
+  if (m.act_next) trn_list_push_n(m.act_next, m.act_next_n, ids, na);
+  m.vdeg[source] = 0;
+  m.alive[source] = 0;
+  for (int a = 0; a < deg; ++a) st[a] = -1;
+  m.deg[source] = 0;
+}
+
+/* where a collapse's newly tagged vertices go: straight onto the lists (one
+ * atomic per warp and push), or, in a grid-wide launch, into the block's
+ * shared buffers, which one atomic each empties (thousands of warps pushing a
+ * few ids each serialise on the two counters in L2) */
+struct DirectSink {
+  __device__ __forceinline__ void fix(const DMesh& m, int v) const { trn_tag_fix(m, v); }
+  __device__ __forceinline__ void act(const DMesh& m, int v) const { trn_activate(m, v); }
+};
+
+constexpr int kSinkAct = 512, kSinkFix = 192;
+struct BlockLists {
+  int act[kSinkAct], fix[kSinkFix];
+  int nact, nfix, act0, fix0;
+};
+struct BlockSink {
+  BlockLists* b;
+  __device__ __forceinline__ void fix(const DMesh& m, int v) const {
+    if (!trn_byte_cas01(m.fixes + v) || !m.fix_list) return;
+    const int k = atomicAdd(&b->nfix, 1);
+    if (k < kSinkFix) b->fix[k] = v;
+    else trn_list_push(m.fix_list, m.fix_n, v);
+  }
+  __device__ __forceinline__ void act(const DMesh& m, int v) const {
+    if (!trn_byte_cas01(m.activ + v) || !m.act_next) return;
+    const int k = atomicAdd(&b->nact, 1);
+    if (k < kSinkAct) b->act[k] = v;
+    else trn_list_push(m.act_next, m.act_next_n, v);
+  }
+};
+
+/* one collapse by 8 lanes, up to four elements a lane: the shell elements are
+ * the first one (boundary source) or two that hold both ends; the others move
+ * to the destination. Every step's gathers and atomics are in flight together,
+ * where one lane went through its elements and its neighbours one after the
+ * other. Levels of a few hundred collapses: 20-29 us -> 6 us inside the level
+ * loop, 14 us as a launch; the first level of the 2M-triangle workload 141 ->
+ * 60 us (a level's pushes through the block's buffers; straight onto the
+ * lists it took twice the one-lane kernel's time). */
+constexpr int kCollapseLanes = 8, kCollapseEach = 4;
+
+template <class Sink>
+__device__ __forceinline__ void collapse_group(const DMesh& m, int source, int destin, const Sink& sink) {
+  const int lane = threadIdx.x & 31, gl = lane & (kCollapseLanes - 1), g0 = lane & ~(kCollapseLanes - 1);
+  const unsigned gm = 0xffu << g0;
+  const int deg = trn_deg(m, source);
+  if (deg > kCollapseLanes * kCollapseEach) {
+    if (gl == 0) collapse_serial(m, source, destin);
+    __syncwarp(gm);
+    return;
+  }
+  const TrnRow st = trn_row(m.stenc, m, source), vc = trn_row(m.vic, m, source);
+  const int nv = m.vdeg[source];
+  const int limit = (m.tags[source] & TRN_TAG_BOUND) ? 1 : 2;
+  int e[kCollapseEach];
+  int4 n[kCollapseEach];
+#pragma unroll
+  for (int c = 0; c < kCollapseEach; ++c) {
+    const int at = c * kCollapseLanes + gl;
+    e[c] = at < deg ? st[at] : -1;
+  }
+#pragma unroll
+  for (int c = 0; c < kCollapseEach; ++c) n[c] = e[c] >= 0 ? m.tri[e[c]] : make_int4(-1, -1, -1, 0);
+  int shells = 0, nr = 0, place[kCollapseEach] = {-1, -1, -1, -1}, opp[kCollapseEach] = {-1, -1, -1, -1};
+  unsigned trash = 0;
+#pragma unroll
+  for (int c = 0; c < kCollapseEach; ++c) {
+    if (c * kCollapseLanes >= deg) break;   /* the same on every lane of the group */
+    int o = -2;
+    if (e[c] >= 0) {
+      if ((source == n[c].x && destin == n[c].y) || (destin == n[c].x && source == n[c].y)) o = n[c].z;
+      else if ((source == n[c].y && destin == n[c].z) || (destin == n[c].y && source == n[c].z)) o = n[c].x;
+      else if ((source == n[c].z && destin == n[c].x) || (destin == n[c].z && source == n[c].x)) o = n[c].y;
     }
-    for (int j = 0; j < k; ++j)
-      if (opp[j] >= 0) trn_tag_fix(m, opp[j]);
-    trn_stenc_append_n(m, destin, rest, nr);
-    for (int a = 0; a < nr; ++a) {
-      int4 n = m.tri[rest[a]];
-      if (n.x == source) n.x = destin;
-      else if (n.y == source) n.y = destin;
-      else if (n.z == source) n.z = destin;
-      m.tri[rest[a]] = n;
+    const unsigned both = (__ballot_sync(gm, o != -2) & gm) >> g0;
+    const bool shell = o != -2 && shells + __popc(both & ((1u << gl) - 1u)) < limit;
+    shells += __popc(both);
+    if (shell) {
+      trash |= 1u << c;
+      opp[c] = o;
     }
-    trn_tag_fix(m, destin);
-    const TrnRow vc = trn_row(m.vic, m, source);
-    const int nv = m.vdeg[source];
-    /* re-activate the 1-ring: independent flag atomics, newly set ids listed
-     * in batches of 16 with one atomic each */
-    int ids[16], na = 0;
-    for (int b = 0; b < nv; ++b) {
-      const int t = vc[b];
-      if (trn_byte_cas01(m.activ + t)) ids[na++] = t;
-      if (na == 16) {
-        if (m.act_next) trn_list_push_n(m.act_next, m.act_next_n, ids, na);
-        na = 0;
-      }
+    const bool live = c * kCollapseLanes + gl < deg && !shell;
+    const unsigned keep = (__ballot_sync(gm, live) & gm) >> g0;
+    if (live) place[c] = nr + __popc(keep & ((1u << gl) - 1u));
+    nr += __popc(keep);
+  }
+  int k = 0;
+  if (gl == 0) k = atomicAdd(m.deg + destin, nr);
+  k = __shfl_sync(gm, k, 0, kCollapseLanes);
+  const bool full = k + nr > m.bucket;
+  if (full && gl == 0) trn_set_error(m.err, TRN_DERR_BUCKET);
+  const TrnRow dst = trn_row(m.stenc, m, destin);
+#pragma unroll
+  for (int c = 0; c < kCollapseEach; ++c) {
+    const int at = c * kCollapseLanes + gl;
+    if (place[c] >= 0) {
+      if (!full) dst[k + place[c]] = e[c];
+      if (n[c].x == source) n[c].x = destin;
+      else if (n[c].y == source) n[c].y = destin;
+      else if (n[c].z == source) n[c].z = destin;
+      if (e[c] >= 0) m.tri[e[c]] = n[c];
+    } else if ((trash >> c) & 1u) {
+      m.tri[e[c]] = make_int4(-1, -1, -1, 0);
+      if (opp[c] >= 0) sink.fix(m, opp[c]);
     }
-    if (m.act_next) trn_list_push_n(m.act_next, m.act_next_n, ids, na);
+    if (at < deg) st[at] = -1;
+  }
+  if (gl == 0) sink.fix(m, destin);
+  for (int b = gl; b < nv; b += kCollapseLanes) sink.act(m, vc[b]);
+  __syncwarp(gm);   /* every lane has read the counts */
+  if (gl == 0) {
     m.vdeg[source] = 0;
     m.alive[source] = 0;
-    for (int a = 0; a < deg; ++a) st[a] = -1;
     m.deg[source] = 0;
   }
+}
+
+__global__ void __launch_bounds__(TRN_THREADS) k_collapse(DMesh m, const int* __restrict__ indep, const int* count,
+                                                         const int* __restrict__ target,
+                                                         const uint8_t* __restrict__ cand_flag) {
+  __shared__ BlockLists lists;
+  if (trn_failed_block(m)) return;
+  const int n_indep = *count;
+  const BlockSink sink{&lists};
+  constexpr int groups = TRN_THREADS / kCollapseLanes;
+  for (int base = blockIdx.x * groups; base < n_indep; base += gridDim.x * groups) {
+    if (threadIdx.x == 0) lists.nact = lists.nfix = 0;
+    __syncthreads();
+    const int q = base + (int) threadIdx.x / kCollapseLanes;
+    if (q < n_indep) {
+      const int source = indep[q];
+      if (source < 0 || source >= m.capa_node || (cand_flag && !cand_flag[source])) {
+        if ((threadIdx.x & (kCollapseLanes - 1)) == 0) trn_set_error(m.err, TRN_DERR_REPLAY);
+      } else {
+        collapse_group(m, source, target[source], sink);
+      }
+    }
+    __syncthreads();
+    const int na = min(lists.nact, kSinkAct), nf = min(lists.nfix, kSinkFix);
+    if (threadIdx.x == 0 && na) lists.act0 = atomicAdd(m.act_next_n, na);
+    if (threadIdx.x == 32 && nf) lists.fix0 = atomicAdd(m.fix_n, nf);
+    __syncthreads();
+    for (int i = threadIdx.x; i < na; i += TRN_THREADS) m.act_next[lists.act0 + i] = lists.act[i];
+    for (int i = threadIdx.x; i < nf; i += TRN_THREADS) m.fix_list[lists.fix0 + i] = lists.fix[i];
+    __syncthreads();
+  }
+}
+
+/* ---- the levels of a short list in one launch (trn_level.cuh) ---- */
+
+/* one candidate of the independent set, kept in registers over the rounds:
+ * its neighbours, of which a round reads the states (in flight together; the
+ * rule is mis_item's of heuristics.cu) */
+struct TailCand {
+  int v = -1, nv = 0;
+  int w[kRowChunk];
+  uint8_t st = 0;
+
+  __device__ __forceinline__ void load(const DMesh& m, int id) {
+    v = id;
+    st = 1;   /* the filter marks every candidate undecided */
+    nv = m.vdeg[v];
+    const int* row = trn_row(m.vic, m, v).p;
+#pragma unroll
+    for (int j = 0; j < kRowChunk; ++j) w[j] = j < nv ? row[j] : -1;
+  }
+  __device__ __forceinline__ void round(const DMesh& m, const uint8_t* in, uint8_t* out, uint64_t seed) {
+    if (st == 1) {
+      const uint64_t pv = trn_prio(seed, v);
+      bool is_max = true, leave = false;
+      uint8_t sw[kRowChunk];
+#pragma unroll
+      for (int j = 0; j < kRowChunk; ++j) sw[j] = w[j] >= 0 ? in[w[j]] : 0;
+#pragma unroll
+      for (int j = 0; j < kRowChunk; ++j) {
+        leave |= sw[j] == 2;
+        if (sw[j] == 1 && trn_prio(seed, w[j]) > pv) is_max = false;
+      }
+      const TrnRow vc = trn_row(m.vic, m, v);
+      for (int b = kRowChunk; b < nv; ++b) {
+        const int x = vc[b];
+        const uint8_t s = in[x];
+        leave |= s == 2;
+        if (s == 1 && trn_prio(seed, x) > pv) is_max = false;
+      }
+      st = leave ? 0 : (is_max ? 2 : 1);
+    }
+    out[v] = st;
+  }
+};
+
+constexpr int kMaxMisRounds = 8;
+
+template <bool F32>
+__global__ void __launch_bounds__(kTailThreads) k_coarsen_tail(DMesh m, int* act0, int* act1, int* status, int* target,
+                                                               int* cand, uint8_t* s0, uint8_t* s1, int* indep,
+                                                               int* open, Seed sd, int rounds, int cap) {
+  const int tid = trn_tid(), stride = trn_grid_stride();
+  for (int level = 0;; ++level) {
+    const int* act = (level & 1) ? act1 : act0;
+    m.act_next = (level & 1) ? act0 : act1;
+    const bool failed = tail_failed(m);
+    /* the filter; the counters of the later steps start empty */
+    if (tid == 0) {
+      trn_level_clear(m, nullptr);
+      status[S_NINDEP] = 0;
+      for (int r = 0; r < kMaxMisRounds; ++r) open[r] = 0;
+    }
+    /* more lanes a vertex while the list leaves lanes idle */
+    const int na = failed ? 0 : status[S_ACT];
+    if (na * 16 <= 2 * stride)
+      search_list<F32, 16>(m, act, na, tid >> 5, stride >> 5, target, cand, status + S_NTASK, s0);
+    else
+      search_list<F32, 8>(m, act, na, tid >> 5, stride >> 5, target, cand, status + S_NTASK, s0);
+    cluster_sync();
+    /* the independent set: rounds until no candidate is undecided (the
+     * rounds after that would only copy the states) */
+    const int nc = status[S_NTASK];
+    const uint64_t base = trn_seed(sd);
+    TailCand mine;
+    if (tid < nc) mine.load(m, cand[tid]);
+    int r = 0;
+    while (r < rounds) {
+      const uint8_t* in = (r & 1) ? s1 : s0;
+      uint8_t* out = (r & 1) ? s0 : s1;
+      const uint64_t seed = base + 0x9e3779b97f4a7c15ULL * r;
+      bool wait = false;
+      if (mine.v >= 0) {
+        mine.round(m, in, out, seed);
+        wait = mine.st == 1;
+      }
+      for (int q = tid + stride; q < nc; q += stride) {   /* more candidates than threads */
+        TailCand c;
+        c.load(m, cand[q]);
+        c.st = in[c.v];
+        c.round(m, in, out, seed);
+        wait |= c.st == 1;
+      }
+      if (wait) open[r] = 1;
+      cluster_sync();
+      if (!tail_word(open + r++)) break;
+    }
+    uint8_t* state = (r & 1) ? s1 : s0;
+    uint8_t* other = (r & 1) ? s0 : s1;
+    for (int q = tid; q < nc; q += stride) {
+      const int v = cand[q];
+      const uint8_t st = q == tid ? mine.st : state[v];
+      if (st == 2) trn_append(indep, status + S_NINDEP, v);
+      else if (st == 1) trn_activate(m, v);
+      state[v] = 0;
+      other[v] = 0;
+    }
+    cluster_sync();
+    const int ni = tail_failed(m) ? 0 : status[S_NINDEP];
+    for (int q = tid / kCollapseLanes; q < ni; q += stride / kCollapseLanes) {
+      const int v = indep[q];
+      collapse_group(m, v, target[v], DirectSink());
+    }
+    cluster_sync();
+    if (tid == 0) tail_level_end(m, status, kLevelCoarsen, cap);
+    if (!tail_failed(m)) {
+      int buf[TRN_MAX_DEG];
+      tail_fix(m, tid, stride, buf);
+    }
+    cluster_sync();
+    if (!tail_word(status + S_CONT)) return;
+  }
+}
+
+bool coarsen_tail(const DMesh& m, int* act0, int* act1, int* status, int* target, int* cand, HeurWs& ws, int* indep,
+                  Seed sd, int rounds, int cap, bool fp32, cudaStream_t s) {
+  if (rounds > kMaxMisRounds) return false;
+  ProfScope ps("coarsen_tail", s, 0.0);
+  int* open = ws.cnt + 112;
+  return fp32 ? cluster_launch(k_coarsen_tail<true>, s, m, act0, act1, status, target, cand, ws.state, ws.state2,
+                               indep, open, sd, rounds, cap)
+              : cluster_launch(k_coarsen_tail<false>, s, m, act0, act1, status, target, cand, ws.state, ws.state2,
+                               indep, open, sd, rounds, cap);
 }
 
 void coarsen_pre(const DMesh& m, int nb_nodes, cudaStream_t s, int* act, int* act_n) {
@@ -455,8 +803,8 @@ void coarsen_filter_append(const DMesh& m, const int* act, const int* act_n, int
 void collapse(const DMesh& m, const int* indep, const int* count, const int* target,
               const uint8_t* cand_flag, cudaStream_t s, long long bound) {
   ProfScope ps("collapse", s, 0.0);
-  k_collapse<<<TRN_RESIDENT(k_collapse, grid_bounded(bound, m.capa_node), TRN_THREADS), TRN_THREADS, 0, s>>>(m, indep, count, target,
-                                                                      cand_flag);
+  const int g = grid_bounded(bound < 0 ? bound : kCollapseLanes * bound, (long long) kCollapseLanes * m.capa_node);
+  k_collapse<<<TRN_RESIDENT(k_collapse, g, TRN_THREADS), TRN_THREADS, 0, s>>>(m, indep, count, target, cand_flag);
   note_launch();
   check_launch("collapse");
 }

@@ -32,6 +32,7 @@
  *                   its vertices grouped by stencil length.
  */
 #include "trn_internal.h"
+#include "trn_match.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -281,114 +282,7 @@ void mis_jp_rounds(const DMesh& m, const int* cand, const int* count, int rounds
   check_launch("mis_jp_rounds");
 }
 
-/* ---------------- matching ---------------- */
-static constexpr int kMatchRounds = 4;
-
-/* The rank of dual edge (row i, slot q) in the upper bits of its weight, and
- * the mask of the lower bits a hash fills. Row order (rank == nullptr): the
- * slot of the edge in the row of its lower-id candidate end, first slots
- * first, as the reference's greedy takes each candidate's first free
- * neighbour. Gain: rank[4 i + q], the quantized quality change of the flip.
- * Both ends of an edge between two candidates compute the same rank. */
-__device__ __forceinline__ uint32_t edge_rank(const int* __restrict__ dual, const int* __restrict__ dual_n,
-                                              const uint32_t* __restrict__ rank, const int* __restrict__ map,
-                                              int ntasks, int i, int q, uint32_t* low) {
-  if (rank) {
-    *low = 0x3ffu;
-    return rank[i * 4 + q];
-  }
-  const int c = dual[i * 4], n = dual[i * 4 + q];
-  int pos = q;
-  if (n < c) {
-    const int x = map[n];
-    if (x >= 0 && x < ntasks && dual[x * 4] == n)
-      for (int e = 1; e < dual_n[x]; ++e)
-        if (dual[x * 4 + e] == c) pos = e;
-  }
-  *low = 0x3fffffffu;
-  return (uint32_t) (4 - pos) << 30;
-}
-
-/* the weight of dual edge (row i, slot q): its rank, then a symmetric hash of
- * the pair, so equal ranks break ties at random and the edge weighs the same
- * from both ends */
-__device__ __forceinline__ uint32_t edge_weight(const int* __restrict__ dual, const int* __restrict__ dual_n,
-                                                const uint32_t* __restrict__ rank, const int* __restrict__ map,
-                                                int ntasks, int i, int q, uint64_t seed, int round) {
-  const int a = dual[i * 4], b = dual[i * 4 + q];
-  const int lo = a < b ? a : b, hi = a < b ? b : a;
-  const uint64_t h = trn_hash64(seed ^ ((uint64_t) (uint32_t) lo << 32 | (uint32_t) hi) ^
-                                ((uint64_t) round * 0xd1b54a32d192ed03ULL));
-  uint32_t low;
-  const uint32_t r = edge_rank(dual, dual_n, rank, map, ntasks, i, q, &low);
-  return (r & ~low) | ((uint32_t) (h >> 32) & low) | 1u;
-}
-
-struct MatchArgs {
-  const int* dual;
-  const int* dual_n;
-  const uint32_t* rank;   /* gain ranks, or nullptr for row order */
-  const int* map;
-  int* mate;
-  unsigned long long* prop;
-  int* choice;
-};
-
-__device__ __forceinline__ void match_reset_item(const MatchArgs& a, int i) {
-  for (int q = 0; q < a.dual_n[i]; ++q) {
-    const int e = a.dual[i * 4 + q];
-    a.mate[e] = -1;
-    a.prop[e] = 0ULL;
-  }
-}
-
-__device__ __forceinline__ void match_propose_item(const MatchArgs& a, int ntasks, int i, uint64_t seed,
-                                                   int round) {
-  const int c = a.dual[i * 4];
-  int best = -1;
-  uint32_t bw = 0;
-  if (a.mate[c] == -1) {
-    for (int q = 1; q < a.dual_n[i]; ++q) {
-      const int n = a.dual[i * 4 + q];
-      if (a.mate[n] != -1) continue;
-      const uint32_t w = edge_weight(a.dual, a.dual_n, a.rank, a.map, ntasks, i, q, seed, round);
-      if (w > bw) { bw = w; best = n; }
-    }
-    if (best >= 0) atomicMax(a.prop + best, ((unsigned long long) bw << 32) | (uint32_t) c);
-  }
-  a.choice[i] = best;
-}
-
-/* a mutual choice between two candidates, or a non-candidate's heaviest
- * proposer, is a match */
-__device__ __forceinline__ void match_accept_item(const MatchArgs& a, int ntasks, int i, uint64_t seed,
-                                                  int round, int* pairs, int* npairs) {
-  const int n = a.choice[i];
-  if (n < 0) return;
-  const int c = a.dual[i * 4];
-  const int x = a.map[n];
-  const bool n_cand = x >= 0 && x < ntasks && a.dual[x * 4] == n;
-  bool ok;
-  if (n_cand) {
-    ok = (a.choice[x] == c) && (c < n);
-  } else {
-    int q = 1;
-    while (q < a.dual_n[i] - 1 && a.dual[i * 4 + q] != n) ++q;
-    const uint32_t w = edge_weight(a.dual, a.dual_n, a.rank, a.map, ntasks, i, q, seed, round);
-    ok = a.prop[n] == (((unsigned long long) w << 32) | (uint32_t) c);
-  }
-  if (ok) {
-    a.mate[c] = n;
-    a.mate[n] = c;
-    const int p = trn_warp_reserve(npairs);
-    pairs[2 * p] = c;
-    pairs[2 * p + 1] = n;
-  }
-}
-
-__device__ __forceinline__ void match_clear_item(const MatchArgs& a, int i) {
-  for (int q = 1; q < a.dual_n[i]; ++q) a.prop[a.dual[i * 4 + q]] = 0ULL;
-}
+/* ---------------- matching (items: trn_match.cuh) ---------------- */
 
 __global__ void k_match_reset(MatchArgs a, const int* ntasks_dev, int min_n) {
   const int ntasks = *ntasks_dev;
@@ -471,125 +365,7 @@ void match_handshake(const DMesh& m, int nb_elems, const int* dual, const int* d
   check_launch("match_handshake");
 }
 
-/* ---------------- greedy matching in interleaved element order ----------------
- *
- * The reference's matching (Match::computeGreedyMatching / matchAndUpdate,
- * matching.cpp:81-135) is a loop over the dual rows in list order, i.e. in
- * increasing candidate id: a row whose candidate is still free marks it
- * taken, then takes its free neighbours in slot order, going past each
- * neighbour that is not itself a candidate (the "continue" of
- * matching.cpp:124) and stopping at the first one that is; the candidate's
- * partner is the last neighbour taken. This is that loop without the
- * degree-1 stack, over the rows in the order (id mod 4, id): four
- * interleaved sweeps of the candidate ids.
- *
- * Its result is computed exactly, in parallel, as the greedy matching of an
- * order is: in each round a row decides once it comes first, under that
- * order, among the undecided rows that list any of its elements; such rows
- * share no element with one another, so they decide independently, and what
- * each finds is what the sequential loop would have found. Rows propose
- * their key with a 64-bit atomicMin on every element of their row into the
- * round's buffer (keys of later rounds compare lower, so no buffer needs
- * clearing between rounds); a row is ready when every element holds its own
- * key. A round decides the ready rows and lets the others propose for the
- * next round into the other buffer, so one launch per round. The rounds
- * run over a compacted list of the undecided rows; once that list is short
- * one block finishes the remaining rounds with block barriers. After
- * kGreedyRounds rounds any row still undecided stays unmatched (a valid, if
- * not maximal, matching). On the 2M-triangle workload the deepest level
- * needs 48 rounds, the mean is 12.
- *
- * The four-way interleave keeps the chains of dependent rows short (a plain
- * increasing-id sweep has chains as long as a row of the grid), and the
- * final meshes' metric edge-length histograms stay within half a point per
- * bin of the reference's, where a maximal handshake matching, which flips
- * more pairs, is a point and a half off. */
-constexpr int kGreedyRounds = 64;
-constexpr int kGreedyTail = 2048;   /* undecided rows left to the one-block rounds */
-/* rows waiting above which a round runs as its own grid launch (measured:
- * such rounds are faster launched than inside the cooperative kernel) */
-constexpr int kGreedyGrid = 1 << 15;
-
-struct GreedyArgs {
-  const int* dual;
-  const int* dual_n;
-  const int* map;
-  int* vis;                 /* per element: -1 free, else taken */
-  unsigned long long* mk0;  /* per element: lowest key proposed, even rounds */
-  unsigned long long* mk1;  /* odd rounds */
-  int* list0;               /* undecided rows, even rounds */
-  int* list1;
-  int* cnt;                 /* [3] list lengths, by round mod 3 */
-  int* ran;                 /* [kGreedyRounds] round r ran on the grid */
-};
-
-__device__ __forceinline__ unsigned long long greedy_key(int r, int c) {
-  return ((unsigned long long) (kGreedyRounds - r) << 40) | ((unsigned long long) (c & 3) << 32) |
-         (uint32_t) c;
-}
-
-/* "is a candidate" as matching.cpp:124 asks it: the element has a row in the
- * map, which keeps the rows of earlier levels of the same call (it is reset
- * once per call, swapping.cpp:161-162) */
-__device__ __forceinline__ bool greedy_is_row(const GreedyArgs& a, int ntasks, int e) {
-  (void) ntasks;
-  return a.map[e] >= 0;
-}
-
-
-__device__ __forceinline__ void greedy_propose(const GreedyArgs& a, int r, int i) {
-  unsigned long long* mk = (r & 1) ? a.mk1 : a.mk0;
-  const unsigned long long key = greedy_key(r, a.dual[i * 4]);
-  for (int q = 0; q < a.dual_n[i]; ++q) atomicMin(mk + a.dual[i * 4 + q], key);
-}
-
-/* is row i first on all its elements in round r? The loads of the row's
- * slots past its length read slot 0 again (always there), so that every
- * load can be issued before any compare */
-__device__ __forceinline__ bool greedy_ready(const GreedyArgs& a, int r, int i) {
-  const unsigned long long* mk = (r & 1) ? a.mk1 : a.mk0;
-  const int4 row = reinterpret_cast<const int4*>(a.dual)[i];
-  const int dn = a.dual_n[i];
-  const unsigned long long key = greedy_key(r, row.x);
-  const unsigned long long k0 = mk[row.x], k1 = mk[dn > 1 ? row.y : row.x];
-  const unsigned long long k2 = mk[dn > 2 ? row.z : row.x], k3 = mk[dn > 3 ? row.w : row.x];
-  return k0 == key && k1 == key && k2 == key && k3 == key;
-}
-
-/* row i in round r, its readiness known: decide it when it is first on all
- * its elements (and return false), else propose it for round r + 1 (and
- * return true) */
-__device__ __forceinline__ bool greedy_act(const GreedyArgs& a, int ntasks, int r, int i, bool ready,
-                                           int* pairs, int* npairs) {
-  const int c = a.dual[i * 4];
-  const int dn = a.dual_n[i];
-  if (!ready) {
-    greedy_propose(a, r + 1, i);
-    return true;
-  }
-  if (a.vis[c] != -1) return false;
-  a.vis[c] = 1;
-  int partner = -1;
-  for (int q = 1; q < dn; ++q) {
-    const int n = a.dual[i * 4 + q];
-    if (a.vis[n] != -1) continue;
-    a.vis[n] = 1;
-    partner = n;
-    if (greedy_is_row(a, ntasks, n)) break;
-  }
-  if (partner >= 0) {
-    const int p = trn_warp_reserve(npairs);
-    pairs[2 * p] = c;
-    pairs[2 * p + 1] = partner;
-  }
-  return false;
-}
-
-__device__ __forceinline__ bool greedy_item(const GreedyArgs& a, int ntasks, int r, int i, int* pairs,
-                                            int* npairs) {
-  return greedy_act(a, ntasks, r, i, greedy_ready(a, r, i), pairs, npairs);
-}
-
+/* ---------------- greedy matching (items: trn_match.cuh) ---------------- */
 
 /* round 0's proposals; every row starts undecided */
 __global__ void k_greedy_start(GreedyArgs a, const int* ntasks_dev, int min_n) {

@@ -22,6 +22,8 @@
  * rows therefore persist across levels.
  */
 #include "trn_internal.h"
+#include "trn_level.cuh"
+#include "trn_match.cuh"
 #include "trn_mixed.cuh"
 
 namespace trn {
@@ -212,8 +214,30 @@ __device__ __forceinline__ uint32_t flip_rank(const DMesh& m, int a, int b) {
 }
 
 /* free mode: filter, dual extraction and (when rank is given) the ranks of
- * each row's flips in one pass; rows are numbered in append order (no use
- * depends on it) */
+ * each row's flips of listed element k; rows are numbered in append order (no
+ * use depends on it) */
+template <bool F32>
+__device__ __forceinline__ void filter_dual_item(const DMesh& m, int k, int* dual, int* dual_n, int* map,
+                                                 uint32_t* rank, int* count, const GreedyReset& gr) {
+  if (!m.activ[k]) return;
+  m.activ[k] = 0;
+  if (!(m.qual[k] < TRN_Q_MIN)) return;
+  const int r = trn_warp_reserve(count);
+  const int dn = dual_row(m, k, r, dual, dual_n, map);
+  if (gr.vis)   /* the greedy matching's state of the row's elements (rows sharing one write the same) */
+    for (int e = 0; e < dn; ++e) {
+      const int x = dual[r * 4 + e];
+      gr.vis[x] = -1;
+      gr.mk0[x] = ~0ULL;
+      gr.mk1[x] = ~0ULL;
+    }
+  if (rank) {
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    for (int e = 1; e < dn; ++e) w[e] = flip_rank<F32>(m, k, dual[r * 4 + e]);
+    reinterpret_cast<uint4*>(rank)[r] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
 template <bool F32>
 __global__ void k_swap_filter_dual(DMesh m, const int* __restrict__ act, const int* act_n,
                                    int* __restrict__ dual, int* __restrict__ dual_n,
@@ -222,30 +246,8 @@ __global__ void k_swap_filter_dual(DMesh m, const int* __restrict__ act, const i
   if (blockIdx.x == 0 && threadIdx.x == 0) trn_level_clear(m, flips);
   if (trn_failed(m)) return;
   const int na = *act_n;
-  for (int q = trn_tid(); q < na; q += trn_grid_stride()) {
-    const int k = act[q];
-    if (!m.activ[k]) continue;
-    m.activ[k] = 0;
-    if (!(m.qual[k] < TRN_Q_MIN)) continue;
-    unsigned mask = __activemask();
-    int lane = threadIdx.x & 31, leader = __ffs(mask) - 1, base = 0;
-    if (lane == leader) base = atomicAdd(count, __popc(mask));
-    base = __shfl_sync(mask, base, leader);
-    const int r = base + __popc(mask & ((1u << lane) - 1));
-    const int dn = dual_row(m, k, r, dual, dual_n, map);
-    if (gr.vis)   /* the greedy matching's state of the row's elements (rows sharing one write the same) */
-      for (int e = 0; e < dn; ++e) {
-        const int x = dual[r * 4 + e];
-        gr.vis[x] = -1;
-        gr.mk0[x] = ~0ULL;
-        gr.mk1[x] = ~0ULL;
-      }
-    if (rank) {
-      uint32_t w[4] = {0u, 0u, 0u, 0u};
-      for (int e = 1; e < dn; ++e) w[e] = flip_rank<F32>(m, k, dual[r * 4 + e]);
-      reinterpret_cast<uint4*>(rank)[r] = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-  }
+  for (int q = trn_tid(); q < na; q += trn_grid_stride())
+    filter_dual_item<F32>(m, act[q], dual, dual_n, map, rank, count, gr);
 }
 
 /* Swap::swap, swapping.cpp:55-149, with the two new qualities on two lanes:
@@ -294,8 +296,31 @@ __device__ int flip_pair2(const DMesh& m, int id1, int id2, int index, const int
   return 2;
 }
 
-/* two lanes per pair; the grid-stride loop keeps the lanes of a pair
- * together (both see the same p), so every shuffle has its partner */
+/* two lanes per pair (both see the same p), so every shuffle has its
+ * partner; the flip's share of the commit count, on the pair's first lane */
+template <bool F32>
+__device__ __forceinline__ int flip_item(const DMesh& m, int k1, int k2, const int* map, const int* dual,
+                                         const int* dual_n, int ntasks, bool strict_map) {
+  const int half = threadIdx.x & 1;
+  const unsigned mask = 3u << (threadIdx.x & 30);
+  bool ok = k1 >= 0 && k1 < m.capa_elem && k2 >= 0 && k2 < m.capa_elem;
+  int index = -1;
+  if (ok) {
+    index = map[k1];
+    ok = index >= 0 && index < ntasks && dual[index * 4] == k1;
+    if (ok) {
+      ok = false;
+      for (int q = 1; q < dual_n[index]; ++q) ok |= (dual[index * 4 + q] == k2);
+    }
+  }
+  if (!ok) {
+    if (!half) trn_set_error(m.err, TRN_DERR_REPLAY);
+    return 0;
+  }
+  const int r = flip_pair2<F32>(m, k1, k2, index, map, dual, dual_n, ntasks, strict_map, half, mask);
+  return half ? 0 : r;
+}
+
 template <bool F32>
 __global__ void k_swap_flip2(DMesh m, const int* __restrict__ pairs, const int* npairs,
                              const int* __restrict__ map, const int* __restrict__ dual,
@@ -304,30 +329,220 @@ __global__ void k_swap_flip2(DMesh m, const int* __restrict__ pairs, const int* 
   if (trn_failed(m)) return;
   const int np = *npairs;
   const int ntasks = *ntasks_dev;
-  const int half = threadIdx.x & 1;
-  const unsigned mask = 3u << (threadIdx.x & 30);
   int local = 0;
   const int stride = (gridDim.x * blockDim.x) >> 1;
-  for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 1; p < np; p += stride) {
-    const int k1 = pairs[2 * p], k2 = pairs[2 * p + 1];
-    bool ok = k1 >= 0 && k1 < m.capa_elem && k2 >= 0 && k2 < m.capa_elem;
-    int index = -1;
-    if (ok) {
-      index = map[k1];
-      ok = index >= 0 && index < ntasks && dual[index * 4] == k1;
-      if (ok) {
-        ok = false;
-        for (int q = 1; q < dual_n[index]; ++q) ok |= (dual[index * 4 + q] == k2);
+  for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 1; p < np; p += stride)
+    local += flip_item<F32>(m, pairs[2 * p], pairs[2 * p + 1], map, dual, dual_n, ntasks, strict_map != 0);
+  trn_warp_add(commit, local);
+}
+
+/* ---- the levels of a short list in one launch (trn_level.cuh) ---- */
+
+/* a matched pair by 8 lanes: the first two run the tests and the two new
+ * qualities as flip_pair2 does, then every lane takes one of the flip's tags
+ * and re-activations, so that a commit is a few rounds of independent atomics
+ * instead of a chain of a dozen */
+constexpr int kFlipLanes = 8;
+
+template <bool F32>
+__device__ __forceinline__ int flip_group(const DMesh& m, int id1, int id2, const int* map, const int* dual,
+                                          const int* dual_n, int ntasks) {
+  const int gl = threadIdx.x & (kFlipLanes - 1);
+  const unsigned gm = 0xffu << ((threadIdx.x & 31) & ~(kFlipLanes - 1));
+  const int index = map[id1], x = map[id2];
+  int c1[3], c2[3];
+  double q0, q1;
+  /* lanes 2 to 7 follow the first two: the same tests, a quality each of
+   * their own pair that nobody reads */
+  const bool ok = flip_eval2<F32>(m, id1, id2, c1, c2, &q0, &q1, threadIdx.x & 1, gm);
+  bool go = false;
+  if (ok) go = !(trn_dmin(q0, q1) < trn_dmin(m.qual[id1], m.qual[id2]));
+  /* this lane's re-activation: 0-3 the row of id1, 4-7 the row of id2 (of
+   * the current level only) */
+  int act = -1;
+  if (go) {
+    const int row = gl < 4 ? index : (x > -1 && x < ntasks && dual[x * 4] == id2 ? x : -1);
+    if (row >= 0 && (gl & 3) < dual_n[row]) act = dual[row * 4 + (gl & 3)];
+  }
+  __syncwarp(gm);   /* every lane has read the old elements */
+  if (!go) return 0;
+  if (gl == 0) {
+    m.tri[id1] = make_int4(c1[0], c1[1], c1[2], 0);
+    m.qual[id1] = q0;
+    trn_stenc_append(m, c2[0], id2);
+  } else if (gl == 1) {
+    m.tri[id2] = make_int4(c2[0], c2[1], c2[2], 0);
+    m.qual[id2] = q1;
+    trn_stenc_append(m, c2[1], id1);
+  }
+  if (gl < 4) trn_tag_fix(m, gl < 3 ? (gl == 0 ? c1[0] : (gl == 1 ? c1[1] : c1[2])) : c2[2]);
+  if (act >= 0) trn_activate(m, act);
+  return gl == 0 ? 2 : 0;
+}
+
+/* a dual row of the greedy matching, kept in registers over the rounds (the
+ * rule is greedy_item's, trn_match.cuh): a round costs its four keys and, once
+ * the row is first on all of them, its four elements' states */
+struct TailRow {
+  int4 row = make_int4(-1, -1, -1, -1);
+  int dn = 0;
+  unsigned rows = 0;   /* bit q: element q has a row itself */
+  bool open = false;
+
+  __device__ __forceinline__ int at(int q) const { return q == 0 ? row.x : (q == 1 ? row.y : (q == 2 ? row.z : row.w)); }
+  __device__ __forceinline__ void load(const GreedyArgs& a, int i) {
+    row = reinterpret_cast<const int4*>(a.dual)[i];
+    dn = a.dual_n[i];
+#pragma unroll
+    for (int q = 1; q < 4; ++q)
+      if (q < dn && a.map[at(q)] >= 0) rows |= 1u << q;
+    open = true;
+  }
+  __device__ __forceinline__ void propose(const GreedyArgs& a, int r) const {
+    unsigned long long* mk = (r & 1) ? a.mk1 : a.mk0;
+    const unsigned long long key = greedy_key(r, row.x);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q < dn) atomicMin(mk + at(q), key);
+  }
+  __device__ __forceinline__ void round(const GreedyArgs& a, int r, int* pairs, int* npairs) {
+    const unsigned long long* mk = (r & 1) ? a.mk1 : a.mk0;
+    const unsigned long long key = greedy_key(r, row.x);
+    bool ready = true;
+    unsigned free = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q < dn) {
+        ready &= mk[at(q)] == key;
+        if (a.vis[at(q)] == -1) free |= 1u << q;
+      }
+    if (!ready) {
+      propose(a, r + 1);
+      return;
+    }
+    open = false;
+    if (!(free & 1u)) return;
+    a.vis[row.x] = 1;
+    int partner = -1;
+    bool done = false;
+#pragma unroll
+    for (int q = 1; q < 4; ++q)
+      if (!done && ((free >> q) & 1u)) {
+        a.vis[at(q)] = 1;
+        partner = at(q);
+        done = (rows >> q) & 1u;
+      }
+    if (partner >= 0) {
+      const int p = trn_warp_reserve(npairs);
+      pairs[2 * p] = row.x;
+      pairs[2 * p + 1] = partner;
+    }
+  }
+};
+
+template <bool F32>
+__global__ void __launch_bounds__(kTailThreads) k_swap_tail(DMesh m, int* act0, int* act1, int* status, int* dual,
+                                                            int* dual_n, int* map, uint32_t* rank, GreedyArgs ga,
+                                                            MatchArgs ma, int greedy, int* pairs, Seed sd, int cap) {
+  const int tid = trn_tid(), stride = trn_grid_stride();
+  GreedyReset gr;
+  if (greedy) gr = GreedyReset{ga.vis, ga.mk0, ga.mk1};
+  int* npairs = status + S_NPAIRS;
+  for (int level = 0;; ++level) {
+    const int* act = (level & 1) ? act1 : act0;
+    m.act_next = (level & 1) ? act0 : act1;
+    const int na = tail_failed(m) ? 0 : status[S_ACT];
+    if (tid == 0) {
+      trn_level_clear(m, status + S_COMMIT);
+      *npairs = 0;
+      ga.cnt[1] = ga.cnt[2] = 0;
+    }
+    for (int q = tid; q < na; q += stride)
+      filter_dual_item<F32>(m, act[q], dual, dual_n, map, rank, status + S_NTASK, gr);
+    cluster_sync();
+    const int ntasks = status[S_NTASK];
+    if (greedy && ntasks <= stride) {
+      TailRow mine;
+      if (tid < ntasks) {
+        mine.load(ga, tid);
+        mine.propose(ga, 0);
+      }
+      cluster_sync();
+      for (int r = 0; r < kGreedyRounds; ++r) {
+        /* rows undecided before this round (round 0: all); the word of the
+         * round after next starts at zero */
+        if (r > 0 && tail_word(ga.cnt + r % 3) == 0) break;
+        if (tid == 0) ga.cnt[(r + 2) % 3] = 0;
+        if (mine.open) {
+          mine.round(ga, r, pairs, npairs);
+          if (mine.open) ga.cnt[(r + 1) % 3] = 1;
+        }
+        cluster_sync();
+      }
+    } else if (greedy) {
+      if (tid == 0) ga.cnt[0] = ntasks;
+      for (int i = tid; i < ntasks; i += stride) {
+        greedy_propose(ga, 0, i);
+        ga.list0[i] = i;
+      }
+      cluster_sync();
+      for (int r = 0; r < kGreedyRounds; ++r) {
+        const int n = tail_word(ga.cnt + r % 3);
+        if (n == 0) break;
+        const int* in = (r & 1) ? ga.list1 : ga.list0;
+        int* out = (r & 1) ? ga.list0 : ga.list1;
+        if (tid == 0) ga.cnt[(r + 2) % 3] = 0;
+        for (int q = tid; q < n; q += stride) {
+          const int i = in[q];
+          if (greedy_item(ga, ntasks, r, i, pairs, npairs)) trn_append(out, ga.cnt + (r + 1) % 3, i);
+        }
+        cluster_sync();
+      }
+    } else {
+      const uint64_t seed = trn_seed(sd);
+      for (int i = tid; i < ntasks; i += stride) match_reset_item(ma, i);
+      cluster_sync();
+      for (int r = 0; r < kMatchRounds; ++r) {
+        for (int i = tid; i < ntasks; i += stride) match_propose_item(ma, ntasks, i, seed, r);
+        cluster_sync();
+        for (int i = tid; i < ntasks; i += stride) match_accept_item(ma, ntasks, i, seed, r, pairs, npairs);
+        cluster_sync();
+        for (int i = tid; i < ntasks; i += stride) match_clear_item(ma, i);
+        cluster_sync();
       }
     }
-    if (!ok) {
-      if (!half) trn_set_error(m.err, TRN_DERR_REPLAY);
-      continue;
+    const int np = tail_failed(m) ? 0 : *npairs;
+    int local = 0;
+    if (np * kFlipLanes <= stride) {
+      if (tid / kFlipLanes < np) {
+        const int p = tid / kFlipLanes;
+        local = flip_group<F32>(m, pairs[2 * p], pairs[2 * p + 1], map, dual, dual_n, ntasks);
+      }
+    } else {
+      for (int p = tid >> 1; p < np; p += stride >> 1)
+        local += flip_item<F32>(m, pairs[2 * p], pairs[2 * p + 1], map, dual, dual_n, ntasks, true);
     }
-    const int r = flip_pair2<F32>(m, k1, k2, index, map, dual, dual_n, ntasks, strict_map != 0, half, mask);
-    if (!half) local += r;
+    trn_warp_add(status + S_COMMIT, local);
+    cluster_sync();
+    if (tid == 0) tail_level_end(m, status, kLevelSwap, cap);
+    if (!tail_failed(m)) {
+      int buf[TRN_MAX_DEG];
+      tail_fix(m, tid, stride, buf);
+    }
+    cluster_sync();
+    if (!tail_word(status + S_CONT)) return;
   }
-  trn_warp_add(commit, local);
+}
+
+bool swap_tail(const DMesh& m, int* act0, int* act1, int* status, int* dual, int* dual_n, int* map, uint32_t* rank,
+               bool greedy, HeurWs& ws, int* pairs, Seed sd, int cap, bool fp32, cudaStream_t s) {
+  ProfScope ps("swap_tail", s, 0.0);
+  const GreedyArgs ga{dual, dual_n, map, ws.mate, ws.prop, ws.prop2, ws.choice, ws.choice2, ws.cnt, ws.cnt + 8};
+  const MatchArgs ma{dual, dual_n, rank, map, ws.mate, ws.prop, ws.choice};
+  return fp32 ? cluster_launch(k_swap_tail<true>, s, m, act0, act1, status, dual, dual_n, map, rank, ga, ma,
+                               greedy ? 1 : 0, pairs, sd, cap)
+              : cluster_launch(k_swap_tail<false>, s, m, act0, act1, status, dual, dual_n, map, rank, ga, ma,
+                               greedy ? 1 : 0, pairs, sd, cap);
 }
 
 void swap_init(const DMesh& m, int nb_nodes, int nb_elems, int* map, bool fp32, cudaStream_t s, int* act,

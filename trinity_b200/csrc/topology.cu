@@ -12,6 +12,7 @@
  *                    the vertex's bucket held in registers/local memory.
  */
 #include "trn_internal.h"
+#include "trn_level.cuh"
 
 #include <algorithm>
 #include "trn_mixed.cuh"
@@ -47,56 +48,6 @@ __global__ void k_build_vicin(DMesh m, int nb_nodes, int only_flagged) {
     if (only_flagged && m.activ[v] == 0) continue;
     build_one_vicin(m, v);
   }
-}
-
-/* repair of one tagged stencil (Mesh::fixTagged, mesh.cpp:716-760): keep the
- * entries whose element still holds v, sorted, without duplicates. Stencils
- * of up to 16 entries stay in registers (the element loads all in flight at
- * once, a sorting network, no local memory); longer ones take the scratch
- * array. Both give the same entries in the same order. */
-constexpr int kFixRegs = 16;
-
-__device__ __forceinline__ void fix_stencil(const DMesh& m, int v, int* buf) {
-  const TrnRow s = trn_row(m.stenc, m, v);
-  const int d = trn_deg(m, v);
-  int k = 0;
-  if (d <= kFixRegs) {
-    int r[kFixRegs];
-#pragma unroll
-    for (int a = 0; a < kFixRegs; ++a) r[a] = (a < d) ? s[a] : -1;
-#pragma unroll
-    for (int a = 0; a < kFixRegs; ++a) {
-      int keep = 0x7fffffff;
-      if (r[a] >= 0) {
-        const int4 nn = m.tri[r[a]];
-        if (v == nn.x || v == nn.y || v == nn.z) keep = r[a];
-      }
-      r[a] = keep;
-    }
-#pragma unroll
-    for (int p = 0; p < kFixRegs; ++p)
-#pragma unroll
-      for (int a = p & 1; a + 1 < kFixRegs; a += 2) {
-        const int lo = min(r[a], r[a + 1]), hi = max(r[a], r[a + 1]);
-        r[a] = lo;
-        r[a + 1] = hi;
-      }
-#pragma unroll
-    for (int a = 0; a < kFixRegs; ++a)
-      if (r[a] != 0x7fffffff && (a == 0 || r[a] != r[a - 1])) s[k++] = r[a];
-  } else {
-    for (int a = 0; a < d; ++a) {
-      const int t = s[a];
-      if (t < 0) continue;
-      const int4 nn = m.tri[t];
-      if (v == nn.x || v == nn.y || v == nn.z) buf[k++] = t;
-    }
-    trn_isort(buf, k);
-    k = trn_iunique(buf, k);
-    for (int a = 0; a < k; ++a) s[a] = buf[a];
-  }
-  for (int a = k; a < d; ++a) s[a] = -1;
-  m.deg[v] = k;
 }
 
 __global__ void k_fix_tagged(DMesh m, int nb_nodes) {

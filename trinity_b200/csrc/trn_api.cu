@@ -1051,7 +1051,11 @@ int trn_coarsen_run(trn_mesh* m, int max_colors, trn_stats* st) {
     enq_coarsen_begin(m, s, false);
     long long bound = m->nb_nodes;
     do {
-      enq_coarsen_level(m, s, bound, 0, false);
+      /* the levels of a short list run in one launch, to the call's end */
+      if (bound > kCoarsenTail ||
+          !coarsen_tail(level_mesh(m), act_list(m, 0), act_list(m, 1), m->status, m->target, m->list, m->hws,
+                        m->indep, seed_of(m, 0x9e37ULL), kMisRounds, m->level_cap, m->fp32, s))
+        enq_coarsen_level(m, s, bound, 0, false);
       int rc = sync_status(m);
       if (rc) return rc;
       bound = m->h_status[S_ACT];
@@ -1093,7 +1097,11 @@ int trn_swap_run(trn_mesh* m, trn_stats* st) {
     enq_swap_begin(m, s, false);
     long long bound = m->nb_elems;
     do {
-      enq_swap_level(m, s, bound, 0, false);
+      if (bound > kSwapTail ||
+          !swap_tail(level_mesh(m), act_list(m, 0), act_list(m, 1), m->status, m->dual, m->dual_n, m->map,
+                     m->swap_match == TRN_SWAP_GAIN ? m->hws.rank : nullptr, m->swap_match == TRN_SWAP_GREEDY, m->hws,
+                     m->pairs, seed_of(m, 0x51edULL), m->level_cap, m->fp32, s))
+        enq_swap_level(m, s, bound, 0, false);
       int rc = sync_status(m);
       if (rc) return rc;
       bound = m->h_status[S_ACT];

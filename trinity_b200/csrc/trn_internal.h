@@ -337,6 +337,19 @@ void color_finish(const DMesh& m, int hint, int max_col, HeurWs& ws, int* parts,
                   unsigned* tick, cudaStream_t s);
 int* color_cont(HeurWs& ws);
 
+/* the coarsening (swapping) levels left, in one launch on one cluster, from
+ * the list act0 (its length in status[S_ACT]); the decision and the call's
+ * statistics end up in status as after the last level. For lists of at most
+ * kCoarsenTail vertices (eight lanes each: four passes of the cluster's 8,192
+ * threads; at 2,048 the 100 x 100 workload's coarsening takes 3.0 ms instead
+ * of 2.6) or kSwapTail elements (a thread each) and streams that are not being
+ * captured; false when it could not launch. */
+constexpr int kCoarsenTail = 4096, kSwapTail = 8192;
+bool coarsen_tail(const DMesh& m, int* act0, int* act1, int* status, int* target, int* cand, HeurWs& ws, int* indep,
+                  Seed sd, int rounds, int cap, bool fp32, cudaStream_t s);
+bool swap_tail(const DMesh& m, int* act0, int* act1, int* status, int* dual, int* dual_n, int* map, uint32_t* rank,
+               bool greedy, HeurWs& ws, int* pairs, Seed sd, int cap, bool fp32, cudaStream_t s);
+
 /* element-quality functional and its adjoint (adjoint.cu) */
 struct AdjWs {
   int cap_v = 0, cap_e = 0;
