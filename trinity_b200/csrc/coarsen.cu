@@ -734,9 +734,9 @@ bool coarsen_tail(const DMesh& m, int* act0, int* act1, int* status, int* target
   if (rounds > kMaxMisRounds) return false;
   ProfScope ps("coarsen_tail", s, 0.0);
   int* open = ws.cnt + 112;
-  return fp32 ? cluster_launch(k_coarsen_tail<true>, s, m, act0, act1, status, target, cand, ws.state, ws.state2,
+  return fp32 ? cluster_launch<k_coarsen_tail<true>>(s, m, act0, act1, status, target, cand, ws.state, ws.state2,
                                indep, open, sd, rounds, cap)
-              : cluster_launch(k_coarsen_tail<false>, s, m, act0, act1, status, target, cand, ws.state, ws.state2,
+              : cluster_launch<k_coarsen_tail<false>>(s, m, act0, act1, status, target, cand, ws.state, ws.state2,
                                indep, open, sd, rounds, cap);
 }
 

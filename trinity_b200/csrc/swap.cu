@@ -539,9 +539,9 @@ bool swap_tail(const DMesh& m, int* act0, int* act1, int* status, int* dual, int
   ProfScope ps("swap_tail", s, 0.0);
   const GreedyArgs ga{dual, dual_n, map, ws.mate, ws.prop, ws.prop2, ws.choice, ws.choice2, ws.cnt, ws.cnt + 8};
   const MatchArgs ma{dual, dual_n, rank, map, ws.mate, ws.prop, ws.choice};
-  return fp32 ? cluster_launch(k_swap_tail<true>, s, m, act0, act1, status, dual, dual_n, map, rank, ga, ma,
+  return fp32 ? cluster_launch<k_swap_tail<true>>(s, m, act0, act1, status, dual, dual_n, map, rank, ga, ma,
                                greedy ? 1 : 0, pairs, sd, cap)
-              : cluster_launch(k_swap_tail<false>, s, m, act0, act1, status, dual, dual_n, map, rank, ga, ma,
+              : cluster_launch<k_swap_tail<false>>(s, m, act0, act1, status, dual, dual_n, map, rank, ga, ma,
                                greedy ? 1 : 0, pairs, sd, cap);
 }
 

@@ -7,6 +7,8 @@
 
 #include "trn_internal.h"
 
+#include <atomic>
+
 namespace trn {
 
 /* repair of one tagged stencil (Mesh::fixTagged, mesh.cpp:716-760): keep the
@@ -179,9 +181,9 @@ __device__ __forceinline__ int tail_word(const int* p) { return *(const volatile
 
 /* launches `kernel` as one cluster; false when it could not (the caller then
  * takes the grid-wide kernels) */
-template <class K, class... Args>
-bool cluster_launch(K kernel, cudaStream_t s, Args... args) {
-  static int size = -1;   /* per kernel; a race writes the same value */
+template <auto kernel, class... Args>
+bool cluster_launch(cudaStream_t s, Args... args) {
+  static std::atomic<int> size{-1};   /* of this kernel; a race writes the same value */
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(kTailThreads);
   cfg.stream = s;
