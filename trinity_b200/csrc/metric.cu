@@ -25,131 +25,22 @@
  * vertices that the first pass lists as not fitting.
  */
 #include "trn_internal.h"
+#include "trn_metric.cuh"
 #include "trn_mixed.cuh"
-#include "trn_patch.cuh"
 
 namespace trn {
 
-/* An element's share of a patch sum depends on the element alone, and an
- * element lies in the patches of about 12 vertices: it is computed once into a
- * 32-byte record (one sector a gather) instead of once per patch. What bounds
- * the patch sums: the record gathers (24 a vertex, mostly L1/L2 hits) and the
- * integer merge of the rows. One vertex a thread that gathered, sorted in
- * local memory and computed every element of its patch took 582 us for the
- * gradient and 650 us for the Hessian of the 2M-triangle mesh; records and
- * register merge take 30 + 194 and 30 + 202 us (cold caches). */
 __global__ void k_elem_gradient(DMesh m, int nb_elems, const double* __restrict__ solut,
                                 double4* __restrict__ rec) {
   if (trn_failed(m)) return;
-  for (int t = trn_tid(); t < nb_elems; t += trn_grid_stride()) {
-    if (m.tri[t].x < 0) {
-      rec[t] = make_double4(0.0, 0.0, 0.0, 0.0);
-      continue;
-    }
-    const ElemGrad g = elem_grad(m, t);
-    const double s0 = solut[g.v.x], s1 = solut[g.v.y], s2 = solut[g.v.z];
-    double ex = 0, ey = 0;
-    ex += s0 * g.d[0];
-    ey += s0 * g.d[1];
-    ex += s1 * g.d[2];
-    ey += s1 * g.d[3];
-    ex += s2 * g.d[4];
-    ey += s2 * g.d[5];
-    rec[t] = make_double4(g.area, g.area * ex, g.area * ey, 0.0);
-  }
+  for (int t = trn_tid(); t < nb_elems; t += trn_grid_stride()) rec[t] = elem_gradient(m, t, solut);
 }
 
 __global__ void k_elem_hessian(DMesh m, int nb_elems, const double2* __restrict__ grad,
                                double4* __restrict__ rec) {
   if (trn_failed(m)) return;
-  for (int t = trn_tid(); t < nb_elems; t += trn_grid_stride()) {
-    if (m.tri[t].x < 0) {
-      rec[t] = make_double4(0.0, 0.0, 0.0, 0.0);
-      continue;
-    }
-    const ElemGrad g = elem_grad(m, t);
-    const double2 g0 = grad[g.v.x], g1 = grad[g.v.y], g2 = grad[g.v.z];
-    double dl[4] = {0, 0, 0, 0};
-    dl[0] += (g0.x * g.d[0]);
-    dl[1] += (g0.x * g.d[1]);
-    dl[2] += (g0.y * g.d[0]);
-    dl[3] += (g0.y * g.d[1]);
-    dl[0] += (g1.x * g.d[2]);
-    dl[1] += (g1.x * g.d[3]);
-    dl[2] += (g1.y * g.d[2]);
-    dl[3] += (g1.y * g.d[3]);
-    dl[0] += (g2.x * g.d[4]);
-    dl[1] += (g2.x * g.d[5]);
-    dl[2] += (g2.y * g.d[4]);
-    dl[3] += (g2.y * g.d[5]);
-    rec[t] = make_double4(g.area * dl[0], g.area * dl[1], g.area * dl[2], g.area * dl[3]);
-  }
+  for (int t = trn_tid(); t < nb_elems; t += trn_grid_stride()) rec[t] = elem_hessian(m, t, grad);
 }
-
-/* the sums over one patch: load() the record of an element, add() them in
- * ascending element order, finish() the vertex. The reference stores the
- * per-element values and sums afterwards in the same element order;
- * interleaving its loops keeps every sum's order. */
-struct GradSum {
-  const double4* rec;
-  double2* grad;
-  double* atot;   /* patch areas, for the Hessian's mean too */
-  double total_area = 0, gx = 0, gy = 0;
-  using Rec = double4;
-  __device__ __forceinline__ void begin(const DMesh&, int) {}
-  __device__ __forceinline__ Rec load(const DMesh&, int t) const { return rec[t]; }
-  __device__ __forceinline__ void add(const Rec& r) {
-    total_area += r.x;
-    gx += r.y;
-    gy += r.z;
-  }
-  __device__ __forceinline__ void finish(const DMesh&, int v) {
-    gx /= total_area;
-    gy /= total_area;
-    grad[v] = make_double2(gx, gy);
-    atot[v] = total_area;
-  }
-};
-
-struct HessSum {
-  const double4* rec;
-  const double* atot;   /* the gradient pass's sums: the same areas in the same order */
-  double scale_exp;
-  double4* hsym;
-  double4* mloc;
-  double h[4] = {0, 0, 0, 0};
-  using Rec = double4;
-  __device__ __forceinline__ void begin(const DMesh&, int) {}
-  __device__ __forceinline__ Rec load(const DMesh&, int t) const { return rec[t]; }
-  __device__ __forceinline__ void add(const Rec& r) {
-    h[0] += r.x;
-    h[1] += r.y;
-    h[2] += r.z;
-    h[3] += r.w;
-  }
-  __device__ __forceinline__ void finish(const DMesh& m, int v) {
-    const double total_area = atot[v];
-    for (int j = 0; j < 4; ++j) h[j] /= total_area;
-    /* symmetrise (hessian.cpp:149-152) */
-    double t0 = h[0];
-    double t1 = 0.5 * (h[1] + h[2]);
-    double t2 = h[3];
-    if (hsym) hsym[v] = make_double4(t0, t1, t2, 0.0);
-    /* normalizeLocally (metric.cpp:107-149) */
-    double mm[4] = {t0, t1, t1, t2};
-    double val[2] = {0, 0}, vec[4] = {0, 0, 0, 0};
-    trn_eigen(mm, val, vec);
-    val[0] = trn_dmax(fabs(val[0]), TRN_EPS);
-    val[1] = trn_dmax(fabs(val[1]), TRN_EPS);
-    double det = val[0] * val[1];
-    double scale_loc = trn_pow(det, scale_exp);
-    val[0] *= scale_loc;
-    val[1] *= scale_loc;
-    const double4 r = trn_recompose(val, vec);
-    m.ten[v] = r;
-    if (mloc) mloc[v] = r;
-  }
-};
 
 /* ---- the mixed-precision form of the recovery ----
  * The same patch means in FP32. Every coordinate difference is taken in
@@ -251,76 +142,27 @@ struct HessSum32 {
   }
 };
 
-/* one thread a vertex, its patch merged in registers; a vertex whose rows do
- * not fit goes onto rest[*rest_n] (when given; the second pass over the same
- * rows finds the same ones) */
 constexpr int kPatchThreads = 128;
 
+/* a vertex whose rows do not fit goes onto rest[*rest_n] (when given; the
+ * second pass over the same rows finds the same ones) */
 template <class Sum, int Batch>
 __global__ void __launch_bounds__(kPatchThreads) k_patch_sum(DMesh m, int nb_nodes, Sum zero, int* rest,
                                                              int* rest_n) {
   if (trn_failed(m)) return;
-  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    int key[kPatchKeys];
-    if (!patch_keys(m, v, key)) {
-      if (rest) trn_append(rest, rest_n, v);
-      continue;
-    }
-    Sum s = zero;
-    s.begin(m, v);
-#pragma unroll
-    for (int c = 0; c < kPatchKeys; c += Batch) {
-      typename Sum::Rec r[Batch];
-#pragma unroll
-      for (int j = 0; j < Batch; ++j)
-        if (key[c + j] != kNoId && (c + j == 0 || key[c + j] != key[c + j - 1])) r[j] = s.load(m, key[c + j]);
-#pragma unroll
-      for (int j = 0; j < Batch; ++j)
-        if (key[c + j] != kNoId && (c + j == 0 || key[c + j] != key[c + j - 1])) s.add(r[j]);
-    }
-    s.finish(m, v);
-  }
+  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride())
+    if (!patch_sum_regs<Sum, Batch>(m, v, zero) && rest) trn_append(rest, rest_n, v);
 }
 
-/* the listed vertices, a warp each: every lane walks the sorted patch (the
- * loads are warp-wide broadcasts) and the first writes */
+/* the listed vertices, a warp each */
 template <class Sum>
 __global__ void __launch_bounds__(kPatchThreads) k_patch_sum_rest(DMesh m, Sum zero, const int* rest,
                                                                   const int* rest_n) {
   __shared__ int s_buf[kPatchThreads / 32][TRN_MAX_PATCH];
   if (trn_failed(m)) return;
   const int n = *rest_n;
-  int* buf = s_buf[threadIdx.x >> 5];
-  for (int q = trn_tid() >> 5; q < n; q += trn_grid_stride() >> 5) {
-    const int v = rest[q];
-    const int k = patch_sort_warp(m, v, buf);
-    Sum s = zero;
-    s.begin(m, v);
-    for (int i = 0; i < k; ++i)
-      if (i == 0 || buf[i] != buf[i - 1]) s.add(s.load(m, buf[i]));
-    if ((threadIdx.x & 31) == 0) s.finish(m, v);
-    __syncwarp();
-  }
-}
-
-__device__ __forceinline__ double complexity_term(const DMesh& m, int i) {
-  const int4 v = m.tri[i];
-  if (v.x < 0) return 0.0;
-  double2 p0 = m.pts[v.x], p1 = m.pts[v.y], p2 = m.pts[v.z];
-  double s0 = p1.x - p0.x;
-  double s1 = p2.x - p0.x;
-  double s2 = p1.y - p0.y;
-  double s3 = p2.y - p0.y;
-  double area = 0.5 * (s0 * s3 - s1 * s2);
-  double rho = 0.;
-  int ids[3] = {v.x, v.y, v.z};
-  for (int j = 0; j < 3; ++j) {
-    double4 t = m.ten[ids[j]];
-    double det = t.x * t.z - trn_pow(t.y, 2);
-    rho += sqrt(det);
-  }
-  rho /= 3;
-  return rho * area;
+  for (int q = trn_tid() >> 5; q < n; q += trn_grid_stride() >> 5)
+    patch_sum_warp(m, rest[q], zero, s_buf[threadIdx.x >> 5]);
 }
 
 __global__ void k_complexity_term(DMesh m, int nb_elems, double* __restrict__ terms) {
@@ -387,17 +229,7 @@ __global__ void k_normalize(DMesh m, int nb_nodes, const double* complexity, dou
   if (trn_failed(m)) return;
   double fact = target / *complexity;
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    double4 t = m.ten[v];
-    double mm[4] = {t.x, t.y, t.y, t.z};
-    double val[2], vec[4];
-    trn_eigen(mm, val, vec);
-    val[0] *= fact;
-    val[1] *= fact;
-    for (int j = 0; j < 2; ++j) {
-      val[j] = trn_dmin(val[j], eig_min);
-      val[j] = trn_dmax(val[j], eig_max);
-    }
-    double4 t4 = trn_recompose(val, vec);
+    const double4 t4 = normalize_tensor(m.ten[v], fact, eig_min, eig_max);
     m.ten[v] = t4;
     if (m.lten) m.lten[v] = trn_log_tensor(t4.x, t4.y, t4.z);
   }

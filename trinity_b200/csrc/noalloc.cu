@@ -16,22 +16,24 @@
  * long as the process lives. Every call on a device shares it: calls that
  * overlap on the GPU (other streams, other host threads) race and corrupt
  * each other's results, so serialise them. The array keeps the last call's
- * contents; each call first clears what must start empty.
+ * contents; each call starts by clearing what must be empty.
  *
  * Host code cannot use the array's name as a device address (in host code it
  * names a host-side stand-in), so the first call on each device looks the
  * address up with cudaGetSymbolAddress while that device is current and keeps
  * it.
  *
- * The computation is the same kernels, in the same order, as trn_metric_run
- * (gradient, Hessian with local L^p scaling, complexity with the fixed-shape
- * tree sum, global scaling), so the tensors are identical to it when that
+ * The computation is trn_metric_run's, step by step (gradient, Hessian with
+ * local L^p scaling, complexity with the fixed-shape tree sum, global
+ * scaling; trn_metric.cuh), so the tensors are identical to it when that
  * mesh also sums with the tree (its default; exact_sum and replay sum in
- * element order). The kernels run on the caller's stream with the address
+ * element order). The kernel runs on the caller's stream with the address
  * looked up for the current device, so the stream must belong to it.
  */
 #include "trn_internal.h"
+#include "trn_level.cuh"
 #include "trn_libm.h"
+#include "trn_metric.cuh"
 #include "../../include/trinity_b200.h"
 
 #include <cmath>
@@ -40,19 +42,12 @@
 
 namespace trn {
 
-/* kernels of topology.cu and metric.cu, reused as they are */
-__global__ void k_fill_stencils(DMesh m, int nb_elems);
-__global__ void k_sort_stencils(DMesh m, int nb_nodes);
-__global__ void k_build_vicin(DMesh m, int nb_nodes, int only_flagged);
-__global__ void k_normalize(DMesh m, int nb_nodes, const double* complexity, double target,
-                            double eig_min, double eig_max);
-
 namespace {
 
 constexpr size_t kMaxN = TRN_NOALLOC_MAX_NODES;
 constexpr size_t kMaxE = TRN_NOALLOC_MAX_ELEMS;
 constexpr size_t kB = TRN_NOALLOC_BUCKET;
-constexpr size_t kPartials = 4096;  /* >= any grid_for() block count */
+constexpr size_t kPartials = 256;  /* one per 256 elements */
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t) 255; }
 
@@ -70,8 +65,7 @@ constexpr size_t oTerms = oGrad + align256(sizeof(double2) * kMaxN);
 constexpr size_t oRec = oTerms + align256(sizeof(double) * kPartials);
 constexpr size_t oAtot = oRec + align256(sizeof(double4) * kMaxE);
 constexpr size_t oRest = oAtot + align256(sizeof(double) * kMaxN);
-constexpr size_t oCplx = oRest + align256(sizeof(int) * (kMaxN + 1));
-constexpr size_t oErr = oCplx + 256;
+constexpr size_t oErr = oRest + align256(sizeof(int) * (kMaxN + 1));
 constexpr size_t kScratchBytes = oErr + 256;
 
 }  // namespace
@@ -103,31 +97,123 @@ int scratch_address(unsigned char** out) {
   return TRN_OK;
 }
 
-__global__ void k_na_expand(const int* __restrict__ tris, int nb_elems, int nb_nodes,
-                            int4* __restrict__ tri4, int* err) {
-  for (int i = trn_tid(); i < nb_elems; i += trn_grid_stride()) {
-    int a = tris[3 * i], b = tris[3 * i + 1], c = tris[3 * i + 2];
-    if (a < 0 || a >= nb_nodes || b < 0 || b >= nb_nodes || c < 0 || c >= nb_nodes) {
-      trn_set_error(err, TRN_DERR_INVALID);
-      a = b = c = -1;
+/* The whole recovery in one launch of one thread-block cluster: at most 16,384
+ * vertices are two a thread, so each step is a few dependent gathers, and as
+ * fifteen launches and four clears they cost five times that. The steps are
+ * separated by the cluster barrier; the error word is read once a warp and
+ * step, so lanes agree about it. The complexity is summed in the tree of
+ * k_sum_terms / k_sum_final: a partial per 256 elements (as metric_run's grid
+ * has for so few), then one tree over the partials, which every block
+ * computes for itself. 441 vertices 105 -> 67 us a call, 16,129
+ * vertices 187 (before the element records) -> 110. */
+constexpr int kNaPart = TRN_THREADS;
+
+__device__ __forceinline__ double na_tree(double* sm, double s, int t) {
+  sm[t] = s;
+  __syncthreads();
+  for (int o = kNaPart / 2; o > 0; o >>= 1) {
+    if (t < o) sm[t] += sm[t + o];
+    __syncthreads();
+  }
+  const double r = sm[0];
+  __syncthreads();
+  return r;
+}
+
+__global__ void __launch_bounds__(kTailThreads) k_na_recover(DMesh d, int nb_nodes, int nb_elems,
+                                                            const double* __restrict__ points,
+                                                            const int* __restrict__ tris,
+                                                            const double* __restrict__ solut, double2* grad,
+                                                            MetricWs ws, double* partial, double target,
+                                                            double scale_exp, double eig_min, double eig_max,
+                                                            double* __restrict__ out) {
+  __shared__ int s_buf[kTailThreads / 32][TRN_MAX_PATCH];
+  __shared__ double s_tree[kTailThreads / kNaPart][kNaPart];
+  const int tid = trn_tid(), stride = trn_grid_stride(), half = threadIdx.x / kNaPart, t = threadIdx.x % kNaPart;
+  if (tid == 0) {
+    *d.err = 0;
+    *ws.rest_n = 0;
+  }
+  for (int v = tid; v < nb_nodes; v += stride) {
+    d.pts[v] = make_double2(points[2 * v], points[2 * v + 1]);
+    d.deg[v] = d.vdeg[v] = 0;
+    d.alive[v] = 1;
+  }
+  cluster_sync();
+  for (int i = tid; i < nb_elems; i += stride) {
+    const int a = tris[3 * i], b = tris[3 * i + 1], c = tris[3 * i + 2];
+    const bool ok = a >= 0 && a < nb_nodes && b >= 0 && b < nb_nodes && c >= 0 && c < nb_nodes;
+    if (!ok) atomicExch(d.err, TRN_DERR_INVALID);   /* before an overfull vertex, whichever is met first */
+    d.tri[i] = ok ? make_int4(a, b, c, 0) : make_int4(-1, -1, -1, 0);
+    if (!ok) continue;
+    trn_stenc_append(d, a, i);
+    trn_stenc_append(d, b, i);
+    trn_stenc_append(d, c, i);
+  }
+  cluster_sync();
+  if (!tail_failed(d)) {
+    for (int v = tid; v < nb_nodes; v += stride) {
+      const TrnRow row = trn_row(d.stenc, d, v);
+      const int n = trn_deg(d, v);
+      if (n <= kRowChunk) {
+        int r[kRowChunk];
+#pragma unroll
+        for (int k = 0; k < kRowChunk; ++k) r[k] = k < n ? row.p[k] : kNoId;
+        patch_sort8(r);
+#pragma unroll
+        for (int k = 0; k < kRowChunk; ++k)
+          if (k < n) row.p[k] = r[k];
+      } else {
+        int r[TRN_NOALLOC_BUCKET];
+        for (int k = 0; k < n; ++k) r[k] = row[k];
+        trn_isort(r, n);
+        for (int k = 0; k < n; ++k) row[k] = r[k];
+      }
+      build_one_vicin(d, v);   /* its own stencil and the elements alone */
     }
-    tri4[i] = make_int4(a, b, c, 0);
+    for (int i = tid; i < nb_elems; i += stride) ws.rec[i] = elem_gradient(d, i, solut);
+  }
+  cluster_sync();
+  const GradSum gsum{ws.rec, grad, ws.atot};
+  const HessSum hsum{ws.rec, ws.atot, scale_exp, nullptr, nullptr};
+  const bool go = !tail_failed(d);
+  if (go)
+    for (int v = tid; v < nb_nodes; v += stride)
+      if (!patch_sum_regs<GradSum, 4>(d, v, gsum)) trn_append(ws.rest, ws.rest_n, v);
+  cluster_sync();
+  const int nr = *ws.rest_n;
+  for (int q = tid >> 5; q < nr; q += stride >> 5)
+    patch_sum_warp(d, ws.rest[q], gsum, s_buf[threadIdx.x >> 5]);
+  cluster_sync();
+  if (go)
+    for (int i = tid; i < nb_elems; i += stride) ws.rec[i] = elem_hessian(d, i, grad);
+  cluster_sync();
+  if (go)
+    for (int v = tid; v < nb_nodes; v += stride) patch_sum_regs<HessSum, 4>(d, v, hsum);
+  for (int q = tid >> 5; q < nr; q += stride >> 5)
+    patch_sum_warp(d, ws.rest[q], hsum, s_buf[threadIdx.x >> 5]);
+  cluster_sync();
+  /* one partial per 256 elements by each half of a block, the same number of
+   * steps for all of them */
+  const int parts = (nb_elems + kNaPart - 1) / kNaPart, halves = stride / kNaPart;
+  for (int b0 = 0; b0 < parts; b0 += halves) {
+    const int b = b0 + tid / kNaPart, i = b * kNaPart + t;
+    const double s = na_tree(s_tree[half], go && b < parts && i < nb_elems ? 0 + complexity_term(d, i) : 0.0, t);
+    if (t == 0 && b < parts) partial[b] = s;
+  }
+  cluster_sync();
+  const double complexity = na_tree(s_tree[half], t < parts ? 0 + partial[t] : 0.0, t);
+  if (tail_failed(d)) return;
+  const double fact = target / complexity;
+  for (int v = tid; v < nb_nodes; v += stride) {
+    const double4 r = normalize_tensor(d.ten[v], fact, eig_min, eig_max);
+    out[3 * v] = r.x;
+    out[3 * v + 1] = r.y;
+    out[3 * v + 2] = r.z;
   }
 }
 
-__global__ void k_na_points(const double* __restrict__ pts, int nb_nodes, double2* __restrict__ out) {
-  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride())
-    out[v] = make_double2(pts[2 * v], pts[2 * v + 1]);
-}
-
-__global__ void k_na_tensor(const double4* __restrict__ ten, int nb_nodes, double* __restrict__ out) {
-  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    double4 t = ten[v];
-    out[3 * v] = t.x;
-    out[3 * v + 1] = t.y;
-    out[3 * v + 2] = t.z;
-  }
-}
+static_assert(kMaxE <= (size_t) kNaPart * kNaPart, "one tree over the partials");
 
 }  // namespace
 }  // namespace trn
@@ -167,22 +253,6 @@ extern "C" int trn_metric_noalloc(int nb_nodes, int nb_elems, const double* d_po
   d.capa_elem = nb_elems;
   double2* grad = reinterpret_cast<double2*>(base + oGrad);
   double* terms = reinterpret_cast<double*>(base + oTerms);
-  double* cplx = reinterpret_cast<double*>(base + oCplx);
-
-  /* what must start empty: degrees and the error word (rows are read up to
-   * their counts) */
-  if (cudaMemsetAsync(d.err, 0, sizeof(int), s) != cudaSuccess ||
-      cudaMemsetAsync(d.deg, 0, sizeof(int) * (size_t) nb_nodes, s) != cudaSuccess ||
-      cudaMemsetAsync(d.vdeg, 0, sizeof(int) * (size_t) nb_nodes, s) != cudaSuccess ||
-      cudaMemsetAsync(d.alive, 1, (size_t) nb_nodes, s) != cudaSuccess)
-    return TRN_ERR_CUDA;
-
-  const int gv = grid_for(nb_nodes), ge = grid_for(nb_elems);
-  k_na_expand<<<ge, TRN_THREADS, 0, s>>>(d_tris, nb_elems, nb_nodes, d.tri, d.err);
-  k_na_points<<<gv, TRN_THREADS, 0, s>>>(d_points, nb_nodes, d.pts);
-  k_fill_stencils<<<ge, TRN_THREADS, 0, s>>>(d, nb_elems);
-  k_sort_stencils<<<gv, TRN_THREADS, 0, s>>>(d, nb_nodes);
-  k_build_vicin<<<gv, TRN_THREADS, 0, s>>>(d, nb_nodes, 0);
 
   const double target = (double) (int) std::floor(nb_nodes * target_factor);
   const double scale_exp = lp_norm ? -1. / (2 * lp_norm + 2) : 0.5;
@@ -190,11 +260,9 @@ extern "C" int trn_metric_noalloc(int nb_nodes, int nb_elems, const double* d_po
   const double eig_max = 1 / trn_pow(h_max, 2);
   int* rest = reinterpret_cast<int*>(base + oRest);
   const MetricWs ws{reinterpret_cast<double4*>(base + oRec), reinterpret_cast<double*>(base + oAtot), rest + 1, rest};
-  metric_patches(d, nb_nodes, nb_elems, d_solut, grad, ws, scale_exp, s);
-  metric_complexity(d, nb_elems, nullptr, terms, cplx, false, s);
-  k_normalize<<<gv, TRN_THREADS, 0, s>>>(d, nb_nodes, cplx, target, eig_min, eig_max);
-  k_na_tensor<<<gv, TRN_THREADS, 0, s>>>(d.ten, nb_nodes, d_tensor);
-  if (cudaPeekAtLastError() != cudaSuccess) return TRN_ERR_CUDA;
+  if (!cluster_launch<k_na_recover>(s, d, nb_nodes, nb_elems, d_points, d_tris, d_solut, grad, ws, terms, target,
+                                    scale_exp, eig_min, eig_max, d_tensor))
+    return TRN_ERR_CUDA;
 
   int err = 0;
   if (cudaMemcpyAsync(&err, d.err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
