@@ -616,6 +616,28 @@ void smooth_pre(const DMesh& m, int nb_nodes, cudaStream_t s) {
   check_launch("smooth_pre");
 }
 
+/* The default shape (2 lanes, the sweep at 128 registers) stands for a choice
+ * by the class's length and the form. A vertex is a chain of gathers and
+ * arithmetic: a class too short to fill the chip takes as long as one chain,
+ * which more lanes shorten; a long one is bound by issue, which the lanes'
+ * shared part (the new tensor) then repeats. Two passes over the classes, ms,
+ * by live vertices (a class is a quarter of them at most):
+ *   FP64   8 lanes   4 lanes   2 lanes      FP32   8, sweep  8, in turn  2, sweep
+ *   10 k   0.42      0.52      0.69         10 k   0.37      0.40        0.57
+ *   103 k  0.72      0.76      0.90         103 k  0.58      0.59        0.74
+ *   187 k  0.98      0.96      1.08         187 k  0.73      0.72        0.89
+ *   294 k  1.35      1.26      1.29         294 k  0.96      0.90        1.03
+ *   578 k  2.39      2.12      2.06         578 k  1.67      1.48        1.63 */
+static void smooth_shape(int n, bool fp32, int* lanes, int* regs) {
+  if (fp32) {
+    *lanes = 8;
+    *regs = n <= 32768 ? 5 : 2;
+  } else if (n <= 65536) {
+    *lanes = n <= 32768 ? 8 : 4;
+    *regs = n <= 8192 ? 7 : (n <= 32768 ? 5 : 7);
+  }
+}
+
 static void smooth_launch(const DMesh& m, const int* list, int n, const int* off, int c, int hint,
                           int* counters, bool fp32, cudaStream_t s) {
   /* per moved vertex: list id, flag, counts, own point/tensor read+write,
@@ -627,9 +649,9 @@ static void smooth_launch(const DMesh& m, const int* list, int n, const int* off
   ByteCount bc;
   ProfScope ps("smooth_move", s, n * own + nbr, &bc);
   const int t = tune().smooth_threads;
-  const int lanes = tune().smooth_lanes;
+  int lanes = tune().smooth_lanes, regs = tune().smooth_regs;
+  if (lanes == 2 && regs == 7) smooth_shape(hint, fp32, &lanes, &regs);
   const int g = grid_for((long long) hint * lanes, t);
-  const int regs = tune().smooth_regs;
   if (lanes == 8 || lanes == 4 || lanes == 2) {
     /* smooth_regs 0, 1, 2 (and 3): the tries in turn, registers capped for
      * two, three, four 256-thread blocks an SM; 4, 5 (and 8), 6 (and 7): the
