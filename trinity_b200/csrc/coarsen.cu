@@ -610,47 +610,6 @@ __global__ void __launch_bounds__(TRN_THREADS) k_collapse(DMesh m, const int* __
 
 /* ---- the levels of a short list in one launch (trn_level.cuh) ---- */
 
-/* one candidate of the independent set, kept in registers over the rounds:
- * its neighbours, of which a round reads the states (in flight together; the
- * rule is mis_item's of heuristics.cu) */
-struct TailCand {
-  int v = -1, nv = 0;
-  int w[kRowChunk];
-  uint8_t st = 0;
-
-  __device__ __forceinline__ void load(const DMesh& m, int id) {
-    v = id;
-    st = 1;   /* the filter marks every candidate undecided */
-    nv = m.vdeg[v];
-    const int* row = trn_row(m.vic, m, v).p;
-#pragma unroll
-    for (int j = 0; j < kRowChunk; ++j) w[j] = j < nv ? row[j] : -1;
-  }
-  __device__ __forceinline__ void round(const DMesh& m, const uint8_t* in, uint8_t* out, uint64_t seed) {
-    if (st == 1) {
-      const uint64_t pv = trn_prio(seed, v);
-      bool is_max = true, leave = false;
-      uint8_t sw[kRowChunk];
-#pragma unroll
-      for (int j = 0; j < kRowChunk; ++j) sw[j] = w[j] >= 0 ? in[w[j]] : 0;
-#pragma unroll
-      for (int j = 0; j < kRowChunk; ++j) {
-        leave |= sw[j] == 2;
-        if (sw[j] == 1 && trn_prio(seed, w[j]) > pv) is_max = false;
-      }
-      const TrnRow vc = trn_row(m.vic, m, v);
-      for (int b = kRowChunk; b < nv; ++b) {
-        const int x = vc[b];
-        const uint8_t s = in[x];
-        leave |= s == 2;
-        if (s == 1 && trn_prio(seed, x) > pv) is_max = false;
-      }
-      st = leave ? 0 : (is_max ? 2 : 1);
-    }
-    out[v] = st;
-  }
-};
-
 constexpr int kMaxMisRounds = 8;
 
 template <bool F32>
@@ -679,7 +638,7 @@ __global__ void __launch_bounds__(kTailThreads) k_coarsen_tail(DMesh m, int* act
      * rounds after that would only copy the states) */
     const int nc = status[S_NTASK];
     const uint64_t base = trn_seed(sd);
-    TailCand mine;
+    MisCand mine;
     if (tid < nc) mine.load(m, cand[tid]);
     int r = 0;
     while (r < rounds) {
@@ -692,7 +651,7 @@ __global__ void __launch_bounds__(kTailThreads) k_coarsen_tail(DMesh m, int* act
         wait = mine.st == 1;
       }
       for (int q = tid + stride; q < nc; q += stride) {   /* more candidates than threads */
-        TailCand c;
+        MisCand c;
         c.load(m, cand[q]);
         c.st = in[c.v];
         c.round(m, in, out, seed);

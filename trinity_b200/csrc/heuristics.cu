@@ -94,9 +94,12 @@ __device__ __forceinline__ bool grid_sync(GridBar* b, int* mesh_err, long long m
  * barrier that gave up keeps its arrivals and failure mark) */
 static GridBar* grid_bar(HeurWs& ws, cudaStream_t s) {
   GridBar* b = reinterpret_cast<GridBar*>(ws.cnt + 100);
-  cudaMemsetAsync(b, 0, sizeof(GridBar), s);
+  cudaMemsetAsync(b, 0, sizeof(int) * 20, s);   /* and the words of mis_open after it */
   return b;
 }
+
+/* one word per independent-set round: a candidate was left undecided */
+static int* mis_open(HeurWs& ws) { return ws.cnt + 112; }
 
 /* A cooperative launch whose first block never reaches the barrier: the
  * others wait max_polls polls, give up and mark the error word (the bounded
@@ -219,27 +222,49 @@ __global__ void __launch_bounds__(kFusedThreads) k_mis_fused(DMesh m, uint8_t* s
   for (int q = threadIdx.x; q < n; q += blockDim.x) mis_finish_item(m, state, other, cand[q], indep, nindep);
 }
 
-/* all the rounds and the collection in one cooperative launch (stopping
- * the rounds once no candidate is undecided was measured slower: the
- * undecided flag's reduction costs more on the long levels than the rounds
- * it saves on the short ones) */
+/* all the rounds and the collection in one cooperative launch, until no
+ * candidate is undecided (the rounds after that would only copy the states):
+ * a block that has one left says so by a plain store before the round's
+ * barrier. A thread's first candidate stays in registers over the rounds; only
+ * lists longer than the grid read the others again. */
 __global__ void __launch_bounds__(kFusedThreads) k_mis_persist(DMesh m, uint8_t* s0, uint8_t* s1,
-                                                               const int* __restrict__ cand, const int* count,
+                                                               const int* cand, const int* count,
                                                                Seed sd, int rounds, int* indep, int* nindep,
-                                                               GridBar* bar) {
+                                                               GridBar* bar, int* open) {
   if (trn_failed_block(m)) return;
   const int n = *count;
   if (trn_tid() == 0) *nindep = 0;
   const uint64_t base = trn_seed(sd);
-  for (int r = 0; r < rounds; ++r) {
+  MisCand mine;
+  if (trn_tid() < n) mine.load(m, cand[trn_tid()]);
+  int r = 0;
+  while (r < rounds) {
     const uint8_t* in = (r & 1) ? s1 : s0;
     uint8_t* out = (r & 1) ? s0 : s1;
     const uint64_t seed = base + 0x9e3779b97f4a7c15ULL * r;
-    for (int q = trn_tid(); q < n; q += trn_grid_stride()) mis_item(m, in, out, cand[q], seed);
+    bool wait = false;
+    if (mine.v >= 0) {
+      mine.round(m, in, out, seed);
+      wait = mine.st == 1;
+    }
+    for (int q = trn_tid() + trn_grid_stride(); q < n; q += trn_grid_stride()) {
+      const int v = cand[q];
+      const uint8_t st = in[v];
+      if (st != 1) {
+        out[v] = st;
+        continue;
+      }
+      MisCand c;
+      c.load(m, v);
+      c.round(m, in, out, seed);
+      wait |= c.st == 1;
+    }
+    if (__syncthreads_or(wait) && threadIdx.x == 0) open[r] = 1;
     if (!grid_sync(bar, m.err)) return;
+    if (!*(volatile int*) (open + r++)) break;
   }
-  uint8_t* state = (rounds & 1) ? s1 : s0;
-  uint8_t* other = (rounds & 1) ? s0 : s1;
+  uint8_t* state = (r & 1) ? s1 : s0;
+  uint8_t* other = (r & 1) ? s0 : s1;
   for (int q = trn_tid(); q < n; q += trn_grid_stride()) mis_finish_item(m, state, other, cand[q], indep, nindep);
 }
 
@@ -249,7 +274,7 @@ void mis_jp_rounds(const DMesh& m, const int* cand, const int* count, int rounds
   uint8_t* buf[2] = {ws.state, ws.state2};
   if (bound > kFusedThreads &&
       coop_launch(k_mis_persist, bound, kFusedThreads, s, m, buf[0], buf[1], cand, count, sd, rounds, indep,
-                  nindep, grid_bar(ws, s))) {
+                  nindep, grid_bar(ws, s), mis_open(ws))) {
     check_launch("mis_jp_rounds");
     return;
   }
@@ -443,55 +468,18 @@ __global__ void __launch_bounds__(kFusedThreads) k_greedy_tail(GreedyArgs a, con
   }
 }
 
-/* the matching of a level in one cooperative launch: with `whole`, the
- * first proposals (the dual filter reset the elements' state), then rounds
- * until no row waits (at most
- * kGreedyRounds); else the rounds from the first one the grid launches did
- * not run. Once kGreedyTail rows or fewer wait, the first block finishes the
- * rounds alone, separated by block barriers, and the others return: a grid
- * barrier costs more than such a round. */
-__global__ void __launch_bounds__(kFusedThreads) k_greedy_persist(GreedyArgs a, const int* ntasks_dev,
-                                                                  int* pairs, int* npairs, GridBar* bar,
-                                                                  int* err, int whole) {
+/* the matching of a level, or with `rest` its rounds after the grid
+ * launches', by one cluster */
+__global__ void __launch_bounds__(kTailThreads) k_greedy_cluster(GreedyArgs a, const int* ntasks_dev, int* pairs,
+                                                                int* npairs, int rest) {
   const int ntasks = *ntasks_dev;
-  int r0 = 0;
-  if (whole) {
-    if (trn_tid() == 0) {
-      *npairs = 0;
-      a.cnt[0] = ntasks;
-      a.cnt[1] = 0;
-      a.cnt[2] = 0;
-    }
-    for (int i = trn_tid(); i < ntasks; i += trn_grid_stride()) {
-      greedy_propose(a, 0, i);
-      a.list0[i] = i;
-    }
-    if (!grid_sync(bar, err)) return;
-  } else {
+  int r0 = -1;
+  if (rest) {
+    r0 = 0;
     while (r0 < kGreedyRounds && a.ran[r0]) ++r0;
+    if (r0 >= kGreedyRounds) return;
   }
-  bool alone = false;
-  for (int r = r0; r < kGreedyRounds; ++r) {
-    const int n = *(volatile int*) (a.cnt + r % 3);
-    if (n == 0) break;
-    if (!alone && n <= kGreedyTail) {
-      if (blockIdx.x != 0) return;
-      alone = true;
-    }
-    const int* in = (r & 1) ? a.list1 : a.list0;
-    int* out = (r & 1) ? a.list0 : a.list1;
-    const int b0 = alone ? 0 : (int) (blockIdx.x * blockDim.x);
-    const int bs = alone ? (int) blockDim.x : trn_grid_stride();
-    if (b0 == 0 && threadIdx.x == 0) a.cnt[(r + 2) % 3] = 0;
-    for (int base = b0; base < n; base += bs) {
-      const int q = base + threadIdx.x;
-      const int i = q < n ? in[q] : -1;
-      const bool wait = q < n && greedy_item(a, ntasks, r, i, pairs, npairs);
-      trn_block_append(out, a.cnt + (r + 1) % 3, i, wait);
-    }
-    if (alone) __syncthreads();
-    else if (!grid_sync(bar, err)) return;
-  }
+  greedy_cluster(a, ntasks, r0, pairs, npairs);
 }
 
 void match_greedy(const DMesh& m, int nb_elems, const int* dual, const int* dual_n, const int* ntasks,
@@ -506,10 +494,14 @@ void match_greedy(const DMesh& m, int nb_elems, const int* dual, const int* dual
     check_launch("match_greedy");
     return;
   }
-  if (bound >= 0 && bound <= kGreedyGrid &&
-      coop_launch(k_greedy_persist, bound, kFusedThreads, s, a, ntasks, pairs, npairs, grid_bar(ws, s), m.err, 1)) {
-    check_launch("match_greedy");
-    return;
+  cudaStreamCaptureStatus cs;
+  const bool live = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+  if (live && bound >= 0 && bound <= kGreedyGrid) {
+    cudaMemsetAsync(npairs, 0, sizeof(int), s);
+    if (cluster_launch<k_greedy_cluster>(s, a, ntasks, pairs, npairs, 0)) {
+      check_launch("match_greedy");
+      return;
+    }
   }
   /* grid rounds, each a launch that returns at once when few rows wait:
    * about two per halving of the list bound down to kGreedyTail rows (on
@@ -528,8 +520,8 @@ void match_greedy(const DMesh& m, int nb_elems, const int* dual, const int* dual
   k_greedy_start<<<g, TRN_THREADS, 0, s>>>(a, ntasks, min_n);
   note_launch();
   /* a long list known: grid launches while more than kGreedyGrid rows wait,
-   * then the cooperative rounds */
-  const bool coop = bound > kGreedyGrid;
+   * then the cluster's rounds */
+  const bool coop = live && bound > kGreedyGrid;
   if (coop) {
     rounds = 0;
     for (long long n = bound; n > kGreedyGrid; n /= 2) rounds += 3;
@@ -539,8 +531,7 @@ void match_greedy(const DMesh& m, int nb_elems, const int* dual, const int* dual
     k_greedy_round<<<TRN_RESIDENT(k_greedy_round, g, TRN_THREADS), TRN_THREADS, 0, s>>>(a, ntasks, r, pairs, npairs, coop ? kGreedyGrid + 1 : 0);
     note_launch();
   }
-  if (coop && coop_launch(k_greedy_persist, bound, kFusedThreads, s, a, ntasks, pairs, npairs, grid_bar(ws, s),
-                          m.err, 0)) {
+  if (coop && cluster_launch<k_greedy_cluster>(s, a, ntasks, pairs, npairs, 1)) {
     check_launch("match_greedy");
     return;
   }

@@ -66,6 +66,18 @@ __global__ void k_swap_filter(DMesh m, int nb_elems, uint8_t* __restrict__ flag)
   }
 }
 
+/* entries base .. base + 7 of a stencil of d, and their elements; t = -1 past
+ * the end */
+__device__ __forceinline__ void row_chunk(const DMesh& m, const TrnRow& s, int base, int d, int* t, int4* v) {
+  const int4* p = reinterpret_cast<const int4*>(s.p + (size_t) (base / kRowChunk) * s.plane);
+  const int4 a = p[0], b = d - base > 4 ? p[1] : make_int4(-1, -1, -1, -1);
+  const int e[kRowChunk] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int j = 0; j < kRowChunk; ++j) t[j] = base + j < d ? e[j] : -1;
+#pragma unroll
+  for (int j = 0; j < kRowChunk; ++j) v[j] = t[j] >= 0 ? m.tri[t[j]] : make_int4(-1, -1, -1, 0);
+}
+
 /* the dual row of candidate k at row index i; returns its length */
 __device__ __forceinline__ int dual_row(const DMesh& m, int k, int i, int* __restrict__ dual,
                                         int* __restrict__ dual_n, int* __restrict__ map) {
@@ -73,27 +85,42 @@ __device__ __forceinline__ int dual_row(const DMesh& m, int k, int i, int* __res
     const int4 n = m.tri[k];
     int row[4] = {k, -1, -1, -1};
     int dn = 1;
-    const TrnRow s0 = trn_row(m.stenc, m, n.x);
-    const int d0 = trn_deg(m, n.x);
-    for (int a = 0; dn < 3 && a < d0; ++a) {
-      int t = s0[a];
-      if (t == k) continue;
-      int4 v = m.tri[t];
-      if ((v.x == n.x && v.y == n.z) || (v.x == n.y && v.y == n.x) ||
-          (v.y == n.x && v.z == n.z) || (v.y == n.y && v.z == n.x) ||
-          (v.z == n.x && v.x == n.z) || (v.z == n.y && v.x == n.x))
-        row[dn++] = t;
+    /* the neighbours at the first vertex, in its stencil's order, then the
+     * one across the opposite edge; a stencil's elements are loaded 8 at a
+     * time, before any is looked at */
+    const TrnRow s0 = trn_row(m.stenc, m, n.x), s2 = trn_row(m.stenc, m, n.z);
+    const int d0 = trn_deg(m, n.x), d2 = trn_deg(m, n.z);
+    for (int base = 0; dn < 3 && base < d0; base += kRowChunk) {
+      int t[kRowChunk];
+      int4 v[kRowChunk];
+      row_chunk(m, s0, base, d0, t, v);
+#pragma unroll
+      for (int j = 0; j < kRowChunk; ++j)
+        if (dn < 3 && t[j] >= 0 && t[j] != k &&
+            ((v[j].x == n.x && v[j].y == n.z) || (v[j].x == n.y && v[j].y == n.x) ||
+             (v[j].y == n.x && v[j].z == n.z) || (v[j].y == n.y && v[j].z == n.x) ||
+             (v[j].z == n.x && v[j].x == n.z) || (v[j].z == n.y && v[j].x == n.x))) {
+          if (dn == 1) row[1] = t[j];
+          else row[2] = t[j];
+          ++dn;
+        }
     }
-    const TrnRow s2 = trn_row(m.stenc, m, n.z);
-    const int d2 = trn_deg(m, n.z);
-    for (int a = 0; a < d2; ++a) {
-      int t = s2[a];
-      if (t == k) continue;
-      int4 v = m.tri[t];
-      if ((v.x == n.z && v.y == n.y) || (v.y == n.z && v.z == n.y) || (v.z == n.z && v.x == n.y)) {
-        row[dn++] = t;
-        break;
-      }
+    bool across = false;
+    for (int base = 0; !across && base < d2; base += kRowChunk) {
+      int t[kRowChunk];
+      int4 v[kRowChunk];
+      row_chunk(m, s2, base, d2, t, v);
+#pragma unroll
+      for (int j = 0; j < kRowChunk; ++j)
+        if (!across && t[j] >= 0 && t[j] != k &&
+            ((v[j].x == n.z && v[j].y == n.y) || (v[j].y == n.z && v[j].z == n.y) ||
+             (v[j].z == n.z && v[j].x == n.y))) {
+          if (dn == 1) row[1] = t[j];
+          else if (dn == 2) row[2] = t[j];
+          else row[3] = t[j];
+          ++dn;
+          across = true;
+        }
     }
     reinterpret_cast<int4*>(dual)[i] = make_int4(row[0], row[1], row[2], row[3]);
     dual_n[i] = dn;
@@ -380,66 +407,6 @@ __device__ __forceinline__ int flip_group(const DMesh& m, int id1, int id2, cons
   return gl == 0 ? 2 : 0;
 }
 
-/* a dual row of the greedy matching, kept in registers over the rounds (the
- * rule is greedy_item's, trn_match.cuh): a round costs its four keys and, once
- * the row is first on all of them, its four elements' states */
-struct TailRow {
-  int4 row = make_int4(-1, -1, -1, -1);
-  int dn = 0;
-  unsigned rows = 0;   /* bit q: element q has a row itself */
-  bool open = false;
-
-  __device__ __forceinline__ int at(int q) const { return q == 0 ? row.x : (q == 1 ? row.y : (q == 2 ? row.z : row.w)); }
-  __device__ __forceinline__ void load(const GreedyArgs& a, int i) {
-    row = reinterpret_cast<const int4*>(a.dual)[i];
-    dn = a.dual_n[i];
-#pragma unroll
-    for (int q = 1; q < 4; ++q)
-      if (q < dn && a.map[at(q)] >= 0) rows |= 1u << q;
-    open = true;
-  }
-  __device__ __forceinline__ void propose(const GreedyArgs& a, int r) const {
-    unsigned long long* mk = (r & 1) ? a.mk1 : a.mk0;
-    const unsigned long long key = greedy_key(r, row.x);
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (q < dn) atomicMin(mk + at(q), key);
-  }
-  __device__ __forceinline__ void round(const GreedyArgs& a, int r, int* pairs, int* npairs) {
-    const unsigned long long* mk = (r & 1) ? a.mk1 : a.mk0;
-    const unsigned long long key = greedy_key(r, row.x);
-    bool ready = true;
-    unsigned free = 0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (q < dn) {
-        ready &= mk[at(q)] == key;
-        if (a.vis[at(q)] == -1) free |= 1u << q;
-      }
-    if (!ready) {
-      propose(a, r + 1);
-      return;
-    }
-    open = false;
-    if (!(free & 1u)) return;
-    a.vis[row.x] = 1;
-    int partner = -1;
-    bool done = false;
-#pragma unroll
-    for (int q = 1; q < 4; ++q)
-      if (!done && ((free >> q) & 1u)) {
-        a.vis[at(q)] = 1;
-        partner = at(q);
-        done = (rows >> q) & 1u;
-      }
-    if (partner >= 0) {
-      const int p = trn_warp_reserve(npairs);
-      pairs[2 * p] = row.x;
-      pairs[2 * p + 1] = partner;
-    }
-  }
-};
-
 template <bool F32>
 __global__ void __launch_bounds__(kTailThreads) k_swap_tail(DMesh m, int* act0, int* act1, int* status, int* dual,
                                                             int* dual_n, int* map, uint32_t* rank, GreedyArgs ga,
@@ -455,49 +422,13 @@ __global__ void __launch_bounds__(kTailThreads) k_swap_tail(DMesh m, int* act0, 
     if (tid == 0) {
       trn_level_clear(m, status + S_COMMIT);
       *npairs = 0;
-      ga.cnt[1] = ga.cnt[2] = 0;
     }
     for (int q = tid; q < na; q += stride)
       filter_dual_item<F32>(m, act[q], dual, dual_n, map, rank, status + S_NTASK, gr);
     cluster_sync();
     const int ntasks = status[S_NTASK];
-    if (greedy && ntasks <= stride) {
-      TailRow mine;
-      if (tid < ntasks) {
-        mine.load(ga, tid);
-        mine.propose(ga, 0);
-      }
-      cluster_sync();
-      for (int r = 0; r < kGreedyRounds; ++r) {
-        /* rows undecided before this round (round 0: all); the word of the
-         * round after next starts at zero */
-        if (r > 0 && tail_word(ga.cnt + r % 3) == 0) break;
-        if (tid == 0) ga.cnt[(r + 2) % 3] = 0;
-        if (mine.open) {
-          mine.round(ga, r, pairs, npairs);
-          if (mine.open) ga.cnt[(r + 1) % 3] = 1;
-        }
-        cluster_sync();
-      }
-    } else if (greedy) {
-      if (tid == 0) ga.cnt[0] = ntasks;
-      for (int i = tid; i < ntasks; i += stride) {
-        greedy_propose(ga, 0, i);
-        ga.list0[i] = i;
-      }
-      cluster_sync();
-      for (int r = 0; r < kGreedyRounds; ++r) {
-        const int n = tail_word(ga.cnt + r % 3);
-        if (n == 0) break;
-        const int* in = (r & 1) ? ga.list1 : ga.list0;
-        int* out = (r & 1) ? ga.list0 : ga.list1;
-        if (tid == 0) ga.cnt[(r + 2) % 3] = 0;
-        for (int q = tid; q < n; q += stride) {
-          const int i = in[q];
-          if (greedy_item(ga, ntasks, r, i, pairs, npairs)) trn_append(out, ga.cnt + (r + 1) % 3, i);
-        }
-        cluster_sync();
-      }
+    if (greedy) {
+      greedy_cluster(ga, ntasks, -1, pairs, npairs);
     } else {
       const uint64_t seed = trn_seed(sd);
       for (int i = tid; i < ntasks; i += stride) match_reset_item(ma, i);

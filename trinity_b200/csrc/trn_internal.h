@@ -342,9 +342,9 @@ int* color_cont(HeurWs& ws);
  * statistics end up in status as after the last level. For lists of at most
  * kCoarsenTail vertices (eight lanes each: four passes of the cluster's 8,192
  * threads; at 2,048 the 100 x 100 workload's coarsening takes 3.0 ms instead
- * of 2.6) or kSwapTail elements (a thread each) and streams that are not being
+ * of 2.6) or kSwapTail elements (up to three a thread) and streams that are not being
  * captured; false when it could not launch. */
-constexpr int kCoarsenTail = 4096, kSwapTail = 8192;
+constexpr int kCoarsenTail = 4096, kSwapTail = 24576;
 bool coarsen_tail(const DMesh& m, int* act0, int* act1, int* status, int* target, int* cand, HeurWs& ws, int* indep,
                   Seed sd, int rounds, int cap, bool fp32, cudaStream_t s);
 bool swap_tail(const DMesh& m, int* act0, int* act1, int* status, int* dual, int* dual_n, int* map, uint32_t* rank,

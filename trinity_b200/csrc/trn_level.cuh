@@ -25,7 +25,14 @@ __device__ __forceinline__ void fix_stencil(const DMesh& m, int v, int* buf) {
   if (d <= kFixRegs) {
     int r[kFixRegs];
 #pragma unroll
-    for (int a = 0; a < kFixRegs; ++a) r[a] = (a < d) ? s[a] : -1;
+    for (int c = 0; c < kFixRegs / 4; ++c) {   /* a chunk of the row is two vector loads */
+      const int4 x = 4 * c < d ? *reinterpret_cast<const int4*>(s.p + (size_t) (c / 2) * s.plane + 4 * (c & 1))
+                               : make_int4(-1, -1, -1, -1);
+      r[4 * c] = 4 * c < d ? x.x : -1;
+      r[4 * c + 1] = 4 * c + 1 < d ? x.y : -1;
+      r[4 * c + 2] = 4 * c + 2 < d ? x.z : -1;
+      r[4 * c + 3] = 4 * c + 3 < d ? x.w : -1;
+    }
 #pragma unroll
     for (int a = 0; a < kFixRegs; ++a) {
       int keep = 0x7fffffff;
@@ -137,6 +144,47 @@ __device__ __forceinline__ void tail_fix(const DMesh& m, int tid, int stride, in
     fix_stencil_group(m, v, gm, buf);
   }
 }
+
+/* one candidate of the independent set, kept in registers over the rounds:
+ * its neighbours, of which a round reads the states (in flight together; the
+ * rule is mis_item's of heuristics.cu) */
+struct MisCand {
+  int v = -1, nv = 0;
+  int w[kRowChunk];
+  uint8_t st = 0;
+
+  __device__ __forceinline__ void load(const DMesh& m, int id) {
+    v = id;
+    st = 1;   /* the filter marks every candidate undecided */
+    nv = m.vdeg[v];
+    const int* row = trn_row(m.vic, m, v).p;
+#pragma unroll
+    for (int j = 0; j < kRowChunk; ++j) w[j] = j < nv ? row[j] : -1;
+  }
+  __device__ __forceinline__ void round(const DMesh& m, const uint8_t* in, uint8_t* out, uint64_t seed) {
+    if (st == 1) {
+      const uint64_t pv = trn_prio(seed, v);
+      bool is_max = true, leave = false;
+      uint8_t sw[kRowChunk];
+#pragma unroll
+      for (int j = 0; j < kRowChunk; ++j) sw[j] = w[j] >= 0 ? in[w[j]] : 0;
+#pragma unroll
+      for (int j = 0; j < kRowChunk; ++j) {
+        leave |= sw[j] == 2;
+        if (sw[j] == 1 && trn_prio(seed, w[j]) > pv) is_max = false;
+      }
+      const TrnRow vc = trn_row(m.vic, m, v);
+      for (int b = kRowChunk; b < nv; ++b) {
+        const int x = vc[b];
+        const uint8_t s = in[x];
+        leave |= s == 2;
+        if (s == 1 && trn_prio(seed, x) > pv) is_max = false;
+      }
+      st = leave ? 0 : (is_max ? 2 : 1);
+    }
+    out[v] = st;
+  }
+};
 
 /* ---- the level loop of short lists ----
  * A level is five steps with a dependence between each (filter, the

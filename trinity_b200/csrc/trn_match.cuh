@@ -7,6 +7,7 @@
 #define TRN_MATCH_CUH
 
 #include "trn_internal.h"
+#include "trn_level.cuh"
 
 namespace trn {
 
@@ -154,8 +155,10 @@ __device__ __forceinline__ void match_clear_item(const MatchArgs& a, int i) {
  * more pairs, is a point and a half off. */
 constexpr int kGreedyRounds = 64;
 constexpr int kGreedyTail = 2048;   /* undecided rows left to the one-block rounds */
-/* rows waiting above which a round runs as its own grid launch (measured:
- * such rounds are faster launched than inside the cooperative kernel) */
+/* rows waiting above which a round runs as its own grid launch: what the
+ * threads of a cluster keep in registers (greedy_cluster). Matching of the
+ * 2M-triangle workload's three rounds 3.80 ms with a cooperative grid for the
+ * rounds after that, 3.22 ms with the cluster. */
 constexpr int kGreedyGrid = 1 << 15;
 
 struct GreedyArgs {
@@ -238,6 +241,136 @@ __device__ __forceinline__ bool greedy_item(const GreedyArgs& a, int ntasks, int
   return greedy_act(a, ntasks, r, i, greedy_ready(a, r, i), pairs, npairs);
 }
 
+
+/* a dual row of the greedy matching, kept in registers over the rounds (the
+ * rule is greedy_item's, trn_match.cuh): a round costs its four keys and, once
+ * the row is first on all of them, its four elements' states */
+struct TailRow {
+  int4 row = make_int4(-1, -1, -1, -1);
+  int dn = 0;
+  unsigned rows = 0;   /* bit q: element q has a row itself */
+  bool open = false;
+
+  __device__ __forceinline__ int at(int q) const { return q == 0 ? row.x : (q == 1 ? row.y : (q == 2 ? row.z : row.w)); }
+  __device__ __forceinline__ void load(const GreedyArgs& a, int i) {
+    row = reinterpret_cast<const int4*>(a.dual)[i];
+    dn = a.dual_n[i];
+#pragma unroll
+    for (int q = 1; q < 4; ++q)
+      if (q < dn && a.map[at(q)] >= 0) rows |= 1u << q;
+    open = true;
+  }
+  __device__ __forceinline__ void propose(const GreedyArgs& a, int r) const {
+    unsigned long long* mk = (r & 1) ? a.mk1 : a.mk0;
+    const unsigned long long key = greedy_key(r, row.x);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q < dn) atomicMin(mk + at(q), key);
+  }
+  __device__ __forceinline__ void round(const GreedyArgs& a, int r, int* pairs, int* npairs) {
+    const unsigned long long* mk = (r & 1) ? a.mk1 : a.mk0;
+    const unsigned long long key = greedy_key(r, row.x);
+    bool ready = true;
+    unsigned free = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q < dn) {
+        ready &= mk[at(q)] == key;
+        if (a.vis[at(q)] == -1) free |= 1u << q;
+      }
+    if (!ready) {
+      propose(a, r + 1);
+      return;
+    }
+    open = false;
+    if (!(free & 1u)) return;
+    a.vis[row.x] = 1;
+    int partner = -1;
+    bool done = false;
+#pragma unroll
+    for (int q = 1; q < 4; ++q)
+      if (!done && ((free >> q) & 1u)) {
+        a.vis[at(q)] = 1;
+        partner = at(q);
+        done = (rows >> q) & 1u;
+      }
+    if (partner >= 0) {
+      const int p = trn_warp_reserve(npairs);
+      pairs[2 * p] = row.x;
+      pairs[2 * p + 1] = partner;
+    }
+  }
+};
+
+/* The rounds of the greedy matching by one cluster, to the end: with r0 < 0
+ * the whole matching of rows 0 .. ntasks - 1, else from round r0, whose
+ * undecided rows are in its list and have proposed. While more rows wait than
+ * the threads can keep (kClusterRows each) the rounds go over the lists as the
+ * grid's do; then every thread keeps its rows in registers, and a round is
+ * their keys, a few stores and a barrier. All threads of the cluster call it;
+ * it ends after a barrier. */
+constexpr int kClusterRows = 4;
+
+__device__ __forceinline__ void greedy_cluster(const GreedyArgs& a, int ntasks, int r0, int* pairs, int* npairs) {
+  const int tid = trn_tid(), stride = trn_grid_stride();
+  const bool whole = r0 < 0;
+  int* more = a.cnt + 4;   /* [3] rows left open, by round mod 3 */
+  int r = whole ? 0 : r0;
+  int n = whole ? ntasks : tail_word(a.cnt + r % 3);
+  const bool lists = n > kClusterRows * stride;
+  if (tid == 0) {
+    more[0] = more[1] = more[2] = 0;
+    if (whole) a.cnt[1] = a.cnt[2] = 0;
+  }
+  if (whole && lists) {
+    if (tid == 0) a.cnt[0] = ntasks;
+    for (int i = tid; i < ntasks; i += stride) {
+      greedy_propose(a, 0, i);
+      a.list0[i] = i;
+    }
+  }
+  cluster_sync();
+  if (lists)
+    for (; r < kGreedyRounds; ++r) {
+      n = tail_word(a.cnt + r % 3);
+      if (n <= kClusterRows * stride) break;
+      const int* in = (r & 1) ? a.list1 : a.list0;
+      int* out = (r & 1) ? a.list0 : a.list1;
+      if (tid == 0) a.cnt[(r + 2) % 3] = 0;
+      for (int q = tid; q < n; q += stride) {
+        const int i = in[q];
+        if (greedy_item(a, ntasks, r, i, pairs, npairs)) trn_append(out, a.cnt + (r + 1) % 3, i);
+      }
+      cluster_sync();
+    }
+  if (r >= kGreedyRounds || n == 0) return;
+  const int* in = (r & 1) ? a.list1 : a.list0;
+  TailRow mine[kClusterRows];
+#pragma unroll
+  for (int k = 0; k < kClusterRows; ++k) {
+    const int q = tid + k * stride;
+    if (q < n) mine[k].load(a, whole && !lists ? q : in[q]);
+  }
+  if (whole && !lists) {
+#pragma unroll
+    for (int k = 0; k < kClusterRows; ++k)
+      if (mine[k].open) mine[k].propose(a, 0);
+    cluster_sync();
+  }
+  for (const int first = r; r < kGreedyRounds; ++r) {
+    if (r > first && tail_word(more + r % 3) == 0) return;
+    if (tid == 0) more[(r + 2) % 3] = 0;   /* the round after next's word */
+    bool left = false;
+#pragma unroll
+    for (int k = 0; k < kClusterRows; ++k)
+      if (mine[k].open) {
+        mine[k].round(a, r, pairs, npairs);
+        left |= mine[k].open;
+      }
+    if (left) more[(r + 1) % 3] = 1;
+    cluster_sync();
+  }
+}
 
 }  // namespace trn
 
