@@ -186,13 +186,11 @@ int trn_smooth_gradient_run(trn_mesh* mesh, int max_colors, int steps, double ma
  * cfg[1] collapse-target search block, cfg[2] lanes per vertex of the
  * grouped search (4, 8, 16; 1: the one-lane search at every level), cfg[3]
  * longest level list the grouped search takes (longer ones run the one-lane
- * search), cfg[4] flip block, cfg[5] lanes per smoothed vertex (1, 2, 4,
- * 8), cfg[6] variant of the smoothing kernel with 2 or more lanes (0: the
- * back-off tries in turn, up to 128 registers, two 256-thread blocks per SM;
- * 1: capped for three; 2, 3: for four; 4: the five tries in one sweep, capped
- * for four; 5, 8: for three; 6, 7: for two; one lane a vertex reads 0-2 only
- * and treats 3-8 as
- * 2). Defaults: 2 lanes, variant 7, 256-thread blocks. Per mesh; a
+ * search), cfg[4] flip block, cfg[5] lanes per smoothed vertex (2, 4 or
+ * 8; 1 runs as 2), cfg[6] registers of the smoothing kernel (0: up to 128,
+ * two 256-thread blocks per SM; 1: capped for three; 2 to 8: for four). With
+ * cfg[5], cfg[6] at 2, 1 (the default) both follow each color class's length
+ * and the arithmetic form. Defaults: 256-thread blocks. Per mesh; a
  * captured round is recaptured when they change. trn_autotune chooses them
  * on the loaded mesh, timing metric + `rounds` rounds from the input (the
  * best of three runs; a candidate replaces the value kept only when at

@@ -4,15 +4,13 @@
  *
  *   k_smooth_pre   live vertices: interior ones active, boundary ones not
  *                  (smoothing.cpp:129-142)
- *   k_smooth_move  one launch per color class: every listed interior vertex
- *                  moves to the mean over its neighbours b of
+ *   k_smooth_move_grp  one launch per color class: every listed interior
+ *                  vertex (by 2, 4 or 8 lanes) moves to the mean over its neighbours b of
  *                  p_a + (p_b - p_a)/L_M(a,b), takes the log-Euclidean mean of
  *                  the neighbours' tensors, and keeps the move only if every
  *                  incident element stays CCW with quality above the old
  *                  stencil minimum, backing off the step 1, 1/2, .., 1/16
  *                  (Smooth::moveSmartLaplacian, smoothing.cpp:40-126).
- *   k_smooth_move_grp  the same with 2, 4 or 8 lanes per vertex (launch shape
- *                  smooth_lanes; the same results)
  * Vertices of one color share no element, so a class moves in parallel; the
  * classes run in order, as in the reference.
  */
@@ -32,110 +30,10 @@ __global__ void k_smooth_pre(DMesh m, int nb_nodes) {
 /* Element metrics of the back-off: the log-Euclidean mean of an element's
  * three tensors (and the square root of its determinant) does not depend on
  * where the moved vertex sits, only on its new tensor, so it is computed once
- * per stencil element before the tries and kept in shared memory (kj slots a
- * thread, stride blockDim.x so that a warp's slots are contiguous); the
- * tries only redo the geometry. Elements past the kj-th (rare: long
- * stencils) take the metric inline. Same operations, same bits as
- * evaluating the whole quality in every try. */
+ * per stencil element before the tries; the tries only redo the geometry.
+ * Same operations, same bits as evaluating the whole quality in every try. */
 template <bool F32>
 using JmT = LogT<F32>;
-
-template <bool F32>
-__device__ int move_laplacian(const DMesh& m, int i, JmT<F32>* jc, int kj) {
-  const TrnRow vc = trn_row(m.vic, m, i);
-  const TrnRow st = trn_row(m.stenc, m, i);
-  const int deg = trn_deg(m, i);
-  const int nb_neigh = m.vdeg[i];
-  double q_min = 1.7976931348623157e308;
-  for (int a = 0; a < deg; ++a) q_min = trn_dmin(q_min, m.qual[st[a]]);
-  const double2 pini = m.pts[i];
-  const double4 tini = m.ten[i];
-  const TenT<F32> tinf = ten_load<F32>(m, i);
-  const LogT<F32> lini = log_load<F32>(m, i);
-  double ox = 0, oy = 0;
-  LogSum<F32> lsum;
-  if constexpr (F32) {
-    /* the mean displacement in single precision, added to the FP64 point */
-    float dx = 0.f, dy = 0.f;
-    for (int k = 0; k < nb_neigh; ++k) {
-      const int nb = vc[k];
-      const double2 pb = m.pts[nb];
-      const float il = __frcp_rn(trnf_dist2(pini, pb, tenf_of(tinf), tenf_of(ten_load<F32>(m, nb))));
-      dx += (float) (pb.x - pini.x) * il;
-      dy += (float) (pb.y - pini.y) * il;
-      lsum.add(log_load<F32>(m, nb));
-    }
-    const float inv = __frcp_rn((float) nb_neigh);
-    ox = pini.x + (double) (dx * inv);
-    oy = pini.y + (double) (dy * inv);
-  } else {
-    for (int k = 0; k < nb_neigh; ++k) {
-      const int nb = vc[k];
-      const double2 pb = m.pts[nb];
-      const double4 tb = m.ten[nb];
-      const double len = length_x<F32>(pini, pb, tini, tb);
-      ox += pini.x + ((pb.x - pini.x) / len);
-      oy += pini.y + ((pb.y - pini.y) / len);
-      lsum.add(log_load<F32>(m, nb));
-    }
-    ox /= nb_neigh;
-    oy /= nb_neigh;
-  }
-  double tn[3];
-  lsum.finish(nb_neigh, tn);
-  const double4 tnew = make_double4(tn[0], tn[1], tn[2], 0.0);
-  const LogT<F32> lnew = log_of<F32>(tn[0], tn[1], tn[2]);
-  ten_store<F32>(m, i, tnew);
-  log_store<F32>(m, i, lnew);
-  const int nj = deg < kj ? deg : kj;
-  for (int a = 0; a < nj; ++a) {
-    const int4 n = m.tri[st[a]];
-    const LogT<F32> l0 = (n.x == i) ? lnew : log_load<F32>(m, n.x);
-    const LogT<F32> l1 = (n.y == i) ? lnew : log_load<F32>(m, n.y);
-    const LogT<F32> l2 = (n.z == i) ? lnew : log_load<F32>(m, n.z);
-    jc[(size_t) a * blockDim.x] = qmetric_x(l0, l1, l2);
-  }
-  double qual[TRN_MAX_DEG];
-  bool valid;
-  int retry = 0;
-  double weight = 1;
-  do {
-    valid = true;
-    double2 pa;
-    pa.x = (1 - weight) * pini.x + weight * ox;
-    pa.y = (1 - weight) * pini.y + weight * oy;
-    m.pts[i] = pa;
-    for (int a = 0; valid && a < deg; ++a) {
-      const int4 n = m.tri[st[a]];
-      const double2 p0 = (n.x == i) ? pa : m.pts[n.x];
-      const double2 p1 = (n.y == i) ? pa : m.pts[n.y];
-      const double2 p2 = (n.z == i) ? pa : m.pts[n.z];
-      valid = false;
-      if (trn_ccw(p0, p1, p2)) {
-        JmT<F32> jm;
-        if (a < nj) {
-          jm = jc[(size_t) a * blockDim.x];
-        } else {
-          const LogT<F32> l0 = (n.x == i) ? lnew : log_load<F32>(m, n.x);
-          const LogT<F32> l1 = (n.y == i) ? lnew : log_load<F32>(m, n.y);
-          const LogT<F32> l2 = (n.z == i) ? lnew : log_load<F32>(m, n.z);
-          jm = qmetric_x(l0, l1, l2);
-        }
-        qual[a] = qgeom_x(p0, p1, p2, jm);
-        valid = (qual[a] > q_min);
-      }
-    }
-    weight *= 0.5;
-  } while (!valid && ++retry < 5);
-  if (valid) {
-    for (int a = 0; a < deg; ++a) m.qual[st[a]] = qual[a];
-  } else {
-    m.pts[i] = pini;
-    ten_store<F32>(m, i, tini);
-    log_store<F32>(m, i, lini);
-  }
-  return valid ? 1 : 0;
-}
 
 /* the algorithmic bytes of one listed vertex (profiled runs only): its list
  * entry and flags; when it moves, its own point, tensor and logarithm read
@@ -161,47 +59,12 @@ __device__ unsigned long long smooth_bytes(const DMesh& m, int v, bool moved, un
   return b;
 }
 
-/* MinB: 256-thread blocks an SM the registers are capped for (2: up to 128,
- * 3: 80, 4: 64); more warps hide more of the gathers' latency, at the cost of
- * spills */
-template <bool F32, int MinB>
-__global__ void __launch_bounds__(256, MinB) k_smooth_move(DMesh m, const int* __restrict__ list,
-                                                                   int n, const int* off, int c, int* counters,
-                                                                   int kj, ByteCount bc) {
-  extern __shared__ __align__(16) unsigned char smooth_smem[];
-  JmT<F32>* jc = reinterpret_cast<JmT<F32>*>(smooth_smem) + threadIdx.x;
-  if (trn_failed(m)) return;
-  if (off) {   /* color class c of a device-side partition */
-    list += off[c];
-    n = off[c + 1] - off[c];
-  }
-  int tasks = 0, commit = 0;
-  unsigned long long bytes = 0;
-  for (int q = trn_tid(); q < n; q += trn_grid_stride()) {
-    const int v = list[q];
-    if (v < 0 || v >= m.capa_node) {
-      trn_set_error(m.err, TRN_DERR_REPLAY);
-      continue;
-    }
-    const bool moved = m.activ[v] && m.vdeg[v] != 0;
-    if (bc.bytes) bytes += smooth_bytes<F32>(m, v, moved, bc.seen);
-    if (!moved) continue;
-    tasks++;
-    commit += move_laplacian<F32>(m, v, jc, kj);
-  }
-  trn_warp_add(counters, tasks);
-  trn_warp_add(counters + 1, commit);
-  if (bytes) atomicAdd(bc.bytes, bytes);
-}
-
-/* The same move with G lanes per vertex: lane j gathers the neighbours
- * j, j+G, ... and evaluates the elements j, j+G, ... of the stencil. The
- * displacement and the tensor-logarithm sums are accumulated in neighbour
- * order by every lane from the lanes' terms (shuffles), the stencil minimum
- * is a min-reduction and validity an all-vote, so the results are the bits
- * of move_laplacian. More loads in flight per vertex and no per-thread
- * quality array: the one-lane form is bound by gather latency, divergence
- * and registers. */
+/* A move by G lanes per vertex: lane j gathers the neighbours j, j+G, ... and
+ * evaluates the elements j, j+G, ... of the stencil. The displacement and the
+ * tensor-logarithm sums are accumulated in neighbour order by every lane from
+ * the lanes' terms (shuffles), the stencil minimum is a min-reduction and
+ * validity a vote, so the results are those of one lane in the reference's
+ * order. */
 template <class T>
 __device__ __forceinline__ T grp_shfl(unsigned mask, T v, int src, int width);
 template <>
@@ -221,40 +84,6 @@ template <>
 __device__ __forceinline__ float4 grp_shfl(unsigned mask, float4 v, int src, int width) {
   return make_float4(__shfl_sync(mask, v.x, src, width), __shfl_sync(mask, v.y, src, width),
                      __shfl_sync(mask, v.z, src, width), __shfl_sync(mask, v.w, src, width));
-}
-
-/* quality of stencil element t of vertex i with i at pa (log lnew); false
- * when it is not CCW */
-template <bool F32>
-__device__ __forceinline__ bool elem_quality_at(const DMesh& m, int i, int4 n, double2 pa, LogT<F32> lnew,
-                                                double* q) {
-  const double2 p0 = (n.x == i) ? pa : m.pts[n.x];
-  const double2 p1 = (n.y == i) ? pa : m.pts[n.y];
-  const double2 p2 = (n.z == i) ? pa : m.pts[n.z];
-  if (!trn_ccw(p0, p1, p2)) return false;
-  const LogT<F32> l0 = (n.x == i) ? lnew : log_load<F32>(m, n.x);
-  const LogT<F32> l1 = (n.y == i) ? lnew : log_load<F32>(m, n.y);
-  const LogT<F32> l2 = (n.z == i) ? lnew : log_load<F32>(m, n.z);
-  *q = quality_x(p0, p1, p2, l0, l1, l2);
-  return true;
-}
-
-/* a[j] of a small register array, j known only at run time: predicated
- * selects, so the array stays in registers */
-template <int K, class T>
-__device__ __forceinline__ T reg_pick(const T (&a)[K], int j) {
-  T r = a[0];
-#pragma unroll
-  for (int k = 1; k < K; ++k)
-    if (j == k) r = a[k];
-  return r;
-}
-
-template <int K, class T>
-__device__ __forceinline__ void reg_put(T (&a)[K], int j, T v) {
-#pragma unroll
-  for (int k = 0; k < K; ++k)
-    if (j == k) a[k] = v;
 }
 
 /* The moved vertex's new tensor (the exponentiated mean of its neighbours'
@@ -410,21 +239,28 @@ __device__ __forceinline__ JmT<F32> elem_metric(const DMesh& m, int i, int4 n, L
                    (n.z == i) ? lnew : log_load<F32>(m, n.z));
 }
 
-/* V selects how the back-off runs:
- *   0  the tries in turn, element metrics in registers;
- *   1  one sweep over the lane's elements decides all five tries (try_mask),
- *      the group ANDs the lanes' five-bit pass masks and keeps the first try
- *      that passes, whose qualities the commit evaluates. A warp of 8 groups
- *      or more almost always runs all five tries in turn anyway (half the
- *      moves fail every try), so this costs no extra issue and turns a serial
- *      chain into parallel ones. The element metrics of the lane's first KQ
- *      elements wait in shared memory (stride blockDim.x), which frees
- *      registers; those of later ones (long stencils) are taken again.
- * Same tries, same arithmetic, same first passing try: the same bits. */
-template <bool F32, int G, int V>
+template <bool F32>
+struct VertexPark {
+  double2 pini, o;
+  double tn[3], q_min;
+  LogT<F32> lnew;
+};
+
+/* One sweep over the lane's elements decides all five tries (try_mask), the
+ * group ANDs the lanes' five-bit pass masks and keeps the first try that
+ * passes, whose qualities the commit evaluates. A warp of 4 groups or more
+ * almost always needs every try of some group anyway (half the moves fail all
+ * five), so this costs no extra issue over trying in turn, and turns a serial
+ * chain into parallel ones. The element metrics of the lane's first KQ elements
+ * wait in shared memory (stride blockDim.x); those of later ones (long
+ * stencils) are taken again. What the elements need of the vertex waits there
+ * too (VertexPark): held in registers over the element loop it took 128 of
+ * them, or spilled; without it 80 hold the kernel, three 256-thread blocks an
+ * SM instead of two, and 64 all but 128 bytes. Two passes over the classes of
+ * the 2M-triangle workload, FP64 / mixed: 6.49 / 4.98 ms before, 5.61 / 4.32. */
+template <bool F32, int G>
 __device__ int move_laplacian_grp(const DMesh& m, int i, int lane, unsigned gmask, unsigned char* smem) {
   static_assert(G >= 2, "lane groups of two or more");
-  constexpr bool SW = V == 1;
   constexpr int KQ = G >= 4 ? 2 : 3;
   JmT<F32>* js = reinterpret_cast<JmT<F32>*>(smem) + threadIdx.x;
   const TrnRow vc = trn_row(m.vic, m, i);
@@ -484,32 +320,38 @@ __device__ int move_laplacian_grp(const DMesh& m, int i, int lane, unsigned gmas
     lsum.finish(nb_neigh, tn);
     lnew = log_of<F32>(tn[0], tn[1], tn[2]);
   }
-  const double4 tnew = make_double4(tn[0], tn[1], tn[2], 0.0);
-  /* the element metrics of this lane's first KQ elements: they do not depend
-   * on where the vertex sits, so the tries below only redo the geometry (a
-   * stencil of 6 elements fits: 2 a lane with 4 lanes, 3 with 2) */
-  if constexpr (SW) {
-    const double2 o = make_double2(ox, oy);
-    unsigned okm = 0x1fu;   /* bit w: every element of this lane passes try w */
-    int j = 0;
-    for (int a = lane; a < deg; a += G, ++j) {
-      const int4 n = m.tri[st[a]];
-      const JmT<F32> q = elem_metric<F32>(m, i, n, lnew);
-      if (j < KQ) js[(size_t) j * blockDim.x] = q;
-      okm &= try_mask<F32>(m, i, n, pini, o, q, q_min);
-    }
+  VertexPark<F32>* park = reinterpret_cast<VertexPark<F32>*>(smem + (size_t) KQ * blockDim.x * sizeof(JmT<F32>)) +
+                          threadIdx.x / G;
+  if (lane == 0) {
+    park->pini = pini;
+    park->o = make_double2(ox, oy);
+    park->q_min = q_min;
+    park->tn[0] = tn[0];
+    park->tn[1] = tn[1];
+    park->tn[2] = tn[2];
+    park->lnew = lnew;
+  }
+  __syncwarp(gmask);
+  unsigned okm = 0x1fu;   /* bit w: every element of this lane passes try w */
+  int j = 0;
+  for (int a = lane; a < deg; a += G, ++j) {
+    const int4 n = m.tri[st[a]];
+    const JmT<F32> q = elem_metric<F32>(m, i, n, park->lnew);
+    if (j < KQ) js[(size_t) j * blockDim.x] = q;
+    okm &= try_mask<F32>(m, i, n, park->pini, park->o, q, park->q_min);
+  }
 #pragma unroll
-    for (int d = G / 2; d > 0; d >>= 1) okm &= __shfl_xor_sync(gmask, okm, d, G);
-    if (!okm) return 0;
+  for (int d = G / 2; d > 0; d >>= 1) okm &= __shfl_xor_sync(gmask, okm, d, G);
+  if (okm) {
     double weight = 1;
     for (int w = __ffs(okm) - 1; w > 0; --w) weight *= 0.5;
     double2 pa;
-    pa.x = (1 - weight) * pini.x + weight * ox;
-    pa.y = (1 - weight) * pini.y + weight * oy;
+    pa.x = (1 - weight) * park->pini.x + weight * park->o.x;
+    pa.y = (1 - weight) * park->pini.y + weight * park->o.y;
     j = 0;
     for (int a = lane; a < deg; a += G, ++j) {
       const int4 n = m.tri[st[a]];
-      const JmT<F32> q = j < KQ ? js[(size_t) j * blockDim.x] : elem_metric<F32>(m, i, n, lnew);
+      const JmT<F32> q = j < KQ ? js[(size_t) j * blockDim.x] : elem_metric<F32>(m, i, n, park->lnew);
       const double2 p0 = (n.x == i) ? pa : m.pts[n.x];
       const double2 p1 = (n.y == i) ? pa : m.pts[n.y];
       const double2 p2 = (n.z == i) ? pa : m.pts[n.z];
@@ -517,66 +359,17 @@ __device__ int move_laplacian_grp(const DMesh& m, int i, int lane, unsigned gmas
     }
     if (lane == 0) {
       m.pts[i] = pa;
-      ten_store<F32>(m, i, tnew);
-      log_store<F32>(m, i, lnew);
+      ten_store<F32>(m, i, make_double4(park->tn[0], park->tn[1], park->tn[2], 0.0));
+      log_store<F32>(m, i, park->lnew);
     }
-    return 1;
-  } else {
-    double qv[KQ];
-    JmT<F32> jv[KQ];
-#pragma unroll
-    for (int j = 0; j < KQ; ++j) {
-      const int a = lane + j * G;
-      if (a < deg) jv[j] = elem_metric<F32>(m, i, m.tri[st[a]], lnew);
-    }
-    bool valid;
-    int retry = 0;
-    double weight = 1;
-    double2 pa;
-    do {
-      pa.x = (1 - weight) * pini.x + weight * ox;
-      pa.y = (1 - weight) * pini.y + weight * oy;
-      bool ok = true;
-      int j = 0;
-      for (int a = lane; ok && a < deg; a += G, ++j) {
-        double q = 0;
-        if (j < KQ) {
-          const int4 n = m.tri[st[a]];
-          const double2 p0 = (n.x == i) ? pa : m.pts[n.x];
-          const double2 p1 = (n.y == i) ? pa : m.pts[n.y];
-          const double2 p2 = (n.z == i) ? pa : m.pts[n.z];
-          ok = trn_ccw(p0, p1, p2);
-          if (ok) {
-            q = qgeom_x(p0, p1, p2, reg_pick(jv, j));
-            ok = q > q_min;
-          }
-          reg_put(qv, j, q);
-        } else {
-          ok = elem_quality_at<F32>(m, i, m.tri[st[a]], pa, lnew, &q) && (q > q_min);
-        }
-      }
-      valid = __all_sync(gmask, ok);
-      weight *= 0.5;
-    } while (!valid && ++retry < 5);
-    if (valid) {
-      int j = 0;
-      for (int a = lane; a < deg; a += G, ++j) {
-        double q = 0;
-        if (j < KQ) q = reg_pick(qv, j);
-        else elem_quality_at<F32>(m, i, m.tri[st[a]], pa, lnew, &q);
-        m.qual[st[a]] = q;
-      }
-      if (lane == 0) {
-        m.pts[i] = pa;
-        ten_store<F32>(m, i, tnew);
-        log_store<F32>(m, i, lnew);
-      }
-    }
-    return valid ? 1 : 0;
   }
+  __syncwarp(gmask);   /* the next vertex reuses the place */
+  return okm ? 1 : 0;
 }
 
-template <bool F32, int G, int MinB, int V>
+/* MinB: 256-thread blocks an SM the registers are capped for (2: 112 are
+ * used, 3: 80, 4: 64) */
+template <bool F32, int G, int MinB>
 __global__ void __launch_bounds__(256, MinB) k_smooth_move_grp(DMesh m, const int* __restrict__ list,
                                                                        int n, const int* off, int c,
                                                                        int* counters, ByteCount bc) {
@@ -602,7 +395,7 @@ __global__ void __launch_bounds__(256, MinB) k_smooth_move_grp(DMesh m, const in
     if (bc.bytes && lane == 0) bytes += smooth_bytes<F32>(m, v, moved, bc.seen);
     if (!moved) continue;
     tasks++;
-    commit += move_laplacian_grp<F32, G, V>(m, v, lane, gmask, smooth_smem);
+    commit += move_laplacian_grp<F32, G>(m, v, lane, gmask, smooth_smem);
   }
   /* the group's tallies sit on its first lane (0 on the others) */
   trn_warp_add(counters, tasks * (lane == 0));
@@ -616,25 +409,28 @@ void smooth_pre(const DMesh& m, int nb_nodes, cudaStream_t s) {
   check_launch("smooth_pre");
 }
 
-/* The default shape (2 lanes, the sweep at 128 registers) stands for a choice
- * by the class's length and the form. A vertex is a chain of gathers and
- * arithmetic: a class too short to fill the chip takes as long as one chain,
- * which more lanes shorten; a long one is bound by issue, which the lanes'
- * shared part (the new tensor) then repeats. Two passes over the classes, ms,
- * by live vertices (a class is a quarter of them at most):
- *   FP64   8 lanes   4 lanes   2 lanes      FP32   8, sweep  8, in turn  2, sweep
- *   10 k   0.42      0.52      0.69         10 k   0.37      0.40        0.57
- *   103 k  0.72      0.76      0.90         103 k  0.58      0.59        0.74
- *   187 k  0.98      0.96      1.08         187 k  0.73      0.72        0.89
- *   294 k  1.35      1.26      1.29         294 k  0.96      0.90        1.03
- *   578 k  2.39      2.12      2.06         578 k  1.67      1.48        1.63 */
-static void smooth_shape(int n, bool fp32, int* lanes, int* regs) {
+/* The default shape (2 lanes, variant 1) stands for a choice by the class's
+ * length and the form. A vertex is a chain of gathers and arithmetic: a class
+ * too short to fill the chip takes as long as one chain, which more lanes
+ * shorten; a long one is bound by issue, which the lanes' shared part (the new
+ * tensor) then repeats. Two passes over the classes, ms, by live vertices (a
+ * class is a quarter of them at most), lanes x 256-thread blocks an SM:
+ *   FP64    8 x 3   4 x 4   2 x 3      mixed   8 x 4   4 x 4   2 x 4
+ *   23 k    0.47    0.59    0.75       23 k    0.41    0.50    0.65
+ *   187 k   0.89    0.92    1.02       187 k   0.69    0.74    0.86
+ *   294 k   1.20    1.13    1.28       294 k   0.86    0.88    0.96
+ *   578 k   2.12    1.86    1.89       578 k   1.41    1.36    1.42
+ *   1181 k  3.95    3.34    3.10       1181 k  2.58    2.38    2.45 */
+static void smooth_shape(int n, bool fp32, int* lanes, int* blocks) {
   if (fp32) {
+    *lanes = n <= 98304 ? 8 : 4;
+    *blocks = 4;
+  } else if (n <= 49152) {
     *lanes = 8;
-    *regs = n <= 32768 ? 5 : 2;
-  } else if (n <= 65536) {
-    *lanes = n <= 32768 ? 8 : 4;
-    *regs = n <= 8192 ? 7 : (n <= 32768 ? 5 : 7);
+    *blocks = 3;
+  } else if (n <= 163840) {
+    *lanes = 4;
+    *blocks = 4;
   }
 }
 
@@ -649,63 +445,37 @@ static void smooth_launch(const DMesh& m, const int* list, int n, const int* off
   ByteCount bc;
   ProfScope ps("smooth_move", s, n * own + nbr, &bc);
   const int t = tune().smooth_threads;
-  int lanes = tune().smooth_lanes, regs = tune().smooth_regs;
-  if (lanes == 2 && regs == 7) smooth_shape(hint, fp32, &lanes, &regs);
+  const int regs = tune().smooth_regs;
+  int lanes = std::max(2, tune().smooth_lanes), blocks = regs == 0 ? 2 : (regs == 1 ? 3 : 4);
+  if (lanes == 2 && blocks == 3) smooth_shape(hint, fp32, &lanes, &blocks);
   const int g = grid_for((long long) hint * lanes, t);
-  if (lanes == 8 || lanes == 4 || lanes == 2) {
-    /* smooth_regs 0, 1, 2 (and 3): the tries in turn, registers capped for
-     * two, three, four 256-thread blocks an SM; 4, 5 (and 8), 6 (and 7): the
-     * sweep, capped for four, three, two, with the element metrics in shared
-     * memory (KQ = 2 slots a thread for 4 or 8 lanes, 3 for 2) */
-    const int kq = lanes >= 4 ? 2 : 3;
-    const size_t js_smem = (size_t) kq * t * (fp32 ? sizeof(float4) : sizeof(double4));
-#define TRN_GRP(F, G, B, V)                                                                   \
-  do {                                                                                        \
-    auto* kern = k_smooth_move_grp<F, G, B, V>;                                               \
-    const size_t sm = V == 1 ? js_smem : 0;                                                   \
-    kern<<<grid_resident(reinterpret_cast<const void*>(kern), t, g, sm), t, sm, s>>>(m, list, n, off, c, \
-                                                                                     counters, bc); \
+  /* KQ element metrics a thread, a VertexPark a vertex */
+  const size_t smem = (size_t) (lanes >= 4 ? 2 : 3) * t * (fp32 ? sizeof(float4) : sizeof(double4)) +
+                      (size_t) (t / lanes) * (fp32 ? sizeof(VertexPark<true>) : sizeof(VertexPark<false>));
+#define TRN_GRP(F, G, B)                                                                         \
+  do {                                                                                           \
+    auto* kern = k_smooth_move_grp<F, G, B>;                                                     \
+    kern<<<grid_resident(reinterpret_cast<const void*>(kern), t, g, smem), t, smem, s>>>(        \
+        m, list, n, off, c, counters, bc);                                                       \
   } while (0)
-#define TRN_GRP_B(F, G)                                                                       \
-  do {                                                                                        \
-    if (regs == 0) TRN_GRP(F, G, 2, 0);                                                       \
-    else if (regs == 1) TRN_GRP(F, G, 3, 0);                                                  \
-    else if (regs <= 3) TRN_GRP(F, G, 4, 0);                                                  \
-    else if (regs == 4) TRN_GRP(F, G, 4, 1);                                                  \
-    else if (regs == 5 || regs == 8) TRN_GRP(F, G, 3, 1);                                     \
-    else TRN_GRP(F, G, 2, 1);                                                                 \
+#define TRN_GRP_B(F, G)                                                                          \
+  do {                                                                                           \
+    if (blocks == 2) TRN_GRP(F, G, 2);                                                           \
+    else if (blocks == 3) TRN_GRP(F, G, 3);                                                      \
+    else TRN_GRP(F, G, 4);                                                                       \
   } while (0)
-    if (lanes == 8) {
-      if (fp32) TRN_GRP_B(true, 8);
-      else TRN_GRP_B(false, 8);
-    } else if (lanes == 4) {
-      if (fp32) TRN_GRP_B(true, 4);
-      else TRN_GRP_B(false, 4);
-    } else {
-      if (fp32) TRN_GRP_B(true, 2);
-      else TRN_GRP_B(false, 2);
-    }
+  if (lanes == 8) {
+    if (fp32) TRN_GRP_B(true, 8);
+    else TRN_GRP_B(false, 8);
+  } else if (lanes == 4) {
+    if (fp32) TRN_GRP_B(true, 4);
+    else TRN_GRP_B(false, 4);
+  } else {
+    if (fp32) TRN_GRP_B(true, 2);
+    else TRN_GRP_B(false, 2);
+  }
 #undef TRN_GRP_B
 #undef TRN_GRP
-  } else {
-    /* element-metric slots a thread: what 40 KB of shared memory a block
-     * holds, at most 8 (FP64) or 12 (FP32) */
-    const int slot = fp32 ? (int) sizeof(float4) : (int) sizeof(double4);
-    const int kj = std::min(fp32 ? 12 : 8, (40 << 10) / (t * slot));
-    const size_t smem = (size_t) kj * t * slot;
-#define TRN_ONE(F, B)                                                                           \
-  do {                                                                                          \
-    auto* kern = k_smooth_move<F, B>;                                                           \
-    kern<<<grid_resident(reinterpret_cast<const void*>(kern), t, g, smem), t, smem, s>>>(m, list, n, off, \
-                                                                                        c, counters, kj, bc); \
-  } while (0)
-#define TRN_ONE_B(F) \
-  do { if (regs == 0) TRN_ONE(F, 2); else if (regs == 1) TRN_ONE(F, 3); else TRN_ONE(F, 4); } while (0)
-    if (fp32) TRN_ONE_B(true);
-    else TRN_ONE_B(false);
-#undef TRN_ONE_B
-#undef TRN_ONE
-  }
   note_launch();
   check_launch("smooth_move");
 }

@@ -1431,8 +1431,7 @@ int trn_set_tune(trn_mesh* m, const int cfg[TRN_TUNE_N]) {
 
 /* Launch shapes timed on this mesh (the best of three runs of metric +
  * rounds from the loaded input, device time of the rounds). First the
- * smoothing's lanes a vertex and register / back-off variant jointly (they
- * interact: two lanes a vertex pay off only with the one-sweep tries), then
+ * smoothing's lanes a vertex and registers jointly (they interact), then
  * coordinate descent over every parameter: the current value and then every
  * other candidate with the others at their best so far. A candidate replaces
  * the value kept only when it is at least 1 % faster (run-to-run noise is
@@ -1470,7 +1469,7 @@ int trn_autotune(trn_mesh* m, double target_factor, int norm, double h_min, doub
                              &m->tune.filter_threads, &m->tune.group_lanes, &m->tune.group_max,
                              &m->tune.flip_threads};
   const std::vector<std::vector<int>> cands = {
-      {1, 2, 4, 8}, {64, 128, 256}, {0, 1, 2, 3, 4, 5, 6, 7, 8}, {128, 256, 512}, {4, 8, 16}, {4096, 16384, 65536}, {128, 256, 512}};
+      {2, 4, 8}, {64, 128, 256}, {0, 1, 2}, {128, 256, 512}, {4, 8, 16}, {4096, 16384, 65536}, {128, 256, 512}};
   {
     int best_l = m->tune.smooth_lanes, best_r = m->tune.smooth_regs;
     double best_ms;
@@ -1478,7 +1477,7 @@ int trn_autotune(trn_mesh* m, double target_factor, int norm, double h_min, doub
     for (int l : cands[0]) {
       for (int r : cands[2]) {
         if (rc != TRN_OK) break;
-        if ((l == best_l && r == best_r) || (l == 1 && r > 2)) continue;  /* one lane: 0-2 only */
+        if (l == best_l && r == best_r) continue;
         m->tune.smooth_lanes = l;
         m->tune.smooth_regs = r;
         double ms;

@@ -85,9 +85,7 @@ void fix_list_level_end(const DMesh& m, const int* list, const int* count, long 
 
 /* launch shapes the autotuner (trn_autotune) chooses; none of them changes
  * a result. The defaults are the tuner's choice on the 2M-triangle workload
- * in FP64 (the smoothing by 2 lanes a vertex in 256-thread blocks, the five
- * back-off tries in one sweep). Each mesh keeps
- * its own table; the C-ABI entry that drives a mesh makes it the calling
+ * in FP64. Each mesh keeps its own table; the C-ABI entry that drives a mesh makes it the calling
  * thread's table for the launchers. */
 struct Tune {
   int smooth_threads = 256;   /* k_smooth_move block: 64, 128, 256 */
@@ -95,10 +93,10 @@ struct Tune {
   int group_lanes = 16;       /* lanes per vertex of the grouped search: 1 (one-lane search), 4, 8, 16 */
   int group_max = 16384;      /* longest level list the grouped search takes */
   int flip_threads = 256;     /* k_swap_flip block: 128, 256, 512 */
-  int smooth_lanes = 2;       /* lanes per smoothed vertex: 1, 2, 4, 8 */
-  int smooth_regs = 7;        /* smoothing variant: 0 the tries in turn, up to 128 registers, 1 capped
-                                 at 80 (three 256-thread blocks an SM), 2 (and 3) at 64 (four); 4, 5
-                                 (and 8), 6 (and 7): the five tries in one sweep, capped at 64, 80, 128 */
+  int smooth_lanes = 2;       /* lanes per smoothed vertex: 2 (or 1, the same), 4, 8 */
+  int smooth_regs = 1;        /* smoothing registers: 0 up to 128 (two 256-thread blocks an SM), 1 capped
+                                 at 80 (three), 2 and more at 64 (four); 2 lanes at 1 (the default) leave
+                                 both to the class's length and the form */
   bool operator==(const Tune& o) const {
     return smooth_threads == o.smooth_threads && filter_threads == o.filter_threads &&
            group_lanes == o.group_lanes && group_max == o.group_max && flip_threads == o.flip_threads &&
