@@ -55,7 +55,7 @@ struct trn_mesh {
   int* dual_n = nullptr;
   int* pairs = nullptr;
   int* parts = nullptr;
-  unsigned char* stage = nullptr;   /* transfer staging: max(24 B/vertex, 12 B/element) */
+  unsigned char* stage = nullptr;   /* transfer staging: max(40 B/vertex, 12 B/element) */
   int* status = nullptr;
   int* h_status = nullptr;
   /* the last loaded input, kept on the device for trn_mesh_reload */
@@ -321,7 +321,7 @@ int trn_mesh_create_ex(const int size[2], int bucket, int depth, int verbosity, 
       (rc = dmalloc(m, &m->indep, cn)) || (rc = dmalloc(m, &m->map, ce)) ||
       (rc = dmalloc(m, &m->dual, ce * 4)) || (rc = dmalloc(m, &m->dual_n, ce)) ||
       (rc = dmalloc(m, &m->pairs, ce * 2)) || (rc = dmalloc(m, &m->parts, cn)) ||
-      (rc = dmalloc(m, &m->stage, std::max(24 * cn, 12 * ce))) ||
+      (rc = dmalloc(m, &m->stage, std::max(40 * cn, 12 * ce))) ||
       (rc = dmalloc(m, &m->status, S_SIZE)))
     return bail(rc);
   d.err = m->status + S_ERR;
