@@ -1,5 +1,8 @@
-"""An export with the tensors where the mesh fills its capacity: points and
-tensors of every vertex wait in the staging buffer."""
+"""Loading in one pass and exporting with one read back: a reload after an
+adaptation has to start as a fresh load does, and an export has to be the
+renumbering of the raw state where the staging buffer holds the vertices and
+the triangles and where it does not (no room to spare, with the tensor), at
+sides whose counts end inside a 16-byte store of flags."""
 import numpy as np
 import pytest
 
@@ -38,4 +41,36 @@ def test_export_without_room_to_spare(side):
     assert same(g.export_compact(), want)
     p, t, ten = g.export_compact(with_tensor=False)
     assert ten is None and same((p, t), want[:2])
+    g.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("side", [15, 47])
+def test_reload_and_export_after_adapting(side):
+    from trinity_b200.api import Coarse, Metrics, Partit, Refine, Smooth, Swap
+    m, g = make(side, 8)
+    h = Partit(g, 8)
+
+    def adapt():
+        Metrics(g, 0.8, 2).run()
+        for k in (Refine(g, 1), Coarse(g, h), Swap(g), Smooth(g, h, 1)):
+            k.run()
+        return renumbered(g)
+
+    first = adapt()
+    nv, ne = first[0].shape[0], first[1].shape[0]
+    assert same(g.export_compact(), first)
+    for extra in (0, 5, 40000):       # exactly enough, less than the slots in use, more
+        out = (np.empty((nv + extra, 2)), np.empty((ne + extra, 3), np.int32), np.empty((nv + extra, 3)))
+        got = g.export_compact(out=out)
+        assert same(got, first) and got[0].base is out[0]
+    for cut in range(3):
+        out = [np.empty((nv, 2)), np.empty((ne, 3), np.int32), np.empty((nv, 3))]
+        out[cut] = out[cut][:-1]
+        with pytest.raises(ValueError):
+            g.export_compact(out=tuple(out))
+    g.reload()
+    p, t, ten = g.export_compact()
+    assert np.array_equal(p, m.points) and np.array_equal(t, m.tris) and not ten.any()
+    assert same(adapt(), first)
     g.close()

@@ -142,19 +142,26 @@ class Mesh:
         Mesh::store: (points[V',2], tris[T',3] 0-based, tensor[V',3] or None).
         out: optional (points, tris, tensor) arrays with at least V' / T' rows
         (e.g. views of pinned host memory); the results are their leading rows."""
-        _, _, nv, ne = self.counts()
+        nn, ne = ctypes.c_int(), ctypes.c_int()
         if out is not None:
-            if out[0].shape[0] < nv or out[1].shape[0] < ne or (with_tensor and out[2].shape[0] < nv):
-                raise ValueError("export_compact: output arrays too small")
-            pts, tri = out[0][:nv], out[1][:ne]
-            ten = out[2][:nv] if with_tensor else None
+            # arrays with room for every slot in use need no live count first
+            self._check(self._L.trn_mesh_counts(self.h, ctypes.byref(nn), ctypes.byref(ne), None, None))
+            rows = min(out[0].shape[0], out[2].shape[0]) if with_tensor else out[0].shape[0]
+            if rows < nn.value or out[1].shape[0] < ne.value:
+                _, _, nv, nt = self.counts()
+                if out[0].shape[0] < nv or out[1].shape[0] < nt or (with_tensor and out[2].shape[0] < nv):
+                    raise ValueError("export_compact: output arrays too small")
+            pts, tri = out[0], out[1]
+            ten = out[2] if with_tensor else None
         else:
-            pts = np.empty((nv, 2)); tri = np.empty((ne, 3), np.int32)
+            _, _, nv, nt = self.counts()
+            pts = np.empty((nv, 2)); tri = np.empty((nt, 3), np.int32)
             ten = np.empty((nv, 3)) if with_tensor else None
-        a, b = ctypes.c_int(), ctypes.c_int()
         self._check(self._L.trn_mesh_export_compact(self.h, _p(pts), _p(tri), _p(ten) if with_tensor else None,
-                                                    ctypes.byref(a), ctypes.byref(b)))
-        assert (a.value, b.value) == (nv, ne)
+                                                    ctypes.byref(nn), ctypes.byref(ne)))
+        pts, tri = pts[:nn.value], tri[:ne.value]
+        if with_tensor:
+            ten = ten[:nn.value]
         return pts, tri, ten
 
     def set_precision(self, mode: str) -> None:

@@ -67,13 +67,24 @@ __global__ void k_tile_sum_i64(const long long* __restrict__ in, int n, const in
   if (threadIdx.x == 0) tile[blockIdx.x] = tot;
 }
 
-__global__ void k_tile_count_u8(const uint8_t* __restrict__ flags, int n, long long* tile) {
+/* what a compaction keeps: flagged items, or live elements */
+struct KeepFlag {
+  const uint8_t* flags;
+  __device__ __forceinline__ bool operator()(long long i) const { return flags[i] != 0; }
+};
+struct KeepTri {
+  const int4* tri;
+  __device__ __forceinline__ bool operator()(long long i) const { return tri[i].x >= 0; }
+};
+
+template <class Keep>
+__global__ void k_tile_count(Keep keep, int n, long long* tile) {
   __shared__ long long ws[TRN_THREADS / 32];
   const long long base = (long long) blockIdx.x * kTile;
   long long c = 0;
   for (int k = threadIdx.x; k < kTile; k += TRN_THREADS) {
     long long i = base + k;
-    if (i < n && flags[i]) ++c;
+    if (i < n && keep(i)) ++c;
   }
   long long tot;
   block_exclusive_scan<long long>(c, ws, &tot);
@@ -131,14 +142,14 @@ __global__ void k_tile_scan_i64(const long long* __restrict__ in, long long* __r
   }
 }
 
-__global__ void k_tile_compact_u8(const uint8_t* __restrict__ flags, int n, int* __restrict__ list,
-                                  const long long* tile) {
+template <class Keep>
+__global__ void k_tile_compact(Keep keep, int n, int* __restrict__ list, const long long* tile) {
   __shared__ uint8_t sf[kTile];
   __shared__ long long ws[TRN_THREADS / 32];
   const long long base = (long long) blockIdx.x * kTile;
   for (int k = threadIdx.x; k < kTile; k += TRN_THREADS) {
     long long i = base + k;
-    sf[k] = (i < n && flags[i]) ? 1 : 0;
+    sf[k] = (i < n && keep(i)) ? 1 : 0;
   }
   __syncthreads();
   long long c = 0;
@@ -179,19 +190,28 @@ void scan_i64(const long long* in, long long* out, int n, ScanWs& ws, cudaStream
   note_launch();
 }
 
-void compact_u8(const uint8_t* flags, int n, int* list, ScanWs& ws, cudaStream_t s) {
+template <class Keep>
+static void compact(const Keep& keep, int n, int* list, ScanWs& ws, int* count, double bytes, cudaStream_t s) {
   int ntiles = (n + kTile - 1) / kTile;
   if (ntiles == 0) {
-    cudaMemsetAsync(ws.count, 0, sizeof(int), s);
+    cudaMemsetAsync(count, 0, sizeof(int), s);
     return;
   }
-  ProfScope ps("compact", s, (double) n * 2);
-  k_tile_count_u8<<<ntiles, TRN_THREADS, 0, s>>>(flags, n, ws.tile);
+  ProfScope ps("compact", s, bytes);
+  k_tile_count<<<ntiles, TRN_THREADS, 0, s>>>(keep, n, ws.tile);
   note_launch();
-  k_scan_tiles<<<1, TRN_THREADS, 0, s>>>(ws.tile, ntiles, nullptr, ws.count);
+  k_scan_tiles<<<1, TRN_THREADS, 0, s>>>(ws.tile, ntiles, nullptr, count);
   note_launch();
-  k_tile_compact_u8<<<ntiles, TRN_THREADS, 0, s>>>(flags, n, list, ws.tile);
+  k_tile_compact<<<ntiles, TRN_THREADS, 0, s>>>(keep, n, list, ws.tile);
   note_launch();
+}
+
+void compact_u8(const uint8_t* flags, int n, int* list, ScanWs& ws, cudaStream_t s, int* count) {
+  compact(KeepFlag{flags}, n, list, ws, count ? count : ws.count, (double) n * 2, s);
+}
+
+void compact_tris(const DMesh& m, int nb_elems, int* list, ScanWs& ws, cudaStream_t s) {
+  compact(KeepTri{m.tri}, nb_elems, list, ws, ws.count, (double) nb_elems * 2 * kTri, s);
 }
 
 static const Tune kDefaultTune;

@@ -3,9 +3,10 @@
  *
  *   k_count_fill   : vertex -> element stencils from the triangle array
  *                    (Mesh::rebuildTopology, mesh.cpp:197-210: atomic append)
- *   k_sort_stencil : sort each stencil (mesh.cpp:244)
- *   k_build_vicin  : sorted unique vertex adjacency from the stencil
- *                    (mesh.cpp:214-243 and Mesh::extractPrimalGraph 297-330)
+ *   k_sort_stencils: sort each stencil (mesh.cpp:244) and build its adjacency
+ *   k_build_vicin  : sorted unique vertex adjacency from the stencil, flagged
+ *                    vertices (mesh.cpp:214-243 and Mesh::extractPrimalGraph
+ *                    297-330)
  *   k_fix_tagged   : the fused stencil repair of Mesh::fixTagged
  *                    (mesh.cpp:716-760): keep the entries whose element still
  *                    holds the vertex, sort, drop duplicates, in one pass over
@@ -29,23 +30,87 @@ __global__ void k_fill_stencils(DMesh m, int nb_elems) {
   }
 }
 
+/* the sorted row of each vertex (the fill's order is arbitrary), and its
+ * adjacency, which needs no other row: up to 8 entries in registers */
 __global__ void k_sort_stencils(DMesh m, int nb_nodes) {
   if (trn_failed(m)) return;
-  int buf[TRN_MAX_DEG];
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    int d = trn_deg(m, v);
+    const int d = trn_deg(m, v);
     const TrnRow s = trn_row(m.stenc, m, v);
-    for (int a = 0; a < d; ++a) buf[a] = s[a];
-    trn_isort(buf, d);
-    for (int a = 0; a < d; ++a) s[a] = buf[a];
+    if (d <= kRowChunk) {
+      int4* p = reinterpret_cast<int4*>(s.p);
+      const int4 a = d > 0 ? p[0] : make_int4(0, 0, 0, 0), b = d > 4 ? p[1] : make_int4(0, 0, 0, 0);
+      int r[kRowChunk] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int k = 0; k < kRowChunk; ++k)
+        if (k >= d) r[k] = 0x7fffffff;
+      patch_sort8(r);
+      if (d > 0) p[0] = make_int4(r[0], r[1], r[2], r[3]);
+      if (d > 4) p[1] = make_int4(r[4], r[5], r[6], r[7]);
+    } else {
+      int buf[TRN_MAX_DEG];
+      for (int a = 0; a < d; ++a) buf[a] = s[a];
+      trn_isort(buf, d);
+      for (int a = 0; a < d; ++a) s[a] = buf[a];
+    }
+    build_one_vicin(m, v);
   }
 }
 
-__global__ void k_build_vicin(DMesh m, int nb_nodes, int only_flagged) {
+/* everything a load sets before the stencils, in one launch where it was a
+ * dozen clears and copies: what is read before it is written. The tensors of
+ * the vertices in use (an export before the first recovery), points, tags and
+ * elements from the input's copies, counts and flags over the capacity. Rows
+ * are read up to their counts; a new vertex or element is written whole when
+ * it gets its slot, but for its flags. 16 flag bytes a store (the flag arrays
+ * have 16 bytes to spare). Bound by launches on small meshes and by
+ * the bytes on large ones. Measured with the rows' sort and adjacency in one
+ * kernel and the export's single read back: reload, one smoothing and export
+ * of a 600 x 600 grid 2057 -> 1929 us, the same with one coarsening of a
+ * 501 x 501 grid (mixed) 2150 -> 2026 us. */
+__global__ void k_load_init(DMesh m, const double2* __restrict__ pts, const int4* __restrict__ tri,
+                            const uint8_t* __restrict__ tags, int nb_nodes, int nb_elems, int* status) {
+  const int tid = trn_tid(), stride = trn_grid_stride();
+  for (int i = tid; i < S_SIZE; i += stride)
+    status[i] = i == S_NB ? nb_nodes : (i == S_NB + 1 ? nb_elems : 0);
+  const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
+  for (int v = tid; v < nb_nodes; v += stride) {
+    m.pts[v] = pts[v];
+    m.ten[v] = zero;
+    m.lten[v] = zero;
+  }
+  for (int e = tid; e < nb_elems; e += stride) {
+    m.tri[e] = tri[e];
+    m.qual[e] = 0.0;
+  }
+  for (int v = tid; v < m.capa_node; v += stride) m.deg[v] = m.vdeg[v] = 0;
+  const uint4 none = make_uint4(0, 0, 0, 0), ones = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
+  const int nv16 = (m.capa_node + 15) / 16, na16 = (max(m.capa_node, m.capa_elem) + 15) / 16;
+  for (int k = tid; k < nv16; k += stride) {
+    reinterpret_cast<uint4*>(m.alive)[k] = ones;
+    reinterpret_cast<uint4*>(m.fixes)[k] = none;
+    uint4 t = none;
+    if (16 * k < nb_nodes) {
+      uint8_t* b = reinterpret_cast<uint8_t*>(&t);
+      for (int j = 0; j < 16 && 16 * k + j < nb_nodes; ++j) b[j] = tags[16 * k + j];
+    }
+    reinterpret_cast<uint4*>(m.tags)[k] = t;
+  }
+  for (int k = tid; k < na16; k += stride) reinterpret_cast<uint4*>(m.activ)[k] = none;
+}
+
+void load_init(const DMesh& m, const double2* pts, const int4* tri, const uint8_t* tags, int nb_nodes, int nb_elems,
+               int* status, cudaStream_t s) {
+  k_load_init<<<grid_for(std::max(m.capa_node, nb_elems)), TRN_THREADS, 0, s>>>(m, pts, tri, tags, nb_nodes, nb_elems,
+                                                                                status);
+  note_launch();
+}
+
+__global__ void k_build_vicin(DMesh m, int nb_nodes) {
   nb_nodes = trn_nodes(m, nb_nodes);
   if (trn_failed(m)) return;
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
-    if (only_flagged && m.activ[v] == 0) continue;
+    if (m.activ[v] == 0) continue;
     build_one_vicin(m, v);
   }
 }
@@ -172,10 +237,6 @@ __global__ void k_pack_nodes(DMesh m, const int* __restrict__ list, const int* c
   }
 }
 
-__global__ void k_flag_live_tris(DMesh m, int nb_elems, uint8_t* __restrict__ flag) {
-  for (int i = trn_tid(); i < nb_elems; i += trn_grid_stride()) flag[i] = m.tri[i].x >= 0 ? 1 : 0;
-}
-
 __global__ void k_pack_tris(DMesh m, const int* __restrict__ list, const int* count,
                             const int* __restrict__ newid, int* __restrict__ out) {
   const int n = *count;
@@ -222,20 +283,15 @@ void pack_tris_load(const DMesh& m, const int* list, const int* count, const int
   note_launch();
 }
 
-void pack_nodes(const DMesh& m, const int* list, const int* count, int* newid, double* pts, double* ten,
+void pack_nodes(const DMesh& m, const int* list, const int* count, int n, int* newid, double* pts, double* ten,
                 cudaStream_t s) {
-  k_pack_nodes<<<grid_for(m.capa_node), TRN_THREADS, 0, s>>>(m, list, count, newid, pts, ten);
+  k_pack_nodes<<<grid_for(n), TRN_THREADS, 0, s>>>(m, list, count, newid, pts, ten);
   note_launch();
 }
 
-void flag_live_tris(const DMesh& m, int nb_elems, uint8_t* flag, cudaStream_t s) {
-  k_flag_live_tris<<<grid_for(nb_elems), TRN_THREADS, 0, s>>>(m, nb_elems, flag);
-  note_launch();
-}
-
-void pack_tris(const DMesh& m, const int* list, const int* count, const int* newid, int* out,
+void pack_tris(const DMesh& m, const int* list, const int* count, int n, const int* newid, int* out,
                cudaStream_t s) {
-  k_pack_tris<<<grid_for(m.capa_elem), TRN_THREADS, 0, s>>>(m, list, count, newid, out);
+  k_pack_tris<<<grid_for(n), TRN_THREADS, 0, s>>>(m, list, count, newid, out);
   note_launch();
 }
 
@@ -247,7 +303,6 @@ void count_live(const DMesh& m, int nb_nodes, int nb_elems, int* out, cudaStream
 
 void build_stencils(const DMesh& m, int nb_nodes, int nb_elems, cudaStream_t s) {
   ProfScope ps("build_stencils", s, 3.0 * nb_elems * (kTri + 2 * kIdx) + 2.0 * nb_nodes * kIdx);
-  cudaMemsetAsync(m.deg, 0, sizeof(int) * (size_t) m.capa_node, s);
   k_fill_stencils<<<TRN_RESIDENT(k_fill_stencils, grid_for(nb_elems), TRN_THREADS), TRN_THREADS, 0, s>>>(m, nb_elems);
   note_launch();
   k_sort_stencils<<<TRN_RESIDENT(k_sort_stencils, grid_for(nb_nodes), TRN_THREADS), TRN_THREADS, 0, s>>>(m, nb_nodes);
@@ -255,9 +310,9 @@ void build_stencils(const DMesh& m, int nb_nodes, int nb_elems, cudaStream_t s) 
   check_launch("build_stencils");
 }
 
-void build_vicin(const DMesh& m, int nb_nodes, bool only_flagged, cudaStream_t s) {
+void build_vicin(const DMesh& m, int nb_nodes, cudaStream_t s) {
   ProfScope ps("build_vicin", s, (double) nb_nodes * (1 + 2 * kIdx + kAvgDeg * (kIdx + kTri + kIdx)));
-  k_build_vicin<<<TRN_RESIDENT(k_build_vicin, grid_for(nb_nodes), TRN_THREADS), TRN_THREADS, 0, s>>>(m, nb_nodes, only_flagged ? 1 : 0);
+  k_build_vicin<<<TRN_RESIDENT(k_build_vicin, grid_for(nb_nodes), TRN_THREADS), TRN_THREADS, 0, s>>>(m, nb_nodes);
   note_launch();
   check_launch("build_vicin");
 }

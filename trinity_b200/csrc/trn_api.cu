@@ -312,7 +312,7 @@ int trn_mesh_create_ex(const int size[2], int bucket, int depth, int verbosity, 
       (rc = dmalloc(m, &d.tri, ce)) ||
       (rc = dmalloc(m, &d.stenc, trn_row_ints(cn, bucket))) || (rc = dmalloc(m, &d.deg, cn)) ||
       (rc = dmalloc(m, &d.vic, trn_row_ints(cn, bucket))) || (rc = dmalloc(m, &d.vdeg, cn)) ||
-      (rc = dmalloc(m, &d.tags, cn)) || (rc = dmalloc(m, &d.alive, cn)) ||
+      (rc = dmalloc(m, &d.tags, cn + 16)) || (rc = dmalloc(m, &d.alive, cn + 16)) ||
       (rc = dmalloc(m, &d.fixes, cn + 16)) || (rc = dmalloc(m, &d.activ, std::max(cn, ce) + 16)) ||
       (rc = dmalloc(m, &d.qual, ce)) || (rc = dmalloc(m, &m->solut, cn)) ||
       (rc = dmalloc(m, &m->grad, cn)) || (rc = dmalloc(m, &m->terms, ce + 8192)) ||
@@ -351,32 +351,13 @@ int trn_mesh_destroy(trn_mesh* m) {
 /* state of a freshly loaded mesh from the device copies pts0/tri0/tags0 */
 static int init_from_device(trn_mesh* m) {
   DMesh& d = m->d;
-  const size_t cn = (size_t) m->capa_node, ce = (size_t) m->capa_elem;
   const int nb_nodes = m->n0_nodes, nb_elems = m->n0_elems;
   cudaStream_t s = m->stream;
-  /* only what is read before it is written: the tensors of the vertices in
-   * use (an export before the first recovery), the counts and the flags.
-   * Rows are read up to their counts; a new vertex or element is written
-   * whole when it gets its slot, but for its flags. */
-  CK(cudaMemsetAsync(d.ten, 0, sizeof(double4) * (size_t) nb_nodes, s));
-  CK(cudaMemsetAsync(d.lten, 0, sizeof(double4) * (size_t) nb_nodes, s));
-  CK(cudaMemsetAsync(d.vdeg, 0, sizeof(int) * cn, s));
-  CK(cudaMemsetAsync(d.tags, 0, cn, s));
-  CK(cudaMemsetAsync(d.alive, 1, cn, s));
-  CK(cudaMemsetAsync(d.fixes, 0, cn, s));
-  CK(cudaMemsetAsync(d.activ, 0, std::max(cn, ce), s));
-  CK(cudaMemsetAsync(d.qual, 0, sizeof(double) * (size_t) nb_elems, s));
-  CK(cudaMemsetAsync(m->status, 0, sizeof(int) * S_SIZE, s));
-  const int counts[2] = {nb_nodes, nb_elems};
-  CK(cudaMemcpyAsync(m->status + S_NB, counts, sizeof(counts), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(d.pts, m->pts0, sizeof(double2) * (size_t) nb_nodes, cudaMemcpyDeviceToDevice, s));
-  CK(cudaMemcpyAsync(d.tri, m->tri0, sizeof(int4) * (size_t) nb_elems, cudaMemcpyDeviceToDevice, s));
-  CK(cudaMemcpyAsync(d.tags, m->tags0, (size_t) nb_nodes, cudaMemcpyDeviceToDevice, s));
+  load_init(d, m->pts0, m->tri0, m->tags0, nb_nodes, nb_elems, m->status, s);
   m->nb_nodes = nb_nodes;
   m->nb_elems = nb_elems;
   m->cursor = 0;
   build_stencils(d, nb_nodes, nb_elems, s);
-  build_vicin(d, nb_nodes, false, s);
   return sync_status(m);
 }
 
@@ -653,22 +634,27 @@ int trn_mesh_export_compact(trn_mesh* m, double* points, int* tris, double* tens
   if (!m || !nb_nodes || !nb_elems) return fail(m, TRN_ERR_INVALID, "export_compact: null argument");
   cudaStream_t s = m->stream;
   DMesh& d = m->d;
-  compact_u8(d.alive, m->nb_nodes, m->list, m->scan, s);
-  int rc = sync_status(m, m->scan.count);
+  /* both lists before the one read back of their lengths; the element list
+   * goes to the matching's pair buffer */
+  int* elist = m->pairs;
+  compact_u8(d.alive, m->nb_nodes, m->list, m->scan, s, m->scan.count + 1);
+  compact_tris(d, m->nb_elems, elist, m->scan, s);
+  CK(cudaMemcpyAsync(m->h_status + H_WIDE, m->scan.count, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  int rc = sync_status(m);
   if (rc) return rc;
-  const int nv = m->h_status[S_COUNT];
+  const int ne = m->h_status[H_WIDE], nv = m->h_status[H_WIDE + 1];
+  const size_t node_bytes = sizeof(double) * (tensor ? 5 : 2) * (size_t) nv;
   double* st_pts = reinterpret_cast<double*>(m->stage);
   double* st_ten = reinterpret_cast<double*>(m->stage) + 2 * (size_t) nv;
-  pack_nodes(d, m->list, m->scan.count, m->target, st_pts, tensor ? st_ten : nullptr, s);
+  pack_nodes(d, m->list, m->scan.count + 1, nv, m->target, st_pts, tensor ? st_ten : nullptr, s);
   if (points) CK(cudaMemcpyAsync(points, st_pts, sizeof(double) * 2 * (size_t) nv, cudaMemcpyDeviceToHost, s));
   if (tensor) CK(cudaMemcpyAsync(tensor, st_ten, sizeof(double) * 3 * (size_t) nv, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  flag_live_tris(d, m->nb_elems, m->flag, s);
-  compact_u8(m->flag, m->nb_elems, m->list, m->scan, s);
-  if ((rc = sync_status(m, m->scan.count))) return rc;
-  const int ne = m->h_status[S_COUNT];
-  int* st_tri = reinterpret_cast<int*>(m->stage);
-  pack_tris(d, m->list, m->scan.count, m->target, st_tri, s);
+  /* the triangles behind the vertices where the staging buffer holds both,
+   * else over them once they are out (the stream's order) */
+  const size_t stage_bytes = std::max(40 * (size_t) m->capa_node, 12 * (size_t) m->capa_elem);
+  const size_t at = node_bytes + sizeof(int) * 3 * (size_t) ne <= stage_bytes ? node_bytes : 0;
+  int* st_tri = reinterpret_cast<int*>(m->stage + at);
+  pack_tris(d, elist, m->scan.count, ne, m->target, st_tri, s);
   if (tris) CK(cudaMemcpyAsync(tris, st_tri, sizeof(int) * 3 * (size_t) ne, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   *nb_nodes = nv;
@@ -695,10 +681,9 @@ int trn_mesh_compact(trn_mesh* m) {
   int rc = sync_status(m, m->scan.count);
   if (rc) return rc;
   const int nv = m->h_status[S_COUNT];
-  flag_live_tris(d, m->nb_elems, m->flag, s);
   /* the element list goes to the stage buffer: m->list still holds the vertices */
   int* elist = reinterpret_cast<int*>(m->stage);
-  compact_u8(m->flag, m->nb_elems, elist, m->scan, s);
+  compact_tris(d, m->nb_elems, elist, m->scan, s);
   if ((rc = sync_status(m, m->scan.count))) return rc;
   const int ne = m->h_status[S_COUNT];
   if (nv <= 0 || ne <= 0) return fail(m, TRN_ERR_INVALID, "compact: empty mesh");
@@ -1065,7 +1050,7 @@ int trn_coarsen_run(trn_mesh* m, int max_colors, trn_stats* st) {
   coarsen_pre(m->d, m->nb_nodes, s);
   int eval = 0, task = 0, nb_indep = 0, level = 0;
   do {
-    build_vicin(m->d, m->nb_nodes, true, s);
+    build_vicin(m->d, m->nb_nodes, s);
     coarsen_filter(m->d, m->nb_nodes, m->target, m->flag, m->fp32, s);
     compact_u8(m->flag, m->nb_nodes, m->list, m->scan, s);
     int rc = sync_status(m, m->scan.count);
@@ -1147,7 +1132,7 @@ int trn_smooth_run(trn_mesh* m, int max_colors, int depth, trn_stats* st) {
   begin_timing(m);
   cudaStream_t s = m->stream;
   smooth_pre(m->d, m->nb_nodes, s);
-  build_vicin(m->d, m->nb_nodes, true, s);
+  build_vicin(m->d, m->nb_nodes, s);
   std::vector<std::pair<const int*, int>> classes;
   if (m->replay) {
     size_t off;
@@ -1239,7 +1224,7 @@ int trn_smooth_gradient_run(trn_mesh* m, int max_colors, int steps, double max_l
   begin_timing(m);
   cudaStream_t s = m->stream;
   smooth_pre(m->d, m->nb_nodes, s);
-  build_vicin(m->d, m->nb_nodes, true, s);
+  build_vicin(m->d, m->nb_nodes, s);
   color_jp(m->d, m->nb_nodes, max_col, seed_of(m, 0xc01dULL), m->hws, m->parts, m->status + S_PARTS,
            reinterpret_cast<unsigned*>(m->status + S_TICK), s);
   int rc = sync_status(m);
@@ -1331,7 +1316,7 @@ int capture_round(trn_mesh* m, int depth) {
     });
   stage_stats(2);
   smooth_pre(m->d, m->capa_node, s);
-  build_vicin(m->d, m->capa_node, true, s);
+  build_vicin(m->d, m->capa_node, s);
   color_begin(m->d, m->capa_node, m->hws, s);
   if (e == cudaSuccess)
     e = capture_loop(s, bs, [&](cudaStream_t b, cudaGraphConditionalHandle h) {

@@ -131,8 +131,10 @@ void scan_ws_free(ScanWs* ws);
 void scan_i64(const long long* in, long long* out, int n, ScanWs& ws, cudaStream_t s,
               const int* dn = nullptr);
 /* ordered compaction: list[k] = i for the k-th i < n with flags[i] != 0;
- * *ws.count receives the number kept */
-void compact_u8(const uint8_t* flags, int n, int* list, ScanWs& ws, cudaStream_t s);
+ * *count (*ws.count when null) receives the number kept */
+void compact_u8(const uint8_t* flags, int n, int* list, ScanWs& ws, cudaStream_t s, int* count = nullptr);
+/* the same of the live elements (tri[i].x >= 0) */
+void compact_tris(const DMesh& m, int nb_elems, int* list, ScanWs& ws, cudaStream_t s);
 
 /* mesh files (mesh_io.cu): an input mesh as loaded (0-based triangles,
  * boundary / corner tags) */
@@ -153,8 +155,14 @@ int write_mesh_binary(const char* path, long nv, long nt, const double* pts, con
                       const int* tris);
 
 /* topology (topology.cu) */
+/* a mesh's state before its stencils, from the device copies of its input */
+void load_init(const DMesh& m, const double2* pts, const int4* tri, const uint8_t* tags, int nb_nodes, int nb_elems,
+               int* status, cudaStream_t s);
+/* stencils of the elements (counts cleared before), their sorted rows and the
+ * adjacency */
 void build_stencils(const DMesh& m, int nb_nodes, int nb_elems, cudaStream_t s);
-void build_vicin(const DMesh& m, int nb_nodes, bool only_flagged, cudaStream_t s);
+/* the adjacency of the flagged vertices */
+void build_vicin(const DMesh& m, int nb_nodes, cudaStream_t s);
 void fix_tagged(const DMesh& m, int nb_nodes, cudaStream_t s);
 void flag_all_alive(const DMesh& m, int nb_nodes, cudaStream_t s);
 void quality_all(const DMesh& m, int nb_elems, bool fp32, cudaStream_t s);
@@ -162,16 +170,15 @@ void quality_all(const DMesh& m, int nb_elems, bool fp32, cudaStream_t s);
 void log_cache(const DMesh& m, int nb_nodes, bool fp32, cudaStream_t s);
 void count_live(const DMesh& m, int nb_nodes, int nb_elems, int* out, cudaStream_t s);
 void expand_tris(const int* raw, int nb_elems, int nb_nodes, int4* out, int* err, cudaStream_t s);
-void pack_nodes(const DMesh& m, const int* list, const int* count, int* newid, double* pts, double* ten,
+void pack_nodes(const DMesh& m, const int* list, const int* count, int n, int* newid, double* pts, double* ten,
                 cudaStream_t s);
-void flag_live_tris(const DMesh& m, int nb_elems, uint8_t* flag, cudaStream_t s);
 /* the listed live vertices (points, tags) and elements (renumbered through
  * newid) packed as a load would place them */
 void pack_nodes_load(const DMesh& m, const int* list, const int* count, int* newid, double2* pts,
                      uint8_t* tags, cudaStream_t s);
 void pack_tris_load(const DMesh& m, const int* list, const int* count, const int* newid, int4* out,
                     cudaStream_t s);
-void pack_tris(const DMesh& m, const int* list, const int* count, const int* newid, int* out,
+void pack_tris(const DMesh& m, const int* list, const int* count, int n, const int* newid, int* out,
                cudaStream_t s);
 
 /* metric (metric.cu) */
