@@ -585,9 +585,16 @@ __device__ __forceinline__ bool color_item(const DMesh& m, int v, int* color, ui
   const int mine = round > 0 ? prev[v] : 0;
   bool keep = mine != 0;
   unsigned used = 0, wanted = 0;
-  for (int b = 0; b < nv; ++b) {
-    const int w = vc[b];
-    const int cw = *(volatile int*) (color + w);
+  /* the row's first chunk in two loads and its neighbours' words before any
+   * of them is looked at; few vertices have more (a coloring of 491 401
+   * vertices 220 -> 194 us, against one word after the other) */
+  const int4* rp = reinterpret_cast<const int4*>(vc.p);
+  const int4 ra = rp[0], rb = nv > 4 ? rp[1] : make_int4(v, v, v, v);
+  const int w8[kRowChunk] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+  int c8[kRowChunk];
+#pragma unroll
+  for (int b = 0; b < kRowChunk; ++b) c8[b] = b < nv ? (int) *(volatile int*) (color + w8[b]) : (int) kNotColored;
+  auto look = [&](int w, int cw) {
     const int rw = cw >> 8;
     if (cw == 0 || rw == round + 1) {
       if (round > 0 && trn_prio(seed, w) > pv) {
@@ -598,6 +605,13 @@ __device__ __forceinline__ bool color_item(const DMesh& m, int v, int* color, ui
     } else {
       used |= 1u << (cw & 0xff & 31);
     }
+  };
+#pragma unroll
+  for (int b = 0; b < kRowChunk; ++b)
+    if (b < nv) look(w8[b], c8[b]);
+  for (int b = kRowChunk; b < nv; ++b) {
+    const int w = vc[b];
+    look(w, *(volatile int*) (color + w));
   }
   if (keep && !(used & (1u << mine))) {
     color[v] = ((round + 1) << 8) | mine;
@@ -875,8 +889,103 @@ __global__ void __launch_bounds__(kFusedThreads) k_color_persist(DMesh m, int* l
   }
 }
 
+/* The whole coloring of a small mesh by one cluster: the vertices that wait
+ * are bits of their thread's mask, a round is the mask's vertices and a
+ * barrier, and the classes are counted, placed and cleared at the end. Every
+ * vertex's rounds are color_item's, so the colors are those of the grid's
+ * rounds. Bound by the rounds' chain of row, colors and tentatives in L2 and
+ * the barrier; the ten launches of the grid's form and its barrier over all
+ * multiprocessors cost more below some 45 000 vertices: 441 vertices 67 ->
+ * 29 us, 10 201 103 -> 56, 32 761 124 -> 82, 48 841 115 -> 109, and the
+ * other way round above, 68 121 120 -> 150 (one cluster then has too few
+ * threads for the first rounds). At most 32 vertices a thread of the smallest
+ * cluster. */
+constexpr int kColorCluster = 40960;
+
+__global__ void __launch_bounds__(kTailThreads) k_color_cluster(DMesh m, int nb_nodes, int* color, uint8_t* tent,
+                                                               int max_col, Seed sd, int* more, int* keys,
+                                                               int* parts, int* part_off, unsigned* tick) {
+  __shared__ int cnt[kColorKeys], base[kColorKeys], off[kColorKeys];
+  const int tid = trn_tid(), stride = trn_grid_stride();
+  const uint64_t seed = trn_seed(sd);
+  for (int k = threadIdx.x; k < kColorKeys; k += blockDim.x) cnt[k] = 0;
+  for (int k = tid; k < kColorKeys; k += stride) keys[k] = 0;
+  if (tid < 3) more[tid] = 0;
+  unsigned open = 0;
+  const bool failed = trn_failed(m);
+  for (int k = 0, v = tid; v < nb_nodes; ++k, v += stride) {
+    if (m.activ[v] == 1 && m.vdeg[v] > 0) open |= 1u << k;
+    else color[v] = kNotColored;
+  }
+  if (failed) open = 0;
+  cluster_sync();
+  for (int round = 0; round < kColorTailRounds; ++round) {
+    if (round > 0 && tail_word(more + round % 3) == 0) break;
+    if (tid == 0) more[(round + 2) % 3] = 0;   /* the round after next's word */
+    for (unsigned left = open; left; left &= left - 1) {
+      const int k = __ffs(left) - 1;
+      if (!color_item(m, tid + k * stride, color, tent, m.capa_node, max_col, seed, round)) open &= ~(1u << k);
+    }
+    if (open) more[(round + 1) % 3] = 1;
+    cluster_sync();
+  }
+  /* the classes: counts by key, each block's share of a key reserved */
+  for (int v = tid; v < nb_nodes; v += stride) {
+    const int cw = color[v];
+    if (cw != 0 && (cw & 0xff) >= 1 && (cw & 0xff) <= max_col) atomicAdd(cnt + color_key(m, v, cw & 0xff), 1);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < kColorKeys; k += blockDim.x) {
+    if (cnt[k] > 0) base[k] = atomicAdd(keys + k, cnt[k]);
+    cnt[k] = 0;
+  }
+  cluster_sync();
+  /* lane c of a block's first warp: where color c's bins begin */
+  if (threadIdx.x < 32) {
+    const int c = threadIdx.x;
+    int n[kDegBins], size = 0;
+    for (int b = 0; b < kDegBins; ++b) {
+      n[b] = *(volatile int*) (keys + c * kDegBins + b);
+      size += n[b];
+    }
+    int end = size;
+    for (int d = 1; d < 32; d <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, end, d);
+      if (c >= d) end += o;
+    }
+    int at = end - size;
+    if (blockIdx.x == 0) {
+      if (c >= 1 && c <= max_col) part_off[c - 1] = at;
+      if (c == max_col) part_off[max_col] = end;
+      if (c == 0 && tick) ++*tick;
+    }
+    for (int b = 0; b < kDegBins; ++b) {
+      off[c * kDegBins + b] = at;
+      at += n[b];
+    }
+  }
+  __syncthreads();
+  for (int v = tid; v < nb_nodes; v += stride) {
+    const int cw = color[v];
+    if (cw != 0 && (cw & 0xff) >= 1 && (cw & 0xff) <= max_col) {
+      const int key = color_key(m, v, cw & 0xff);
+      parts[off[key] + base[key] + atomicAdd(cnt + key, 1)] = v;
+    }
+    color[v] = 0;
+  }
+}
+
 void color_jp(const DMesh& m, int hint, int max_col, Seed sd, HeurWs& ws, int* parts, int* part_off,
               unsigned* tick, cudaStream_t s) {
+  cudaStreamCaptureStatus cs;
+  if (hint <= kColorCluster && cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
+    ProfScope ps("color_jp", s, 0.0);
+    if (cluster_launch<k_color_cluster>(s, m, hint, ws.color, ws.tent, max_col, sd, ws.cnt + 104, ws.color_keys, parts,
+                                        part_off, tick)) {
+      check_launch("color_jp");
+      return;
+    }
+  }
   color_begin(m, hint, ws, s);
   bool done;
   {

@@ -329,9 +329,11 @@ void mis_jp_rounds(const DMesh& m, const int* cand, const int* count, int rounds
 /* speculative first-fit coloring of interior vertices (tentative colors,
  * priority conflicts resolved round by round), colors 1..max_col;
  * parts: vertex ids grouped by color, part_off[c] offsets (c = 0..max_col).
- * hint: grid size (at least the vertex count). color_jp runs batches of 8
- * rounds while vertices wait (at most 8 batches), reading the decision back
- * after each; a captured round runs color_batch inside a loop node instead.
+ * hint: grid size (at least the vertex count). color_jp colors a small mesh in
+ * one cluster launch, a larger one in one cooperative launch; where neither
+ * can run, batches of 8 rounds while vertices wait (at most 8 batches),
+ * reading the decision back after each; a captured round runs color_batch
+ * inside a loop node instead.
  * color_finish advances *tick (the seeds' counter). */
 void color_jp(const DMesh& m, int hint, int max_col, Seed seed, HeurWs& ws, int* parts,
               int* part_off, unsigned* tick, cudaStream_t s);
