@@ -33,13 +33,13 @@ namespace trn {
 __global__ void k_elem_gradient(DMesh m, int nb_elems, const double* __restrict__ solut,
                                 double4* __restrict__ rec) {
   if (trn_failed(m)) return;
-  for (int t = trn_tid(); t < nb_elems; t += trn_grid_stride()) rec[t] = elem_gradient(m, t, solut);
+  for (int t = trn_tid(); t < nb_elems; t += trn_grid_stride()) rec_store(rec, t, kRecMix, elem_gradient(m, t, solut));
 }
 
 __global__ void k_elem_hessian(DMesh m, int nb_elems, const double2* __restrict__ grad,
                                double4* __restrict__ rec) {
   if (trn_failed(m)) return;
-  for (int t = trn_tid(); t < nb_elems; t += trn_grid_stride()) rec[t] = elem_hessian(m, t, grad);
+  for (int t = trn_tid(); t < nb_elems; t += trn_grid_stride()) rec_store(rec, t, kRecMix, elem_hessian(m, t, grad));
 }
 
 /* ---- the mixed-precision form of the recovery ----
@@ -66,9 +66,10 @@ __global__ void k_elem_edges(DMesh m, int nb_elems, float4* __restrict__ rec) {
     /* rotated edges: area x d[2j] = 2 ey[j], area x d[2j+1] = 2 ex[j] */
     const float c0 = (float) (p1.x - p0.x), c1 = (float) (p2.x - p0.x);
     const float c2 = (float) (p1.y - p0.y), c3 = (float) (p2.y - p0.y);
-    rec[2 * (size_t) i] = make_float4(0.5f * (c0 * c3 - c1 * c2), (float) (p1.y - p2.y), (float) (p2.y - p0.y),
+    const size_t at = rec_slot(i, kRecMix);
+    rec[at] = make_float4(0.5f * (c0 * c3 - c1 * c2), (float) (p1.y - p2.y), (float) (p2.y - p0.y),
                                       (float) (p0.y - p1.y));
-    rec[2 * (size_t) i + 1] = make_float4((float) (p2.x - p1.x), (float) (p0.x - p2.x), (float) (p1.x - p0.x), 0.f);
+    rec[at ^ 1] = make_float4((float) (p2.x - p1.x), (float) (p0.x - p2.x), (float) (p1.x - p0.x), 0.f);
   }
 }
 
@@ -85,7 +86,8 @@ struct GradSum32 {
   __device__ __forceinline__ void begin(const DMesh&, int v) { uv = solut[v]; }
   __device__ __forceinline__ Rec load(const DMesh& m, int i) const {
     const int4 t = m.tri[i];
-    return Rec{{rec[2 * (size_t) i], rec[2 * (size_t) i + 1]}, {solut[t.x], solut[t.y], solut[t.z]}};
+    const size_t at = rec_slot(i, kRecMix);
+    return Rec{{rec[at], rec[at ^ 1]}, {solut[t.x], solut[t.y], solut[t.z]}};
   }
   __device__ __forceinline__ void add(const Rec& r) {
     const float s[3] = {(float) (r.u[0] - uv), (float) (r.u[1] - uv), (float) (r.u[2] - uv)};
@@ -112,7 +114,8 @@ struct HessSum32 {
   __device__ __forceinline__ void begin(const DMesh&, int v) { gv = grad[v]; }
   __device__ __forceinline__ Rec load(const DMesh& m, int i) const {
     const int4 t = m.tri[i];
-    return Rec{{rec[2 * (size_t) i], rec[2 * (size_t) i + 1]}, {grad[t.x], grad[t.y], grad[t.z]}};
+    const size_t at = rec_slot(i, kRecMix);
+    return Rec{{rec[at], rec[at ^ 1]}, {grad[t.x], grad[t.y], grad[t.z]}};
   }
   __device__ __forceinline__ void add(const Rec& r) {
     tot += r.e.a.x;
@@ -143,15 +146,26 @@ struct HessSum32 {
 };
 
 constexpr int kPatchThreads = 128;
+constexpr int kPatchIds = 48;   /* an interior patch of these rows has 42 at most */
+constexpr int kPatchBatch = 4;  /* records in flight a thread (2: 5% slower at 100 k vertices; 8: spills) */
 
-/* a vertex whose rows do not fit goes onto rest[*rest_n] (when given; the
+/* The merged ids go to shared memory, so that the sums are a loop over the
+ * patch instead of 64 predicated slots and the merge's registers are free
+ * again: 5 blocks a multiprocessor where the sums over the registers had 3 (4
+ * are as fast, 6 spill in single precision). Bound by the shared-memory data
+ * path's wavefronts (80% of its peak before rec_slot mixed the records'
+ * banks). Recovery of 1 002 001 vertices 517 us, 480 with the column, 445 with
+ * the mixed records; of 101 124 vertices in single precision 140, 126, 116.
+ * A vertex whose rows do not fit goes onto rest[*rest_n] (when given; the
  * second pass over the same rows finds the same ones) */
-template <class Sum, int Batch>
-__global__ void __launch_bounds__(kPatchThreads) k_patch_sum(DMesh m, int nb_nodes, Sum zero, int* rest,
-                                                             int* rest_n) {
+template <class Sum>
+__global__ void __launch_bounds__(kPatchThreads, 5) k_patch_sum(DMesh m, int nb_nodes, Sum zero, int* rest,
+                                                                int* rest_n) {
+  __shared__ int s_ids[kPatchIds * kPatchThreads];
   if (trn_failed(m)) return;
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride())
-    if (!patch_sum_regs<Sum, Batch>(m, v, zero) && rest) trn_append(rest, rest_n, v);
+    if (!patch_sum_column<Sum, kPatchBatch, kPatchIds, kPatchThreads>(m, v, zero, s_ids + threadIdx.x) && rest)
+      trn_append(rest, rest_n, v);
 }
 
 /* the listed vertices, a warp each */
@@ -264,10 +278,10 @@ void sum_tree(const double* in, int n, double* partial, double* out, cudaStream_
 /* a patch mean: the elements' records are ready in ws.rec; the vertices
  * that the register merge cannot take are listed by the first pass (collect)
  * and served by the second kernel, which returns at once when there are none */
-template <int Batch, class Sum>
+template <class Sum>
 static void patch_sum(const DMesh& m, int nb_nodes, const Sum& zero, const MetricWs& ws, bool collect,
                       cudaStream_t s) {
-  auto* fast = k_patch_sum<Sum, Batch>;
+  auto* fast = k_patch_sum<Sum>;
   auto* rest = k_patch_sum_rest<Sum>;
   fast<<<TRN_RESIDENT(fast, grid_for(nb_nodes, kPatchThreads), kPatchThreads), kPatchThreads, 0, s>>>(
       m, nb_nodes, zero, collect ? ws.rest : nullptr, ws.rest_n);
@@ -289,11 +303,11 @@ void metric_patches(const DMesh& m, int nb_nodes, int nb_elems, const double* so
     k_elem_edges<<<ge, TRN_THREADS, 0, s>>>(m, nb_elems, rec);
     note_launch();
     GradSum32 z{rec, solut, grad};
-    patch_sum<2>(m, nb_nodes, z, ws, true, s);
+    patch_sum(m, nb_nodes, z, ws, true, s);
     }
     ProfScope ps("metric_hessian", s, V * (2 * kIdx + kAvgDeg * kIdx * 2 + 16 + kPt + kTen) + E * kTri);
     HessSum32 z{rec, grad, (float) scale_exp};
-    patch_sum<2>(m, nb_nodes, z, ws, false, s);
+    patch_sum(m, nb_nodes, z, ws, false, s);
     return;
   }
   double* atot = keep && keep->atot ? keep->atot : ws.atot;
@@ -301,14 +315,14 @@ void metric_patches(const DMesh& m, int nb_nodes, int nb_elems, const double* so
   ProfScope ps("metric_gradient", s, V * (2 * kIdx + kAvgDeg * kIdx * 2 + 8 + kPt + 16) + E * kTri);
   k_elem_gradient<<<ge, TRN_THREADS, 0, s>>>(m, nb_elems, solut, ws.rec);
   note_launch();
-  GradSum z{ws.rec, grad, atot};
-  patch_sum<4>(m, nb_nodes, z, ws, true, s);
+  GradSum z{ws.rec, kRecMix, grad, atot};
+  patch_sum(m, nb_nodes, z, ws, true, s);
   }
   ProfScope ps("metric_hessian", s, V * (2 * kIdx + kAvgDeg * kIdx * 2 + 16 + kPt + kTen) + E * kTri);
   k_elem_hessian<<<ge, TRN_THREADS, 0, s>>>(m, nb_elems, grad, ws.rec);
   note_launch();
-  HessSum z{ws.rec, atot, scale_exp, keep ? keep->hsym : nullptr, keep ? keep->mloc : nullptr};
-  patch_sum<4>(m, nb_nodes, z, ws, false, s);
+  HessSum z{ws.rec, kRecMix, atot, scale_exp, keep ? keep->hsym : nullptr, keep ? keep->mloc : nullptr};
+  patch_sum(m, nb_nodes, z, ws, false, s);
 }
 
 void metric_complexity(const DMesh& m, int nb_elems, double* terms, double* partial, double* complexity,

@@ -174,8 +174,8 @@ __global__ void __launch_bounds__(kTailThreads) k_na_recover(DMesh d, int nb_nod
     for (int i = tid; i < nb_elems; i += stride) ws.rec[i] = elem_gradient(d, i, solut);
   }
   cluster_sync();
-  const GradSum gsum{ws.rec, grad, ws.atot};
-  const HessSum hsum{ws.rec, ws.atot, scale_exp, nullptr, nullptr};
+  const GradSum gsum{ws.rec, 0, grad, ws.atot};
+  const HessSum hsum{ws.rec, 0, ws.atot, scale_exp, nullptr, nullptr};
   const bool go = !tail_failed(d);
   if (go)
     for (int v = tid; v < nb_nodes; v += stride)

@@ -223,7 +223,8 @@ void refine_ws_alloc(RefineWs* ws, int capa_node, int capa_elem) {
   /* one block of 32 bytes an element: the metric recovery keeps its element
    * records there between refinements */
   const size_t ce = (size_t) capa_elem;
-  cudaMalloc(&ws->info, (sizeof(int4) + 2 * sizeof(long long)) * ce);
+  /* with the rest of a 128-byte line: the metric's records are mixed within one */
+  cudaMalloc(&ws->info, (sizeof(int4) + 2 * sizeof(long long)) * ce + 128);
   ws->cnt = reinterpret_cast<long long*>(ws->info + ce);
   ws->off = ws->cnt + ce;
   unsigned long long cap = 1024;

@@ -18,7 +18,31 @@ namespace trn {
  * integer merge of the rows. One vertex a thread that gathered, sorted in
  * local memory and computed every element of its patch took 582 us for the
  * gradient and 650 us for the Hessian of the 2M-triangle mesh; records and
- * register merge take 30 + 194 and 30 + 202 us (cold caches). */
+ * register merge take 163 and 175 us, the records' kernels included. */
+/* Where the first 16 bytes of element i's record are, in units of 16 bytes;
+ * the second are at the slot ^ 1. With `mix` (kRecMix; the buffer then has
+ * room for a multiple of 4 records) the 8 slots of a 128-byte line are
+ * exchanged by the line's number: the threads of a warp gather the records of
+ * neighbouring vertices' elements, about two elements and so 64 bytes apart,
+ * and would meet in two of the eight slots of a line, a quarter of the banks.
+ * A record keeps its sector. */
+constexpr unsigned kRecMix = 7;
+__device__ __forceinline__ size_t rec_slot(int i, unsigned mix) { return ((size_t) i * 2) ^ (((unsigned) i >> 2) & mix); }
+
+__device__ __forceinline__ void rec_store(double4* rec, int i, unsigned mix, const double4& r) {
+  double2* p = reinterpret_cast<double2*>(rec);
+  const size_t at = rec_slot(i, mix);
+  p[at] = make_double2(r.x, r.y);
+  p[at ^ 1] = make_double2(r.z, r.w);
+}
+
+__device__ __forceinline__ double4 rec_load(const double4* rec, int i, unsigned mix) {
+  const double2* p = reinterpret_cast<const double2*>(rec);
+  const size_t at = rec_slot(i, mix);
+  const double2 a = p[at], b = p[at ^ 1];
+  return make_double4(a.x, a.y, b.x, b.y);
+}
+
 __device__ __forceinline__ double4 elem_gradient(const DMesh& m, int t, const double* solut) {
   if (m.tri[t].x < 0) return make_double4(0.0, 0.0, 0.0, 0.0);
   const ElemGrad g = elem_grad(m, t);
@@ -59,12 +83,13 @@ __device__ __forceinline__ double4 elem_hessian(const DMesh& m, int t, const dou
  * interleaving its loops keeps every sum's order. */
 struct GradSum {
   const double4* rec;
+  unsigned mix;   /* of the records (rec_slot) */
   double2* grad;
   double* atot;   /* patch areas, for the Hessian's mean too */
   double total_area = 0, gx = 0, gy = 0;
   using Rec = double4;
   __device__ __forceinline__ void begin(const DMesh&, int) {}
-  __device__ __forceinline__ Rec load(const DMesh&, int t) const { return rec[t]; }
+  __device__ __forceinline__ Rec load(const DMesh&, int t) const { return rec_load(rec, t, mix); }
   __device__ __forceinline__ void add(const Rec& r) {
     total_area += r.x;
     gx += r.y;
@@ -80,6 +105,7 @@ struct GradSum {
 
 struct HessSum {
   const double4* rec;
+  unsigned mix;
   const double* atot;   /* the gradient pass's sums: the same areas in the same order */
   double scale_exp;
   double4* hsym;
@@ -87,7 +113,7 @@ struct HessSum {
   double h[4] = {0, 0, 0, 0};
   using Rec = double4;
   __device__ __forceinline__ void begin(const DMesh&, int) {}
-  __device__ __forceinline__ Rec load(const DMesh&, int t) const { return rec[t]; }
+  __device__ __forceinline__ Rec load(const DMesh&, int t) const { return rec_load(rec, t, mix); }
   __device__ __forceinline__ void add(const Rec& r) {
     h[0] += r.x;
     h[1] += r.y;
@@ -135,6 +161,37 @@ __device__ __forceinline__ bool patch_sum_regs(const DMesh& m, int v, const Sum&
 #pragma unroll
     for (int j = 0; j < Batch; ++j)
       if (key[c + j] != kNoId && (c + j == 0 || key[c + j] != key[c + j - 1])) s.add(r[j]);
+  }
+  s.finish(m, v);
+  return true;
+}
+
+/* the same with the patch's ids, duplicates dropped, in the thread's own
+ * column of shared memory (Ids entries, Stride apart); false also when they
+ * are more */
+template <class Sum, int Batch, int Ids, int Stride>
+__device__ __forceinline__ bool patch_sum_column(const DMesh& m, int v, const Sum& zero, int* col) {
+  int n = 0;
+  {
+    int key[kPatchKeys];
+    if (!patch_keys(m, v, key)) return false;
+#pragma unroll
+    for (int c = 0; c < kPatchKeys; ++c)
+      if (key[c] != kNoId && (c == 0 || key[c] != key[c - 1])) {
+        if (n < Ids) col[n * Stride] = key[c];
+        ++n;
+      }
+  }
+  if (n > Ids) return false;
+  Sum s = zero;
+  s.begin(m, v);
+  for (int c = 0; c < n; c += Batch) {
+    typename Sum::Rec r[Batch];
+#pragma unroll
+    for (int j = 0; j < Batch; ++j) r[j] = s.load(m, col[min(c + j, n - 1) * Stride]);
+#pragma unroll
+    for (int j = 0; j < Batch; ++j)
+      if (c + j < n) s.add(r[j]);
   }
   s.finish(m, v);
   return true;
