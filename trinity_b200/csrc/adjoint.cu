@@ -897,14 +897,44 @@ __global__ void __launch_bounds__(128) k_smooth_gradient(DMesh m, const int* __r
   trn_warp_add(counters + 1, commit * (gl == 0));
 }
 
+/* A class longer than this is moved by one lane a vertex: it fills the chip
+ * so, and the eight lanes' idle two and their shuffles only cost. Five steps,
+ * one lane / eight lanes / by the rule: 500 x 500 quads 4.5 / 4.0 / 4.0 ms,
+ * 700 x 700 7.2 / 7.7 / 6.9, 1000 x 1000 12.3 / 15.8 / 11.7; in single precision
+ * 2.7 / 2.3 / 2.3, 4.1 / 4.1 / 3.2, 6.7 / 8.0 / 5.8. The one-lane form is bound by
+ * its chain of dependent loads and arithmetic: four blocks a multiprocessor
+ * (128 registers; at 142 three fit: 14.0 ms) and in single precision eight. */
+constexpr int kGradOne64 = 90112, kGradOne32 = 73728;
+
+template <bool F32>
+__global__ void __launch_bounds__(128, F32 ? 8 : 4) k_smooth_gradient_one(DMesh m, const int* __restrict__ list, int n,
+                                                             double max_len, int mode, int* counters) {
+  if (trn_failed_block(m)) return;
+  int tasks = 0, commit = 0;
+  for (int q = trn_tid(); q < n; q += trn_grid_stride()) {
+    const int v = list[q];
+    if (v < 0 || v >= m.capa_node) {
+      trn_set_error(m.err, TRN_DERR_INVALID);
+      continue;
+    }
+    if (!m.activ[v] || trn_deg(m, v) == 0) continue;
+    tasks++;
+    commit += move_gradient<F32>(m, v, max_len, mode);
+  }
+  trn_warp_add(counters, tasks);
+  trn_warp_add(counters + 1, commit);
+}
+
 void smooth_gradient_color(const DMesh& m, const int* list, int n, double max_len, int mode,
                            int* counters, bool fp32, cudaStream_t s) {
   if (n <= 0) return;
   const double own = 4 + 1 + 4 + 2 * kPt + kTen + kAvgDeg * (kIdx + kTri + 2 * kQ);
   const double nbr = (double) std::min<long long>((long long) m.capa_node, 6LL * n) * (kPt + kTen);
   ProfScope ps("smooth_gradient", s, n * own + nbr);
-  auto* kern = fp32 ? k_smooth_gradient<true> : k_smooth_gradient<false>;
-  kern<<<grid_for((long long) kGradLanes * n, 128), 128, 0, s>>>(m, list, n, max_len, mode, counters);
+  const bool one = n > (fp32 ? kGradOne32 : kGradOne64);
+  auto* kern = one ? (fp32 ? k_smooth_gradient_one<true> : k_smooth_gradient_one<false>)
+                   : (fp32 ? k_smooth_gradient<true> : k_smooth_gradient<false>);
+  kern<<<grid_for(one ? n : (long long) kGradLanes * n, 128), 128, 0, s>>>(m, list, n, max_len, mode, counters);
   note_launch();
   check_launch("smooth_gradient");
 }

@@ -88,7 +88,7 @@ void fix_list_level_end(const DMesh& m, const int* list, const int* count, long 
  * in FP64. Each mesh keeps its own table; the C-ABI entry that drives a mesh makes it the calling
  * thread's table for the launchers. */
 struct Tune {
-  int smooth_threads = 256;   /* k_smooth_move block: 64, 128, 256 */
+  int smooth_threads = 256;   /* k_smooth_move_grp block: 64, 128, 256 */
   int filter_threads = 128;   /* one-lane collapse-target search block: 128, 256, 512 */
   int group_lanes = 16;       /* lanes per vertex of the grouped search: 1 (one-lane search), 4, 8, 16 */
   int group_max = 16384;      /* longest level list the grouped search takes */
