@@ -505,7 +505,9 @@ template <class Sink>
 __device__ __forceinline__ void collapse_group(const DMesh& m, int source, int destin, const Sink& sink) {
   const int lane = threadIdx.x & 31, gl = lane & (kCollapseLanes - 1), g0 = lane & ~(kCollapseLanes - 1);
   const unsigned gm = 0xffu << g0;
-  const int deg = trn_deg(m, source);
+  /* through a shuffle: every lane has read the count before the first lane's
+   * serial collapse can clear it, and all of them take the same branch */
+  const int deg = __shfl_sync(gm, trn_deg(m, source), 0, kCollapseLanes);
   if (deg > kCollapseLanes * kCollapseEach) {
     if (gl == 0) collapse_serial(m, source, destin);
     __syncwarp(gm);

@@ -75,7 +75,9 @@ constexpr int kFixLanes = 16;
 
 __device__ __forceinline__ void fix_stencil_group(const DMesh& m, int v, unsigned gm, int* buf) {
   const int gl = threadIdx.x & (kFixLanes - 1);
-  const int d = trn_deg(m, v);
+  /* through a shuffle: every lane has read the count before the first lane's
+   * serial repair can change it, and all of them take the same branch */
+  const int d = __shfl_sync(gm, trn_deg(m, v), 0, kFixLanes);
   if (d > 2 * kFixLanes) {
     if (gl == 0) fix_stencil(m, v, buf);
     __syncwarp(gm);
