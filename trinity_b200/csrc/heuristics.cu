@@ -747,13 +747,13 @@ __global__ void k_color_offsets(const int* cnt, int* part_off, int* cursor, int 
   if (tick) ++*tick;
   int acc = 0;
   for (int c = 1; c <= max_col; ++c) {
-    part_off[c - 1] = acc;
+    if (c <= kClasses + 1) part_off[c - 1] = acc;
     for (int b = 0; b < kDegBins; ++b) {
       cursor[c * kDegBins + b] = acc;
       acc += cnt[c * kDegBins + b];
     }
   }
-  part_off[max_col] = acc;
+  if (max_col <= kClasses) part_off[max_col] = acc;
 }
 
 /* vertices into their color's part, by degree bin; per block, the slots are
@@ -955,8 +955,8 @@ __global__ void __launch_bounds__(kTailThreads) k_color_cluster(DMesh m, int nb_
     }
     int at = end - size;
     if (blockIdx.x == 0) {
-      if (c >= 1 && c <= max_col) part_off[c - 1] = at;
-      if (c == max_col) part_off[max_col] = end;
+      if (c >= 1 && c <= max_col && c <= kClasses + 1) part_off[c - 1] = at;
+      if (c == max_col && c <= kClasses) part_off[c] = end;
       if (c == 0 && tick) ++*tick;
     }
     for (int b = 0; b < kDegBins; ++b) {

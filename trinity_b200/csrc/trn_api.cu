@@ -1150,7 +1150,7 @@ int trn_smooth_run(trn_mesh* m, int max_colors, int depth, trn_stats* st) {
              reinterpret_cast<unsigned*>(m->status + S_TICK), s);
     int rc = sync_status(m);
     if (rc) return rc;
-    for (int c = 0; c < max_col && c < 8; ++c) {
+    for (int c = 0; c < max_col && c < kClasses; ++c) {
       int a = m->h_status[S_PARTS + c], b = m->h_status[S_PARTS + c + 1];
       classes.emplace_back(m->parts + a, b - a);
     }
@@ -1230,7 +1230,7 @@ int trn_smooth_gradient_run(trn_mesh* m, int max_colors, int steps, double max_l
   int rc = sync_status(m);
   if (rc) return rc;
   std::vector<std::pair<const int*, int>> classes;
-  for (int c = 0; c < max_col && c < 8; ++c) {
+  for (int c = 0; c < max_col && c < kClasses; ++c) {
     int a = m->h_status[S_PARTS + c], b = m->h_status[S_PARTS + c + 1];
     classes.emplace_back(m->parts + a, b - a);
   }
@@ -1326,7 +1326,7 @@ int capture_round(trn_mesh* m, int depth) {
   quality_all(m->d, m->capa_elem, m->fp32, s);
   cudaMemsetAsync(m->status + S_SMOOTH_TASKS, 0, sizeof(int) * 2, s);
   for (int level = 0; level < depth; ++level)
-    for (int c = 0; c < max_col && c < 8; ++c)
+    for (int c = 0; c < max_col && c < kClasses; ++c)
       smooth_class(m->d, m->parts, m->status + S_PARTS, c, m->capa_node, m->status + S_SMOOTH_TASKS,
                    m->fp32, s);
   cudaMemcpyAsync(m->rstats + 6, m->status + S_SMOOTH_TASKS, sizeof(int) * 2, cudaMemcpyDeviceToDevice, s);

@@ -40,6 +40,9 @@ enum StatusSlot {
   S_RDONE = 31,    /* and refinement's "a level split nothing" */
   S_SIZE = 32,
 };
+/* the color classes that are smoothed: S_PARTS has an offset for each and the
+ * last one's end. Colors above (Partit allows 30) are given but not smoothed. */
+constexpr int kClasses = 8;
 constexpr int kLevelCoarsen = 0, kLevelSwap = 1;
 constexpr int kLevelCap = 100000;
 
@@ -328,7 +331,8 @@ void mis_jp_rounds(const DMesh& m, const int* cand, const int* count, int rounds
                    HeurWs& ws, int* indep, int* nindep, cudaStream_t s, long long bound = -1);
 /* speculative first-fit coloring of interior vertices (tentative colors,
  * priority conflicts resolved round by round), colors 1..max_col;
- * parts: vertex ids grouped by color, part_off[c] offsets (c = 0..max_col).
+ * parts: vertex ids grouped by color, part_off[c] offsets (c = 0 .. max_col, at
+ * most kClasses).
  * hint: grid size (at least the vertex count). color_jp colors a small mesh in
  * one cluster launch, a larger one in one cooperative launch; where neither
  * can run, batches of 8 rounds while vertices wait (at most 8 batches),
