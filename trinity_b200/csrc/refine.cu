@@ -161,6 +161,10 @@ __global__ void k_ref_cut(DMesh m, int nb_elems, const int4* __restrict__ info,
     const int s[3] = {h_get(hkey, hval, hcap, n[1], n[2]), h_get(hkey, hval, hcap, n[2], n[0]),
                       h_get(hkey, hval, hcap, n[0], n[1])};
     int offset = nb_elems + (int) (off[id] & 0xffffffffLL);
+    /* a split count that disagrees with the edge map (possible only when the
+     * two sides of an edge measure it differently) leaves the element uncut
+     * instead of reading vertex -1, and the slots it had reserved erased */
+    bool cut = false;
     if (pattern == 1) {
       const int t[2] = {id, offset};
       for (int i = 0; i < 3; ++i) {
@@ -171,6 +175,7 @@ __global__ void k_ref_cut(DMesh m, int nb_elems, const int4* __restrict__ info,
           trn_stenc_append(m, n[k], t[1]);
           put_tri(m, t[0], n[i], n[j], s[i]);
           put_tri(m, t[1], n[i], s[i], n[k]);
+          cut = true;
           break;
         }
       }
@@ -179,9 +184,6 @@ __global__ void k_ref_cut(DMesh m, int nb_elems, const int4* __restrict__ info,
       for (int i = 0; i < 3; ++i) {
         if (s[i] < 0) {
           int j = (i + 1) % 3, k = (i + 2) % 3;
-          /* a split count that disagrees with the edge map (possible only when
-           * the two sides of an edge measure it differently) leaves the
-           * element uncut instead of reading vertex -1 */
           if (s[j] < 0 || s[k] < 0) break;
           double diag0 = length_x<F32>(m.pts[n[j]], m.pts[s[j]], ten_load<F32>(m, n[j]), ten_load<F32>(m, s[j]));
           double diag1 = length_x<F32>(m.pts[n[k]], m.pts[s[k]], ten_load<F32>(m, n[k]), ten_load<F32>(m, s[k]));
@@ -197,11 +199,11 @@ __global__ void k_ref_cut(DMesh m, int nb_elems, const int4* __restrict__ info,
           put_tri(m, t[0], n[i], s[k], s[j]);
           put_tri(m, t[1], n[j], n[k], s[v]);
           put_tri(m, t[2], s[j], s[k], n[v]);
+          cut = true;
           break;
         }
       }
-    } else {
-      if (s[0] < 0 || s[1] < 0 || s[2] < 0) continue;
+    } else if (s[0] >= 0 && s[1] >= 0 && s[2] >= 0) {
       const int t[4] = {id, offset, offset + 1, offset + 2};
       const int a0[3] = {t[1], t[2], t[3]};
       const int a1[3] = {t[0], t[2], t[3]};
@@ -215,7 +217,10 @@ __global__ void k_ref_cut(DMesh m, int nb_elems, const int4* __restrict__ info,
       put_tri(m, t[1], n[1], s[0], s[2]);
       put_tri(m, t[2], n[2], s[1], s[0]);
       put_tri(m, t[3], s[0], s[1], s[2]);
+      cut = true;
     }
+    if (!cut)
+      for (int k = 0; k < pattern; ++k) put_tri(m, offset + k, -1, -1, -1);
   }
 }
 
