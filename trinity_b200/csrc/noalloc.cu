@@ -27,7 +27,8 @@
  * local L^p scaling, complexity with the fixed-shape tree sum, global
  * scaling; trn_metric.cuh), so the tensors are identical to it when that
  * mesh also sums with the tree (its default; exact_sum and replay sum in
- * element order). The kernel runs on the caller's stream with the address
+ * element order): in one launch of one cluster, or by its kernels where many
+ * vertices have long rows. They run on the caller's stream with the address
  * looked up for the current device, so the stream must belong to it.
  */
 #include "trn_internal.h"
@@ -47,7 +48,7 @@ namespace {
 constexpr size_t kMaxN = TRN_NOALLOC_MAX_NODES;
 constexpr size_t kMaxE = TRN_NOALLOC_MAX_ELEMS;
 constexpr size_t kB = TRN_NOALLOC_BUCKET;
-constexpr size_t kPartials = 256;  /* one per 256 elements */
+constexpr size_t kPartials = 256;  /* one per 256 elements; the sum behind them (grid form) */
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t) 255; }
 
@@ -62,10 +63,10 @@ constexpr size_t oVdeg = oDeg + align256(sizeof(int) * kMaxN);
 constexpr size_t oAlive = oVdeg + align256(sizeof(int) * kMaxN);
 constexpr size_t oGrad = oAlive + align256(kMaxN);
 constexpr size_t oTerms = oGrad + align256(sizeof(double2) * kMaxN);
-constexpr size_t oRec = oTerms + align256(sizeof(double) * kPartials);
+constexpr size_t oRec = oTerms + align256(sizeof(double) * (kPartials + 1));
 constexpr size_t oAtot = oRec + align256(sizeof(double4) * kMaxE);
 constexpr size_t oRest = oAtot + align256(sizeof(double) * kMaxN);
-constexpr size_t oErr = oRest + align256(sizeof(int) * (kMaxN + 1));
+constexpr size_t oErr = oRest + align256(sizeof(int) * kMaxN);   /* the error word, the length of the list at oRest */
 constexpr size_t kScratchBytes = oErr + 256;
 
 }  // namespace
@@ -97,6 +98,53 @@ int scratch_address(unsigned char** out) {
   return TRN_OK;
 }
 
+/* the steps before the recovery, for one vertex or element; the calls of one
+ * step before any of the next */
+__device__ __forceinline__ void na_vertex(const DMesh& d, int v, const double* points) {
+  d.pts[v] = make_double2(points[2 * v], points[2 * v + 1]);
+  d.deg[v] = d.vdeg[v] = 0;
+  d.alive[v] = 1;
+}
+
+__device__ __forceinline__ void na_elem(const DMesh& d, int i, int nb_nodes, const int* tris) {
+  const int a = tris[3 * i], b = tris[3 * i + 1], c = tris[3 * i + 2];
+  const bool ok = a >= 0 && a < nb_nodes && b >= 0 && b < nb_nodes && c >= 0 && c < nb_nodes;
+  if (!ok) atomicExch(d.err, TRN_DERR_INVALID);   /* before an overfull vertex, whichever is met first */
+  d.tri[i] = ok ? make_int4(a, b, c, 0) : make_int4(-1, -1, -1, 0);
+  if (!ok) return;
+  trn_stenc_append(d, a, i);
+  trn_stenc_append(d, b, i);
+  trn_stenc_append(d, c, i);
+}
+
+/* the sorted row, and the adjacency from it and the elements alone */
+__device__ __forceinline__ void na_row(const DMesh& d, int v) {
+  const TrnRow row = trn_row(d.stenc, d, v);
+  const int n = trn_deg(d, v);
+  if (n <= kRowChunk) {
+    int r[kRowChunk];
+#pragma unroll
+    for (int k = 0; k < kRowChunk; ++k) r[k] = k < n ? row.p[k] : kNoId;
+    patch_sort8(r);
+#pragma unroll
+    for (int k = 0; k < kRowChunk; ++k)
+      if (k < n) row.p[k] = r[k];
+  } else {
+    int r[TRN_NOALLOC_BUCKET];
+    for (int k = 0; k < n; ++k) r[k] = row[k];
+    trn_isort(r, n);
+    for (int k = 0; k < n; ++k) row[k] = r[k];
+  }
+  build_one_vicin(d, v);
+}
+
+__device__ __forceinline__ void na_out(const DMesh& d, int v, double fact, double eig_min, double eig_max, double* out) {
+  const double4 r = normalize_tensor(d.ten[v], fact, eig_min, eig_max);
+  out[3 * v] = r.x;
+  out[3 * v + 1] = r.y;
+  out[3 * v + 2] = r.z;
+}
+
 /* The whole recovery in one launch of one thread-block cluster: at most 16,384
  * vertices are two a thread, so each step is a few dependent gathers, and as
  * fifteen launches and four clears they cost five times that. The steps are
@@ -107,6 +155,16 @@ int scratch_address(unsigned char** out) {
  * computes for itself. 441 vertices 105 -> 67 us a call, 16,129
  * vertices 187 (before the element records) -> 110. */
 constexpr int kNaPart = TRN_THREADS;
+
+/* vertices of long rows that the cluster's 256 warps take, one after the
+ * other: with more of them the kernel stops and the call goes on with
+ * metric_run's kernels over the whole chip (na_recover_grid). Every triangle
+ * of a grid cut into three at its centre (no row fits the registers), us a
+ * call, cluster / grid after the cluster's start: 1,241 vertices 197 / 201,
+ * 2,761 332 / 204, 10,921 1,100 / 289, 15,697 1,566 / 336; adapted meshes, a
+ * quarter of whose rows are long: 4,083 vertices 128 / 183, 8,186 159 / 198,
+ * 10,923 197 / 211. */
+constexpr int kNaRest = 2048;
 
 __device__ __forceinline__ double na_tree(double* sm, double s, int t) {
   sm[t] = s;
@@ -134,43 +192,12 @@ __global__ void __launch_bounds__(kTailThreads) k_na_recover(DMesh d, int nb_nod
     *d.err = 0;
     *ws.rest_n = 0;
   }
-  for (int v = tid; v < nb_nodes; v += stride) {
-    d.pts[v] = make_double2(points[2 * v], points[2 * v + 1]);
-    d.deg[v] = d.vdeg[v] = 0;
-    d.alive[v] = 1;
-  }
+  for (int v = tid; v < nb_nodes; v += stride) na_vertex(d, v, points);
   cluster_sync();
-  for (int i = tid; i < nb_elems; i += stride) {
-    const int a = tris[3 * i], b = tris[3 * i + 1], c = tris[3 * i + 2];
-    const bool ok = a >= 0 && a < nb_nodes && b >= 0 && b < nb_nodes && c >= 0 && c < nb_nodes;
-    if (!ok) atomicExch(d.err, TRN_DERR_INVALID);   /* before an overfull vertex, whichever is met first */
-    d.tri[i] = ok ? make_int4(a, b, c, 0) : make_int4(-1, -1, -1, 0);
-    if (!ok) continue;
-    trn_stenc_append(d, a, i);
-    trn_stenc_append(d, b, i);
-    trn_stenc_append(d, c, i);
-  }
+  for (int i = tid; i < nb_elems; i += stride) na_elem(d, i, nb_nodes, tris);
   cluster_sync();
   if (!tail_failed(d)) {
-    for (int v = tid; v < nb_nodes; v += stride) {
-      const TrnRow row = trn_row(d.stenc, d, v);
-      const int n = trn_deg(d, v);
-      if (n <= kRowChunk) {
-        int r[kRowChunk];
-#pragma unroll
-        for (int k = 0; k < kRowChunk; ++k) r[k] = k < n ? row.p[k] : kNoId;
-        patch_sort8(r);
-#pragma unroll
-        for (int k = 0; k < kRowChunk; ++k)
-          if (k < n) row.p[k] = r[k];
-      } else {
-        int r[TRN_NOALLOC_BUCKET];
-        for (int k = 0; k < n; ++k) r[k] = row[k];
-        trn_isort(r, n);
-        for (int k = 0; k < n; ++k) row[k] = r[k];
-      }
-      build_one_vicin(d, v);   /* its own stencil and the elements alone */
-    }
+    for (int v = tid; v < nb_nodes; v += stride) na_row(d, v);
     for (int i = tid; i < nb_elems; i += stride) ws.rec[i] = elem_gradient(d, i, solut);
   }
   cluster_sync();
@@ -182,6 +209,7 @@ __global__ void __launch_bounds__(kTailThreads) k_na_recover(DMesh d, int nb_nod
       if (!patch_sum_regs<GradSum, 4>(d, v, gsum)) trn_append(ws.rest, ws.rest_n, v);
   cluster_sync();
   const int nr = *ws.rest_n;
+  if (nr > kNaRest) return;   /* every thread: too many for the cluster's warps */
   for (int q = tid >> 5; q < nr; q += stride >> 5)
     patch_sum_warp(d, ws.rest[q], gsum, s_buf[threadIdx.x >> 5]);
   cluster_sync();
@@ -205,15 +233,49 @@ __global__ void __launch_bounds__(kTailThreads) k_na_recover(DMesh d, int nb_nod
   const double complexity = na_tree(s_tree[half], t < parts ? 0 + partial[t] : 0.0, t);
   if (tail_failed(d)) return;
   const double fact = target / complexity;
-  for (int v = tid; v < nb_nodes; v += stride) {
-    const double4 r = normalize_tensor(d.ten[v], fact, eig_min, eig_max);
-    out[3 * v] = r.x;
-    out[3 * v + 1] = r.y;
-    out[3 * v + 2] = r.z;
-  }
+  for (int v = tid; v < nb_nodes; v += stride) na_out(d, v, fact, eig_min, eig_max, out);
 }
 
 static_assert(kMaxE <= (size_t) kNaPart * kNaPart, "one tree over the partials");
+
+/* the same steps as launches of their own, around metric_run's kernels */
+__global__ void k_na_vertices(DMesh d, int nb_nodes, const double* __restrict__ points) {
+  if (trn_tid() == 0) *d.err = 0;
+  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) na_vertex(d, v, points);
+}
+
+__global__ void k_na_elems(DMesh d, int nb_nodes, int nb_elems, const int* __restrict__ tris) {
+  for (int i = trn_tid(); i < nb_elems; i += trn_grid_stride()) na_elem(d, i, nb_nodes, tris);
+}
+
+__global__ void k_na_rows(DMesh d, int nb_nodes) {
+  if (trn_failed(d)) return;
+  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) na_row(d, v);
+}
+
+__global__ void k_na_tensors(DMesh d, int nb_nodes, const double* complexity, double target, double eig_min,
+                             double eig_max, double* __restrict__ out) {
+  if (trn_failed(d)) return;
+  const double fact = target / *complexity;
+  for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) na_out(d, v, fact, eig_min, eig_max, out);
+}
+
+void na_recover_grid(const DMesh& d, int nb_nodes, int nb_elems, const double* points, const int* tris,
+                     const double* solut, double2* grad, const MetricWs& ws, double* partial, double target,
+                     double scale_exp, double eig_min, double eig_max, double* out, cudaStream_t s) {
+  const int gv = grid_for(nb_nodes), ge = grid_for(nb_elems);
+  double* complexity = partial + kPartials;
+  k_na_vertices<<<gv, TRN_THREADS, 0, s>>>(d, nb_nodes, points);
+  note_launch();
+  k_na_elems<<<ge, TRN_THREADS, 0, s>>>(d, nb_nodes, nb_elems, tris);
+  note_launch();
+  k_na_rows<<<gv, TRN_THREADS, 0, s>>>(d, nb_nodes);
+  note_launch();
+  metric_patches(d, nb_nodes, nb_elems, solut, grad, ws, scale_exp, s);
+  metric_complexity(d, nb_elems, nullptr, partial, complexity, false, s);
+  k_na_tensors<<<gv, TRN_THREADS, 0, s>>>(d, nb_nodes, complexity, target, eig_min, eig_max, out);
+  note_launch();
+}
 
 }  // namespace
 }  // namespace trn
@@ -259,15 +321,23 @@ extern "C" int trn_metric_noalloc(int nb_nodes, int nb_elems, const double* d_po
   const double eig_min = 1 / trn_pow(h_min, 2);
   const double eig_max = 1 / trn_pow(h_max, 2);
   int* rest = reinterpret_cast<int*>(base + oRest);
-  const MetricWs ws{reinterpret_cast<double4*>(base + oRec), reinterpret_cast<double*>(base + oAtot), rest + 1, rest};
+  const MetricWs ws{reinterpret_cast<double4*>(base + oRec), reinterpret_cast<double*>(base + oAtot), rest, d.err + 1};
   if (!cluster_launch<k_na_recover>(s, d, nb_nodes, nb_elems, d_points, d_tris, d_solut, grad, ws, terms, target,
                                     scale_exp, eig_min, eig_max, d_tensor))
     return TRN_ERR_CUDA;
 
-  int err = 0;
-  if (cudaMemcpyAsync(&err, d.err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-      cudaStreamSynchronize(s) != cudaSuccess)
-    return TRN_ERR_CUDA;
+  int word[2] = {0, 0};   /* the error word, the vertices that the cluster's warps had to take */
+  const int& err = word[0];
+  auto read_back = [&](size_t n) {
+    return cudaMemcpyAsync(word, d.err, n, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+           cudaStreamSynchronize(s) == cudaSuccess;
+  };
+  if (!read_back(sizeof(word))) return TRN_ERR_CUDA;
+  if (!err && word[1] > kNaRest) {
+    na_recover_grid(d, nb_nodes, nb_elems, d_points, d_tris, d_solut, grad, ws, terms, target, scale_exp, eig_min,
+                    eig_max, d_tensor, s);
+    if (cudaPeekAtLastError() != cudaSuccess || !read_back(sizeof(int))) return TRN_ERR_CUDA;
+  }
   if (err == TRN_DERR_CAPACITY || err == TRN_DERR_BUCKET) {
     std::fprintf(stderr, "trn_metric_noalloc: a vertex has more than %d incident triangles\n",
                  TRN_NOALLOC_BUCKET);
