@@ -21,8 +21,8 @@
  * Patch order matters: the reference sums over the patch in ascending element
  * id (std::set order, mesh.cpp:396-432), so the union of the stencils of the
  * vertex and of its neighbours is sorted and deduplicated first
- * (trn_patch.cuh): in registers where the rows are short, by a warp for the
- * vertices that the first pass lists as not fitting.
+ * (trn_patch.cuh): in registers where the rows are short, by a warp or a lane
+ * for the vertices that the first pass lists as not fitting.
  */
 #include "trn_internal.h"
 #include "trn_metric.cuh"
@@ -168,13 +168,47 @@ __global__ void __launch_bounds__(kPatchThreads, 5) k_patch_sum(DMesh m, int nb_
       trn_append(rest, rest_n, v);
 }
 
-/* the listed vertices, a warp each */
+/* The listed vertices, a warp each, or, where they are many and a good part of
+ * the mesh, a lane each. A warp is quick about one patch but spends 32 lanes on
+ * its serial sum: 2.4 to 6 ns a vertex, by the patch's length and the form,
+ * against a lane's 1 ns behind some 100 us of latency. Lists that are long but
+ * a small part of the mesh are spread over it, and a lane's gathers are then
+ * alone on their cache lines. us a recovery, warps / lanes, FP64 and (mixed):
+ * triangles cut in three (every vertex listed) 19,361 vertices 261 / 224 (343 /
+ * 237), 36,521 386 / 253 (594 / 299), 270,601 2,208 / 683 (3,604 / 846); random
+ * points (45 % listed) 60,000 302 / 409 (483 / 494), 250,000 866 / 743 (1,588 /
+ * 1,071); an adapted mesh (15 %) of 354,918 453 / 611 (634 / 772). */
+constexpr int kRestWarps = 32768;
+/* records in flight a lane: at 4 the 80-byte records of the mixed form take 102
+ * registers, and the warps' branch of the same kernel pays (1,611 -> 2,078 us
+ * at 120,401 listed vertices) */
 template <class Sum>
-__global__ void __launch_bounds__(kPatchThreads) k_patch_sum_rest(DMesh m, Sum zero, const int* rest,
-                                                                  const int* rest_n) {
+constexpr int kRestBatch = sizeof(typename Sum::Rec) > 32 ? 2 : 4;
+
+template <class Sum>
+__global__ void __launch_bounds__(kPatchThreads) k_patch_sum_rest(DMesh m, int nb_nodes, Sum zero,
+                                                                  const int* rest, const int* rest_n) {
   __shared__ int s_buf[kPatchThreads / 32][TRN_MAX_PATCH];
   if (trn_failed(m)) return;
   const int n = *rest_n;
+  if (n > kRestWarps && 4LL * n > nb_nodes) {
+    int ids[TRN_MAX_PATCH];
+    for (int q = trn_tid(); q < n; q += trn_grid_stride()) {
+      const int v = rest[q], k = patch_sort_lane(m, v, ids);
+      Sum s = zero;
+      s.begin(m, v);
+      for (int c = 0; c < k; c += kRestBatch<Sum>) {
+        typename Sum::Rec r[kRestBatch<Sum>];
+#pragma unroll
+        for (int j = 0; j < kRestBatch<Sum>; ++j) r[j] = s.load(m, ids[min(c + j, k - 1)]);
+#pragma unroll
+        for (int j = 0; j < kRestBatch<Sum>; ++j)
+          if (c + j < k) s.add(r[j]);
+      }
+      s.finish(m, v);
+    }
+    return;
+  }
   for (int q = trn_tid() >> 5; q < n; q += trn_grid_stride() >> 5)
     patch_sum_warp(m, rest[q], zero, s_buf[threadIdx.x >> 5]);
 }
@@ -287,7 +321,7 @@ static void patch_sum(const DMesh& m, int nb_nodes, const Sum& zero, const Metri
       m, nb_nodes, zero, collect ? ws.rest : nullptr, ws.rest_n);
   note_launch();
   rest<<<TRN_RESIDENT(rest, grid_for(32LL * nb_nodes, kPatchThreads), kPatchThreads), kPatchThreads, 0, s>>>(
-      m, zero, ws.rest, ws.rest_n);
+      m, nb_nodes, zero, ws.rest, ws.rest_n);
   note_launch();
 }
 

@@ -132,4 +132,35 @@ __device__ __forceinline__ int patch_sort_warp(const DMesh& m, int v, int* buf) 
   return k;
 }
 
+/* the same by one lane, in its own array: the ids without duplicates. Every
+ * id is searched among those kept so far, so the array holds a third of what
+ * the rows hold (an element is in the rows of its three vertices). */
+__device__ __forceinline__ int patch_sort_lane(const DMesh& m, int v, int* ids) {
+  const int nv = m.vdeg[v];
+  int k = 0, gathered = 0;
+  for (int b = -1; b < nv; ++b) {
+    const int w = b < 0 ? v : trn_row(m.vic, m, v)[b];
+    const int dw = trn_deg(m, w);
+    const TrnRow s = trn_row(m.stenc, m, w);
+    const int room = TRN_MAX_PATCH - gathered;
+    if (dw > room) trn_set_error(m.err, TRN_DERR_BUCKET);
+    const int n = dw < room ? dw : room;
+    gathered += n;
+    for (int a = 0; a < n; ++a) {
+      const int x = s[a];
+      int lo = 0, hi = k;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (ids[mid] < x) lo = mid + 1;
+        else hi = mid;
+      }
+      if (lo < k && ids[lo] == x) continue;
+      for (int j = k; j > lo; --j) ids[j] = ids[j - 1];
+      ids[lo] = x;
+      ++k;
+    }
+  }
+  return k;
+}
+
 #endif
