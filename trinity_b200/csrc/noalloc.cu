@@ -28,7 +28,7 @@
  * scaling; trn_metric.cuh), so the tensors are identical to it when that
  * mesh also sums with the tree (its default; exact_sum and replay sum in
  * element order): in one launch of one cluster, or by its kernels where many
- * vertices have long rows. They run on the caller's stream with the address
+ * vertices have long rows or the device has no room for a cluster. They run on the caller's stream with the address
  * looked up for the current device, so the stream must belong to it.
  */
 #include "trn_internal.h"
@@ -322,18 +322,17 @@ extern "C" int trn_metric_noalloc(int nb_nodes, int nb_elems, const double* d_po
   const double eig_max = 1 / trn_pow(h_max, 2);
   int* rest = reinterpret_cast<int*>(base + oRest);
   const MetricWs ws{reinterpret_cast<double4*>(base + oRec), reinterpret_cast<double*>(base + oAtot), rest, d.err + 1};
-  if (!cluster_launch<k_na_recover>(s, d, nb_nodes, nb_elems, d_points, d_tris, d_solut, grad, ws, terms, target,
-                                    scale_exp, eig_min, eig_max, d_tensor))
-    return TRN_ERR_CUDA;
-
   int word[2] = {0, 0};   /* the error word, the vertices that the cluster's warps had to take */
   const int& err = word[0];
   auto read_back = [&](size_t n) {
     return cudaMemcpyAsync(word, d.err, n, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
            cudaStreamSynchronize(s) == cudaSuccess;
   };
-  if (!read_back(sizeof(word))) return TRN_ERR_CUDA;
-  if (!err && word[1] > kNaRest) {
+  const bool cluster = cluster_launch<k_na_recover>(s, d, nb_nodes, nb_elems, d_points, d_tris, d_solut, grad, ws,
+                                                    terms, target, scale_exp, eig_min, eig_max, d_tensor);
+  if (cluster && !read_back(sizeof(word))) return TRN_ERR_CUDA;
+  /* no cluster fits this device (a part of one), or too much for the cluster */
+  if (!cluster || (!err && word[1] > kNaRest)) {
     na_recover_grid(d, nb_nodes, nb_elems, d_points, d_tris, d_solut, grad, ws, terms, target, scale_exp, eig_min,
                     eig_max, d_tensor, s);
     if (cudaPeekAtLastError() != cudaSuccess || !read_back(sizeof(int))) return TRN_ERR_CUDA;

@@ -5,9 +5,8 @@
 #ifndef TRN_LEVEL_CUH
 #define TRN_LEVEL_CUH
 
+#include "trn_cluster.h"
 #include "trn_internal.h"
-
-#include <atomic>
 
 namespace trn {
 
@@ -207,7 +206,6 @@ struct MisCand {
  * and a read back; a swapping level 35 us instead of 165. The 100 x 100
  * workload's three rounds: coarsening 4.67 -> 2.64 ms, swapping 2.26 -> 1.56. */
 constexpr int kTailThreads = 512;
-constexpr int kTailCluster = 16;   /* 8 where 16 cannot be resident */
 
 __device__ __forceinline__ void cluster_sync() {
   __syncwarp();
@@ -229,11 +227,13 @@ __device__ __forceinline__ bool tail_failed(const DMesh& m) {
 /* a word that decides a branch around a barrier */
 __device__ __forceinline__ int tail_word(const int* p) { return *(const volatile int*) p; }
 
-/* launches `kernel` as one cluster; false when it could not (the caller then
- * takes the grid-wide kernels) */
+/* launches `kernel` as one cluster on the current device; false when it could
+ * not (the caller then takes the grid-wide kernels) */
 template <auto kernel, class... Args>
 bool cluster_launch(cudaStream_t s, Args... args) {
-  static std::atomic<int> size{-1};   /* of this kernel; a race writes the same value */
+  static ClusterSizes sizes;   /* of this kernel */
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(kTailThreads);
   cfg.stream = s;
@@ -242,25 +242,24 @@ bool cluster_launch(cudaStream_t s, Args... args) {
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (size < 0) {
-    int fit = 0;
-    for (int c = kTailCluster; c >= 8 && !fit; c >>= 1) {
-      int n = 0;
-      cfg.gridDim = dim3(c);
-      at[0].val.clusterDim.x = c;
-      if (c > 8) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0) fit = c;
-    }
-    cudaGetLastError();
-    size = fit;
-  }
-  if (!size) return false;
-  cfg.gridDim = dim3(size);
-  at[0].val.clusterDim.x = size;
-  if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
+  /* an error of these calls is answered here and not left for the next check */
+  auto ok = [](cudaError_t e) {
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
+  };
+  auto probe = [&](int c) {
+    int n = 0;
+    cfg.gridDim = dim3(c);
+    at[0].val.clusterDim.x = c;
+    return (c <= 8 || ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) &&
+           ok(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg)) && n > 0;
+  };
+  auto launch = [&](int c) {
+    cfg.gridDim = dim3(c);
+    at[0].val.clusterDim.x = c;
+    return ok(cudaLaunchKernelEx(&cfg, kernel, args...));
+  };
+  if (!sizes.launch(dev, probe, launch)) return false;
   note_launch();
   return true;
 }
