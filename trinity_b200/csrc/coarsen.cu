@@ -69,15 +69,28 @@ __device__ __forceinline__ bool collapse_valid(const DMesh& m, int source, int d
   return true;
 }
 
+/* A lane's array for whichever serial path it takes: the device reserves the
+ * deepest stack for every thread it can hold (0.3 GB a KB on 148
+ * multiprocessors), so the paths share one. Candidates are places in the
+ * source's row, which a byte holds (bucket <= 256). */
+union SerialBuf {
+  int ids[2 * TRN_MAX_DEG];   /* build_one_vicin; the repair and the collapse use half */
+  struct {
+    float lo[TRN_MAX_DEG], hi[TRN_MAX_DEG];
+    uint8_t at[TRN_MAX_DEG];
+  } cand;
+};
+
 /* The candidates are tried by increasing upper bound of their length
  * (length_below), and the exact length is computed only between two valid
  * ones whose bounds overlap: the pick is the valid one of smallest (length,
  * adjacency index), as the reference's multimap gives it. */
 template <bool F32>
-__device__ int identify_target(const DMesh& m, int source) {
+__device__ __forceinline__ int identify_target(const DMesh& m, int source, SerialBuf& buf) {
   const bool bound_source = (m.tags[source] & TRN_TAG_BOUND) != 0;
-  float lo[TRN_MAX_DEG], hi[TRN_MAX_DEG];
-  int cands[TRN_MAX_DEG];
+  float* lo = buf.cand.lo;
+  float* hi = buf.cand.hi;
+  uint8_t* at = buf.cand.at;
   int nc = 0;
   const TrnRow vc = trn_row(m.vic, m, source);
   const int nv = m.vdeg[source];
@@ -92,12 +105,12 @@ __device__ int identify_target(const DMesh& m, int source) {
       while (p > 0 && hi[p - 1] > h) {
         hi[p] = hi[p - 1];
         lo[p] = lo[p - 1];
-        cands[p] = cands[p - 1];
+        at[p] = at[p - 1];
         --p;
       }
       hi[p] = h;
       lo[p] = l;
-      cands[p] = neigh;
+      at[p] = (uint8_t) b;
       nc++;
     }
   }
@@ -107,7 +120,7 @@ __device__ int identify_target(const DMesh& m, int source) {
   float best_hi = 0.f;
   for (int k = 0; k < nc; ++k) {
     if (best >= 0 && lo[k] > best_hi) continue;   /* certainly longer */
-    const int c = cands[k];
+    const int c = vc[at[k]];
     const bool both = bound_source && (m.tags[c] & TRN_TAG_BOUND) != 0;
     const double2 pc = m.pts[c];
     const TenT<F32> tc = ten_load<F32>(m, c);
@@ -134,11 +147,12 @@ __global__ void k_coarse_filter(DMesh m, int nb_nodes, int* __restrict__ target,
                                 uint8_t* __restrict__ flag) {
   nb_nodes = trn_nodes(m, nb_nodes);
   if (trn_failed(m)) return;
+  SerialBuf buf;
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
     uint8_t f = 0;
     if (m.activ[v] > 0) {
       m.activ[v] = 0;
-      int t = identify_target<F32>(m, v);
+      int t = identify_target<F32>(m, v, buf);
       target[v] = t;
       f = t > -1 ? 1 : 0;
     }
@@ -165,14 +179,15 @@ __global__ void __launch_bounds__(kSearchThreads) k_coarse_filter_append(DMesh m
   if (trn_failed(m)) return;
   const int n = *act_n;
   if (n < min_n) return;
+  SerialBuf buf;
   /* warp-aggregated appends: a block-wide one would make every thread wait
    * for its block's longest search at each step */
   for (int q = trn_tid(); q < n; q += trn_grid_stride()) {
     const int v = act[q];
     if (m.activ[v] <= 0) continue;
     m.activ[v] = 0;
-    build_one_vicin(m, v);
-    const int t = identify_target<F32>(m, v);
+    build_one_vicin(m, v, buf.ids);
+    const int t = identify_target<F32>(m, v, buf);
     target[v] = t;
     if (t > -1) {
       state[v] = 1;
@@ -187,7 +202,7 @@ __global__ void __launch_bounds__(kSearchThreads) k_coarse_filter_append(DMesh m
  * ones, counted by shuffles. Longer or irregular stencils by the group's first
  * lane. v < 0: no vertex; all lanes of the warp call it. */
 template <int G>
-__device__ __forceinline__ void build_vicin_group(const DMesh& m, int v) {
+__device__ __forceinline__ void build_vicin_group(const DMesh& m, int v, SerialBuf& buf) {
   const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
   const unsigned gm = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << g0;
   const int deg = v >= 0 && m.alive[v] ? trn_deg(m, v) : 0;
@@ -248,7 +263,7 @@ __device__ __forceinline__ void build_vicin_group(const DMesh& m, int v) {
     }
     if (gl == 0) m.vdeg[v] = deg + extra;
   } else if (serial && gl == 0) {
-    build_one_vicin(m, v);
+    build_one_vicin(m, v, buf.ids);
   }
   __syncwarp();
 }
@@ -265,10 +280,10 @@ __device__ __forceinline__ void build_vicin_group(const DMesh& m, int v) {
  * group, < 0: no vertex) gets its adjacency row too; all lanes of the warp
  * call it, and the group's first lane receives the target. */
 template <bool F32, int G>
-__device__ __forceinline__ int search_group(const DMesh& m, int v) {
+__device__ __forceinline__ int search_group(const DMesh& m, int v, SerialBuf& buf) {
   const int lane = threadIdx.x & 31;
   const int gl = lane & (G - 1);
-  build_vicin_group<G>(m, v);
+  build_vicin_group<G>(m, v, buf);
   const int nv = v >= 0 ? m.vdeg[v] : 0;
   const bool serial = nv > 32;
   const bool grp = v >= 0 && !serial;
@@ -364,13 +379,13 @@ __device__ __forceinline__ int search_group(const DMesh& m, int v) {
     }
   }
   if (gl != 0 || v < 0) return -1;
-  return serial ? identify_target<F32>(m, v) : (bestb >= 0 ? vc[bestb] : -1);
+  return serial ? identify_target<F32>(m, v, buf) : (bestb >= 0 ? vc[bestb] : -1);
 }
 
 /* the listed vertices by the groups of the warps warp, warp + nwarps, ... */
 template <bool F32, int G>
 __device__ __forceinline__ void search_list(const DMesh& m, const int* act, int n, int warp, int nwarps, int* target,
-                                            int* cand, int* count, uint8_t* state) {
+                                            int* cand, int* count, uint8_t* state, SerialBuf& buf) {
   constexpr int per_warp = 32 / G;
   const int lane = threadIdx.x & 31, gl = lane & (G - 1);
   for (int base = warp * per_warp; base < n; base += nwarps * per_warp) {
@@ -379,7 +394,7 @@ __device__ __forceinline__ void search_list(const DMesh& m, const int* act, int 
     if (v >= 0 && m.activ[v] <= 0) v = -1;
     __syncwarp();
     if (gl == 0 && v >= 0) m.activ[v] = 0;
-    const int t = search_group<F32, G>(m, v);
+    const int t = search_group<F32, G>(m, v, buf);
     if (gl == 0 && v >= 0) {
       target[v] = t;
       if (t > -1) {
@@ -398,11 +413,12 @@ __global__ void k_coarse_filter_group(DMesh m, const int* __restrict__ act, cons
   if (trn_failed(m)) return;
   const int n = *act_n;
   if (n > max_n) return;
-  search_list<F32, G>(m, act, n, trn_tid() >> 5, trn_grid_stride() >> 5, target, cand, count, state);
+  SerialBuf buf;
+  search_list<F32, G>(m, act, n, trn_tid() >> 5, trn_grid_stride() >> 5, target, cand, count, state, buf);
 }
 
 /* one collapse (Coarse::collapseEdge) by one lane: long stencils */
-__device__ __noinline__ void collapse_serial(const DMesh& m, int source, int destin) {
+__device__ __noinline__ void collapse_serial(const DMesh& m, int source, int destin, int* rest) {
   const TrnRow st = trn_row(m.stenc, m, source);
   const int deg = trn_deg(m, source);
   const int limit = (m.tags[source] & TRN_TAG_BOUND) ? 1 : 2;
@@ -420,7 +436,6 @@ __device__ __noinline__ void collapse_serial(const DMesh& m, int source, int des
       ++k;
     }
   }
-  int rest[TRN_MAX_DEG];
   int nr = 0;
   for (int a = 0; a < deg; ++a) {
     int e = st[a];
@@ -502,14 +517,14 @@ struct BlockSink {
 constexpr int kCollapseLanes = 8, kCollapseEach = 4;
 
 template <class Sink>
-__device__ __forceinline__ void collapse_group(const DMesh& m, int source, int destin, const Sink& sink) {
+__device__ __forceinline__ void collapse_group(const DMesh& m, int source, int destin, const Sink& sink, int* buf) {
   const int lane = threadIdx.x & 31, gl = lane & (kCollapseLanes - 1), g0 = lane & ~(kCollapseLanes - 1);
   const unsigned gm = 0xffu << g0;
   /* through a shuffle: every lane has read the count before the first lane's
    * serial collapse can clear it, and all of them take the same branch */
   const int deg = __shfl_sync(gm, trn_deg(m, source), 0, kCollapseLanes);
   if (deg > kCollapseLanes * kCollapseEach) {
-    if (gl == 0) collapse_serial(m, source, destin);
+    if (gl == 0) collapse_serial(m, source, destin, buf);
     __syncwarp(gm);
     return;
   }
@@ -586,6 +601,7 @@ __global__ void __launch_bounds__(TRN_THREADS) k_collapse(DMesh m, const int* __
   if (trn_failed_block(m)) return;
   const int n_indep = *count;
   const BlockSink sink{&lists};
+  int buf[TRN_MAX_DEG];
   constexpr int groups = TRN_THREADS / kCollapseLanes;
   for (int base = blockIdx.x * groups; base < n_indep; base += gridDim.x * groups) {
     if (threadIdx.x == 0) lists.nact = lists.nfix = 0;
@@ -596,7 +612,7 @@ __global__ void __launch_bounds__(TRN_THREADS) k_collapse(DMesh m, const int* __
       if (source < 0 || source >= m.capa_node || (cand_flag && !cand_flag[source])) {
         if ((threadIdx.x & (kCollapseLanes - 1)) == 0) trn_set_error(m.err, TRN_DERR_REPLAY);
       } else {
-        collapse_group(m, source, target[source], sink);
+        collapse_group(m, source, target[source], sink, buf);
       }
     }
     __syncthreads();
@@ -618,6 +634,7 @@ template <bool F32>
 __global__ void __launch_bounds__(kTailThreads) k_coarsen_tail(DMesh m, int* act0, int* act1, int* status, int* target,
                                                                int* cand, uint8_t* s0, uint8_t* s1, int* indep,
                                                                int* open, Seed sd, int rounds, int cap) {
+  SerialBuf buf;
   const int tid = trn_tid(), stride = trn_grid_stride();
   for (int level = 0;; ++level) {
     const int* act = (level & 1) ? act1 : act0;
@@ -632,9 +649,9 @@ __global__ void __launch_bounds__(kTailThreads) k_coarsen_tail(DMesh m, int* act
     /* more lanes a vertex while the list leaves lanes idle */
     const int na = failed ? 0 : status[S_ACT];
     if (na * 16 <= 2 * stride)
-      search_list<F32, 16>(m, act, na, tid >> 5, stride >> 5, target, cand, status + S_NTASK, s0);
+      search_list<F32, 16>(m, act, na, tid >> 5, stride >> 5, target, cand, status + S_NTASK, s0, buf);
     else
-      search_list<F32, 8>(m, act, na, tid >> 5, stride >> 5, target, cand, status + S_NTASK, s0);
+      search_list<F32, 8>(m, act, na, tid >> 5, stride >> 5, target, cand, status + S_NTASK, s0, buf);
     cluster_sync();
     /* the independent set: rounds until no candidate is undecided (the
      * rounds after that would only copy the states) */
@@ -677,14 +694,11 @@ __global__ void __launch_bounds__(kTailThreads) k_coarsen_tail(DMesh m, int* act
     const int ni = tail_failed(m) ? 0 : status[S_NINDEP];
     for (int q = tid / kCollapseLanes; q < ni; q += stride / kCollapseLanes) {
       const int v = indep[q];
-      collapse_group(m, v, target[v], DirectSink());
+      collapse_group(m, v, target[v], DirectSink(), buf.ids);
     }
     cluster_sync();
     if (tid == 0) tail_level_end(m, status, kLevelCoarsen, cap);
-    if (!tail_failed(m)) {
-      int buf[TRN_MAX_DEG];
-      tail_fix(m, tid, stride, buf);
-    }
+    if (!tail_failed(m)) tail_fix(m, tid, stride, buf.ids);
     cluster_sync();
     if (!tail_word(status + S_CONT)) return;
   }

@@ -119,6 +119,7 @@ __device__ __forceinline__ void na_elem(const DMesh& d, int i, int nb_nodes, con
 
 /* the sorted row, and the adjacency from it and the elements alone */
 __device__ __forceinline__ void na_row(const DMesh& d, int v) {
+  int buf[2 * TRN_NOALLOC_BUCKET];
   const TrnRow row = trn_row(d.stenc, d, v);
   const int n = trn_deg(d, v);
   if (n <= kRowChunk) {
@@ -130,12 +131,11 @@ __device__ __forceinline__ void na_row(const DMesh& d, int v) {
     for (int k = 0; k < kRowChunk; ++k)
       if (k < n) row.p[k] = r[k];
   } else {
-    int r[TRN_NOALLOC_BUCKET];
-    for (int k = 0; k < n; ++k) r[k] = row[k];
-    trn_isort(r, n);
-    for (int k = 0; k < n; ++k) row[k] = r[k];
+    for (int k = 0; k < n; ++k) buf[k] = row[k];
+    trn_isort(buf, n);
+    for (int k = 0; k < n; ++k) row[k] = buf[k];
   }
-  build_one_vicin(d, v);
+  build_one_vicin(d, v, buf);
 }
 
 __device__ __forceinline__ void na_out(const DMesh& d, int v, double fact, double eig_min, double eig_max, double* out) {

@@ -34,6 +34,7 @@ __global__ void k_fill_stencils(DMesh m, int nb_elems) {
  * adjacency, which needs no other row: up to 8 entries in registers */
 __global__ void k_sort_stencils(DMesh m, int nb_nodes) {
   if (trn_failed(m)) return;
+  int buf[2 * TRN_MAX_DEG];
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
     const int d = trn_deg(m, v);
     const TrnRow s = trn_row(m.stenc, m, v);
@@ -48,12 +49,11 @@ __global__ void k_sort_stencils(DMesh m, int nb_nodes) {
       if (d > 0) p[0] = make_int4(r[0], r[1], r[2], r[3]);
       if (d > 4) p[1] = make_int4(r[4], r[5], r[6], r[7]);
     } else {
-      int buf[TRN_MAX_DEG];
       for (int a = 0; a < d; ++a) buf[a] = s[a];
       trn_isort(buf, d);
       for (int a = 0; a < d; ++a) s[a] = buf[a];
     }
-    build_one_vicin(m, v);
+    build_one_vicin(m, v, buf);
   }
 }
 
@@ -109,9 +109,10 @@ void load_init(const DMesh& m, const double2* pts, const int4* tri, const uint8_
 __global__ void k_build_vicin(DMesh m, int nb_nodes) {
   nb_nodes = trn_nodes(m, nb_nodes);
   if (trn_failed(m)) return;
+  int buf[2 * TRN_MAX_DEG];
   for (int v = trn_tid(); v < nb_nodes; v += trn_grid_stride()) {
     if (m.activ[v] == 0) continue;
-    build_one_vicin(m, v);
+    build_one_vicin(m, v, buf);
   }
 }
 

@@ -251,7 +251,7 @@ __device__ __forceinline__ int trn_iunique(int* a, int n) {
  * Otherwise a stencil of up to 12 elements
  * stays in registers (its element loads all in flight, an odd-even
  * transposition network over the 24 ids, no local memory); longer ones sort
- * in a local array. Both give the same rows. */
+ * in the caller's array of twice the bucket. Both give the same rows. */
 constexpr int kVicRegs = 24;
 
 __device__ __forceinline__ void patch_cmp(int& a, int& b) {
@@ -304,7 +304,7 @@ __device__ __forceinline__ bool build_vicin_ring(const DMesh& m, int v, int d) {
   return true;
 }
 
-__device__ __forceinline__ void build_one_vicin(const DMesh& m, int v) {
+__device__ __forceinline__ void build_one_vicin(const DMesh& m, int v, int* buf) {
   if (m.alive[v] && trn_deg(m, v) <= kRowChunk && build_vicin_ring(m, v, trn_deg(m, v))) return;
   if (m.alive[v] && trn_deg(m, v) <= kVicRegs / 2) {
     const TrnRow s = trn_row(m.stenc, m, v);
@@ -345,7 +345,6 @@ __device__ __forceinline__ void build_one_vicin(const DMesh& m, int v) {
     m.vdeg[v] = k;
     return;
   }
-  int buf[2 * TRN_MAX_DEG];
   int k = 0;
   if (m.alive[v]) {
     const TrnRow s = trn_row(m.stenc, m, v);
