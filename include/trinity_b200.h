@@ -186,7 +186,8 @@ int trn_smooth_gradient_run(trn_mesh* mesh, int max_colors, int steps, double ma
  * cfg[1] collapse-target search block, cfg[2] lanes per vertex of the
  * grouped search (4, 8, 16; 1: the one-lane search at every level), cfg[3]
  * longest level list the grouped search takes (longer ones run the one-lane
- * search), cfg[4] flip block, cfg[5] lanes per smoothed vertex (2, 4 or
+ * search; from a list of at most 4,096 vertices that it takes, the levels left
+ * run in one launch, with 8 or 16 lanes), cfg[4] flip block, cfg[5] lanes per smoothed vertex (2, 4 or
  * 8; 1 runs as 2), cfg[6] registers of the smoothing kernel (0: up to 128,
  * two 256-thread blocks per SM; 1: capped for three; 2 to 8: for four). With
  * cfg[5], cfg[6] at 2, 1 (the default) both follow each color class's length

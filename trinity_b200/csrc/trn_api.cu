@@ -1036,8 +1036,10 @@ int trn_coarsen_run(trn_mesh* m, int max_colors, trn_stats* st) {
     enq_coarsen_begin(m, s, false);
     long long bound = m->nb_nodes;
     do {
-      /* the levels of a short list run in one launch, to the call's end */
-      if (bound > kCoarsenTail ||
+      /* the levels of a short list run in one launch, to the call's end, where
+       * the launch shapes give such a list to the grouped search (which is what
+       * that launch holds) */
+      if (bound > kCoarsenTail || bound > m->tune.group_max || m->tune.group_lanes == 1 ||
           !coarsen_tail(level_mesh(m), act_list(m, 0), act_list(m, 1), m->status, m->target, m->list, m->hws,
                         m->indep, seed_of(m, 0x9e37ULL), kMisRounds, m->level_cap, m->fp32, s))
         enq_coarsen_level(m, s, bound, 0, false);
