@@ -188,10 +188,10 @@ int trn_smooth_gradient_run(trn_mesh* mesh, int max_colors, int steps, double ma
  * longest level list the grouped search takes (longer ones run the one-lane
  * search; from a list of at most 4,096 vertices that it takes, the levels left
  * run in one launch, with 8 or 16 lanes), cfg[4] flip block, cfg[5] lanes per smoothed vertex (2, 4 or
- * 8; 1 runs as 2), cfg[6] registers of the smoothing kernel (0: up to 128,
- * two 256-thread blocks per SM; 1: capped for three; 2 to 8: for four). With
- * cfg[5], cfg[6] at 2, 1 (the default) both follow each color class's length
- * and the arithmetic form. Defaults: 256-thread blocks. Per mesh; a
+ * 8; 1 runs as 2), cfg[6] registers of the smoothing kernel (0, 6, 7: up to
+ * 128, two 256-thread blocks per SM; 1, 5, 8: capped for three; 2, 3, 4: for
+ * four). With cfg[5], cfg[6] at 2, 7 (the default) both follow each color
+ * class's length and the arithmetic form. Defaults: 256-thread blocks. Per mesh; a
  * captured round is recaptured when they change. trn_autotune chooses them
  * on the loaded mesh, timing metric + `rounds` rounds from the input (the
  * best of three runs; a candidate replaces the value kept only when at

@@ -409,7 +409,10 @@ void smooth_pre(const DMesh& m, int nb_nodes, cudaStream_t s) {
   check_launch("smooth_pre");
 }
 
-/* The default shape (2 lanes, variant 1) stands for a choice by the class's
+/* the blocks an SM that the values of smooth_regs cap the registers for */
+static constexpr int kRegsBlocks[9] = {2, 3, 4, 4, 4, 3, 2, 2, 3};
+
+/* The default shape (2 lanes, smooth_regs 7) stands for a choice by the class's
  * length and the form. A vertex is a chain of gathers and arithmetic: a class
  * too short to fill the chip takes as long as one chain, which more lanes
  * shorten; a long one is bound by issue, which the lanes' shared part (the new
@@ -431,6 +434,9 @@ static void smooth_shape(int n, bool fp32, int* lanes, int* blocks) {
   } else if (n <= 163840) {
     *lanes = 4;
     *blocks = 4;
+  } else {
+    *lanes = 2;
+    *blocks = 3;
   }
 }
 
@@ -446,8 +452,8 @@ static void smooth_launch(const DMesh& m, const int* list, int n, const int* off
   ProfScope ps("smooth_move", s, n * own + nbr, &bc);
   const int t = tune().smooth_threads;
   const int regs = tune().smooth_regs;
-  int lanes = std::max(2, tune().smooth_lanes), blocks = regs == 0 ? 2 : (regs == 1 ? 3 : 4);
-  if (lanes == 2 && blocks == 3) smooth_shape(hint, fp32, &lanes, &blocks);
+  int lanes = std::max(2, tune().smooth_lanes), blocks = kRegsBlocks[regs];
+  if (tune().smooth_lanes == 2 && regs == 7) smooth_shape(hint, fp32, &lanes, &blocks);
   const int g = grid_for((long long) hint * lanes, t);
   /* KQ element metrics a thread, a VertexPark a vertex */
   const size_t smem = (size_t) (lanes >= 4 ? 2 : 3) * t * (fp32 ? sizeof(float4) : sizeof(double4)) +

@@ -1456,7 +1456,7 @@ int trn_autotune(trn_mesh* m, double target_factor, int norm, double h_min, doub
                              &m->tune.filter_threads, &m->tune.group_lanes, &m->tune.group_max,
                              &m->tune.flip_threads};
   const std::vector<std::vector<int>> cands = {
-      {2, 4, 8}, {64, 128, 256}, {0, 1, 2}, {128, 256, 512}, {4, 8, 16}, {4096, 16384, 65536}, {128, 256, 512}};
+      {2, 4, 8}, {64, 128, 256}, {0, 1, 2, 7}, {128, 256, 512}, {4, 8, 16}, {4096, 16384, 65536}, {128, 256, 512}};
   {
     int best_l = m->tune.smooth_lanes, best_r = m->tune.smooth_regs;
     double best_ms;
@@ -1464,7 +1464,7 @@ int trn_autotune(trn_mesh* m, double target_factor, int norm, double h_min, doub
     for (int l : cands[0]) {
       for (int r : cands[2]) {
         if (rc != TRN_OK) break;
-        if (l == best_l && r == best_r) continue;
+        if ((l == best_l && r == best_r) || (l != 2 && r == 7)) continue;   /* 7: the rule, with 2 */
         m->tune.smooth_lanes = l;
         m->tune.smooth_regs = r;
         double ms;

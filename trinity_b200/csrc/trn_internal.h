@@ -97,9 +97,9 @@ struct Tune {
   int group_max = 16384;      /* longest level list the grouped search takes */
   int flip_threads = 256;     /* k_swap_flip block: 128, 256, 512 */
   int smooth_lanes = 2;       /* lanes per smoothed vertex: 2 (or 1, the same), 4, 8 */
-  int smooth_regs = 1;        /* smoothing registers: 0 up to 128 (two 256-thread blocks an SM), 1 capped
-                                 at 80 (three), 2 and more at 64 (four); 2 lanes at 1 (the default) leave
-                                 both to the class's length and the form */
+  int smooth_regs = 7;        /* smoothing registers: 0, 6, 7 up to 128 (two 256-thread blocks an SM),
+                                 1, 5, 8 capped at 80 (three), 2, 3, 4 at 64 (four); 2 lanes at 7 (the
+                                 default) leave both to the class's length and the form */
   bool operator==(const Tune& o) const {
     return smooth_threads == o.smooth_threads && filter_threads == o.filter_threads &&
            group_lanes == o.group_lanes && group_max == o.group_max && flip_threads == o.flip_threads &&
