@@ -256,7 +256,7 @@ __device__ __forceinline__ double length_x(double2 pa, double2 pb, T ta, T tb) {
  *      is 5e-6 of the length in the FP64 form, 2e-5 in the FP32 form, whose
  *      own length is good to about 1e-6. Where the two lengths all but agree
  *      (the computed ratio may be 1) the FP32 form is left to step 3.
- *   3. The computed length (length_above). A NaN fails every test before and
+ *   3. The computed length (length_for). A NaN fails every test before and
  *      ends here.
  * Steps 2 and 3 are met by the edges whose endpoints put the threshold
  * between them, some 5 % on graded meshes: with step 3 alone nearly every warp
@@ -290,21 +290,17 @@ static __device__ __noinline__ float length_of_squares(float s0, float s1) {
   return trnf_dist2_finish(sqrtf(s0), sqrtf(s1));
 }
 
-/* is the computed length above thresh; rarely reached too. In single precision
- * the ratio of two lengths that differ by a unit in the last place can round to
- * 1, and the length computed from it is not a number: two lengths on one side
- * answer before (step 1's margin on the squares, 1.5e-5 of the length, is wider
- * than these 1e-5 and would leave some such edges unsplit) */
-static __device__ __forceinline__ bool length_above(double s0, double s1, double thresh) {
-  return length_of_squares(s0, s1) > thresh;
-}
-static __device__ __noinline__ bool length_above(float s0, float s1, double thresh) {
-  const float l0 = sqrtf(s0), l1 = sqrtf(s1), t = (float) thresh;
-  if (l0 == l0 && l1 == l1) {
-    if (trnf_max(l0, l1) < t * (1.f - 1.e-5f)) return false;
-    if (trnf_min(l0, l1) > t * (1.f + 1.e-5f)) return true;
-  }
-  return (double) trnf_dist2_finish(l0, l1) > thresh;
+/* What a test compares with its threshold t in step 3; rarely reached too. In
+ * single precision the ratio of two lengths that differ by a unit in the last
+ * place can round to 1, and the length computed from it is not a number: two
+ * lengths on one side of t answer before, by either of them (step 1's margin on
+ * the squares, 1.5e-5 of the length, is wider than these 1e-5, and without
+ * this step some such edges would not count as long). */
+static __device__ __forceinline__ double length_for(double s0, double s1, double) { return length_of_squares(s0, s1); }
+static __device__ __noinline__ float length_for(float s0, float s1, float t) {
+  const float l0 = sqrtf(s0), l1 = sqrtf(s1), below = t * (1.f - 1.e-5f), above = t * (1.f + 1.e-5f);
+  if ((l0 < below && l1 < below) || (l0 > above && l1 > above)) return l0;
+  return trnf_dist2_finish(l0, l1);
 }
 
 template <bool F32>
@@ -335,7 +331,7 @@ __device__ __forceinline__ bool length_gt(double2 pa, double2 pb, TenT<F32> ta, 
   const LenT<F32> s0 = length_squares<F32>(pa, pb, ta, tb, &s1);
   const int side = length_test<F32>(s0, s1, thresh);
   if (side) return side > 0;
-  return length_above(s0, s1, thresh);
+  return (double) length_for(s0, s1, (LenT<F32>) thresh) > thresh;
 }
 
 /* length_x < thresh, and float bounds of that length: the geometric mean of
