@@ -44,9 +44,9 @@ WORKLOAD = "c2"
 # DRAM traffic per launch of the kernel that dominates the 2M-triangle step,
 # measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum, caches
 # flushed before each launch, the 7 class launches of the timed step's first
-# pass, default shape); a live run has no hardware counters, so the figure is
-# carried here
-MEASURED_TRAFFIC = {"smooth_move": 408.1e6}
+# pass, default shape; profiles/dram_traffic_top_kernels.md); a live run has no
+# hardware counters, so the figure is carried here
+MEASURED_TRAFFIC = {"smooth_move": 411.7e6}
 METRIC = "adapted triangles/s per full round"
 UNIT = "triangles/s"
 REF_BIN = os.path.join(REPO, "oracle", "_ref", "trinity_ref")

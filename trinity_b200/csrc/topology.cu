@@ -1,7 +1,7 @@
 /*
  * topology.cu — incidence build and repair.
  *
- *   k_count_fill   : vertex -> element stencils from the triangle array
+ *   k_fill_stencils: vertex -> element stencils from the triangle array
  *                    (Mesh::rebuildTopology, mesh.cpp:197-210: atomic append)
  *   k_sort_stencils: sort each stencil (mesh.cpp:244) and build its adjacency
  *   k_build_vicin  : sorted unique vertex adjacency from the stencil, flagged

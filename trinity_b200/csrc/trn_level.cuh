@@ -204,7 +204,8 @@ struct MisCand {
  * some hundred vertices takes about 30 us here (search 7, four or five rounds
  * of the independent set 10, collapse 6, repair 5), 110 us as four launches
  * and a read back; a swapping level 35 us instead of 165. The 100 x 100
- * workload's three rounds: coarsening 4.67 -> 2.64 ms, swapping 2.26 -> 1.56. */
+ * workload's three rounds, before any cluster and now: coarsening 5.02 -> 2.58
+ * ms, swapping 2.22 -> 1.27. */
 constexpr int kTailThreads = 512;
 
 __device__ __forceinline__ void cluster_sync() {

@@ -17,8 +17,9 @@ namespace trn {
  * the patch sums: the record gathers (24 a vertex, mostly L1/L2 hits) and the
  * integer merge of the rows. One vertex a thread that gathered, sorted in
  * local memory and computed every element of its patch took 582 us for the
- * gradient and 650 us for the Hessian of the 2M-triangle mesh; records and
- * register merge take 163 and 175 us, the records' kernels included. */
+ * gradient and 650 us for the Hessian of the 2M-triangle mesh; records, the
+ * merge in registers and the ids in a shared column (metric.cu) take 165 and
+ * 180 us, the records' kernels included. */
 /* Where the first 16 bytes of element i's record are, in units of 16 bytes;
  * the second are at the slot ^ 1. With `mix` (kRecMix; the buffer then has
  * room for a multiple of 4 records) the 8 slots of a 128-byte line are

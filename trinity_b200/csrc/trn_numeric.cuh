@@ -101,11 +101,6 @@ __device__ __forceinline__ void trn_interp_addl(double* log_mat, double4 l) {
   log_mat[3] += l.w;
 }
 
-/* one term of the log-Euclidean sum of numeric::interpolateTensor */
-__device__ __forceinline__ void trn_interp_add(double* log_mat, double t0, double t1, double t2) {
-  trn_interp_addl(log_mat, trn_log_tensor(t0, t1, t2));
-}
-
 /* the exponentiation half of numeric::interpolateTensor (numeric.cpp:189-216) */
 __device__ __forceinline__ void trn_interp_finish(double* log_mat, int nb, double* res) {
   double cache[4], val[2], vec[4];
@@ -168,13 +163,6 @@ __device__ __forceinline__ double trn_quality_geom(double2 pa, double2 pb, doubl
 __device__ __forceinline__ double trn_quality_l(double2 pa, double2 pb, double2 pc,
                                                 double4 la, double4 lb, double4 lc) {
   return trn_quality_geom(pa, pb, pc, trn_quality_metric(la, lb, lc));
-}
-
-/* numeric::computeQuality from the tensors themselves */
-__device__ __forceinline__ double trn_quality(double2 pa, double2 pb, double2 pc,
-                                              double4 ta, double4 tb, double4 tc) {
-  return trn_quality_l(pa, pb, pc, trn_log_tensor(ta.x, ta.y, ta.z),
-                       trn_log_tensor(tb.x, tb.y, tb.z), trn_log_tensor(tc.x, tc.y, tc.z));
 }
 
 /* numeric::approxRiemannDist(a, b, M), numeric.cpp:450-461 */

@@ -94,8 +94,8 @@ __device__ __forceinline__ bool patch_keys(const DMesh& m, int v, int* key) {
 }
 
 /* The general path, one warp a vertex: the patch gathered into `buf` (shared,
- * TRN_MAX_PATCH ids), sorted, duplicates dropped as the caller walks it
- * (patch_walk). Returns the ids gathered; a longer patch sets the error word.
+ * TRN_MAX_PATCH ids), sorted, duplicates left for the caller to skip. Returns
+ * the ids gathered; a longer patch sets the error word.
  * All 32 lanes take part. */
 __device__ __forceinline__ int patch_sort_warp(const DMesh& m, int v, int* buf) {
   const int lane = threadIdx.x & 31;
